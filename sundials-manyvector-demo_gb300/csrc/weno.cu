@@ -12,55 +12,129 @@
 // The float-float forms (weno_f2*.cu) use divergence_f2_kernel below as their pass 2.  Also
 // here: the CFL wave speed, the pack1D stencil gather and the conservation totals.
 #include "common.cuh"
+#include "weno64.cuh"
 #include "weno_face.cuh"
 #include "weno_sweep.cuh"
 #include "weno.cuh"
 
 namespace gbmv {
 
-template <int NCHEM, int DIR>
-__global__ void __launch_bounds__(128) face_flux_kernel(Grid g, Fields w, double* __restrict__ F,
-                                                        long nfaces) {
-  for (long f = blockIdx.x * (long)blockDim.x + threadIdx.x; f < nfaces;
-       f += (long)gridDim.x * blockDim.x) {
-    long cell[6], ijk[3];
+// Primitives of every cell -- half the pressure, the velocities, half the sound speed -- and the
+// legal-state flags (src/euler3D.hpp:1405-1414).  A cell is read by 18 stencil positions, and
+// forming its primitives there cost ~45 of a face's FP64 instructions six times over.
+__global__ void __launch_bounds__(256) prims64_kernel(Grid g, Fields w, double* ph, double* ux,
+                                                      double* uy, double* uz, double* hc,
+                                                      int* __restrict__ status) {
+  int bad = 0;
+  for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < g.ncell;
+       c += (long)gridDim.x * blockDim.x) {
+    const double rho = w.f[0][c], mx = w.f[1][c], my = w.f[2][c], mz = w.f[3][c], et = w.f[4][c];
+    double p, a;
+    point_prims64(g.gamma, rho, mx, my, mz, et, p, a);
+    bad |= (!(rho > 0.0) ? 1 : 0) | (!(et > 0.0) ? 2 : 0) | (!(p > 0.0) ? 4 : 0);
+    if (ph) {
+      ph[c] = p;
+      ux[c] = mx / rho;
+      uy[c] = my / rho;
+      uz[c] = mz / rho;
+      hc[c] = a;
+    }
+  }
+  bad = __reduce_or_sync(0xffffffffu, bad);
+  if (bad && (threadIdx.x & 31) == 0) atomicOr(status, bad);
+}
+
+// Face fluxes of the three directions (one launch).  Bound by the FP64 pipe: ~1550 instructions
+// a face at NVAR 15.  PRE: the primitives are read from the cell pass, else formed per stencil
+// point.  SPLIT: two neighbouring threads share a face, each with one Lax-Friedrichs side (the
+// second reads its stencil reversed, which makes its side the plus formula); the same bits.
+template <int NCHEM, bool PRE, bool SPLIT>
+__global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant__ SweepSet S) {
+  const int dir = sweep_dir(S);
+  const SweepDir& D = S.d[dir];
+  const int nblk = (dir == 2 ? (int)gridDim.x : S.d[dir + 1].block0) - D.block0;
+  const long first = (blockIdx.x - D.block0) * (long)blockDim.x + threadIdx.x;
+  const int side = SPLIT ? (int)(threadIdx.x & 1) : 0;
+  // SPLIT: one pass (the launch covers every face); surplus threads repeat the last face so that
+  // both threads of a pair and the whole warp reach the exchanges
+  for (long f = SPLIT ? (first >> 1) : first; SPLIT || f < D.nfaces;
+       f += (long)nblk * blockDim.x) {
+    const bool live = f < D.nfaces;
+    if (SPLIT && !live) f = D.nfaces - 1;
+    long cell[6];
     bool nall[6], nnorm[6];
-    stencil<DIR>(g, f, cell, nall, nnorm, ijk);
-    double Wd[6][5];
+    stencil_of(S, D, f, side, cell, nall, nnorm);
+    Stencil64 T;
 #pragma unroll
-    for (int l = 0; l < 6; ++l) load_point<DIR>(w, cell[l], nall[l], nnorm[l], Wd[l]);
-    FaceState<double> S;
-    double out[5];
-    fluid_face_flux<double>(Wd, g.gamma, S, out);
-    // undo the direction swap
-    const double o1 = out[1], oD = out[1 + DIR];
-    out[1] = oD;
-    out[1 + DIR] = o1;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) F[v * nfaces + f] = out[v];
-#pragma unroll 1
-    for (int c = 0; c < NCHEM; ++c) {
-      double cv[6];
-#pragma unroll
-      for (int l = 0; l < 6; ++l) {
-        const double x = __ldg(w.f[5] + c + (long)NCHEM * cell[l]);
-        cv[l] = nall[l] ? -x : x;
+    for (int l = 0; l < 6; ++l) {
+      load_point(D, cell[l], nall[l], nnorm[l], T.W[l]);
+      if (PRE) {
+        const double p = __ldg(S.ph + cell[l]), u = __ldg(D.u + cell[l]);
+        T.ph[l] = nall[l] ? -p : p;
+        T.u[l] = nnorm[l] ? -u : u;
+        T.hc[l] = __ldg(S.hc + cell[l]);
+      } else {
+        point_prims64(S.gamma, T.W[l][0], T.W[l][1], T.W[l][2], T.W[l][3], T.W[l][4], T.ph[l],
+                      T.hc[l]);
+        T.u[l] = T.W[l][1] / T.W[l][0];
       }
-      F[(5 + c) * nfaces + f] = tracer_face_flux<double>(S, cv);
+    }
+    if constexpr (!SPLIT) {
+      Split64 H;
+      double out[5];
+      fluid_face_flux64(T, S.gamma, H, out);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) D.F[D.slot[v] * D.nfaces + f] = out[v];
+#pragma unroll 1
+      for (int c = 0; c < NCHEM; ++c) {
+        double cv[6];
+#pragma unroll
+        for (int l = 0; l < 6; ++l) {
+          const double x = __ldg(S.chem + c + (long)NCHEM * cell[l]);
+          cv[l] = nall[l] ? -x : x;
+        }
+        D.F[(5 + c) * D.nfaces + f] = tracer_face_flux64(H, cv);
+      }
+    } else {
+      Roe64 R;
+      roe64(T, S.gamma, R);
+      const double ha = half_alpha64(T);
+      double h[5], ff[5], out[5];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) h[k] = fma(0.5, T.u[k], side ? -ha : ha);
+      fluid_side64<0>(T, R, h, ff);
+#pragma unroll
+      for (int i = 0; i < 5; ++i) ff[i] += __shfl_xor_sync(0xffffffffu, ff[i], 1);
+      fluid_back64(R, ff, out);
+#pragma unroll
+      for (int v = 0; v < 5; ++v)
+        if (live && (v & 1) == side) D.F[D.slot[v] * D.nfaces + f] = out[v];
+#pragma unroll 1
+      for (int c = 0; c < NCHEM; ++c) {
+        double cv[5];
+#pragma unroll
+        for (int l = 0; l < 5; ++l) {
+          const double x = __ldg(S.chem + c + (long)NCHEM * cell[l]);
+          cv[l] = nall[l] ? -x : x;
+        }
+        Weno64 q;
+        double r = weno_prod64(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
+        r += __shfl_xor_sync(0xffffffffu, r, 1);
+        if (live && (c & 1) == side) D.F[(5 + c) * D.nfaces + f] = r;
+      }
+      break;
     }
   }
 }
 
-
 template <int NCHEM>
-__global__ void __launch_bounds__(256) divergence_kernel(Grid g, Fields w, Fields wdot,
+__global__ void __launch_bounds__(256) divergence_kernel(Grid g, Fields wdot,
                                                          const double* __restrict__ Fx,
                                                          const double* __restrict__ Fy,
                                                          const double* __restrict__ Fz,
-                                                         ForceTerm G, int* __restrict__ status) {
+                                                         ForceTerm G) {
   const long nx = g.n[0], ny = g.n[1], nz = g.n[2];
   const long nfx = (nx + 1) * ny * nz, nfy = nx * (ny + 1) * nz, nfz = nx * ny * (nz + 1);
-  int bad = 0;
   for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < g.ncell;
        c += (long)gridDim.x * blockDim.x) {
     long i, j, k;
@@ -68,15 +142,6 @@ __global__ void __launch_bounds__(256) divergence_kernel(Grid g, Fields w, Field
     const long fx = i + (nx + 1) * (j + ny * k);
     const long fy = i + nx * (j + (ny + 1) * k);
     const long fz = c;
-    {
-      const double rho = w.f[0][c], mx = w.f[1][c], my = w.f[2][c], mz = w.f[3][c],
-                   et = w.f[4][c];
-      int s = 0;
-      if (!(rho > 0.0)) s |= 1;
-      if (!(et > 0.0)) s |= 2;
-      if (!(eos64(g.gamma, rho, mx, my, mz, et) > 0.0)) s |= 4;
-      bad |= s;
-    }
 #pragma unroll
     for (int v = 0; v < 5 + NCHEM; ++v) {
       // (F+ - F-) / d as a multiply by 1/d: the reference divides; the difference is one
@@ -89,22 +154,19 @@ __global__ void __launch_bounds__(256) divergence_kernel(Grid g, Fields w, Field
       *dst = base - div;
     }
   }
-  // warp-aggregated status
-  bad = __reduce_or_sync(0xffffffffu, bad);
-  if (bad && (threadIdx.x & 31) == 0) atomicOr(status, bad);
 }
 
-int divergence(const Grid& g, const Fields& w, const Fields& wdot, double* const (&F)[3],
-               const ForceTerm& G, int* d_status, cudaStream_t s) {
+int divergence(const Grid& g, const Fields& wdot, double* const (&F)[3], const ForceTerm& G,
+               cudaStream_t s) {
   ProfScope ps("divergence", s);
   const int t = spread_threads(g.ncell, 256);
   const int b = sweep_blocks(g.ncell, t);
   switch (g.nchem) {
-    case 0: divergence_kernel<0><<<b, t, 0, s>>>(g, w, wdot, F[0], F[1], F[2], G, d_status); break;
-    case 2: divergence_kernel<2><<<b, t, 0, s>>>(g, w, wdot, F[0], F[1], F[2], G, d_status); break;
-    case 4: divergence_kernel<4><<<b, t, 0, s>>>(g, w, wdot, F[0], F[1], F[2], G, d_status); break;
-    case 6: divergence_kernel<6><<<b, t, 0, s>>>(g, w, wdot, F[0], F[1], F[2], G, d_status); break;
-    case 10: divergence_kernel<10><<<b, t, 0, s>>>(g, w, wdot, F[0], F[1], F[2], G, d_status); break;
+    case 0: divergence_kernel<0><<<b, t, 0, s>>>(g, wdot, F[0], F[1], F[2], G); break;
+    case 2: divergence_kernel<2><<<b, t, 0, s>>>(g, wdot, F[0], F[1], F[2], G); break;
+    case 4: divergence_kernel<4><<<b, t, 0, s>>>(g, wdot, F[0], F[1], F[2], G); break;
+    case 6: divergence_kernel<6><<<b, t, 0, s>>>(g, wdot, F[0], F[1], F[2], G); break;
+    case 10: divergence_kernel<10><<<b, t, 0, s>>>(g, wdot, F[0], F[1], F[2], G); break;
     default: set_error("nchem=%d not compiled (0,2,4,6,10)", g.nchem); return GBMV_EUNSUPPORTED;
   }
   GBMV_LAUNCH_CHECK("divergence_kernel");
@@ -170,32 +232,55 @@ int divergence_f2(const Grid& g, const Fields& wdot, float2* const (&F)[3], cons
   return GBMV_OK;
 }
 
+// Cells of w and of the five fluid tendencies that share memory (an in-place call)
+static bool overlap(const Grid& g, const Fields& w, const Fields& wdot) {
+  for (int a = 0; a < 5; ++a)
+    for (int b = 0; b < (g.nchem ? 6 : 5); ++b) {
+      const uintptr_t x = (uintptr_t)wdot.f[a], y = (uintptr_t)w.f[b];
+      const uintptr_t nx = 8 * (uintptr_t)g.ncell, ny = nx * (b == 5 ? g.nchem : 1);
+      if (x < y + ny && y < x + nx) return true;
+    }
+  return false;
+}
+
 template <int NCHEM>
 static int launch_fp64(const Grid& g, const Fields& w, const Fields& wdot, const ForceTerm& G,
                        double* scratch, int* d_status, cudaStream_t s) {
   long nf[3];
   face_counts(g, nf);
+  const long nfaces = nf[0] + nf[1] + nf[2];
   double* F[3] = {scratch, scratch + (long)(5 + NCHEM) * nf[0],
                   scratch + (long)(5 + NCHEM) * (nf[0] + nf[1])};
+  // The primitives live in the five fluid tendencies, which the divergence overwrites last: no
+  // memory of their own.  Where those hold the caller's forcing, or are the state itself, the
+  // sweep forms the primitives per stencil point instead.
+  const bool pre = !G.in_wdot && !overlap(g, w, wdot);
   {
-    ProfScope ps("face_flux", s);
-    const int t = sweep_threads(g, nf[0], 128);
-    face_flux_kernel<NCHEM, 0><<<sweep_blocks(nf[0], t), t, 0, s>>>(g, w, F[0], nf[0]);
-    GBMV_LAUNCH_CHECK("face_flux_kernel<x>");
+    ProfScope ps("prims", s);
+    const int t = spread_threads(g.ncell, 256);
+    double* const none = nullptr;
+    prims64_kernel<<<sweep_blocks(g.ncell, t), t, 0, s>>>(
+        g, w, pre ? wdot.f[0] : none, pre ? wdot.f[1] : none, pre ? wdot.f[2] : none,
+        pre ? wdot.f[3] : none, pre ? wdot.f[4] : none, d_status);
+    GBMV_LAUNCH_CHECK("prims64_kernel");
   }
   {
     ProfScope ps("face_flux", s);
-    const int t = sweep_threads(g, nf[1], 128);
-    face_flux_kernel<NCHEM, 1><<<sweep_blocks(nf[1], t), t, 0, s>>>(g, w, F[1], nf[1]);
-    GBMV_LAUNCH_CHECK("face_flux_kernel<y>");
+    const bool split = pre && nfaces <= kSplitFaces;
+    const int t = sweep_threads(g, split ? 2 * nfaces : nfaces, 128);
+    SweepSet S;
+    const int b = sweep_set(g, w, F, split ? 2 : 1, t, split ? 1L << 30 : (long)kSM * 16, S);
+    if (pre) {
+      S.ph = wdot.f[0];
+      S.hc = wdot.f[4];
+      for (int d = 0; d < 3; ++d) S.d[d].u = wdot.f[1 + d];
+    }
+    if (split) face_flux64_kernel<NCHEM, true, true><<<b, t, 0, s>>>(S);
+    else if (pre) face_flux64_kernel<NCHEM, true, false><<<b, t, 0, s>>>(S);
+    else face_flux64_kernel<NCHEM, false, false><<<b, t, 0, s>>>(S);
+    GBMV_LAUNCH_CHECK("face_flux64_kernel");
   }
-  {
-    ProfScope ps("face_flux", s);
-    const int t = sweep_threads(g, nf[2], 128);
-    face_flux_kernel<NCHEM, 2><<<sweep_blocks(nf[2], t), t, 0, s>>>(g, w, F[2], nf[2]);
-    GBMV_LAUNCH_CHECK("face_flux_kernel<z>");
-  }
-  return divergence(g, w, wdot, F, G, d_status, s);
+  return divergence(g, wdot, F, G, s);
 }
 
 size_t feuler_fp64_scratch_doubles(const Grid& g) {

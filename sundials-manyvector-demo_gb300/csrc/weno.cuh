@@ -21,8 +21,8 @@ int feuler_fp64(const Grid& g, const Fields& w, const Fields& wdot, const ForceT
                 double* scratch, int* d_status, cudaStream_t s);
 
 // pass 2 of every form: wdot = G - div F from the three per-direction face-flux arrays
-int divergence(const Grid& g, const Fields& w, const Fields& wdot, double* const (&F)[3],
-               const ForceTerm& G, int* d_status, cudaStream_t s);
+int divergence(const Grid& g, const Fields& wdot, double* const (&F)[3], const ForceTerm& G,
+               cudaStream_t s);
 // the same from fluxes stored as float pairs (hi, lo), differenced in float-float
 // (no legal-state check: the float-float forms set those flags in prims_f2)
 int divergence_f2(const Grid& g, const Fields& wdot, float2* const (&F)[3], const ForceTerm& G,

@@ -73,6 +73,58 @@ __device__ __forceinline__ void load_point(const Fields& w, long c, bool nall, b
   W[4] = q[4];
 }
 
+// One direction of a sweep that takes the direction at run time: one kernel body serves the
+// three, and one launch covers the faces of all of them (SweepSet), so small grids wait for one
+// sweep instead of three in a row.  Field order as load_point: normal momentum in slot 1.
+struct SweepDir {
+  const double* f[5];  // rho, m_normal, m_t1, m_t2, et
+  int slot[5];         // their field numbers
+  const double* u;     // normal velocity (null: no primitives)
+  double* F;           // face fluxes [field][face]
+  long nfaces, ex, ey; // extents of the face grid along x and y
+  long n, stride;      // cells along the direction and their spacing in memory
+  int dir, bc_lo, bc_hi;
+  int block0;          // first block of the direction
+};
+struct SweepSet {
+  SweepDir d[3];
+  const double* ph;    // half pressure, half sound speed (null: no primitives)
+  const double* hc;
+  const double* chem;
+  long nx, ny;
+  double gamma;
+};
+__device__ __forceinline__ int sweep_dir(const SweepSet& S) {
+  return (int)blockIdx.x >= S.d[2].block0 ? 2 : ((int)blockIdx.x >= S.d[1].block0 ? 1 : 0);
+}
+
+// cells and ghost signs of the six stencil points of face f of a direction, point l at stencil
+// position l, or 5 - l when reversed
+__device__ __forceinline__ void stencil_of(const SweepSet& S, const SweepDir& D, long f,
+                                           bool reversed, long (&cell)[6], bool (&nall)[6],
+                                           bool (&nnorm)[6]) {
+  long i, j, k;
+  split3(f, D.ex, D.ey, i, j, k);
+  const long pos = D.dir == 0 ? i : (D.dir == 1 ? j : k);
+  const long base = i + S.nx * (j + S.ny * k) - pos * D.stride;
+#pragma unroll
+  for (int l = 0; l < 6; ++l)
+    cell[l] = base + D.stride * ghost_src(pos - 3 + (reversed ? 5 - l : l), D.n, D.bc_lo, D.bc_hi,
+                                          &nall[l], &nnorm[l]);
+}
+
+// the fluid values of a stencil point in face order, ghost signs applied
+__device__ __forceinline__ void load_point(const SweepDir& D, long c, bool nall, bool nnorm,
+                                           double (&W)[5]) {
+#pragma unroll
+  for (int v = 0; v < 5; ++v) W[v] = __ldg(D.f[v] + c);
+  if (nall) {
+#pragma unroll
+    for (int v = 0; v < 5; ++v) W[v] = -W[v];
+  }
+  if (nnorm) W[1] = -W[1];
+}
+
 // grid-stride launch size: ceil(n / t) blocks, at least 1, at most 16 per SM
 inline int sweep_blocks(long n, int t) {
   long b = (n + t - 1) / t;
@@ -103,6 +155,42 @@ inline void face_counts(const Grid& g, long (&nf)[3]) {
   nf[0] = (nx + 1) * ny * nz;
   nf[1] = nx * (ny + 1) * nz;
   nf[2] = nx * ny * (nz + 1);
+}
+
+// The three directions of w for a sweep of `per_face` threads a face in blocks of t threads,
+// fluxes to F (null: none); returns the number of blocks (at most cap per direction).
+inline int sweep_set(const Grid& g, const Fields& w, double* const* F, int per_face, int t,
+                     long cap, SweepSet& S) {
+  long nf[3], b = 0;
+  face_counts(g, nf);
+  const long stride[3] = {1, g.n[0], g.n[0] * g.n[1]};
+  for (int d = 0; d < 3; ++d) {
+    SweepDir& D = S.d[d];
+    const int slot[5] = {0, 1 + d, d == 1 ? 1 : 2, d == 2 ? 1 : 3, 4};
+    for (int v = 0; v < 5; ++v) {
+      D.slot[v] = slot[v];
+      D.f[v] = w.f[slot[v]];
+    }
+    D.u = nullptr;
+    D.F = F ? F[d] : nullptr;
+    D.nfaces = nf[d];
+    D.ex = g.n[0] + (d == 0);
+    D.ey = g.n[1] + (d == 1);
+    D.n = g.n[d];
+    D.stride = stride[d];
+    D.dir = d;
+    D.bc_lo = g.bc[2 * d];
+    D.bc_hi = g.bc[2 * d + 1];
+    D.block0 = (int)b;
+    const long nb = (nf[d] * per_face + t - 1) / t;
+    b += nb < cap ? nb : cap;
+  }
+  S.ph = S.hc = nullptr;
+  S.chem = w.f[5];
+  S.nx = g.n[0];
+  S.ny = g.n[1];
+  S.gamma = g.gamma;
+  return (int)b;
 }
 
 }  // namespace gbmv

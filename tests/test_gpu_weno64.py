@@ -1,0 +1,59 @@
+"""The FP64 flux divergence's launch forms against the oracle: two threads a face on small grids,
+one on larger ones (both sides of the line, and face counts that leave a partial warp), the
+primitives from the cell pass or formed per stencil point (a forcing already in wdot, an in-place
+call).  Tolerance: the FP64 parity bar, 1e-12 of each field's largest magnitude; the largest
+difference expected is ~1e-13 (a few roundings of a flux, divided by the spacing)."""
+import numpy as np
+import pytest
+
+import oracle_py as O
+import workloads as W
+from conftest import maxnorm_err
+
+pytestmark = pytest.mark.gpu
+
+# 9728 faces is the line: (16, 16, 11) has 9056, (16, 16, 12) 9856; the others leave odd remainders
+SHAPES = [(3, 3, 3), (7, 5, 3), (16, 16, 11), (16, 16, 12), (33, 17, 21)]
+BCS = [(0, 0, 0, 0, 0, 0), (3, 3, 1, 3, 0, 0)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("nchem", [0, 10])
+@pytest.mark.parametrize("bc", BCS)
+def test_fp64_forms_match_oracle(cuda, shape, nchem, bc):
+    torch = cuda
+    import gbmv
+    wl = W.rayleigh_taylor(shape=shape, nchem=nchem, seed=W.SEED_BASE + 700)
+    st, ref = O.feuler(wl["fields"], nchem, bc, wl["gamma"], None)
+    assert st == 0
+    h = gbmv.Hydro(shape, nchem, bc, wl["gamma"], None)
+    w = [torch.from_numpy(np.ascontiguousarray(f)).cuda() for f in wl["fields"]]
+    plain = [torch.full_like(f, np.nan) for f in w]
+    assert h.fEuler(0.0, w, plain) == 0
+    forced = [torch.full_like(f, 0.25) for f in w]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    h.fEuler_async(0.0, w, forced, status, gbmv.FP64, gbmv.FORCE_IN_WDOT)
+    inplace = [f.clone() for f in w]
+    assert h.fEuler(0.0, inplace, inplace) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for a, b, c, r in zip(plain, forced, inplace, ref):
+        assert maxnorm_err(a.cpu().numpy(), r) <= 1e-12
+        assert maxnorm_err(b.cpu().numpy(), r + 0.25) <= 1e-12
+        assert maxnorm_err(c.cpu().numpy(), r) <= 1e-12
+
+
+def test_fp64_forms_flag_illegal_states(cuda):
+    torch = cuda
+    import gbmv
+    wl = W.rayleigh_taylor(shape=(9, 8, 7), nchem=2, seed=W.SEED_BASE + 701)
+    h = gbmv.Hydro((9, 8, 7), 2, wl["bc"], wl["gamma"], None)
+    for field, bit in ((0, 1), (4, 2)):
+        bad = [f.copy() for f in wl["fields"]]
+        bad[field][3, 2, 1] = -1.0
+        w = [torch.from_numpy(f).cuda() for f in bad]
+        for flags in (0, gbmv.FORCE_IN_WDOT):
+            out = [torch.zeros_like(f) for f in w]
+            status = torch.zeros(1, dtype=torch.int32, device="cuda")
+            h.fEuler_async(0.0, w, out, status, gbmv.FP64, flags)
+            assert int(status.item()) & bit
