@@ -41,7 +41,17 @@ __global__ void __launch_bounds__(256) prims64_kernel(Grid g, Fields w, double* 
     }
   }
   bad = __reduce_or_sync(0xffffffffu, bad);
-  if (bad && (threadIdx.x & 31) == 0) atomicOr(status, bad);
+  if (status && bad && (threadIdx.x & 31) == 0) atomicOr(status, bad);
+}
+
+int prims64(const Grid& g, const Fields& w, double* const (&out)[5], int* d_status,
+            cudaStream_t s) {
+  ProfScope ps("prims", s);
+  const int t = spread_threads(g.ncell, 256);
+  prims64_kernel<<<sweep_blocks(g.ncell, t), t, 0, s>>>(g, w, out[0], out[1], out[2], out[3],
+                                                        out[4], d_status);
+  GBMV_LAUNCH_CHECK("prims64_kernel");
+  return GBMV_OK;
 }
 
 // Face fluxes of the three directions (one launch).  Bound by the FP64 pipe: ~1550 instructions
@@ -67,9 +77,9 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
     Stencil64 T;
 #pragma unroll
     for (int l = 0; l < 6; ++l) {
-      load_point(D, cell[l], nall[l], nnorm[l], T.W[l]);
+      load_point(D.f, cell[l], nall[l], nnorm[l], T.W[l]);
       if (PRE) {
-        const double p = __ldg(S.ph + cell[l]), u = __ldg(D.u + cell[l]);
+        const double p = __ldg(S.ph + cell[l]), u = __ldg(D.vel[0] + cell[l]);
         T.ph[l] = nall[l] ? -p : p;
         T.u[l] = nnorm[l] ? -u : u;
         T.hc[l] = __ldg(S.hc + cell[l]);
@@ -232,8 +242,8 @@ int divergence_f2(const Grid& g, const Fields& wdot, float2* const (&F)[3], cons
   return GBMV_OK;
 }
 
-// Cells of w and of the five fluid tendencies that share memory (an in-place call)
-static bool overlap(const Grid& g, const Fields& w, const Fields& wdot) {
+// Whether w and the five fluid tendencies share memory (an in-place call)
+bool fields_overlap(const Grid& g, const Fields& w, const Fields& wdot) {
   for (int a = 0; a < 5; ++a)
     for (int b = 0; b < (g.nchem ? 6 : 5); ++b) {
       const uintptr_t x = (uintptr_t)wdot.f[a], y = (uintptr_t)w.f[b];
@@ -254,15 +264,12 @@ static int launch_fp64(const Grid& g, const Fields& w, const Fields& wdot, const
   // The primitives live in the five fluid tendencies, which the divergence overwrites last: no
   // memory of their own.  Where those hold the caller's forcing, or are the state itself, the
   // sweep forms the primitives per stencil point instead.
-  const bool pre = !G.in_wdot && !overlap(g, w, wdot);
+  const bool pre = !G.in_wdot && !fields_overlap(g, w, wdot);
   {
-    ProfScope ps("prims", s);
-    const int t = spread_threads(g.ncell, 256);
-    double* const none = nullptr;
-    prims64_kernel<<<sweep_blocks(g.ncell, t), t, 0, s>>>(
-        g, w, pre ? wdot.f[0] : none, pre ? wdot.f[1] : none, pre ? wdot.f[2] : none,
-        pre ? wdot.f[3] : none, pre ? wdot.f[4] : none, d_status);
-    GBMV_LAUNCH_CHECK("prims64_kernel");
+    double* const none[5] = {};
+    double* const out[5] = {wdot.f[0], wdot.f[1], wdot.f[2], wdot.f[3], wdot.f[4]};
+    const int rc = prims64(g, w, pre ? out : none, d_status, s);
+    if (rc) return rc;
   }
   {
     ProfScope ps("face_flux", s);
@@ -271,9 +278,8 @@ static int launch_fp64(const Grid& g, const Fields& w, const Fields& wdot, const
     SweepSet S;
     const int b = sweep_set(g, w, F, split ? 2 : 1, t, split ? 1L << 30 : (long)kSM * 16, S);
     if (pre) {
-      S.ph = wdot.f[0];
-      S.hc = wdot.f[4];
-      for (int d = 0; d < 3; ++d) S.d[d].u = wdot.f[1 + d];
+      const double* const u[3] = {wdot.f[1], wdot.f[2], wdot.f[3]};
+      sweep_prims(S, wdot.f[0], u, wdot.f[4]);
     }
     if (split) face_flux64_kernel<NCHEM, true, true><<<b, t, 0, s>>>(S);
     else if (pre) face_flux64_kernel<NCHEM, true, false><<<b, t, 0, s>>>(S);

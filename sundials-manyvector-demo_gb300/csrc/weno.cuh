@@ -20,6 +20,13 @@ size_t feuler_fp64_scratch_doubles(const Grid& g);
 int feuler_fp64(const Grid& g, const Fields& w, const Fields& wdot, const ForceTerm& G,
                 double* scratch, int* d_status, cudaStream_t s);
 
+// cell primitives of the FP64 sweeps (half pressure, velocities, half sound speed; null: none),
+// legal-state flags OR-ed into *d_status (null: none)
+int prims64(const Grid& g, const Fields& w, double* const (&out)[5], int* d_status,
+            cudaStream_t s);
+// whether w and the five fluid fields of wdot share memory
+bool fields_overlap(const Grid& g, const Fields& w, const Fields& wdot);
+
 // pass 2 of every form: wdot = G - div F from the three per-direction face-flux arrays
 int divergence(const Grid& g, const Fields& wdot, double* const (&F)[3], const ForceTerm& G,
                cudaStream_t s);

@@ -1,105 +1,218 @@
 // Derivatives of the WENO flux divergence (the FP64 form of fEuler, src/utilities.cpp:17-253):
 //
-//   JVP  jv = (d fEuler / d w) dw : forward mode -- the face flux evaluated on dual numbers
-//        (value, tangent), the same templated code as the FP64 form, so the tangent is the
-//        exact linearisation of what the FP64 kernel computes; then the (linear) divergence.
+//   JVP  jv = (d fEuler / d w) dw : forward mode -- the FP64 face flux (weno64.cuh) carried with
+//        its directional derivative, then the (linear) divergence.
 // The external forcing is constant in w, so it has no derivative.  Kinks (max over the
 // stencil of |u| + c, |u|, the positivity guard of sqrt) take the branch the forward pass took.
+//
+// Bound by the FP64 pipe, so the tangents are written out where a generic dual number would
+// spend instructions on constants' zero tangents and on quotients: 40 instructions for the
+// tangent of a reconstruction on top of its 38 (weno_tan64).  96^3 x 9: 5330 -> ~2600 FP64
+// instructions a face.
 #include "common.cuh"
 #include "weno.cuh"
-#include "weno_face.cuh"
+#include "weno64.cuh"
 #include "weno_sweep.cuh"
 
 namespace gbmv {
 
-// ------------------------------------------------------------------ dual numbers (JVP)
-
+// a value and its tangent
 struct Dual {
   double v, d;
   Dual() = default;
-  __host__ __device__ constexpr Dual(double x) : v(x), d(0.0) {}
-  __host__ __device__ constexpr Dual(double x, double y) : v(x), d(y) {}
+  __device__ Dual(double x, double y) : v(x), d(y) {}
 };
 __device__ __forceinline__ Dual operator+(Dual a, Dual b) { return Dual(a.v + b.v, a.d + b.d); }
 __device__ __forceinline__ Dual operator-(Dual a, Dual b) { return Dual(a.v - b.v, a.d - b.d); }
 __device__ __forceinline__ Dual operator-(Dual a) { return Dual(-a.v, -a.d); }
 __device__ __forceinline__ Dual operator*(Dual a, Dual b) {
-  return Dual(a.v * b.v, a.v * b.d + a.d * b.v);
+  return Dual(a.v * b.v, fma(a.v, b.d, a.d * b.v));
 }
-__device__ __forceinline__ Dual operator/(Dual a, Dual b) {
-  const double q = a.v / b.v;
-  return Dual(q, (a.d - q * b.d) / b.v);
+__device__ __forceinline__ Dual operator*(double a, Dual b) { return Dual(a * b.v, a * b.d); }
+__device__ __forceinline__ Dual dfma(Dual a, Dual b, Dual c) {
+  return Dual(fma(a.v, b.v, c.v), fma(a.v, b.d, fma(a.d, b.v, c.d)));
 }
-__device__ __forceinline__ bool operator<(Dual a, Dual b) { return a.v < b.v; }
-__device__ __forceinline__ bool operator<=(Dual a, Dual b) { return a.v <= b.v; }
-__device__ __forceinline__ Dual num_from(double x, Dual*) { return Dual(x); }
-__device__ __forceinline__ Dual num_sqrt(Dual x) {
-  const double s = sqrt(x.v);
-  return Dual(s, x.d / (2.0 * s));
+__device__ __forceinline__ Dual dfma(double a, Dual b, Dual c) {
+  return Dual(fma(a, b.v, c.v), fma(a, b.d, c.d));
 }
-__device__ __forceinline__ Dual num_fabs(Dual x) { return x.v < 0.0 ? -x : x; }
-__device__ __forceinline__ Dual num_fma(Dual a, Dual b, Dual c) {
-  return Dual(fma(a.v, b.v, c.v), a.v * b.d + a.d * b.v + c.d);
+__device__ __forceinline__ Dual drcp(Dual a) {
+  const double r = 1.0 / a.v;
+  return Dual(r, -(a.d * (r * r)));
 }
-// the FP64 weight combination (product form, one division) on duals
-__device__ __forceinline__ Dual weno_combine(Dual bA, Dual bB, Dual bC, Dual qA, Dual qB, Dual qC,
-                                             Dual dA, Dual dB, Dual dC) {
-  const Dual eps(1e-6);
-  Dual aA = eps + bA, aB = eps + bB, aC = eps + bC;
-  aA = aA * aA;
-  aB = aB * aB;
-  aC = aC * aC;
-  const Dual tA = dA * (aB * aC), tB = dB * (aA * aC), tC = dC * (aA * aB);
-  return (tA * qA + tB * qB + tC * qC) / (tA + tB + tC);
+
+// roe64 with tangents
+struct RoeDual {
+  Dual u, v, w, H, q, c, L00, L01, L02, L03, L04, L30, L31, L40, L41;
+};
+__device__ __forceinline__ void roe_dual(const Dual (&W)[6][5], const Dual (&ph)[6], double gamma,
+                                         RoeDual& R) {
+  const double gm = gamma - 1.0;
+  const double sL = sqrt0_64(W[2][0].v), sR = sqrt0_64(W[3][0].v);
+  const double rL = 1.0 / sL, rR = 1.0 / sR;
+  const double tL = 0.5 * W[2][0].d * rL, tR = 0.5 * W[3][0].d * rR;  // tangents of the roots
+  const Dual iL(rL, -(tL * (rL * rL))), iR(rR, -(tR * (rR * rR)));
+  const Dual is = drcp(Dual(sL + sR, tL + tR));
+  R.u = dfma(W[2][1], iL, W[3][1] * iR) * is;
+  R.v = dfma(W[2][2], iL, W[3][2] * iR) * is;
+  R.w = dfma(W[2][3], iL, W[3][3] * iR) * is;
+  R.H = dfma(dfma(2.0, ph[2], W[2][4]), iL, dfma(2.0, ph[3], W[3][4]) * iR) * is;
+  R.q = Dual(0.5 * fma(R.u.v, R.u.v, fma(R.v.v, R.v.v, R.w.v * R.w.v)),
+             fma(R.u.v, R.u.d, fma(R.v.v, R.v.d, R.w.v * R.w.d)));
+  R.c = gm * (R.H - R.q);
+  const Dual hc = 0.5 * drcp(R.c), hgc = gm * hc, gq = gm * R.q, gu = gm * R.u;
+  R.L00 = hc * (R.u + gq);
+  R.L40 = hc * (gq - R.u);
+  R.L01 = -dfma(gu, hc, hc);
+  R.L41 = hc - gu * hc;
+  R.L02 = -(R.v * hgc);
+  R.L03 = -(R.w * hgc);
+  R.L04 = hgc;
+  R.L30 = 2.0 * (hgc * dfma(-2.0, R.q, R.H));
+  R.L31 = 2.0 * (R.u * hgc);
 }
-template <bool Plus>
-__device__ __forceinline__ Dual weno_safe(Dual f0, Dual f1, Dual f2_, Dual f3, Dual f4) {
-  return weno_side<Plus>(f0, f1, f2_, f3, f4);
+
+// reconstruction of five duals
+__device__ __forceinline__ Dual weno_dual(Dual f0, Dual f1, Dual f2, Dual f3, Dual f4) {
+  Weno64 w;
+  const double r = weno_diff64(f2.v, f0.v - f1.v, f1.v - f2.v, f2.v - f3.v, f3.v - f4.v, w);
+  return Dual(r, weno_tan64(w, f2.d, f0.d - f1.d, f1.d - f2.d, f2.d - f3.d, f3.d - f4.d));
+}
+
+// fluid_side64 with tangents
+template <int SIDE>
+__device__ __forceinline__ void fluid_side_dual(const Dual (&W)[6][5], const Dual (&ph)[6],
+                                                const Dual (&u)[6], const RoeDual& R,
+                                                const Dual (&h)[5], Dual (&ff)[5]) {
+  Dual P[5][5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int j = SIDE ? 5 - k : k;
+    const Dual f0 = W[j][0] * h[k], f1 = dfma(W[j][1], h[k], ph[j]), f2 = W[j][2] * h[k],
+               f3 = W[j][3] * h[k], f4 = dfma(W[j][4], h[k], u[j] * ph[j]);
+    const Dual X = dfma(R.L02, f2, dfma(R.L03, f3, R.L04 * f4));
+    P[k][0] = dfma(R.L00, f0, dfma(R.L01, f1, X));
+    P[k][1] = dfma(-R.v, f0, f2);
+    P[k][2] = dfma(-R.w, f0, f3);
+    P[k][3] = dfma(R.L30, f0, dfma(-2.0, X, R.L31 * f1));
+    P[k][4] = dfma(R.L40, f0, dfma(R.L41, f1, X));
+  }
+#pragma unroll
+  for (int i = 0; i < 5; ++i) ff[i] = weno_dual(P[0][i], P[1][i], P[2][i], P[3][i], P[4][i]);
+}
+
+// one tracer's tangent: both sides of c h, the outer points in one difference each
+__device__ __forceinline__ double tracer_side_tan(Dual c0, Dual h0, Dual c1, Dual h1, Dual c2,
+                                                  Dual h2, Dual c3, Dual h3, Dual c4, Dual h4) {
+  const Dual f1 = c1 * h1, f2 = c2 * h2, f3 = c3 * h3;
+  const Dual D01 = dfma(c0, h0, -f1), D12 = f1 - f2, D23 = f2 - f3, D34 = dfma(-c4, h4, f3);
+  Weno64 w;
+  weno_diff64(f2.v, D01.v, D12.v, D23.v, D34.v, w);
+  return weno_tan64(w, f2.d, D01.d, D12.d, D23.d, D34.d);
 }
 
 // ------------------------------------------------------------------ JVP
 
-template <int NCHEM, int DIR>
-__global__ void __launch_bounds__(128) face_flux_jvp_kernel(Grid g, Fields w, Fields dw,
-                                                            double* __restrict__ dF, long nfaces) {
-  Dual* tag = nullptr;
-  for (long f = blockIdx.x * (long)blockDim.x + threadIdx.x; f < nfaces;
-       f += (long)gridDim.x * blockDim.x) {
-    long cell[6], ijk[3];
+// Tangents of the face fluxes, the three directions in one launch.  PRE: the cell primitives
+// are read (they live in the fluid part of the result until the divergence), else formed here.
+template <int NCHEM, bool PRE>
+__global__ void __launch_bounds__(128) face_flux_jvp_kernel(const __grid_constant__ SweepSet S) {
+  const int dir = sweep_dir(S);
+  const SweepDir& D = S.d[dir];
+  const int nblk = (dir == 2 ? (int)gridDim.x : S.d[dir + 1].block0) - D.block0;
+  const double gm = S.gamma - 1.0;
+  for (long f = (blockIdx.x - D.block0) * (long)blockDim.x + threadIdx.x; f < D.nfaces;
+       f += (long)nblk * blockDim.x) {
+    long cell[6];
     bool nall[6], nnorm[6];
-    stencil<DIR>(g, f, cell, nall, nnorm, ijk);
-    Dual W[6][5];
+    stencil_of(S, D, f, false, cell, nall, nnorm);
+    Stencil64 T;
+    Dual W[6][5], ph[6], u[6];
+    double ir[6];
 #pragma unroll
     for (int l = 0; l < 6; ++l) {
-      double a[5], b[5];
-      load_point<DIR>(w, cell[l], nall[l], nnorm[l], a);
-      load_point<DIR>(dw, cell[l], nall[l], nnorm[l], b);
+      double t[5], v1, v2;
+      load_point(D.f, cell[l], nall[l], nnorm[l], T.W[l]);
+      load_point(D.g, cell[l], nall[l], nnorm[l], t);
+      ir[l] = rcp64(T.W[l][0]);
+      if (PRE) {
+        const double p = __ldg(S.ph + cell[l]), x = __ldg(D.vel[0] + cell[l]);
+        T.ph[l] = nall[l] ? -p : p;
+        T.u[l] = nnorm[l] ? -x : x;
+        T.hc[l] = __ldg(S.hc + cell[l]);
+        v1 = __ldg(D.vel[1] + cell[l]);
+        v2 = __ldg(D.vel[2] + cell[l]);
+      } else {
+        point_prims64(S.gamma, T.W[l][0], T.W[l][1], T.W[l][2], T.W[l][3], T.W[l][4], T.ph[l],
+                      T.hc[l]);
+        T.u[l] = T.W[l][1] / T.W[l][0];
+        v1 = T.W[l][2] / T.W[l][0];
+        v2 = T.W[l][3] / T.W[l][0];
+      }
 #pragma unroll
-      for (int v = 0; v < 5; ++v) W[l][v] = Dual(a[v], b[v]);
+      for (int v = 0; v < 5; ++v) W[l][v] = Dual(T.W[l][v], t[v]);
+      // u = m / rho;  p/2 = (gamma-1)/2 (E - |m|^2 / (2 rho))
+      const double x = T.u[l], q = 0.5 * fma(x, x, fma(v1, v1, v2 * v2));
+      u[l] = Dual(x, fma(-x, t[0], t[1]) * ir[l]);
+      ph[l] = Dual(T.ph[l], 0.5 * gm *
+                   fma(q, t[0], fma(-x, t[1], fma(-v1, t[2], fma(-v2, t[3], t[4])))));
     }
-    FaceState<Dual> S;
-    Dual out[5];
-    fluid_face_flux<Dual>(W, g.gamma, S, out);
-    double o[5];
+    // half the Lax-Friedrichs speed and its tangent at the point that attains the maximum:
+    // (c/2)^2 = gamma (p/2) / (2 rho), so d(c/2) = gamma / (4 rho) (dp/2 - (p/2) drho/rho) / (c/2)
+    int am;
+    const double ha = half_alpha64(T, &am);
+    double su = T.u[0], du = u[0].d, sp = T.ph[0], dp = ph[0].d, sr = W[0][0].d, si = ir[0],
+           sc = T.hc[0];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) o[v] = out[v].d;
-    const double o1 = o[1];
-    o[1] = o[1 + DIR];
-    o[1 + DIR] = o1;
+    for (int l = 1; l < 6; ++l) {
+      const bool m = l == am;
+      su = m ? T.u[l] : su;
+      du = m ? u[l].d : du;
+      sp = m ? T.ph[l] : sp;
+      dp = m ? ph[l].d : dp;
+      sr = m ? W[l][0].d : sr;
+      si = m ? ir[l] : si;
+      sc = m ? T.hc[l] : sc;
+    }
+    double dha = su < 0.0 ? -0.5 * du : 0.5 * du;
+    if (sc > 0.0) dha += 0.25 * S.gamma * si * fma(-(sp * si), sr, dp) / sc;
+    Dual hp[6], hm[6];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) dF[v * nfaces + f] = o[v];
+    for (int l = 0; l < 6; ++l) {
+      hp[l] = dfma(0.5, u[l], Dual(ha, dha));
+      hm[l] = dfma(0.5, u[l], Dual(-ha, -dha));
+    }
+    RoeDual R;
+    roe_dual(W, ph, S.gamma, R);
+    Dual ff[5], fm[5];
+    {
+      const Dual h[5] = {hp[0], hp[1], hp[2], hp[3], hp[4]};
+      fluid_side_dual<0>(W, ph, u, R, h, ff);
+    }
+    {
+      const Dual h[5] = {hm[5], hm[4], hm[3], hm[2], hm[1]};
+      fluid_side_dual<1>(W, ph, u, R, h, fm);
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i) ff[i] = ff[i] + fm[i];
+    const Dual t = ff[0] + ff[4], s = t + ff[3], cd = R.c * (ff[4] - ff[0]);
+    const double o[5] = {
+        s.d, dfma(R.u, s, cd).d, dfma(R.v, s, ff[1]).d, dfma(R.w, s, ff[2]).d,
+        dfma(R.H, t, dfma(R.u, cd, dfma(R.v, ff[1], dfma(R.w, ff[2], R.q * ff[3])))).d};
+#pragma unroll
+    for (int v = 0; v < 5; ++v) D.F[D.slot[v] * D.nfaces + f] = o[v];
 #pragma unroll 1
     for (int c = 0; c < NCHEM; ++c) {
       Dual cv[6];
 #pragma unroll
       for (int l = 0; l < 6; ++l) {
-        const double x = __ldg(w.f[5] + c + (long)NCHEM * cell[l]);
-        const double dx = __ldg(dw.f[5] + c + (long)NCHEM * cell[l]);
+        const double x = __ldg(S.chem + c + (long)NCHEM * cell[l]);
+        const double dx = __ldg(S.gchem + c + (long)NCHEM * cell[l]);
         cv[l] = nall[l] ? Dual(-x, -dx) : Dual(x, dx);
       }
-      dF[(5 + c) * nfaces + f] = tracer_face_flux<Dual>(S, cv).d;
+      D.F[(5 + c) * D.nfaces + f] =
+          tracer_side_tan(cv[0], hp[0], cv[1], hp[1], cv[2], hp[2], cv[3], hp[3], cv[4], hp[4]) +
+          tracer_side_tan(cv[5], hm[5], cv[4], hm[4], cv[3], hm[3], cv[2], hm[2], cv[1], hm[1]);
     }
-    (void)tag;
   }
 }
 
@@ -139,12 +252,24 @@ static int jvp_t(const Grid& g, const Fields& w, const Fields& dw, const Fields&
   double* F[3] = {scratch, scratch + (long)(5 + NCHEM) * nf[0],
                   scratch + (long)(5 + NCHEM) * (nf[0] + nf[1])};
   ProfScope ps("jvp", s);
-  face_flux_jvp_kernel<NCHEM, 0><<<sweep_blocks(nf[0], 128), 128, 0, s>>>(g, w, dw, F[0], nf[0]);
-  GBMV_LAUNCH_CHECK("face_flux_jvp_kernel<x>");
-  face_flux_jvp_kernel<NCHEM, 1><<<sweep_blocks(nf[1], 128), 128, 0, s>>>(g, w, dw, F[1], nf[1]);
-  GBMV_LAUNCH_CHECK("face_flux_jvp_kernel<y>");
-  face_flux_jvp_kernel<NCHEM, 2><<<sweep_blocks(nf[2], 128), 128, 0, s>>>(g, w, dw, F[2], nf[2]);
-  GBMV_LAUNCH_CHECK("face_flux_jvp_kernel<z>");
+  // the primitives live in the fluid part of the result, which the divergence writes last,
+  // unless the call is in place
+  const bool pre = !fields_overlap(g, w, out) && !fields_overlap(g, dw, out);
+  const int t = spread_threads(nf[0] + nf[1] + nf[2], 128);
+  SweepSet S;
+  const int b = sweep_set(g, w, F, 1, t, (long)kSM * 16, S);
+  sweep_second(S, dw);
+  if (pre) {
+    double* const p[5] = {out.f[0], out.f[1], out.f[2], out.f[3], out.f[4]};
+    const int rc = prims64(g, w, p, nullptr, s);
+    if (rc) return rc;
+    const double* const u[3] = {p[1], p[2], p[3]};
+    sweep_prims(S, p[0], u, p[4]);
+    face_flux_jvp_kernel<NCHEM, true><<<b, t, 0, s>>>(S);
+  } else {
+    face_flux_jvp_kernel<NCHEM, false><<<b, t, 0, s>>>(S);
+  }
+  GBMV_LAUNCH_CHECK("face_flux_jvp_kernel");
   divergence_lin_kernel<NCHEM><<<sweep_blocks(g.ncell, 256), 256, 0, s>>>(g, out, F[0], F[1], F[2]);
   GBMV_LAUNCH_CHECK("divergence_lin_kernel");
   return GBMV_OK;

@@ -79,7 +79,8 @@ __device__ __forceinline__ void load_point(const Fields& w, long c, bool nall, b
 struct SweepDir {
   const double* f[5];  // rho, m_normal, m_t1, m_t2, et
   int slot[5];         // their field numbers
-  const double* u;     // normal velocity (null: no primitives)
+  const double* g[5];  // a second ManyVector in the same order (tangents; null: none)
+  const double* vel[3];  // velocities: normal, t1, t2 (null: no primitives)
   double* F;           // face fluxes [field][face]
   long nfaces, ex, ey; // extents of the face grid along x and y
   long n, stride;      // cells along the direction and their spacing in memory
@@ -91,6 +92,7 @@ struct SweepSet {
   const double* ph;    // half pressure, half sound speed (null: no primitives)
   const double* hc;
   const double* chem;
+  const double* gchem; // the second ManyVector's tracers
   long nx, ny;
   double gamma;
 };
@@ -114,10 +116,10 @@ __device__ __forceinline__ void stencil_of(const SweepSet& S, const SweepDir& D,
 }
 
 // the fluid values of a stencil point in face order, ghost signs applied
-__device__ __forceinline__ void load_point(const SweepDir& D, long c, bool nall, bool nnorm,
-                                           double (&W)[5]) {
+__device__ __forceinline__ void load_point(const double* const (&f)[5], long c, bool nall,
+                                           bool nnorm, double (&W)[5]) {
 #pragma unroll
-  for (int v = 0; v < 5; ++v) W[v] = __ldg(D.f[v] + c);
+  for (int v = 0; v < 5; ++v) W[v] = __ldg(f[v] + c);
   if (nall) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) W[v] = -W[v];
@@ -157,6 +159,25 @@ inline void face_counts(const Grid& g, long (&nf)[3]) {
   nf[2] = nx * ny * (nz + 1);
 }
 
+// the cell primitives (half pressure, three velocities, half sound speed) of a sweep
+inline void sweep_prims(SweepSet& S, const double* ph, const double* const (&u)[3],
+                        const double* hc) {
+  S.ph = ph;
+  S.hc = hc;
+  for (int d = 0; d < 3; ++d) {
+    S.d[d].vel[0] = u[d];
+    S.d[d].vel[1] = u[d == 0 ? 1 : (d == 1 ? 0 : 1)];
+    S.d[d].vel[2] = u[d == 2 ? 0 : 2];
+  }
+}
+
+// a second ManyVector read beside w
+inline void sweep_second(SweepSet& S, const Fields& v) {
+  for (int d = 0; d < 3; ++d)
+    for (int k = 0; k < 5; ++k) S.d[d].g[k] = v.f[S.d[d].slot[k]];
+  S.gchem = v.f[5];
+}
+
 // The three directions of w for a sweep of `per_face` threads a face in blocks of t threads,
 // fluxes to F (null: none); returns the number of blocks (at most cap per direction).
 inline int sweep_set(const Grid& g, const Fields& w, double* const* F, int per_face, int t,
@@ -171,7 +192,8 @@ inline int sweep_set(const Grid& g, const Fields& w, double* const* F, int per_f
       D.slot[v] = slot[v];
       D.f[v] = w.f[slot[v]];
     }
-    D.u = nullptr;
+    for (int v = 0; v < 5; ++v) D.g[v] = nullptr;
+    for (int v = 0; v < 3; ++v) D.vel[v] = nullptr;
     D.F = F ? F[d] : nullptr;
     D.nfaces = nf[d];
     D.ex = g.n[0] + (d == 0);
@@ -187,6 +209,7 @@ inline int sweep_set(const Grid& g, const Fields& w, double* const* F, int per_f
   }
   S.ph = S.hc = nullptr;
   S.chem = w.f[5];
+  S.gchem = nullptr;
   S.nx = g.n[0];
   S.ny = g.n[1];
   S.gamma = g.gamma;

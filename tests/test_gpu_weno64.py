@@ -57,3 +57,21 @@ def test_fp64_forms_flag_illegal_states(cuda):
             status = torch.zeros(1, dtype=torch.int32, device="cuda")
             h.fEuler_async(0.0, w, out, status, gbmv.FP64, flags)
             assert int(status.item()) & bit
+
+
+@pytest.mark.parametrize("nchem", [0, 4])
+def test_jvp_in_place_matches_out_of_place(cuda, nchem):
+    """jv may be dw itself: the primitives are then formed per stencil point instead of in jv.
+    The two forms differ by the rounding of the velocities and the pressure (~1e-15 per flux)."""
+    torch = cuda
+    import gbmv
+    wl = W.rayleigh_taylor(shape=(13, 9, 7), nchem=nchem, seed=W.SEED_BASE + 702)
+    h = gbmv.Hydro((13, 9, 7), nchem, (3, 3, 0, 0, 1, 3), wl["gamma"], None)
+    w = [torch.from_numpy(np.ascontiguousarray(f)).cuda() for f in wl["fields"]]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    d = [torch.rand(f.shape, generator=gen, device="cuda", dtype=torch.float64) - 0.5 for f in w]
+    out = [torch.empty_like(f) for f in w]
+    h.fEuler_jvp(0.0, w, d, out)
+    h.fEuler_jvp(0.0, w, d, d)
+    for a, b in zip(d, out):
+        assert maxnorm_err(a.cpu().numpy(), b.cpu().numpy()) <= 1e-12
