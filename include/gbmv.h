@@ -154,7 +154,8 @@ int gbmv_stability(gbmv_hydro h, const double* const* w, double cfl, double* dt_
  * All arguments are ManyVectors laid out like w.  The constant external force has no
  * derivative.  At kinks (the Lax-Friedrichs max over the stencil, |u|) the branch the forward
  * evaluation took is differentiated.  The first VJP call on a handle allocates
- * 6 (5+nchem) x (faces of one direction) doubles: make it before any stream capture.
+ * 6 (5+nchem) x (faces of one direction) + 5 x (cells) doubles: make it before any stream
+ * capture.
  * Asynchronous; returns 0 or < 0. */
 int gbmv_feuler_jvp(gbmv_hydro h, double t, const double* const* w, const double* const* dw,
                     double* const* jv, void* stream);

@@ -8,430 +8,328 @@
 //        deterministic result) sums them into u.
 // The external forcing is constant in w, so it has no derivative.  Kinks (max over the
 // stencil of |u| + c, |u|, the positivity guard of sqrt) take the branch the forward pass took.
+//
+// Bound by the FP64 pipe.  The adjoint of a reconstruction works on the neighbour differences
+// and takes the forward weights' products (weno_adj64: 47 instructions after the forward 38; the
+// adjoint of the literal formula took ~250 with its seven divisions), the primitives come from
+// a cell pass, and each point's reciprocal density is formed once.  96^3 x 9: 6120 -> ~2500
+// FP64 instructions a face.
 #include "common.cuh"
 #include "weno.cuh"
-#include "weno_face.cuh"
+#include "weno64.cuh"
 #include "weno_sweep.cuh"
 
 namespace gbmv {
 
 // ------------------------------------------------------------------ VJP
 
-// Reverse sweep of the WENO5 reconstruction weno_side<Plus, double>: fb += (dr/df)^T rb.
-template <bool Plus>
-__device__ __forceinline__ void weno_side_adj(const double (&f)[5], double rb, double (&fb)[5]) {
-  const double dA = f[2] - 2.0 * f[3] + f[4], eA = 3.0 * f[2] - 4.0 * f[3] + f[4];
-  const double dB = f[1] - 2.0 * f[2] + f[3], eB = f[1] - f[3];
-  const double dC = f[0] - 2.0 * f[1] + f[2], eC = f[0] - 4.0 * f[1] + 3.0 * f[2];
-  const double aA = 1e-6 + ((13.0 / 12.0) * (dA * dA) + 0.25 * (eA * eA));
-  const double aB = 1e-6 + ((13.0 / 12.0) * (dB * dB) + 0.25 * (eB * eB));
-  const double aC = 1e-6 + ((13.0 / 12.0) * (dC * dC) + 0.25 * (eC * eC));
-  // candidate polynomials and linear weights (coefficients of f0..f4)
-  const double c13 = 1.0 / 3.0, c56 = 5.0 / 6.0, c16 = 1.0 / 6.0, c76 = 7.0 / 6.0,
-               c116 = 11.0 / 6.0;
-  double QA[5], QB[5], QC[5], wA, wB, wC;
-  if (Plus) {
-    const double a[5] = {0.0, 0.0, c13, c56, -c16}, b[5] = {0.0, -c16, c56, c13, 0.0},
-                 c[5] = {c13, -c76, c116, 0.0, 0.0};
-#pragma unroll
-    for (int m = 0; m < 5; ++m) { QA[m] = a[m]; QB[m] = b[m]; QC[m] = c[m]; }
-    wA = 0.3; wB = 0.6; wC = 0.1;
-  } else {
-    const double a[5] = {0.0, 0.0, c116, -c76, c13}, b[5] = {0.0, c13, c56, -c16, 0.0},
-                 c[5] = {-c16, c56, c13, 0.0, 0.0};
-#pragma unroll
-    for (int m = 0; m < 5; ++m) { QA[m] = a[m]; QB[m] = b[m]; QC[m] = c[m]; }
-    wA = 0.1; wB = 0.6; wC = 0.3;
-  }
-  double qA = 0.0, qB = 0.0, qC = 0.0;
-#pragma unroll
-  for (int m = 0; m < 5; ++m) {
-    qA += QA[m] * f[m];
-    qB += QB[m] * f[m];
-    qC += QC[m] * f[m];
-  }
-  const double tA = wA / (aA * aA), tB = wB / (aB * aB), tC = wC / (aC * aC);
-  const double S = tA + tB + tC, iS = 1.0 / S;
-  const double r = (tA * qA + tB * qB + tC * qC) * iS;
-  // r = sum w_k q_k, w_k = t_k / S;  dr/dq_k = w_k;  dr/dt_k = (q_k - r) / S;
-  // t_k = d_k / a_k^2 -> dt_k/da_k = -2 t_k / a_k;  a_k = eps + 13/12 d^2 + 1/4 e^2
-  const double gA = rb * (qA - r) * iS * (-2.0 * tA / aA);
-  const double gB = rb * (qB - r) * iS * (-2.0 * tB / aB);
-  const double gC = rb * (qC - r) * iS * (-2.0 * tC / aC);
-  const double wqA = rb * tA * iS, wqB = rb * tB * iS, wqC = rb * tC * iS;
-  const double DA[5] = {0.0, 0.0, 1.0, -2.0, 1.0}, EA[5] = {0.0, 0.0, 3.0, -4.0, 1.0};
-  const double DB[5] = {0.0, 1.0, -2.0, 1.0, 0.0}, EB[5] = {0.0, 1.0, 0.0, -1.0, 0.0};
-  const double DC[5] = {1.0, -2.0, 1.0, 0.0, 0.0}, EC[5] = {1.0, -4.0, 3.0, 0.0, 0.0};
-  const double kdA = gA * (13.0 / 6.0) * dA, keA = gA * 0.5 * eA;
-  const double kdB = gB * (13.0 / 6.0) * dB, keB = gB * 0.5 * eB;
-  const double kdC = gC * (13.0 / 6.0) * dC, keC = gC * 0.5 * eC;
-#pragma unroll
-  for (int m = 0; m < 5; ++m)
-    fb[m] += wqA * QA[m] + wqB * QB[m] + wqC * QC[m] + kdA * DA[m] + keA * EA[m] + kdB * DB[m] +
-             keB * EB[m] + kdC * DC[m] + keC * EC[m];
+// the five split fluxes of a point, as fluid_side64 forms them
+__device__ __forceinline__ void split_point64(const Stencil64& S, int j, double h,
+                                              double (&f)[5]) {
+  f[0] = S.W[j][0] * h;
+  f[1] = fma(S.W[j][1], h, S.ph[j]);
+  f[2] = S.W[j][2] * h;
+  f[3] = S.W[j][3] * h;
+  f[4] = fma(S.W[j][4], h, S.u[j] * S.ph[j]);
 }
 
-// Adjoint of fluid_face_flux<double> + tracer_face_flux<double> for one face.
-//   W[6][5]  stencil (face order, signed), ob[5] cotangent of the five fluid fluxes (face
-//   order).  Tracers are handled by the caller through hpb/hmb (cotangents of the split
-//   factors 0.5 (u_j +- alpha)); this returns Wb[6][5] += the fluid-state cotangents.
-struct FluidFwd {
-  double p[6], uj[6], sL, sR, sbar, u, v, ww, H, qsq, c, ci;
-  double L00, L01, L02, L03, L04, L30, L31, L32, L33, L34, L40, L41;
-  double hc, hgc, gc, alpha, ha;
-  int amax;
+// Cotangents gathered over the face: of the Roe values and eigenvector entries, of the points'
+// state, half pressure, velocity and of half the Lax-Friedrichs speed.
+struct Adj64 {
+  double W[6][5], ph[6], u[6], ha;
+  double v, w;
+  double L00, L01, L02, L03, L04, L30, L31, L40, L41;
 };
 
-__device__ __forceinline__ void fluid_forward(const double (&W)[6][5], double gamma, FluidFwd& F) {
-  const double gm = gamma - 1.0;
+// characteristic values of one side, points in upwind order as fluid_side64
+template <int SIDE>
+__device__ __forceinline__ void fluid_side_project(const Stencil64& S, const Roe64& R,
+                                                   const double (&h)[5], double (&P)[5][5]) {
 #pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    F.p[j] = eos_t(gm, W[j][0], W[j][1], W[j][2], W[j][3], W[j][4]);
-    F.uj[j] = W[j][1] / W[j][0];
+  for (int k = 0; k < 5; ++k) {
+    double f[5];
+    split_point64(S, SIDE ? 5 - k : k, h[k], f);
+    const double X = fma(R.L02, f[2], fma(R.L03, f[3], R.L04 * f[4]));
+    P[k][0] = fma(R.L00, f[0], fma(R.L01, f[1], X));
+    P[k][1] = fma(-R.v, f[0], f[2]);
+    P[k][2] = fma(-R.w, f[0], f[3]);
+    P[k][3] = fma(R.L30, f[0], fma(-2.0, X, R.L31 * f[1]));
+    P[k][4] = fma(R.L40, f[0], fma(R.L41, f[1], X));
   }
-  F.sL = sqrt0(W[2][0]);
-  F.sR = sqrt0(W[3][0]);
-  F.sbar = 0.5 * (F.sL + F.sR);
-  F.u = 0.5 * (W[2][1] / F.sL + W[3][1] / F.sR) / F.sbar;
-  F.v = 0.5 * (W[2][2] / F.sL + W[3][2] / F.sR) / F.sbar;
-  F.ww = 0.5 * (W[2][3] / F.sL + W[3][3] / F.sR) / F.sbar;
-  F.H = 0.5 * ((F.p[2] + W[2][4]) / F.sL + (F.p[3] + W[3][4]) / F.sR) / F.sbar;
-  F.qsq = F.u * F.u + F.v * F.v + F.ww * F.ww;
-  F.c = gm * (F.H - 0.5 * F.qsq);
-  F.ci = 1.0 / F.c;
-  F.hgc = 0.5 * gm * F.ci;
-  F.hc = 0.5 * F.ci;
-  F.gc = gm * F.ci;
-  const double u = F.u, v = F.v, ww = F.ww, qsq = F.qsq, H = F.H;
-  F.L00 = F.hc * (u + 0.5 * gm * qsq);
-  F.L01 = -F.hc * (gm * u + 1.0);
-  F.L02 = -v * F.hgc;
-  F.L03 = -ww * F.hgc;
-  F.L04 = F.hgc;
-  F.L30 = -F.gc * (qsq - H);
-  F.L31 = u * F.gc;
-  F.L32 = v * F.gc;
-  F.L33 = ww * F.gc;
-  F.L34 = -F.gc;
-  F.L40 = -F.hc * (u - 0.5 * gm * qsq);
-  F.L41 = -F.hc * (gm * u - 1.0);
-  double alpha = 0.0;
-  int am = 0;
-#pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    const double s = fabs(F.uj[j]) + sqrt0(gamma * F.p[j] / W[j][0]);
-    if (alpha < s) { alpha = s; am = j; }
-  }
-  F.alpha = alpha;
-  F.amax = am;
-  F.ha = 0.5 * alpha;
 }
 
-__device__ __forceinline__ void split_point(const FluidFwd& F, const double (&W)[6][5], int pt,
-                                            double sa, double (&fs)[5]) {
-  const double uj = F.uj[pt], p = F.p[pt];
-  const double hf[5] = {0.5 * W[pt][1], 0.5 * (uj * W[pt][1] + p), 0.5 * (uj * W[pt][2]),
-                        0.5 * (uj * W[pt][3]), 0.5 * (uj * (W[pt][4] + p))};
+// The forward reconstruction of component i and, in place of its five points, their cotangents
+__device__ __forceinline__ double weno_fwd_adj(double (&P)[5][5], int i, double rb) {
+  Weno64 w;
+  const double r = weno_diff64(P[2][i], P[0][i] - P[1][i], P[1][i] - P[2][i], P[2][i] - P[3][i],
+                               P[3][i] - P[4][i], w);
+  double b[5];
+  weno_adj64(w, rb, b);
 #pragma unroll
-  for (int m = 0; m < 5; ++m) fs[m] = fma(sa, W[pt][m], hf[m]);
+  for (int k = 0; k < 5; ++k) P[k][i] = b[k];
+  return r;
 }
 
-__device__ __forceinline__ void project(const FluidFwd& F, const double (&fs)[5], double (&pr)[5]) {
-  pr[0] = F.L00 * fs[0] + F.L01 * fs[1] + F.L02 * fs[2] + F.L03 * fs[3] + F.L04 * fs[4];
-  pr[1] = fs[2] - F.v * fs[0];
-  pr[2] = fs[3] - F.ww * fs[0];
-  pr[3] = F.L30 * fs[0] + F.L31 * fs[1] + F.L32 * fs[2] + F.L33 * fs[3] + F.L34 * fs[4];
-  pr[4] = F.L40 * fs[0] + F.L41 * fs[1] + F.L02 * fs[2] + F.L03 * fs[3] + F.L04 * fs[4];
+// One side of the fluid part: from the cotangents ffb of its reconstructions, their values into
+// ff and the adjoint of projection and splitting into B.
+template <int SIDE>
+__device__ __forceinline__ void fluid_side_adj(const Stencil64& S, const Roe64& R,
+                                               const double (&h)[5], const double (&ffb)[5],
+                                               double (&ff)[5], Adj64& B) {
+  double P[5][5];
+  fluid_side_project<SIDE>(S, R, h, P);
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const double r = weno_fwd_adj(P, i, ffb[i]);
+    ff[i] = SIDE ? ff[i] + r : r;
+  }
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int j = SIDE ? 5 - k : k;
+    const double(&b)[5] = P[k];
+    double f[5], fb[5];
+    split_point64(S, j, h[k], f);
+    const double Xb = fma(-2.0, b[3], b[0] + b[4]);
+    B.L00 = fma(b[0], f[0], B.L00);
+    B.L01 = fma(b[0], f[1], B.L01);
+    B.L02 = fma(Xb, f[2], B.L02);
+    B.L03 = fma(Xb, f[3], B.L03);
+    B.L04 = fma(Xb, f[4], B.L04);
+    B.L30 = fma(b[3], f[0], B.L30);
+    B.L31 = fma(b[3], f[1], B.L31);
+    B.L40 = fma(b[4], f[0], B.L40);
+    B.L41 = fma(b[4], f[1], B.L41);
+    B.v = fma(-b[1], f[0], B.v);
+    B.w = fma(-b[2], f[0], B.w);
+    fb[0] = fma(R.L00, b[0], fma(R.L40, b[4], fma(R.L30, b[3], fma(-R.v, b[1], -R.w * b[2]))));
+    fb[1] = fma(R.L01, b[0], fma(R.L41, b[4], R.L31 * b[3]));
+    fb[2] = fma(R.L02, Xb, b[1]);
+    fb[3] = fma(R.L03, Xb, b[2]);
+    fb[4] = R.L04 * Xb;
+    double hb = 0.0;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      B.W[j][m] = fma(h[k], fb[m], B.W[j][m]);
+      hb = m ? fma(S.W[j][m], fb[m], hb) : S.W[j][0] * fb[0];
+    }
+    B.ph[j] += fma(S.u[j], fb[4], fb[1]);
+    B.u[j] = fma(S.ph[j], fb[4], fma(0.5, hb, B.u[j]));
+    B.ha = SIDE ? B.ha - hb : B.ha + hb;
+  }
 }
 
-__device__ void fluid_face_adjoint(const double (&W)[6][5], double gamma, const FluidFwd& F,
-                                   const double (&ob)[5], const double (&hpb)[6],
-                                   const double (&hmb)[6], double (&Wb)[6][5]) {
-  const double gm = gamma - 1.0;
-  const double u = F.u, v = F.v, ww = F.ww, H = F.H, qsq = F.qsq, c = F.c;
-  // forward characteristic values and reconstructions
-  double pr[2][5][5], ff[5];
+// one side of a tracer: cotangents of its values and of the split factors
+__device__ __forceinline__ void tracer_side_adj(const double (&c)[5], const double (&h)[5],
+                                                double rb, double (&cb)[5], double (&hb)[5]) {
+  Weno64 w;
+  weno_prod64(c[0], h[0], c[1], h[1], c[2], h[2], c[3], h[3], c[4], h[4], w);
+  double b[5];
+  weno_adj64(w, rb, b);
 #pragma unroll
-  for (int side = 0; side < 2; ++side) {
-    const double sa = side == 0 ? F.ha : -F.ha;
-#pragma unroll
-    for (int j = 0; j < 5; ++j) {
-      double fs[5];
-      split_point(F, W, j + side, sa, fs);
-      project(F, fs, pr[side][j]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 5; ++i)
-    ff[i] = weno_side<true>(pr[0][0][i], pr[0][1][i], pr[0][2][i], pr[0][3][i], pr[0][4][i]) +
-            weno_side<false>(pr[1][0][i], pr[1][1][i], pr[1][2][i], pr[1][3][i], pr[1][4][i]);
-  // back-projection: out = R ff
-  double ub = 0.0, vb = 0.0, wwb = 0.0, Hb = 0.0, qb = 0.0, cb = 0.0;
-  const double s034 = ff[0] + ff[3] + ff[4], d04 = ff[4] - ff[0];
-  ub += ob[1] * s034 + ob[4] * c * d04;
-  cb += ob[1] * d04 + ob[4] * u * d04;
-  vb += ob[2] * s034 + ob[4] * ff[1];
-  wwb += ob[3] * s034 + ob[4] * ff[2];
-  Hb += ob[4] * (ff[0] + ff[4]);
-  qb += ob[4] * 0.5 * ff[3];
-  double ffb[5];
-  ffb[0] = ob[0] + ob[1] * (u - c) + ob[2] * v + ob[3] * ww + ob[4] * (H - u * c);
-  ffb[1] = ob[2] + ob[4] * v;
-  ffb[2] = ob[3] + ob[4] * ww;
-  ffb[3] = ob[0] + ob[1] * u + ob[2] * v + ob[3] * ww + ob[4] * (0.5 * qsq);
-  ffb[4] = ob[0] + ob[1] * (u + c) + ob[2] * v + ob[3] * ww + ob[4] * (H + u * c);
-  // WENO reconstructions, projections, splitting
-  double Lb[13] = {0};  // L00 L01 L02 L03 L04 L30 L31 L32 L33 L34 L40 L41, [12] unused
-  double hab = 0.0;
-  double hfb[6][5] = {{0}};
-#pragma unroll
-  for (int side = 0; side < 2; ++side) {
-    double prb[5][5] = {{0}};
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      const double col[5] = {pr[side][0][i], pr[side][1][i], pr[side][2][i], pr[side][3][i],
-                             pr[side][4][i]};
-      double cb5[5] = {0, 0, 0, 0, 0};
-      if (side == 0) weno_side_adj<true>(col, ffb[i], cb5);
-      else weno_side_adj<false>(col, ffb[i], cb5);
-#pragma unroll
-      for (int j = 0; j < 5; ++j) prb[j][i] = cb5[j];
-    }
-    const double sa = side == 0 ? F.ha : -F.ha;
-#pragma unroll
-    for (int j = 0; j < 5; ++j) {
-      const int pt = j + side;
-      double fs[5];
-      split_point(F, W, pt, sa, fs);
-      const double* b = prb[j];
-      Lb[0] += b[0] * fs[0];
-      Lb[1] += b[0] * fs[1];
-      Lb[2] += (b[0] + b[4]) * fs[2];
-      Lb[3] += (b[0] + b[4]) * fs[3];
-      Lb[4] += (b[0] + b[4]) * fs[4];
-      Lb[5] += b[3] * fs[0];
-      Lb[6] += b[3] * fs[1];
-      Lb[7] += b[3] * fs[2];
-      Lb[8] += b[3] * fs[3];
-      Lb[9] += b[3] * fs[4];
-      Lb[10] += b[4] * fs[0];
-      Lb[11] += b[4] * fs[1];
-      vb -= b[1] * fs[0];
-      wwb -= b[2] * fs[0];
-      double fsb[5];
-      fsb[0] = F.L00 * b[0] - v * b[1] - ww * b[2] + F.L30 * b[3] + F.L40 * b[4];
-      fsb[1] = F.L01 * b[0] + F.L31 * b[3] + F.L41 * b[4];
-      fsb[2] = F.L02 * b[0] + b[1] + F.L32 * b[3] + F.L02 * b[4];
-      fsb[3] = F.L03 * b[0] + b[2] + F.L33 * b[3] + F.L03 * b[4];
-      fsb[4] = F.L04 * b[0] + F.L34 * b[3] + F.L04 * b[4];
-      double sab = 0.0;
-#pragma unroll
-      for (int m = 0; m < 5; ++m) {
-        Wb[pt][m] += sa * fsb[m];
-        hfb[pt][m] += fsb[m];
-        sab += fsb[m] * W[pt][m];
-      }
-      hab += side == 0 ? sab : -sab;
-    }
-  }
-  // tracer split factors hp = 0.5 u_j + ha, hm = 0.5 u_j - ha
-  double ujb[6], pb[6];
-#pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    ujb[j] = 0.5 * (hpb[j] + hmb[j]);
-    hab += hpb[j] - hmb[j];
-    pb[j] = 0.0;
-  }
-  // ha = alpha / 2, alpha = max_j (|u_j| + sqrt0(gamma p_j / rho_j))
-  {
-    const int j = F.amax;
-    const double sb = 0.5 * hab;
-    ujb[j] += (F.uj[j] < 0.0 ? -sb : sb);
-    const double x = gamma * F.p[j] / W[j][0];
-    if (x > 0.0) {
-      const double xb = sb * 0.5 / sqrt(x);
-      pb[j] += xb * gamma / W[j][0];
-      Wb[j][0] -= xb * x / W[j][0];
-    }
-  }
-  // halved point fluxes
-#pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    const double uj = F.uj[j], p = F.p[j];
-    const double* hb = hfb[j];
-    Wb[j][1] += 0.5 * hb[0] + 0.5 * uj * hb[1];
-    ujb[j] += 0.5 * (hb[1] * W[j][1] + hb[2] * W[j][2] + hb[3] * W[j][3] + hb[4] * (W[j][4] + p));
-    pb[j] += 0.5 * (hb[1] + uj * hb[4]);
-    Wb[j][2] += 0.5 * uj * hb[2];
-    Wb[j][3] += 0.5 * uj * hb[3];
-    Wb[j][4] += 0.5 * uj * hb[4];
-    // u_j = m_j / rho_j
-    Wb[j][1] += ujb[j] / W[j][0];
-    Wb[j][0] -= ujb[j] * uj / W[j][0];
-  }
-  // left eigenvector entries -> (hc, hgc, gc, u, v, ww, qsq, H)
-  double hcb = 0.0, hgcb = 0.0, gcb = 0.0;
-  hcb += Lb[0] * (u + 0.5 * gm * qsq);
-  ub += Lb[0] * F.hc;
-  qb += Lb[0] * F.hc * 0.5 * gm;
-  hcb -= Lb[1] * (gm * u + 1.0);
-  ub -= Lb[1] * F.hc * gm;
-  vb -= Lb[2] * F.hgc;
-  hgcb -= Lb[2] * v;
-  wwb -= Lb[3] * F.hgc;
-  hgcb -= Lb[3] * ww;
-  hgcb += Lb[4];
-  gcb -= Lb[5] * (qsq - H);
-  qb -= Lb[5] * F.gc;
-  Hb += Lb[5] * F.gc;
-  ub += Lb[6] * F.gc;
-  gcb += Lb[6] * u;
-  vb += Lb[7] * F.gc;
-  gcb += Lb[7] * v;
-  wwb += Lb[8] * F.gc;
-  gcb += Lb[8] * ww;
-  gcb -= Lb[9];
-  hcb -= Lb[10] * (u - 0.5 * gm * qsq);
-  ub -= Lb[10] * F.hc;
-  qb += Lb[10] * F.hc * 0.5 * gm;
-  hcb -= Lb[11] * (gm * u - 1.0);
-  ub -= Lb[11] * F.hc * gm;
-  const double cib = 0.5 * hcb + 0.5 * gm * hgcb + gm * gcb;
-  cb -= cib * F.ci * F.ci;
-  // c = gm (H - qsq / 2)
-  Hb += gm * cb;
-  qb -= 0.5 * gm * cb;
-  // qsq = u^2 + v^2 + ww^2
-  ub += 2.0 * u * qb;
-  vb += 2.0 * v * qb;
-  wwb += 2.0 * ww * qb;
-  // Roe averages: X = a/sL + b/sR, value = X / (2 sbar)
-  double sLb = 0.0, sRb = 0.0, sbb = 0.0;
-  const double ib = 0.5 / F.sbar;
-  auto roe = [&](double val, double vb_, double a, double b, double& ab, double& bb) {
-    const double Xb = vb_ * ib;
-    sbb -= vb_ * val / F.sbar;
-    ab += Xb / F.sL;
-    sLb -= Xb * a / (F.sL * F.sL);
-    bb += Xb / F.sR;
-    sRb -= Xb * b / (F.sR * F.sR);
-  };
-  roe(u, ub, W[2][1], W[3][1], Wb[2][1], Wb[3][1]);
-  roe(v, vb, W[2][2], W[3][2], Wb[2][2], Wb[3][2]);
-  roe(ww, wwb, W[2][3], W[3][3], Wb[2][3], Wb[3][3]);
-  {
-    double a2 = 0.0, a3 = 0.0;
-    roe(H, Hb, F.p[2] + W[2][4], F.p[3] + W[3][4], a2, a3);
-    pb[2] += a2;
-    Wb[2][4] += a2;
-    pb[3] += a3;
-    Wb[3][4] += a3;
-  }
-  sLb += 0.5 * sbb;
-  sRb += 0.5 * sbb;
-  if (W[2][0] > 0.0) Wb[2][0] += sLb * 0.5 / F.sL;
-  if (W[3][0] > 0.0) Wb[3][0] += sRb * 0.5 / F.sR;
-  // p_j = gm (E - (mx^2 + my^2 + mz^2) / (2 rho))
-#pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    const double rho = W[j][0];
-    const double K = (W[j][1] * W[j][1] + W[j][2] * W[j][2] + W[j][3] * W[j][3]) * 0.5 / rho;
-    const double Kb = -gm * pb[j];
-    Wb[j][4] += gm * pb[j];
-    Wb[j][1] += Kb * W[j][1] / rho;
-    Wb[j][2] += Kb * W[j][2] / rho;
-    Wb[j][3] += Kb * W[j][3] / rho;
-    Wb[j][0] -= Kb * K / rho;
+  for (int k = 0; k < 5; ++k) {
+    cb[k] = b[k] * h[k];
+    hb[k] = fma(b[k], c[k], hb[k]);
   }
 }
 
 // Face cotangents -> per-face stencil cotangents A[(l * NVAR + v) * nfaces + f] (original
-// field order, ghost signs applied, so each entry belongs to the source cell of slot l).
-template <int NCHEM, int DIR>
-__global__ void __launch_bounds__(128) face_flux_vjp_kernel(Grid g, Fields w, Fields vb,
-                                                            double* __restrict__ A, long nfaces) {
+// field order, ghost signs applied, so each entry belongs to the source cell of slot l), for the
+// one direction the launch covers.  S.d[dir].g: the cotangent ManyVector in face order.
+template <int NCHEM>
+__global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constant__ SweepSet S,
+                                                            int dir, double inv_d,
+                                                            double* __restrict__ A) {
   constexpr int NV = 5 + NCHEM;
-  const long nd = g.n[DIR];
-  const long stride[3] = {1, g.n[0], g.n[0] * g.n[1]};
+  const SweepDir& D = S.d[dir];
+  const long nfaces = D.nfaces;
+  const double gm = S.gamma - 1.0;
   for (long f = blockIdx.x * (long)blockDim.x + threadIdx.x; f < nfaces;
        f += (long)gridDim.x * blockDim.x) {
-    long cell[6], ijk[3];
+    long cell[6];
     bool nall[6], nnorm[6];
-    stencil<DIR>(g, f, cell, nall, nnorm, ijk);
+    stencil_of(S, D, f, false, cell, nall, nnorm);
     // face cotangent: + v_i / d for the cell above (i < n), - v_{i-1} / d for the one below
-    const long id = ijk[DIR];
-    const long cup = ijk[0] + g.n[0] * (ijk[1] + g.n[1] * ijk[2]);  // valid when id < nd
-    const long cdn = cup - stride[DIR];
-    double cF[NV];
+    long i0, j0, k0;
+    split3(f, D.ex, D.ey, i0, j0, k0);
+    const long id = dir == 0 ? i0 : (dir == 1 ? j0 : k0);
+    const long cup = i0 + S.nx * (j0 + S.ny * k0);  // valid when id < n
+    const long cdn = cup - D.stride;
+    double ob[5];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
+    for (int v = 0; v < 5; ++v) {
       double a = 0.0;
-      if (id < nd) a += (v < 5) ? vb.f[v][cup] : vb.f[5][(v - 5) + (long)NCHEM * cup];
-      if (id >= 1) a -= (v < 5) ? vb.f[v][cdn] : vb.f[5][(v - 5) + (long)NCHEM * cdn];
-      cF[v] = a * g.inv_d[DIR];
+      if (id < D.n) a = D.g[v][cup];
+      if (id >= 1) a -= D.g[v][cdn];
+      ob[v] = a * inv_d;
     }
-    double W[6][5];
-#pragma unroll
-    for (int l = 0; l < 6; ++l) load_point<DIR>(w, cell[l], nall[l], nnorm[l], W[l]);
-    FluidFwd F;
-    fluid_forward(W, g.gamma, F);
-    // tracers first: their cotangents of the split factors feed the fluid adjoint
-    double hpb[6] = {0}, hmb[6] = {0};
-#pragma unroll 1
-    for (int c = 0; c < NCHEM; ++c) {
-      const double rb = cF[5 + c];
-      double cv[6], gp[5], gmv[5];
-#pragma unroll
-      for (int l = 0; l < 6; ++l) {
-        const double x = __ldg(w.f[5] + c + (long)NCHEM * cell[l]);
-        cv[l] = nall[l] ? -x : x;
-      }
-      double hp[6], hm[6];
-#pragma unroll
-      for (int l = 0; l < 6; ++l) {
-        hp[l] = 0.5 * F.uj[l] + F.ha;
-        hm[l] = 0.5 * F.uj[l] - F.ha;
-      }
-#pragma unroll
-      for (int l = 0; l < 5; ++l) {
-        gp[l] = cv[l] * hp[l];
-        gmv[l] = cv[l + 1] * hm[l + 1];
-      }
-      double gpb[5] = {0, 0, 0, 0, 0}, gmb[5] = {0, 0, 0, 0, 0};
-      weno_side_adj<true>(gp, rb, gpb);
-      weno_side_adj<false>(gmv, rb, gmb);
-      double cvb[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-      for (int l = 0; l < 5; ++l) {
-        cvb[l] += gpb[l] * hp[l];
-        hpb[l] += gpb[l] * cv[l];
-        cvb[l + 1] += gmb[l] * hm[l + 1];
-        hmb[l + 1] += gmb[l] * cv[l + 1];
-      }
-#pragma unroll
-      for (int l = 0; l < 6; ++l)
-        A[((long)l * NV + 5 + c) * nfaces + f] = nall[l] ? -cvb[l] : cvb[l];
-    }
-    // fluid: cotangent of the five fluxes in face order
-    double ob[5] = {cF[0], cF[1 + DIR], DIR == 1 ? cF[1] : cF[2], DIR == 2 ? cF[1] : cF[3], cF[4]};
-    double Wb[6][5] = {{0}};
-    fluid_face_adjoint(W, g.gamma, F, ob, hpb, hmb, Wb);
+    Stencil64 T;
 #pragma unroll
     for (int l = 0; l < 6; ++l) {
+      load_point(D.f, cell[l], nall[l], nnorm[l], T.W[l]);
+      const double p = __ldg(S.ph + cell[l]), x = __ldg(D.vel[0] + cell[l]);
+      T.ph[l] = nall[l] ? -p : p;
+      T.u[l] = nnorm[l] ? -x : x;
+      T.hc[l] = __ldg(S.hc + cell[l]);
+    }
+    int am;
+    const double ha = half_alpha64(T, &am);
+    double hp[5], hm[5];  // both sides in upwind order (hm[k] belongs to point 5 - k)
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      hp[k] = fma(0.5, T.u[k], ha);
+      hm[k] = fma(0.5, T.u[5 - k], -ha);
+    }
+    // tracers first: their cotangents of the split factors join the fluid part's
+    double hpb[5] = {0, 0, 0, 0, 0}, hmb[5] = {0, 0, 0, 0, 0};
+#pragma unroll 1
+    for (int c = 0; c < NCHEM; ++c) {
+      double rb = 0.0;
+      if (id < D.n) rb = S.gchem[c + (long)NCHEM * cup];
+      if (id >= 1) rb -= S.gchem[c + (long)NCHEM * cdn];
+      rb *= inv_d;
+      double cv[6];
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        const double x = __ldg(S.chem + c + (long)NCHEM * cell[l]);
+        cv[l] = nall[l] ? -x : x;
+      }
+      double pb[5], mb[5];
+      {
+        const double a[5] = {cv[0], cv[1], cv[2], cv[3], cv[4]};
+        tracer_side_adj(a, hp, rb, pb, hpb);
+      }
+      {
+        const double a[5] = {cv[5], cv[4], cv[3], cv[2], cv[1]};
+        tracer_side_adj(a, hm, rb, mb, hmb);
+      }
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        const double b = l == 0 ? pb[0] : (l == 5 ? mb[0] : pb[l] + mb[5 - l]);
+        A[((long)l * NV + 5 + c) * nfaces + f] = nall[l] ? -b : b;
+      }
+    }
+    Adj64 B;
+#pragma unroll
+    for (int l = 0; l < 6; ++l) {
+      B.ph[l] = B.u[l] = 0.0;
+#pragma unroll
+      for (int m = 0; m < 5; ++m) B.W[l][m] = 0.0;
+    }
+    B.ha = 0.0;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      B.u[k] = fma(0.5, hpb[k], B.u[k]);
+      B.u[5 - k] = fma(0.5, hmb[k], B.u[5 - k]);
+      B.ha += hpb[k] - hmb[k];
+    }
+    Roe64 R;
+    roe64(T, S.gamma, R);
+    const double u = R.u, v = R.v, w = R.w, c = R.c;
+    // back-projection (fluid_back64): s = ff0 + ff3 + ff4, t = ff0 + ff4, cd = c (ff4 - ff0)
+    const double sb = fma(ob[1], u, fma(ob[2], v, fma(ob[3], w, ob[0])));
+    const double tb = sb + ob[4] * R.H, cdb = fma(ob[4], u, ob[1]), db = cdb * c;
+    const double ffb[5] = {tb - db, fma(ob[4], v, ob[2]), fma(ob[4], w, ob[3]),
+                           fma(ob[4], R.q, sb), tb + db};
+    B.v = B.w = B.L00 = B.L01 = B.L02 = B.L03 = B.L04 = B.L30 = B.L31 = B.L40 = B.L41 = 0.0;
+    double ff[5];
+    fluid_side_adj<0>(T, R, hp, ffb, ff, B);
+    fluid_side_adj<1>(T, R, hm, ffb, ff, B);
+    const double t = ff[0] + ff[4], s = t + ff[3], d = ff[4] - ff[0];
+    double ub = fma(ob[1], s, ob[4] * (c * d)), vb = B.v + fma(ob[2], s, ob[4] * ff[1]),
+           wb = B.w + fma(ob[3], s, ob[4] * ff[2]), Hb = ob[4] * t, qb = ob[4] * ff[3],
+           cb = cdb * d;
+    // left eigenvector entries; hc = 1/(2c), hgc = gm hc, gc = 2 hgc
+    const double hc = 0.5 / c, hgc = gm * hc, gq = gm * R.q, gu = gm * u;
+    double hcb = fma(B.L00, u + gq, fma(B.L40, gq - u, -fma(B.L01, gu + 1.0, B.L41 * (gu - 1.0))));
+    ub = fma(hc, (B.L00 - B.L40) - gm * (B.L01 + B.L41), ub);
+    qb = fma(hgc, B.L00 + B.L40, qb);
+    double hgcb = B.L04 - fma(v, B.L02, w * B.L03);
+    vb = fma(-hgc, B.L02, vb);
+    wb = fma(-hgc, B.L03, wb);
+    hgcb = fma(2.0, fma(B.L30, fma(-2.0, R.q, R.H), B.L31 * u), hgcb);
+    Hb = fma(2.0 * hgc, B.L30, Hb);
+    qb = fma(-4.0 * hgc, B.L30, qb);
+    ub = fma(2.0 * hgc, B.L31, ub);
+    hcb = fma(gm, hgcb, hcb);
+    cb = fma(-2.0 * (hc * hc), hcb, cb);  // d(1/(2c)) = -2 hc^2 dc
+    // c = gm (H - q),  q = (u^2 + v^2 + w^2) / 2
+    Hb = fma(gm, cb, Hb);
+    qb = fma(-gm, cb, qb);
+    ub = fma(u, qb, ub);
+    vb = fma(v, qb, vb);
+    wb = fma(w, qb, wb);
+    // Roe averages X = (a iL + b iR) is, iL = 1/sqrt(rhoL), is = 1/(sL + sR)
+    {
+      const double sL = sqrt0_64(T.W[2][0]), sR = sqrt0_64(T.W[3][0]);
+      const double iL = 1.0 / sL, iR = 1.0 / sR, is = 1.0 / __dadd_rn(sL, sR);
+      const double eL = fma(2.0, T.ph[2], T.W[2][4]), eR = fma(2.0, T.ph[3], T.W[3][4]);
+      const double xu = ub * is, xv = vb * is, xw = wb * is, xH = Hb * is;
+      B.W[2][1] = fma(xu, iL, B.W[2][1]);
+      B.W[3][1] = fma(xu, iR, B.W[3][1]);
+      B.W[2][2] = fma(xv, iL, B.W[2][2]);
+      B.W[3][2] = fma(xv, iR, B.W[3][2]);
+      B.W[2][3] = fma(xw, iL, B.W[2][3]);
+      B.W[3][3] = fma(xw, iR, B.W[3][3]);
+      B.W[2][4] = fma(xH, iL, B.W[2][4]);
+      B.W[3][4] = fma(xH, iR, B.W[3][4]);
+      B.ph[2] = fma(2.0 * xH, iL, B.ph[2]);
+      B.ph[3] = fma(2.0 * xH, iR, B.ph[3]);
+      const double iLb = fma(xu, T.W[2][1], fma(xv, T.W[2][2], fma(xw, T.W[2][3], xH * eL)));
+      const double iRb = fma(xu, T.W[3][1], fma(xv, T.W[3][2], fma(xw, T.W[3][3], xH * eR)));
+      // every X carries the factor is: is b = sum X b X / is, d(is) = -is^2 (dsL + dsR)
+      const double sb2 = -is * fma(ub, u, fma(vb, v, fma(wb, w, Hb * R.H)));
+      // d iL = -iL^2 dsL, dsL = drho iL / 2
+      if (T.W[2][0] > 0.0)
+        B.W[2][0] = fma(0.5 * iL, fma(-(iL * iL), iLb, sb2), B.W[2][0]);
+      if (T.W[3][0] > 0.0)
+        B.W[3][0] = fma(0.5 * iR, fma(-(iR * iR), iRb, sb2), B.W[3][0]);
+    }
+    // half the Lax-Friedrichs speed at its point: ha = |u|/2 + c/2,
+    // d(c/2) = gamma / (4 rho) (d(p/2) - (p/2) drho / rho) / (c/2)
+    {
+      double sr = T.W[0][0], sp = T.ph[0], sc = T.hc[0], su = T.u[0];
+#pragma unroll
+      for (int l = 1; l < 6; ++l) {
+        const bool m = l == am;
+        sr = m ? T.W[l][0] : sr;
+        sp = m ? T.ph[l] : sp;
+        sc = m ? T.hc[l] : sc;
+        su = m ? T.u[l] : su;
+      }
+      const double uadd = su < 0.0 ? -0.5 * B.ha : 0.5 * B.ha;
+      double padd = 0.0, radd = 0.0;
+      if (sc > 0.0) {
+        const double ir = 1.0 / sr;
+        padd = 0.25 * S.gamma * ir * B.ha / sc;
+        radd = -(padd * sp) * ir;
+      }
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        const bool m = l == am;
+        B.u[l] += m ? uadd : 0.0;
+        B.ph[l] += m ? padd : 0.0;
+        B.W[l][0] += m ? radd : 0.0;
+      }
+    }
+    // points' primitives: u = m / rho, p/2 = gm/2 (E - |m|^2 / (2 rho))
+#pragma unroll
+    for (int l = 0; l < 6; ++l) {
+      const double ir = rcp64(T.W[l][0]), x = T.u[l], v1 = __ldg(D.vel[1] + cell[l]),
+                   v2 = __ldg(D.vel[2] + cell[l]);
+      const double k = 0.5 * gm * B.ph[l], m = B.u[l] * ir;
       double q[5];
-      q[0] = Wb[l][0];
-      q[4] = Wb[l][4];
-      q[1 + DIR] = Wb[l][1];
-      if (DIR == 0) { q[2] = Wb[l][2]; q[3] = Wb[l][3]; }
-      if (DIR == 1) { q[1] = Wb[l][2]; q[3] = Wb[l][3]; }
-      if (DIR == 2) { q[2] = Wb[l][2]; q[1] = Wb[l][3]; }
+      q[0] = fma(k, 0.5 * fma(x, x, fma(v1, v1, v2 * v2)), fma(-m, x, B.W[l][0]));
+      q[1] = fma(-k, x, B.W[l][1] + m);
+      q[2] = fma(-k, v1, B.W[l][2]);
+      q[3] = fma(-k, v2, B.W[l][3]);
+      q[4] = B.W[l][4] + k;
       if (nall[l]) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) q[v] = -q[v];
+        for (int e = 0; e < 5; ++e) q[e] = -q[e];
       }
-      if (nnorm[l]) q[1 + DIR] = -q[1 + DIR];
+      if (nnorm[l]) q[1] = -q[1];
 #pragma unroll
-      for (int v = 0; v < 5; ++v) A[((long)l * NV + v) * nfaces + f] = q[v];
+      for (int e = 0; e < 5; ++e) A[((long)l * NV + D.slot[e]) * nfaces + f] = q[e];
     }
   }
 }
@@ -489,25 +387,36 @@ __global__ void __launch_bounds__(256) vjp_gather_kernel(Grid g, const double* _
 
 // ------------------------------------------------------------------ launcher
 
+template <int NCHEM, int DIR>
+static int vjp_dir(const Grid& g, const SweepSet& S, const Fields& out, double* A,
+                   cudaStream_t s) {
+  const long nf = S.d[DIR].nfaces;
+  const int t = spread_threads(nf, 128);
+  face_flux_vjp_kernel<NCHEM><<<sweep_blocks(nf, t), t, 0, s>>>(S, DIR, g.inv_d[DIR], A);
+  GBMV_LAUNCH_CHECK("face_flux_vjp_kernel");
+  vjp_gather_kernel<NCHEM, DIR><<<sweep_blocks(g.ncell, 256), 256, 0, s>>>(g, A, out, nf, DIR == 0);
+  GBMV_LAUNCH_CHECK("vjp_gather_kernel");
+  return GBMV_OK;
+}
+
 template <int NCHEM>
 static int vjp_t(const Grid& g, const Fields& w, const Fields& v, const Fields& out, double* A,
                  cudaStream_t s) {
-  long nf[3];
-  face_counts(g, nf);
   ProfScope ps("vjp", s);
-  face_flux_vjp_kernel<NCHEM, 0><<<sweep_blocks(nf[0], 128), 128, 0, s>>>(g, w, v, A, nf[0]);
-  GBMV_LAUNCH_CHECK("face_flux_vjp_kernel<x>");
-  vjp_gather_kernel<NCHEM, 0><<<sweep_blocks(g.ncell, 256), 256, 0, s>>>(g, A, out, nf[0], 1);
-  GBMV_LAUNCH_CHECK("vjp_gather_kernel<x>");
-  face_flux_vjp_kernel<NCHEM, 1><<<sweep_blocks(nf[1], 128), 128, 0, s>>>(g, w, v, A, nf[1]);
-  GBMV_LAUNCH_CHECK("face_flux_vjp_kernel<y>");
-  vjp_gather_kernel<NCHEM, 1><<<sweep_blocks(g.ncell, 256), 256, 0, s>>>(g, A, out, nf[1], 0);
-  GBMV_LAUNCH_CHECK("vjp_gather_kernel<y>");
-  face_flux_vjp_kernel<NCHEM, 2><<<sweep_blocks(nf[2], 128), 128, 0, s>>>(g, w, v, A, nf[2]);
-  GBMV_LAUNCH_CHECK("face_flux_vjp_kernel<z>");
-  vjp_gather_kernel<NCHEM, 2><<<sweep_blocks(g.ncell, 256), 256, 0, s>>>(g, A, out, nf[2], 0);
-  GBMV_LAUNCH_CHECK("vjp_gather_kernel<z>");
-  return GBMV_OK;
+  // cell primitives after the stencil cotangents (not in the flux scratch: a flux divergence on
+  // the same handle may run beside the adjoint on another stream)
+  double* const q = A + feuler_vjp_scratch_doubles(g) - 5 * g.ncell;
+  double* const p[5] = {q, q + g.ncell, q + 2 * g.ncell, q + 3 * g.ncell, q + 4 * g.ncell};
+  int rc = prims64(g, w, p, nullptr, s);
+  SweepSet S;
+  sweep_set(g, w, nullptr, 1, 128, (long)kSM * 16, S);
+  sweep_second(S, v);
+  const double* const u[3] = {p[1], p[2], p[3]};
+  sweep_prims(S, p[0], u, p[4]);
+  if (!rc) rc = vjp_dir<NCHEM, 0>(g, S, out, A, s);
+  if (!rc) rc = vjp_dir<NCHEM, 1>(g, S, out, A, s);
+  if (!rc) rc = vjp_dir<NCHEM, 2>(g, S, out, A, s);
+  return rc;
 }
 
 size_t feuler_vjp_scratch_doubles(const Grid& g) {
@@ -515,7 +424,7 @@ size_t feuler_vjp_scratch_doubles(const Grid& g) {
   long m = (nx + 1) * ny * nz;
   if (nx * (ny + 1) * nz > m) m = nx * (ny + 1) * nz;
   if (nx * ny * (nz + 1) > m) m = nx * ny * (nz + 1);
-  return (size_t)6 * (5 + g.nchem) * (size_t)m;
+  return (size_t)6 * (5 + g.nchem) * (size_t)m + 5 * (size_t)g.ncell;
 }
 
 int feuler_vjp(const Grid& g, const Fields& w, const Fields& v, const Fields& out, double* A,
