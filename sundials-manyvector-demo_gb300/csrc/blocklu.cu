@@ -4,61 +4,83 @@
 // src/multirate_chem_hydro_main.cpp:1312-1411, src/imex_chem_hydro_main.cpp:1075-1194).
 //
 // One thread owns one block; the whole 10x10 block lives in registers (fully unrolled through
-// template recursion, compile-time indices), row interchanges are predicated selects.  A CTA
-// stages 128 consecutive blocks (102 KB, contiguous in HBM) through shared memory with
-// 16-byte coalesced accesses; two CTAs per SM overlap one tile's traffic with the other's
-// arithmetic.
+// template recursion, compile-time indices), row interchanges are predicated selects.  A CTA is
+// one warp with a tile of 32 consecutive blocks (25.6 KB, contiguous in HBM) brought into shared
+// memory by 16-byte asynchronous copies, all in flight at once; eight such CTAs per SM overlap
+// one tile's traffic with the others' arithmetic.  (Two-warp CTAs filling their tile with plain
+// loads, a few in flight, left the FP64 pipe 54 % busy in the factorisation and 20 % in the
+// solve: 192,000 blocks 286 and 164 us, now 172 and 64.)
 #include "chem.cuh"
+#include "weno64.cuh"
 
 namespace gbmv {
 
-constexpr int kLuThreads = 64;   // blocks per tile = threads per CTA
-constexpr int kLuStride = 101;   // padded per-block stride of the shared tile (doubles)
+constexpr int kLuThreads = 32;   // blocks per tile = threads per CTA
+constexpr int kLuStride = 102;   // per-block stride of the shared tile (doubles): a multiple of 16
+                                 // bytes, and two-way bank conflicts at most
 constexpr int kVecStride = 11;   // the same for the right-hand-side tile
 
-// Coalesced copy of `nb` consecutive blocks of NE doubles between global memory and a shared
-// tile with per-block stride SS (16-byte global accesses when NE is even and the address is
-// 16-byte aligned -- caller arrays need only be 8-byte aligned).
-template <int NE, int SS = kLuStride>
-__device__ __forceinline__ void tile_in(const double* __restrict__ g, double* sh, long blk0, int nb) {
-  const double* src = g + blk0 * NE;
-  if (NE % 2 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    const double2* s2 = reinterpret_cast<const double2*>(src);
-    for (int c = threadIdx.x; c < nb * NE / 2; c += blockDim.x) {
-      const double2 v = s2[c];
-      const int b = (2 * c) / NE, e = (2 * c) % NE;
-      sh[b * SS + e] = v.x;
-      sh[b * SS + e + 1] = v.y;
+// Copy of `nb` consecutive blocks of 100 doubles into the shared tile; waits for nothing.
+// 16-byte asynchronous copies where the address allows (caller arrays need only be 8-byte
+// aligned).
+__device__ __forceinline__ void tile_in_async(const double* __restrict__ g, double* sh, long blk0,
+                                              int nb) {
+  const double* src = g + blk0 * 100;
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    const unsigned base = (unsigned)__cvta_generic_to_shared(sh);
+#pragma unroll 10
+    for (int c = threadIdx.x; c < nb * 50; c += kLuThreads) {
+      const int b = c / 50, e = c - b * 50;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       base + (unsigned)(b * (kLuStride * 8) + e * 16)),
+                   "l"(src + 2 * c)
+                   : "memory");
     }
   } else {
-    for (int c = threadIdx.x; c < nb * NE; c += blockDim.x) sh[(c / NE) * SS + c % NE] = src[c];
+    for (int c = threadIdx.x; c < nb * 100; c += kLuThreads)
+      sh[(c / 100) * kLuStride + c % 100] = src[c];
   }
 }
-template <int NE, int SS = kLuStride>
-__device__ __forceinline__ void tile_out(double* __restrict__ g, const double* sh, long blk0, int nb) {
-  double* dst = g + blk0 * NE;
-  if (NE % 2 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-    double2* d2 = reinterpret_cast<double2*>(dst);
-    for (int c = threadIdx.x; c < nb * NE / 2; c += blockDim.x) {
-      const int b = (2 * c) / NE, e = (2 * c) % NE;
-      d2[c] = make_double2(sh[b * SS + e], sh[b * SS + e + 1]);
+__device__ __forceinline__ void tile_in_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+}
+__device__ __forceinline__ void tile_out(double* __restrict__ g, const double* sh, long blk0,
+                                         int nb) {
+  double* dst = g + blk0 * 100;
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll 10
+    for (int c = threadIdx.x; c < nb * 50; c += kLuThreads) {
+      const int b = c / 50, e = c - b * 50;
+      reinterpret_cast<double2*>(dst)[c] =
+          *reinterpret_cast<const double2*>(sh + b * kLuStride + 2 * e);
     }
   } else {
-    for (int c = threadIdx.x; c < nb * NE; c += blockDim.x) dst[c] = sh[(c / NE) * SS + c % NE];
+    for (int c = threadIdx.x; c < nb * 100; c += kLuThreads)
+      dst[c] = sh[(c / 100) * kLuStride + c % 100];
   }
+}
+
+// |x| as an ordered integer; NaN counts as 0, as a comparison with it is false.  (Comparisons of
+// doubles run on the FP64 pipe, which bounds the factorisation.)
+__device__ __forceinline__ unsigned long long abs_order(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+  return b > 0x7ff0000000000000ULL ? 0ULL : b;
 }
 
 // One elimination step KK of LU with partial pivoting (first maximal |pivot|, full-row
 // interchange, the dgetf2 order), fully unrolled through template recursion so the block
 // stays in registers.  The factor keeps 1/U(k,k) on the diagonal (the solve only multiplies);
 // the factored matrix is private to this solver, as MAGMA's is to its own getrs.
-template <int KK, typename R>
-__device__ __forceinline__ void lu_step(R (&A)[100], int (&piv)[10], int& info) {
+template <int KK>
+__device__ __forceinline__ void lu_step(double (&A)[100], int (&piv)[10], int& info) {
   int p = KK;
-  R amax = fabs(A[KK * 10 + KK]);
+  // (a NaN diagonal keeps its place: no comparison with it is true)
+  unsigned long long amax =
+      (unsigned long long)__double_as_longlong(A[KK * 10 + KK]) & 0x7fffffffffffffffULL;
 #pragma unroll
   for (int r = KK + 1; r < 10; ++r) {
-    const R v = fabs(A[KK * 10 + r]);
+    const unsigned long long v = abs_order(A[KK * 10 + r]);
     if (v > amax) { amax = v; p = r; }
   }
   piv[KK] = p;
@@ -67,22 +89,22 @@ __device__ __forceinline__ void lu_step(R (&A)[100], int (&piv)[10], int& info) 
     const bool sw = (r == p);
 #pragma unroll
     for (int col = 0; col < 10; ++col) {
-      const R a = A[col * 10 + KK], b = A[col * 10 + r];
+      const double a = A[col * 10 + KK], b = A[col * 10 + r];
       A[col * 10 + KK] = sw ? b : a;
       A[col * 10 + r] = sw ? a : b;
     }
   }
-  const R d = A[KK * 10 + KK];
-  if (d == R(0)) {
+  const double d = A[KK * 10 + KK];
+  if ((__double_as_longlong(d) & 0x7fffffffffffffffLL) == 0) {
     if (!info) info = KK + 1;
   } else {
-    const R rp = R(1) / d;
+    const double rp = rcp64_any(d);
     A[KK * 10 + KK] = rp;
 #pragma unroll
     for (int r = KK + 1; r < 10; ++r) A[KK * 10 + r] *= rp;
 #pragma unroll
     for (int col = KK + 1; col < 10; ++col) {
-      const R a = A[col * 10 + KK];
+      const double a = A[col * 10 + KK];
 #pragma unroll
       for (int r = KK + 1; r < 10; ++r) A[col * 10 + r] -= A[KK * 10 + r] * a;
     }
@@ -90,8 +112,7 @@ __device__ __forceinline__ void lu_step(R (&A)[100], int (&piv)[10], int& info) 
   if constexpr (KK < 9) lu_step<KK + 1>(A, piv, info);
 }
 
-template <typename R>
-__device__ __forceinline__ int lu10_regs(R (&A)[100], int (&piv)[10]) {
+__device__ __forceinline__ int lu10_regs(double (&A)[100], int (&piv)[10]) {
   int info = 0;
   lu_step<0>(A, piv, info);
   return info;
@@ -99,14 +120,14 @@ __device__ __forceinline__ int lu10_regs(R (&A)[100], int (&piv)[10]) {
 
 // Solve with the factor of lu10_regs (row interchanges, unit-lower forward substitution,
 // upper back substitution multiplying by the stored reciprocal pivots).
-template <typename R, typename X>
-__device__ __forceinline__ void lus10_regs(const R (&A)[100], const int (&piv)[10], X (&x)[10]) {
+__device__ __forceinline__ void lus10(const double* __restrict__ A, const int (&piv)[10],
+                                      double (&x)[10]) {
 #pragma unroll
   for (int kk = 0; kk < 10; ++kk) {
 #pragma unroll
     for (int r = kk + 1; r < 10; ++r) {
       const bool sw = (r == piv[kk]);
-      const X a = x[kk], b = x[r];
+      const double a = x[kk], b = x[r];
       x[kk] = sw ? b : a;
       x[r] = sw ? a : b;
     }
@@ -114,91 +135,113 @@ __device__ __forceinline__ void lus10_regs(const R (&A)[100], const int (&piv)[1
 #pragma unroll
   for (int col = 0; col < 10; ++col)
 #pragma unroll
-    for (int r = col + 1; r < 10; ++r) x[r] -= X(A[col * 10 + r]) * x[col];
+    for (int r = col + 1; r < 10; ++r) x[r] -= A[col * 10 + r] * x[col];
 #pragma unroll
   for (int col = 9; col >= 0; --col) {
-    x[col] *= X(A[col * 10 + col]);
+    x[col] *= A[col * 10 + col];
 #pragma unroll
-    for (int r = 0; r < col; ++r) x[r] -= X(A[col * 10 + r]) * x[col];
+    for (int r = 0; r < col; ++r) x[r] -= A[col * 10 + r] * x[col];
   }
 }
 
-__global__ void __launch_bounds__(kLuThreads, 4) block_lu_factor_kernel(long nb, double* __restrict__ A,
+__global__ void __launch_bounds__(kLuThreads, 8) block_lu_factor_kernel(long nb, double* A,
                                                                         int* __restrict__ piv,
                                                                         int* __restrict__ info_out) {
-  extern __shared__ double sh[];  // [kLuThreads][kLuStride]
+  extern __shared__ __align__(16) double sh[];  // [kLuThreads][kLuStride]
   int bad = 0;
   for (long blk0 = (long)blockIdx.x * kLuThreads; blk0 < nb; blk0 += (long)gridDim.x * kLuThreads) {
     const int nb_here = (int)((nb - blk0) < kLuThreads ? (nb - blk0) : kLuThreads);
-    tile_in<100>(A, sh, blk0, nb_here);
-    __syncthreads();
+    tile_in_async(A, sh, blk0, nb_here);
+    tile_in_wait();
     if (threadIdx.x < nb_here) {
       double a[100];
       int p[10];
-      const double* mine = sh + threadIdx.x * kLuStride;
+      double* mine = sh + threadIdx.x * kLuStride;
 #pragma unroll
       for (int e = 0; e < 100; ++e) a[e] = mine[e];
       if (lu10_regs(a, p)) bad = 1;
-      double* out = sh + threadIdx.x * kLuStride;
 #pragma unroll
-      for (int e = 0; e < 100; ++e) out[e] = a[e];
+      for (int e = 0; e < 100; ++e) mine[e] = a[e];
       int* pg = piv + (blk0 + threadIdx.x) * 10;
 #pragma unroll
       for (int e = 0; e < 10; ++e) pg[e] = p[e];
     }
-    __syncthreads();
-    tile_out<100>(A, sh, blk0, nb_here);
-    __syncthreads();
+    __syncwarp();
+    tile_out(A, sh, blk0, nb_here);
+    __syncwarp();
   }
   if (bad) atomicMax(info_out, 1);
 }
 
-__global__ void __launch_bounds__(kLuThreads, 4) block_lu_solve_kernel(long nb,
-                                                                       const double* __restrict__ LU,
-                                                                       const int* __restrict__ piv,
-                                                                       const double* b, double* x) {
-  extern __shared__ double sh[];  // LU tile, then the right-hand sides
-  double* shb = sh + kLuThreads * kLuStride;  // [kLuThreads][kVecStride]
+__global__ void __launch_bounds__(kLuThreads) block_lu_solve_kernel(long nb,
+                                                                    const double* __restrict__ LU,
+                                                                    const int* __restrict__ piv,
+                                                                    const double* b, double* x) {
+  extern __shared__ __align__(16) double sh[];  // LU tile, then the right-hand sides
+  double* shb = sh + kLuThreads * kLuStride;    // [kLuThreads][kVecStride]
   for (long blk0 = (long)blockIdx.x * kLuThreads; blk0 < nb; blk0 += (long)gridDim.x * kLuThreads) {
     const int nb_here = (int)((nb - blk0) < kLuThreads ? (nb - blk0) : kLuThreads);
-    tile_in<100>(LU, sh, blk0, nb_here);
-    tile_in<10, kVecStride>(b, shb, blk0, nb_here);
-    __syncthreads();
+    tile_in_async(LU, sh, blk0, nb_here);
+    double t[10];  // the right-hand sides: 10 nb_here consecutive doubles
+#pragma unroll
+    for (int e = 0; e < 10; ++e) {
+      const int c = threadIdx.x + e * kLuThreads;
+      t[e] = c < 10 * nb_here ? b[blk0 * 10 + c] : 0.0;
+    }
+    int p[10];
+    const int* pg = piv + (blk0 + (threadIdx.x < nb_here ? threadIdx.x : 0)) * 10;
+#pragma unroll
+    for (int e = 0; e < 10; ++e) p[e] = __ldg(pg + e);
+#pragma unroll
+    for (int e = 0; e < 10; ++e) {
+      const int c = threadIdx.x + e * kLuThreads;
+      shb[(c / 10) * kVecStride + c % 10] = t[e];
+    }
+    tile_in_wait();
     if (threadIdx.x < nb_here) {
-      double a[100], v[10];
-      int p[10];
-      const double* mine = sh + threadIdx.x * kLuStride;
+      double v[10];
 #pragma unroll
-      for (int e = 0; e < 100; ++e) a[e] = mine[e];
-      const int* pg = piv + (blk0 + threadIdx.x) * 10;
-#pragma unroll
-      for (int e = 0; e < 10; ++e) {
-        p[e] = pg[e];
-        v[e] = shb[threadIdx.x * kVecStride + e];
-      }
-      lus10_regs(a, p, v);
+      for (int e = 0; e < 10; ++e) v[e] = shb[threadIdx.x * kVecStride + e];
+      lus10(sh + threadIdx.x * kLuStride, p, v);
 #pragma unroll
       for (int e = 0; e < 10; ++e) shb[threadIdx.x * kVecStride + e] = v[e];
     }
-    __syncthreads();
-    tile_out<10, kVecStride>(x, shb, blk0, nb_here);
-    __syncthreads();
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 10; ++e) {
+      const int c = threadIdx.x + e * kLuThreads;
+      if (c < 10 * nb_here) x[blk0 * 10 + c] = shb[(c / 10) * kVecStride + c % 10];
+    }
+    __syncwarp();
   }
 }
 
-// SUNMatScaleAddI(-gamma, J): A = -gamma*J + I on every block.
+// SUNMatScaleAddI(-gamma, J): A = -gamma*J + I on every block.  One fused multiply-add per
+// element: adding -0 off the diagonal leaves the product as it is.  (A product and a predicated
+// addition issued two FP64 instructions per warp for the three diagonal lanes in it.)
+__device__ __forceinline__ double form_newton(double c, double v, int r) {
+  return fma(c, v, (r % 11 == 0) ? 1.0 : -0.0);
+}
+template <bool PAIRS>
 __global__ void block_form_newton_kernel(long nel, double* __restrict__ J, double c) {
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < nel;
-       e += (long)gridDim.x * blockDim.x) {
-    const int r = (int)(e % 100);
-    const double v = c * J[e];
-    J[e] = (r % 11 == 0) ? v + 1.0 : v;
+  const long step = (long)gridDim.x * blockDim.x;
+  if (PAIRS) {
+    double2* const J2 = reinterpret_cast<double2*>(J);
+    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < nel / 2; e += step) {
+      const int r = 2 * (int)((unsigned long)e % 50u);
+      const double2 v = J2[e];
+      J2[e] = make_double2(form_newton(c, v.x, r), form_newton(c, v.y, r + 1));
+    }
+  } else {
+    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < nel; e += step)
+      J[e] = form_newton(c, J[e], (int)(e % 100));
   }
 }
 
-static int lu_grid(long nb) {
+// persistent grid: as many CTAs as are resident (a few more would run alone at the end)
+static int lu_grid(long nb, int per_sm) {
   long b = (nb + kLuThreads - 1) / kLuThreads;
-  const long cap = (long)kSM * 4;
+  const long cap = (long)kSM * per_sm;
   if (b < 1) b = 1;
   return (int)(b < cap ? b : cap);
 }
@@ -208,7 +251,7 @@ int block_lu_factor(long nb, double* A, int* piv, int* d_info, cudaStream_t s) {
   GBMV_CUDA_TRY(cudaFuncSetAttribute(block_lu_factor_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
   ProfScope ps("block_lu_factor", s);
-  block_lu_factor_kernel<<<lu_grid(nb), kLuThreads, shm, s>>>(nb, A, piv, d_info);
+  block_lu_factor_kernel<<<lu_grid(nb, 8), kLuThreads, shm, s>>>(nb, A, piv, d_info);
   GBMV_LAUNCH_CHECK("block_lu_factor_kernel");
   return GBMV_OK;
 }
@@ -219,18 +262,20 @@ int block_lu_solve(long nb, const double* LU, const int* piv, const double* b, d
   GBMV_CUDA_TRY(cudaFuncSetAttribute(block_lu_solve_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
   ProfScope ps("block_lu_solve", s);
-  block_lu_solve_kernel<<<lu_grid(nb), kLuThreads, shm, s>>>(nb, LU, piv, b, x);
+  block_lu_solve_kernel<<<lu_grid(nb, 7), kLuThreads, shm, s>>>(nb, LU, piv, b, x);
   GBMV_LAUNCH_CHECK("block_lu_solve_kernel");
   return GBMV_OK;
 }
 
 int block_form_newton(long nb, double* J, double gamma, cudaStream_t s) {
   const long nel = 100 * nb;
-  long g = (nel + 255) / 256;
+  const bool pairs = (reinterpret_cast<uintptr_t>(J) & 15) == 0;
+  long g = ((pairs ? nel / 2 : nel) + 255) / 256;
   if (g > (long)kSM * 32) g = (long)kSM * 32;
   if (g < 1) g = 1;
   ProfScope ps("glue", s);
-  block_form_newton_kernel<<<(int)g, 256, 0, s>>>(nel, J, -gamma);
+  if (pairs) block_form_newton_kernel<true><<<(int)g, 256, 0, s>>>(nel, J, -gamma);
+  else block_form_newton_kernel<false><<<(int)g, 256, 0, s>>>(nel, J, -gamma);
   GBMV_LAUNCH_CHECK("block_form_newton_kernel");
   return GBMV_OK;
 }
