@@ -18,12 +18,12 @@ __global__ void __launch_bounds__(128) chem_rhs_kernel(ChemParams P, ChemState S
     double ya[10];
 #pragma unroll
     for (int s = 0; s < 10; ++s) ya[s] = y[j + s] * S.scale[j + s];
-    double Ts = S.Ts[i], dTs = 0.0;
-    chem_temperature(P, ya, Ts, dTs);
+    double Ts = S.Ts[i], dTs = 0.0, logT;
+    chem_temperature(P, ya, Ts, dTs, logT);
     S.Ts[i] = Ts;
     S.dTs_ge[i] = dTs;
     double k[kNRates], dk[kNRates];
-    chem_rates<false>(P, Ts, k, dk);
+    chem_rates<false>(P, logT, k, dk);
     double r[21], sp[9];
     chem_fluxes(k, ya, r);
     chem_species(r, sp);
@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(128) chem_rhs_kernel(ChemParams P, ChemState S
     double out[10];
 #pragma unroll
     for (int s = 0; s < 9; ++s) out[s] = sp[s] * S.inv_scale[j + s];
-    out[9] = chem_ge_source(P, k, ya, Ts, A) * S.inv_scale[j + 9];
+    out[9] = chem_ge_source(P, k, ya, Ts, A, ge_terms(k, ya)) * S.inv_scale[j + 9];
     out[9] *= A.imdens;
 #pragma unroll
     for (int s = 0; s < 10; ++s) ydot[j + s] = out[s] * tunit;
@@ -51,12 +51,13 @@ __global__ void __launch_bounds__(128) chem_jac_kernel(ChemParams P, ChemState S
     for (int s = 0; s < 10; ++s) ya[s] = y[j + s] * sc[s];
     const double T = S.Ts[i];
     double k[kNRates], dk[kNRates];
-    chem_rates<true>(P, T, k, dk);
+    chem_rates<true>(P, log(T), k, dk);
+    const double Tge = S.dTs_ge[i] * (P.idbin / T);
     const ChemAux A{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
     double* out = J + 100 * i;
 #pragma unroll
     for (int e = 0; e < 100; ++e) out[e] = 0.0;
-    chem_jacobian(P, k, dk, ya, T, S.dTs_ge[i], A, [&](int row, int col, double v) {
+    chem_jacobian(P, k, dk, ya, T, Tge, A, ge_terms(k, ya), [&](int row, int col, double v) {
       out[col * 10 + row] = (v * (isc[row] * sc[col])) * tunit;
     });
   }
@@ -85,9 +86,10 @@ __global__ void __launch_bounds__(128) chem_jvp_kernel(ChemParams P, ChemState S
     }
     const double T = S.Ts[i];
     double k[kNRates], dk[kNRates];
-    chem_rates<true>(P, T, k, dk);
+    chem_rates<true>(P, log(T), k, dk);
+    const double Tge = S.dTs_ge[i] * (P.idbin / T);
     const ChemAux A{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
-    chem_jacobian(P, k, dk, ya, T, S.dTs_ge[i], A, [&](int row, int col, double v) {
+    chem_jacobian(P, k, dk, ya, T, Tge, A, ge_terms(k, ya), [&](int row, int col, double v) {
       const double e = (v * (isc[row] * sc[col])) * tunit;
       if (TRANS) acc[col] += e * xv[row];
       else acc[row] += e * xv[col];

@@ -41,7 +41,7 @@
 
 #include "chem.cuh"
 #include "chem_lu.cuh"
-#include "chem_net.cuh"
+#include "chem_net_literal.cuh"
 
 namespace gbmv {
 
@@ -64,18 +64,18 @@ __device__ __forceinline__ void dirk_F(const ChemParams& P, const ChemState& S, 
 #pragma unroll
   for (int s = 0; s < 10; ++s) ya[s] = X[s * BS] * S.scale[j + s];
   if (mixed_temp)
-    chem_temperature_mixed(P, ya, Ts, dTs, 9);  // up to 9 FP32 + 1 FP64 iteration
+    literal::chem_temperature_mixed(P, ya, Ts, dTs, 9);  // up to 9 FP32 + 1 FP64 iteration
   else
-    chem_temperature(P, ya, Ts, dTs);
+    literal::chem_temperature(P, ya, Ts, dTs);
   double k[kNRates], dk[kNRates];
-  chem_rates<false>(P, Ts, k, dk);
+  literal::chem_rates<false>(P, Ts, k, dk);
   double r[21], sp[9];
   chem_fluxes(k, ya, r);
-  chem_species(r, sp);
+  literal::chem_species(r, sp);
   const ChemAux Ax{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
 #pragma unroll
   for (int s = 0; s < 9; ++s) f[s] = (sp[s] * S.inv_scale[j + s]) * tunit;
-  double ge = chem_ge_source(P, k, ya, Ts, Ax) * S.inv_scale[j + 9];
+  double ge = literal::chem_ge_source(P, k, ya, Ts, Ax) * S.inv_scale[j + 9];
   ge *= Ax.imdens;
   f[9] = ge * tunit;
   if (O.nforcing > 0) {
@@ -166,7 +166,7 @@ __device__ __forceinline__ int dirk_setup(const ChemParams& P, const ChemState& 
 #pragma unroll
   for (int s = 0; s < 10; ++s) ya[s] = Y[s * BS] * S.scale[j + s];
   double k[kNRates], dk[kNRates];
-  chem_rates<true>(P, Tsy, k, dk);
+  literal::chem_rates<true>(P, Tsy, k, dk);
   const ChemAux Ax{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
   const double* __restrict__ sc = S.scale + j;
   const double* __restrict__ isc = S.inv_scale + j;
@@ -178,7 +178,7 @@ __device__ __forceinline__ int dirk_setup(const ChemParams& P, const ChemState& 
     return (row == col ? 1.0 : 0.0) + mg * ((v * isc[row]) * sc[col]);
   };
   if (sizeof(LU) == 8) {
-    chem_jacobian(P, k, dk, ya, Tsy, dTsy, Ax, [&](int row, int col, double v) {
+    literal::chem_jacobian(P, k, dk, ya, Tsy, dTsy, Ax, [&](int row, int col, double v) {
       L[(col * 10 + row) * BS] = (LU)entry(row, col, v);
     });
   } else {
@@ -189,13 +189,13 @@ __device__ __forceinline__ int dirk_setup(const ChemParams& P, const ChemState& 
 #pragma unroll
     for (int s = 0; s < 10; ++s) rmax[s] = cmax[s] = 0.0;
     if (REF) {
-      chem_jacobian(P, k, dk, ya, Tsy, dTsy, Ax, [&](int row, int col, double v) {
+      literal::chem_jacobian(P, k, dk, ya, Tsy, dTsy, Ax, [&](int row, int col, double v) {
         const double a = entry(row, col, v);
         A[(col * 10 + row) * BS] = a;
         rmax[row] = fmax(rmax[row], fabs(a));
       });
     } else {
-      chem_jacobian(P, k, dk, ya, Tsy, dTsy, Ax, [&](int row, int col, double v) {
+      literal::chem_jacobian(P, k, dk, ya, Tsy, dTsy, Ax, [&](int row, int col, double v) {
         rmax[row] = fmax(rmax[row], fabs(entry(row, col, v)));
       });
     }
@@ -228,7 +228,7 @@ __device__ __forceinline__ int dirk_setup(const ChemParams& P, const ChemState& 
             to_lu<LU>(A[(col * 10 + row) * BS] * pow2(er[row] + ec[col]));
       }
     } else {
-      chem_jacobian(P, k, dk, ya, Tsy, dTsy, Ax, [&](int row, int col, double v) {
+      literal::chem_jacobian(P, k, dk, ya, Tsy, dTsy, Ax, [&](int row, int col, double v) {
         L[(col * 10 + row) * BS] = to_lu<LU>(entry(row, col, v) * pow2(er[row] + ec[col]));
       });
     }

@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "df64.cuh"
+#include "weno64.cuh"
 
 namespace gbmv {
 
@@ -40,50 +41,104 @@ struct ChemParams {
   int nbins;
 };
 
-__device__ __forceinline__ int chem_bin(const ChemParams& P, double logT, double& t1, double& t2) {
-  int b = (int)(P.idbin * (logT - P.lb));
-  if (b <= 0) b = 0;
-  else if (b >= P.nbins) b = P.nbins - 1;
-  t1 = P.lb + b * P.dbin;
-  t2 = P.lb + (b + 1) * P.dbin;
-  return b;
+// Table position of a temperature: bin b (clamped to the table) and the interpolation weight
+// inside it, log T / dbin = b + w (the tables start at T = 1).  The floor is the product rounded
+// down at the unit digit of a large constant, so no conversion instruction (they run at the FP64
+// rate) and no division by the bin width is needed.
+struct ChemPos {
+  int b;
+  double w;
+};
+__device__ __forceinline__ ChemPos chem_pos(const ChemParams& P, double logT) {
+  constexpr double kUnit = 6755399441055744.0;  // 1.5 2^52: the last bit is the unit digit
+  const double y = __fma_rd(logT, P.idbin, kUnit);
+  ChemPos q;
+  q.b = __double2loint(y);
+  double bd = y - kUnit;
+  if ((unsigned)q.b >= (unsigned)P.nbins) {
+    q.b = q.b < 0 ? 0 : P.nbins - 1;
+    bd = (double)q.b;
+  }
+  q.w = fma(logT, P.idbin, -bd);
+  return q;
 }
 
-// cvklu_calculate_temperature: ten Newton iterations from the previous T, then clamp.
-__device__ __forceinline__ void chem_temperature(const ChemParams& P, const double (&y)[10],
-                                                 double& Ts, double& dTs_ge) {
+// One Newton step of the temperature solve ge(T) = ge (src/raja_primordial_network.cpp:908-1011)
+// at T: returns dT (the step is T - dT) and the slope of T nsum, so that dge/dT = kb / (rho mh)
+// slope.  S: the particles with constant adiabatic index over gamma - 1; gk = ge rho mh / kb.
+// The reference's expression divided through by kb / (rho mh): one reciprocal for both adiabatic
+// indices and one for the slope where it has seven divisions (~55 FP64 instructions, was 122).
+struct ChemTemp {
+  double H2_1, H2_2, S, gk, dmh;
+};
+__device__ __forceinline__ ChemTemp chem_temp_setup(const double (&y)[10]) {
   const double kb = 1.3806504e-16, mh = 1.67e-24, gm1 = 1.0 / (5.e0 / 3.e0 - 1);
-  const double H2_1 = y[0], H2_2 = y[1], H_1 = y[2], H_2 = y[3], H_m0 = y[4], He_1 = y[5],
-               He_2 = y[6], He_3 = y[7], de = y[8], ge = y[9];
-  const double density = 2.0 * H2_1 + 2.0 * H2_2 + 1.00794 * H_1 + 1.00794 * H_2 +
-                         1.00794 * H_m0 + 4.002602 * He_1 + 4.002602 * He_2 + 4.002602 * He_3;
-  const double dmh = density * mh;
-  double T = Ts, Tnew = 0.0, dge_dT = 0.0;
+  ChemTemp c;
+  c.H2_1 = y[0];
+  c.H2_2 = y[1];
+  const double h = y[2] + y[3] + y[4], he = y[5] + y[6] + y[7];
+  c.dmh = fma(2.0, y[0] + y[1], fma(1.00794, h, 4.002602 * he)) * mh;
+  c.S = gm1 * (h + he + y[8]);
+  c.gk = y[9] * (c.dmh * (1.0 / kb));
+  return c;
+}
+__device__ __forceinline__ double chem_temp_step(const ChemParams& P, const ChemTemp& c, double T,
+                                                 double logT, double& slope) {
+  const ChemPos q = chem_pos(P, logT);
+  const double* lo = P.tab + (long)q.b * kNT;
+  const double* dl = P.dtab + (long)q.b * kNT;
+  const double x1 = fma(q.w, dl[GAMMAH2_1], lo[GAMMAH2_1]) - 1.0;
+  const double x2 = fma(q.w, dl[GAMMAH2_2], lo[GAMMAH2_2]) - 1.0;
+  const double dg1 = fma(q.w, dl[DGAMMAH2_1], lo[DGAMMAH2_1]);
+  const double dg2 = fma(q.w, dl[DGAMMAH2_2], lo[DGAMMAH2_2]);
+  const double r = rcp64_any(x1 * x2);
+  const double i1 = r * x2, i2 = r * x1;
+  const double a1 = c.H2_1 * i1, a2 = c.H2_2 * i2;
+  const double nsum = c.S + (a1 + a2);
+  slope = fma(-T, fma(a1 * i1, dg1, (a2 * i2) * dg2), nsum);
+  return fma(T, nsum, -c.gk) * rcp64_any(slope);
+}
+// clamp to the table range; dT/dge from the last slope; log T for the rates: logT + l, the log
+// at the last iterate plus that of the last ratio, unless the clamp moved T
+__device__ __forceinline__ void chem_temp_finish(const ChemParams& P, const ChemTemp& c,
+                                                 double slope, double& Ts, double& logT,
+                                                 bool known, double& dTs_ge) {
+  const double kb = 1.3806504e-16;
+  if (Ts < P.tlo) {
+    Ts = P.tlo;
+    known = false;
+  } else if (Ts > P.thi) {
+    Ts = P.thi;
+    known = false;
+  }
+  if (!known) logT = log(Ts);
+  dTs_ge = c.dmh * rcp64_any(kb * slope);
+}
+
+// cvklu_calculate_temperature: ten Newton iterations from the previous T, then clamp.  The
+// iterations stop once a step is below 2e-15 T: Newton's error falls by at least 80 per step on
+// these tables (interpolated gamma and dgamma/dT are not quite consistent, so the convergence
+// ends linear with that factor), so the remaining iterations only move the last bit.  From the
+// temperature of a nearby state five iterations reach it where ten ran.
+__device__ __forceinline__ void chem_temperature(const ChemParams& P, const double (&y)[10],
+                                                 double& Ts, double& dTs_ge, double& logT) {
+  const ChemTemp c = chem_temp_setup(y);
+  double T = Ts, slope = 0.0;
+  bool known = false;
 #pragma unroll 1
   for (int it = 0; it < 10; ++it) {
-    T = Ts;
-    double t1, t2;
-    const double logT = log(Ts);
-    const int b = chem_bin(P, logT, t1, t2);
-    const double Tdef = (logT - t1) / (t2 - t1);
-    const double* lo = P.tab + (long)b * kNT;
-    const double* dl = P.dtab + (long)b * kNT;
-    const double g2 = lo[GAMMAH2_2] + Tdef * dl[GAMMAH2_2];
-    const double dg2 = lo[DGAMMAH2_2] + Tdef * dl[DGAMMAH2_2];
-    const double g1 = lo[GAMMAH2_1] + Tdef * dl[GAMMAH2_1];
-    const double dg1 = lo[DGAMMAH2_1] + Tdef * dl[DGAMMAH2_1];
-    const double i1 = 1.0 / (g1 - 1.0), i2 = 1.0 / (g2 - 1.0);
-    const double nsum = H2_1 * i1 + H2_2 * i2 + H_1 * gm1 + H_2 * gm1 + H_m0 * gm1 + He_1 * gm1 +
-                        He_2 * gm1 + He_3 * gm1 + gm1 * de;
-    dge_dT = T * kb * (-H2_1 * i1 * i1 * dg1 - H2_2 * i2 * i2 * dg2) / dmh + kb * nsum / dmh;
-    const double dge = T * kb * nsum / dmh - ge;
-    Tnew = T - dge / dge_dT;
-    Ts = Tnew;
+    logT = log(T);
+    const double dT = chem_temp_step(P, c, T, logT, slope);
+    const double T0 = T;
+    T -= dT;
+    if (fabs(dT) <= 2e-15 * T0) {
+      logT = fma(-dT, rcp_seed(T0), logT);  // log(T / T0) = -dT / T0 to 1e-30
+      known = true;
+      break;
+    }
   }
-  Ts = Tnew;
-  if (Ts < P.tlo) Ts = P.tlo;
-  else if (Ts > P.thi) Ts = P.thi;
-  dTs_ge = 1.0 / dge_dT;
+  Ts = T;
+  chem_temp_finish(P, c, slope, Ts, logT, known, dTs_ge);
 }
 
 // The same Newton solve with up to `nfloat` iterations in FP32 (table lookups on float copies
@@ -98,7 +153,8 @@ __device__ __forceinline__ void chem_temperature(const ChemParams& P, const doub
 // converge.  From the carried temperature of a nearby state (successive stages, Newton
 // iterates) one FP32 iteration usually suffices.
 __device__ __forceinline__ void chem_temperature_mixed(const ChemParams& P, const double (&y)[10],
-                                                       double& Ts, double& dTs_ge, int nfloat) {
+                                                       double& Ts, double& dTs_ge, double& logT,
+                                                       int nfloat) {
   const float kb = 1.3806504e-16f, mh = 1.67e-24f, gm1 = 1.5f;
   const float H2_1 = (float)y[0], H2_2 = (float)y[1], H_1 = (float)y[2], H_2 = (float)y[3],
               H_m0 = (float)y[4], He_1 = (float)y[5], He_2 = (float)y[6], He_3 = (float)y[7],
@@ -110,11 +166,11 @@ __device__ __forceinline__ void chem_temperature_mixed(const ChemParams& P, cons
   float T = (float)Ts;
 #pragma unroll 1
   for (int it = 0; it < nfloat; ++it) {
-    const float logT = logf(T);
-    int b = (int)(idbin * (logT - lb));
+    const float logTf = logf(T);
+    int b = (int)(idbin * (logTf - lb));
     b = b <= 0 ? 0 : (b >= P.nbins ? P.nbins - 1 : b);
     const float t1 = lb + b * dbin;
-    const float Tdef = (logT - t1) / dbin;
+    const float Tdef = (logTf - t1) / dbin;
     const float4 ga = __ldg(reinterpret_cast<const float4*>(P.gtab + (long)b * 8));
     const float4 gb = __ldg(reinterpret_cast<const float4*>(P.gtab + (long)b * 8 + 4));
     const float g2 = ga.x + Tdef * ga.y;
@@ -130,64 +186,39 @@ __device__ __forceinline__ void chem_temperature_mixed(const ChemParams& P, cons
     T = T - dT;
     if (fabsf(dT) <= 1e-5f * T) break;
   }
-  Ts = (double)T;
   // remaining iterations (and dT/dge) in FP64: exactly chem_temperature's loop body
-  const double kbd = 1.3806504e-16, mhd = 1.67e-24, gm1d = 1.0 / (5.e0 / 3.e0 - 1);
-  const double dH2_1 = y[0], dH2_2 = y[1], dH_1 = y[2], dH_2 = y[3], dH_m0 = y[4], dHe_1 = y[5],
-               dHe_2 = y[6], dHe_3 = y[7], dde = y[8], dge0 = y[9];
-  const double ddensity = 2.0 * dH2_1 + 2.0 * dH2_2 + 1.00794 * dH_1 + 1.00794 * dH_2 +
-                          1.00794 * dH_m0 + 4.002602 * dHe_1 + 4.002602 * dHe_2 + 4.002602 * dHe_3;
-  const double dmh = ddensity * mhd;
-  // the FP64 tail multiplies by reciprocals where the FP64 form divides (one rounding apart;
-  // each FP64 division costs about as much as ten multiplies on this part)
-  const double kdmd = kbd / dmh;
-  double Tc = Ts, Tnew = Ts, dge_dTd = 0.0;
+  const ChemTemp c = chem_temp_setup(y);
+  double Td = (double)T, T0 = Td, slope = 0.0, dT = 0.0;
 #pragma unroll 1
   for (int it = nfloat; it < 10; ++it) {
-    Tc = Ts;
-    double t1, t2;
-    const double logT = log(Ts);
-    const int b = chem_bin(P, logT, t1, t2);
-    const double Tdef = (logT - t1) * P.idbin;
-    const double* lo = P.tab + (long)b * kNT;
-    const double* dl = P.dtab + (long)b * kNT;
-    const double g2 = lo[GAMMAH2_2] + Tdef * dl[GAMMAH2_2];
-    const double dg2 = lo[DGAMMAH2_2] + Tdef * dl[DGAMMAH2_2];
-    const double g1 = lo[GAMMAH2_1] + Tdef * dl[GAMMAH2_1];
-    const double dg1 = lo[DGAMMAH2_1] + Tdef * dl[DGAMMAH2_1];
-    const double i1 = 1.0 / (g1 - 1.0), i2 = 1.0 / (g2 - 1.0);
-    const double nsum = dH2_1 * i1 + dH2_2 * i2 + dH_1 * gm1d + dH_2 * gm1d + dH_m0 * gm1d +
-                        dHe_1 * gm1d + dHe_2 * gm1d + dHe_3 * gm1d + gm1d * dde;
-    dge_dTd = kdmd * (Tc * (-dH2_1 * i1 * i1 * dg1 - dH2_2 * i2 * i2 * dg2) + nsum);
-    const double dgev = kdmd * Tc * nsum - dge0;
-    Tnew = Tc - dgev / dge_dTd;
-    Ts = Tnew;
+    T0 = Td;
+    logT = log(T0);
+    dT = chem_temp_step(P, c, T0, logT, slope);
+    Td = T0 - dT;
   }
-  Ts = Tnew;
-  if (Ts < P.tlo) Ts = P.tlo;
-  else if (Ts > P.thi) Ts = P.thi;
-  dTs_ge = 1.0 / dge_dTd;
+  Ts = Td;
+  // log(T / T0) by its series: |dT / T0| is ~1e-5 at most after the FP32 stage, and the first
+  // term dropped is below 3e-17 up to 1e-4
+  const double e = -dT * rcp64_any(T0);
+  const bool known = fabs(e) < 1e-4;
+  logT = fma(e, fma(e, fma(e, 1.0 / 3.0, -0.5), 1.0), logT);
+  chem_temp_finish(P, c, slope, Ts, logT, known, dTs_ge);
 }
 
-// Rates at temperature Ts (and their T-derivatives when WithSlopes).  Reciprocal: the
-// interpolation weight and the slope factor multiply by 1 / dbin instead of dividing by the
-// bin width t2 - t1 (one division per cell instead of three, within an ulp or two of the
-// quotients; the mixed forms' choice -- the FP64 forms divide, as the reference does).
-template <bool WithSlopes, bool Reciprocal = false>
-__device__ __forceinline__ void chem_rates(const ChemParams& P, double Ts, double (&k)[kNRates],
+// Rates at the temperature of log logT; WithSlopes: also dk, the rates' differences over the
+// table bin, which times idbin / T are their T-derivatives (the Jacobian applies that factor
+// once per entry that is linear in them).
+template <bool WithSlopes>
+__device__ __forceinline__ void chem_rates(const ChemParams& P, double logT, double (&k)[kNRates],
                                            double (&dk)[kNRates]) {
-  double t1, t2;
-  const double logT = log(Ts);
-  const int b = chem_bin(P, logT, t1, t2);
-  const double Tdef = Reciprocal ? (logT - t1) * P.idbin : (logT - t1) / (t2 - t1);
-  const double Tfactor = Reciprocal ? P.idbin / Ts : (1.0 / Ts) / (t2 - t1);
-  const double* lo = P.tab + (long)b * kNT;
-  const double* dl = P.dtab + (long)b * kNT;
+  const ChemPos q = chem_pos(P, logT);
+  const double* lo = P.tab + (long)q.b * kNT;
+  const double* dl = P.dtab + (long)q.b * kNT;
 #pragma unroll
   for (int r = 0; r < kNRates; ++r) {
     const double a = __ldg(lo + r), d = __ldg(dl + r);
-    k[r] = a + Tdef * d;
-    if (WithSlopes) dk[r] = d * Tfactor;
+    k[r] = fma(q.w, d, a);
+    if (WithSlopes) dk[r] = d;
   }
 }
 
@@ -219,93 +250,72 @@ __device__ __forceinline__ void chem_fluxes(const double (&k)[kNRates], const do
   r[20] = k[K22] * H_1 * H_1 * H_1;
 }
 
-// Net species sources from reaction fluxes (net stoichiometry, reaction order).
+// Net species sources from reaction fluxes (net stoichiometry).
 __device__ __forceinline__ void chem_species(const double (&r)[21], double (&s)[9]) {
-  s[0] = r[7] + r[9] - r[10] - r[11] - r[12] + r[18] + r[19] + r[20];
-  s[1] = r[8] - r[9] + r[10] + r[16] - r[17] - r[18];
-  s[2] = -r[0] + r[1] - r[6] - r[7] - r[8] - r[9] + r[10] + 2 * r[11] + 2 * r[12] + r[13] + r[14] +
-         2 * r[15] + 2 * r[17] + r[18] - 2 * r[19] - 2 * r[20];
-  s[3] = r[0] - r[1] - r[8] + r[9] - r[10] - r[15] - r[16];
-  s[4] = r[6] - r[7] - r[13] - r[14] - r[15] - r[16] - r[18];
-  s[5] = -r[2] + r[3];
-  s[6] = r[2] - r[3] - r[4] + r[5];
-  s[7] = r[4] - r[5];
-  s[8] = r[0] - r[1] + r[2] - r[3] + r[4] - r[5] - r[6] + r[7] + r[13] + r[14] + r[16] - r[17];
+  // sums that several rows share
+  const double p = r[0] - r[1], q = r[9] - r[10], t = r[2] - r[3], u = r[4] - r[5],
+               v = r[13] + r[14], x = r[11] + r[12], y = r[19] + r[20];
+  s[0] = r[7] + q - x + r[18] + y;
+  s[1] = r[8] - q + r[16] - r[17] - r[18];
+  s[2] = fma(2.0, x - y + r[15] + r[17], v - p - r[6] - r[7] - r[8] - q + r[18]);
+  s[3] = p - r[8] + q - r[15] - r[16];
+  s[4] = r[6] - r[7] - v - r[15] - r[16] - r[18];
+  s[5] = -t;
+  s[6] = t - u;
+  s[7] = u;
+  s[8] = p + t + u - r[6] + r[7] + v + r[16] - r[17];
 }
 
 struct ChemAux {
   double mdens, imdens, cie, h2;
 };
 
-// Gas-energy source (cooling/heating), src/raja_primordial_network.cpp:1371-1375.
+// Shared by the gas-energy source and its Jacobian row: G and N, the densities-weighted sums of
+// the H2 cooling and of the three-body terms, and the two reciprocals behind the reference's
+// quotients 1/G, 1/D, 1/N, 1/F (D = h2lte / G + 1, F = ncrn / N + 1):
+//   1/D = G / (h2lte + G),  1/F = N / (ncrn + N).
+struct GeTerms {
+  double G, N, i1, i2, H13, Hf;
+};
+__device__ __forceinline__ GeTerms ge_terms(const double (&k)[kNRates], const double (&y)[10]) {
+  const double H2_1 = y[0], H_1 = y[2], H_2 = y[3], He_1 = y[5], de = y[8];
+  GeTerms t;
+  t.G = H2_1 * k[GAH2] + H_1 * k[GAHI] + H_2 * k[GAHP] + He_1 * k[GAHE] + de * k[GAEL];
+  t.N = H2_1 * k[NCRD2] + H_1 * k[NCRD1];
+  t.i1 = rcp64_any(k[H2LTE] + t.G);
+  t.i2 = rcp64_any(k[NCRN] + t.N);
+  t.H13 = H_1 * H_1 * H_1;
+  t.Hf = t.H13 * k[H2MHEAT] - H2_1 * H_1 * k[H2MCOOL];
+  return t;
+}
+
+// Gas-energy source (cooling/heating), src/raja_primordial_network.cpp:1371-1375, the terms
+// proportional to the electron density summed before the common factor.
 __device__ __forceinline__ double chem_ge_source(const ChemParams& P, const double (&k)[kNRates],
                                                  const double (&y)[10], double T,
-                                                 const ChemAux& A) {
+                                                 const ChemAux& A, const GeTerms& t) {
   const double H2_1 = y[0], H_1 = y[2], H_2 = y[3], He_1 = y[5], He_2 = y[6], He_3 = y[7],
                de = y[8];
-  const double z = P.z, cie = A.cie, h2oda = A.h2, mdens = A.mdens;
-  const double G = H2_1 * k[GAH2] + H_1 * k[GAHI] + H_2 * k[GAHP] + He_1 * k[GAHE] + de * k[GAEL];
-  const double D = k[H2LTE] / G + 1.0;
-  const double F = k[NCRN] / (H2_1 * k[NCRD2] + H_1 * k[NCRD1]) + 1.0;
-  const double H13 = H_1 * H_1 * H_1;
-  const double Hf = -H2_1 * H_1 * k[H2MCOOL] + H13 * k[H2MHEAT];
-  const double de2 = de * de;
-  return -2.01588 * H2_1 * k[CIECO] * cie * mdens - H2_1 * cie * k[H2LTE] * h2oda / D -
-         H_1 * k[CEHI] * cie * de - H_1 * k[CIHI] * cie * de - H_2 * cie * de * k[REHII] -
-         He_1 * k[CIHEI] * cie * de - He_2 * k[CEHEII] * cie * de - He_2 * k[CEHEI] * cie * de2 -
-         He_2 * k[CIHEII] * cie * de - He_2 * k[CIHEIS] * cie * de2 -
-         He_2 * cie * de * k[REHEII1] - He_2 * cie * de * k[REHEII2] -
-         He_3 * cie * de * k[REHEIII] - k[BREM] * cie * de * (H_2 + He_2 + 4.0 * He_3) -
-         cie * k[COMPTON] * de * P.zp1_4 * (T - 2.73 * z - 2.73) + 0.5 / F * Hf;
-}
-
-// The four reciprocals of the cooling/heating terms (1/G, 1/D, 1/N, 1/F), shared by the gas-
-// energy source and its Jacobian row when both are evaluated together.
-struct GeRecip {
-  double iG, iD, iN, iF;
-};
-__device__ __forceinline__ GeRecip ge_recip(const double (&k)[kNRates], const double (&y)[10]) {
-  const double H2_1 = y[0], H_1 = y[2], H_2 = y[3], He_1 = y[5], de = y[8];
-  GeRecip r;
-  const double G = H2_1 * k[GAH2] + H_1 * k[GAHI] + H_2 * k[GAHP] + He_1 * k[GAHE] + de * k[GAEL];
-  r.iG = 1.0 / G;
-  r.iD = 1.0 / (k[H2LTE] * r.iG + 1.0);
-  r.iN = 1.0 / (H2_1 * k[NCRD2] + H_1 * k[NCRD1]);
-  r.iF = 1.0 / (k[NCRN] * r.iN + 1.0);
-  return r;
-}
-
-// chem_ge_source with the shared reciprocals (the fused kernels: one rounding apart from the
-// reference's divisions).
-__device__ __forceinline__ double chem_ge_source_r(const ChemParams& P, const double (&k)[kNRates],
-                                                   const double (&y)[10], double T,
-                                                   const ChemAux& A, const GeRecip& R) {
-  const double H2_1 = y[0], H_1 = y[2], H_2 = y[3], He_1 = y[5], He_2 = y[6], He_3 = y[7],
-               de = y[8];
-  const double z = P.z, cie = A.cie, h2oda = A.h2, mdens = A.mdens;
-  const double H13 = H_1 * H_1 * H_1;
-  const double Hf = -H2_1 * H_1 * k[H2MCOOL] + H13 * k[H2MHEAT];
-  const double de2 = de * de;
-  return -2.01588 * H2_1 * k[CIECO] * cie * mdens - H2_1 * cie * k[H2LTE] * h2oda * R.iD -
-         H_1 * k[CEHI] * cie * de - H_1 * k[CIHI] * cie * de - H_2 * cie * de * k[REHII] -
-         He_1 * k[CIHEI] * cie * de - He_2 * k[CEHEII] * cie * de - He_2 * k[CEHEI] * cie * de2 -
-         He_2 * k[CIHEII] * cie * de - He_2 * k[CIHEIS] * cie * de2 -
-         He_2 * cie * de * k[REHEII1] - He_2 * cie * de * k[REHEII2] -
-         He_3 * cie * de * k[REHEIII] - k[BREM] * cie * de * (H_2 + He_2 + 4.0 * He_3) -
-         cie * k[COMPTON] * de * P.zp1_4 * (T - 2.73 * z - 2.73) + 0.5 * R.iF * Hf;
+  const double he2 = k[CEHEII] + k[CIHEII] + k[REHEII1] + k[REHEII2] + de * (k[CEHEI] + k[CIHEIS]);
+  const double L = H_1 * (k[CEHI] + k[CIHI]) + H_2 * k[REHII] + He_1 * k[CIHEI] + He_2 * he2 +
+                   He_3 * k[REHEIII] + k[BREM] * (H_2 + He_2 + 4.0 * He_3) +
+                   k[COMPTON] * P.zp1_4 * (T - (2.73 * P.z + 2.73));
+  const double h2 = 2.01588 * k[CIECO] * A.mdens + k[H2LTE] * A.h2 * (t.G * t.i1);
+  return 0.5 * (t.N * t.i2) * t.Hf - A.cie * (H2_1 * h2 + de * L);
 }
 
 // Analytic Jacobian in physical units, before the inv_scale*scale and time-unit factors;
-// rates k and slopes dk at the cell temperature.  Each of the 64 nonzeros is handed to
+// rates k and bin differences dk (chem_rates) at the cell temperature.  Each of the 64 nonzeros is handed to
 // put(row, col, value) once, already multiplied by the factors the reference applies to that
 // entry (1/mdensity on the ge row, dT/dge on the ge column); entries never put are zero.
-// Raw: those two factors are left out, for a caller that folds them into its own row and
-// column scaling (one multiply per cell instead of one per entry).
+// Raw: the ge row's factor and the ge column's, with the idbin / T of the slopes, are left out,
+// for a caller that folds them into its own row and column scaling (one multiply per cell
+// instead of one per entry); else Tge holds dT/dge times idbin / T.
 template <bool Raw = false, class Put>
 __device__ __forceinline__ void chem_jacobian(const ChemParams& P, const double (&k)[kNRates],
                                               const double (&dk)[kNRates], const double (&y)[10],
-                                              double T, double Tge, const ChemAux& A, Put&& put,
-                                              const GeRecip* shared = nullptr) {
+                                              double T, double Tge, const ChemAux& A,
+                                              const GeTerms& t, Put&& put) {
   const double H2_1 = y[0], H2_2 = y[1], H_1 = y[2], H_2 = y[3], H_m0 = y[4], He_1 = y[5],
                He_2 = y[6], He_3 = y[7], de = y[8];
   const double z = P.z, h2oda = A.h2, md = A.mdens, imd = A.imdens;
@@ -371,40 +381,34 @@ __device__ __forceinline__ void chem_jacobian(const ChemParams& P, const double 
 #pragma unroll
     for (int q = 0; q < 9; ++q) put(q, 9, Raw ? s[q] : s[q] * Tge);
   }
-  // four reciprocals serve every ge-row entry (the reference divides ~20 times)
-  const GeRecip R = shared ? *shared : ge_recip(k, y);
-  const double iG = R.iG, iD = R.iD, iN = R.iN, iF = R.iF;
-  const double H13 = H1sq * H_1;
-  const double Hf = -H2_1 * H_1 * k[H2MCOOL] + H13 * k[H2MHEAT];
-  const double lte2 = k[H2LTE] * k[H2LTE];
-  const double iDG2 = (iD * iD) * (iG * iG);
-  const double iF2 = iF * iF;
-  const double iN2 = iN * iN;
-  const double lteh = lte2 * h2oda * iDG2;  // h2lte^2 * h2oda / (D^2 G^2)
-  SETG(0, -H2_1 * k[GAH2] * lteh - 0.5 * H_1 * k[H2MCOOL] * iF - 2.01588 * k[CIECO] * md -
-              k[H2LTE] * h2oda * iD + 0.5 * k[NCRD2] * k[NCRN] * iF2 * Hf * iN2);
-  SETG(2, -H2_1 * k[GAHI] * lteh - k[CEHI] * de - k[CIHI] * de +
-              0.5 * k[NCRD1] * k[NCRN] * iF2 * Hf * iN2 +
-              0.5 * (-H2_1 * k[H2MCOOL] + 3 * H1sq * k[H2MHEAT]) * iF);
-  SETG(3, -H2_1 * k[GAHP] * lteh - k[BREM] * de - de * k[REHII]);
-  SETG(5, -H2_1 * k[GAHE] * lteh - k[CIHEI] * de);
-  SETG(6, -k[BREM] * de - k[CEHEII] * de - k[CEHEI] * (de * de) - k[CIHEII] * de -
-              k[CIHEIS] * (de * de) - de * k[REHEII1] - de * k[REHEII2]);
-  SETG(7, -4.0 * k[BREM] * de - de * k[REHEIII]);
-  SETG(8, -H2_1 * k[GAEL] * lteh - H_1 * k[CEHI] - H_1 * k[CIHI] - H_2 * k[REHII] -
-              He_1 * k[CIHEI] - He_2 * k[CEHEII] - 2 * He_2 * k[CEHEI] * de - He_2 * k[CIHEII] -
-              2 * He_2 * k[CIHEIS] * de - He_2 * k[REHEII1] - He_2 * k[REHEII2] -
-              He_3 * k[REHEIII] - k[BREM] * (H_2 + He_2 + 4.0 * He_3) -
-              k[COMPTON] * P.zp1_4 * (T - 2.73 * z - 2.73));
-  const double dGn = -H2_1 * dk[GAH2] - H_1 * dk[GAHI] - H_2 * dk[GAHP] - He_1 * dk[GAHE] -
-                     de * dk[GAEL];
-  const double gg = -H2_1 * k[H2LTE] * h2oda * (-k[H2LTE] * dGn * (iG * iG) - dk[H2LTE] * iG) *
-                        (iD * iD) -
-                    H2_1 * h2oda * dk[H2LTE] * iD +
-                    0.5 * iF2 * Hf *
-                        (-1.0 * k[NCRN] * (-H2_1 * dk[NCRD2] - H_1 * dk[NCRD1]) * iN2 -
-                         1.0 * dk[NCRN] * iN) +
-                    0.5 * iF * (-H2_1 * H_1 * dk[H2MCOOL] + H13 * dk[H2MHEAT]);
+  // With D = h2lte / G + 1 and F = ncrn / N + 1 every quotient of the ge row is in G, N and the
+  // two reciprocals: 1/D = G i1, 1/(D G) = i1, 1/F = N i2, 1/(F N) = i2.
+  const double iF = t.N * t.i2, i1h = t.i1 * t.i1 * h2oda, i22 = t.i2 * t.i2;
+  const double lteh = k[H2LTE] * k[H2LTE] * i1h;  // h2lte^2 h2oda / (D G)^2
+  const double hlteh = H2_1 * lteh;
+  const double nf = 0.5 * k[NCRN] * i22 * t.Hf;
+  const double chi = k[CEHI] + k[CIHI], h2c = k[CEHEII] + k[CIHEII] + k[REHEII1] + k[REHEII2],
+               h2d = k[CEHEI] + k[CIHEIS], bd = k[BREM] * de;
+  SETG(0, nf * k[NCRD2] - k[GAH2] * hlteh - 0.5 * H_1 * k[H2MCOOL] * iF -
+              2.01588 * k[CIECO] * md - k[H2LTE] * h2oda * (t.G * t.i1));
+  SETG(2, nf * k[NCRD1] - k[GAHI] * hlteh - chi * de +
+              0.5 * (3 * H1sq * k[H2MHEAT] - H2_1 * k[H2MCOOL]) * iF);
+  SETG(3, -k[GAHP] * hlteh - bd - de * k[REHII]);
+  SETG(5, -k[GAHE] * hlteh - k[CIHEI] * de);
+  SETG(6, -bd - de * (h2c + h2d * de));
+  SETG(7, -4.0 * bd - de * k[REHEIII]);
+  SETG(8, -k[GAEL] * hlteh - H_1 * chi - H_2 * k[REHII] - He_1 * k[CIHEI] -
+              He_2 * (h2c + 2 * h2d * de) - He_3 * k[REHEIII] -
+              k[BREM] * (H_2 + He_2 + 4.0 * He_3) -
+              k[COMPTON] * P.zp1_4 * (T - (2.73 * z + 2.73)));
+  const double dG = H2_1 * dk[GAH2] + H_1 * dk[GAHI] + H_2 * dk[GAHP] + He_1 * dk[GAHE] +
+                    de * dk[GAEL];
+  const double dN = H2_1 * dk[NCRD2] + H_1 * dk[NCRD1];
+  // d/dT of -H2 h2oda h2lte / D and of Hf / (2 F)
+  const double gg = 0.5 * (k[NCRN] * dN - dk[NCRN] * t.N) * i22 * t.Hf +
+                    0.5 * iF * (t.H13 * dk[H2MHEAT] - H2_1 * H_1 * dk[H2MCOOL]) -
+                    H2_1 * (k[H2LTE] * (k[H2LTE] * dG - t.G * dk[H2LTE]) * i1h +
+                            h2oda * dk[H2LTE] * (t.G * t.i1));
   put(9, 9, Raw ? gg : gg * imd * Tge);
 #undef SETG
 #undef SETJ

@@ -61,30 +61,30 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       double ya[10];
 #pragma unroll
       for (int s = 0; s < 10; ++s) ya[s] = y[j + s] * sc[s];
-      double Ts = S.Ts[i], dTs = 0.0;
+      double Ts = S.Ts[i], dTs = 0.0, logT;
       // mixed form: up to 8 FP32 iterations, then two in FP64.  (One FP64 iteration where
       // the FP32 stage converged measured 5 % faster but left the carried temperature up to
       // 4e-10 off the FP64 form's ten-iteration value: the adiabatic-index tables are linear
       // in log T per bin, so near a bin edge Newton converges only linearly.)
       if (sizeof(LU) == 4)
-        chem_temperature_mixed(P, ya, Ts, dTs, 8);
+        chem_temperature_mixed(P, ya, Ts, dTs, logT, 8);
       else
-        chem_temperature(P, ya, Ts, dTs);
+        chem_temperature(P, ya, Ts, dTs, logT);
       S.Ts[i] = Ts;
       S.dTs_ge[i] = dTs;
       const ChemAux Ax{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
       double f[10];
       {  // source and Newton matrix from one rate evaluation (rates and T slopes)
         double k[kNRates], dk[kNRates];
-        chem_rates<true, kMixed>(P, Ts, k, dk);
-        const GeRecip Rg = ge_recip(k, ya);  // shared by the source and the Jacobian's ge row
+        chem_rates<true>(P, logT, k, dk);
+        const GeTerms Rg = ge_terms(k, ya);  // shared by the source and the Jacobian's ge row
         {
           double r[21], sp[9];
           chem_fluxes(k, ya, r);
           chem_species(r, sp);
 #pragma unroll
           for (int s = 0; s < 9; ++s) f[s] = (sp[s] * isc[s]) * tunit;
-          double ge = chem_ge_source_r(P, k, ya, Ts, Ax, Rg) * isc[9];
+          double ge = chem_ge_source(P, k, ya, Ts, Ax, Rg) * isc[9];
           ge *= Ax.imdens;
           f[9] = ge * tunit;
         }
@@ -96,11 +96,11 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
 #pragma unroll
         for (int r = 0; r < 10; ++r) rf[r] = (-gamma * tunit) * isc[r];
         rf[9] *= Ax.imdens;
-        const double sc9 = sc[9] * dTs;
+        const double sc9 = sc[9] * dTs * (P.idbin * rcp64_any(Ts));
 #pragma unroll
         for (int e = 0; e < 100; ++e) L[e * BS] = LU(0);  // structural zeros
         // every structural entry (the diagonal included) is put exactly once
-        chem_jacobian<true>(P, k, dk, ya, Ts, dTs, Ax, [&](int row, int col, double v) {
+        chem_jacobian<true>(P, k, dk, ya, Ts, dTs, Ax, Rg, [&](int row, int col, double v) {
           const double a = (v * rf[row]) * (col == 9 ? sc9 : sc[col]) + (row == col ? 1.0 : 0.0);
           if (kMixed) {
             const int e = kJacIndex[row][col];
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
           } else {
             L[(col * 10 + row) * BS] = to_lu<LU>(a);
           }
-        }, &Rg);
+        });
         if constexpr (kMixed) {  // the FP32 factor's entries, converted with integer
           // instructions after the Jacobian (off the FP64 pipe, which bounds this kernel, and off
           // the Jacobian's dependency chains: 5.45 -> 5.34 ms per 128^3 call; converting inside
