@@ -84,15 +84,32 @@ __device__ __forceinline__ f2 f2_from_double(double d) {
 // Conversion instructions with a 64-bit operand run at the FP64 rate, 1/64 of the FP32 rate on
 // GB300, so in passes that mostly convert (the float-float primitives, the FP32 factors of the
 // Newton matrices) they set the time.  Each helper returns exactly what the round-to-nearest
-// hardware conversion returns: the integer path covers every normal float result, anything
-// else (zero, subnormal, overflow, inf, NaN) takes the hardware conversion.
+// hardware conversion returns: the integer path covers every normal float result and zeros,
+// anything else (subnormal, overflow, inf, NaN) takes the hardware conversion.  In the passes
+// bound by the FP64 pipe (f2_split, f2_to_double: RARE) that conversion is a volatile statement:
+// the compiler otherwise executes it on every call and selects, and its pipe time is spent after
+// all (128^3 x 15: primitives 314 -> 241 us).  The fused Newton is bound by latency: there the
+// select is 3 % faster than the branch.
+__device__ __forceinline__ float cvt_f32_rare(double d) {
+  float f;
+  asm volatile("cvt.rn.f32.f64 %0, %1;" : "=f"(f) : "d"(d));
+  return f;
+}
+__device__ __forceinline__ double cvt_f64_rare(float f) {
+  double d;
+  asm volatile("cvt.f64.f32 %0, %1;" : "=d"(d) : "f"(f));
+  return d;
+}
 
 // double -> float, round to nearest even: drop 29 mantissa bits on the pattern (a carry into
 // the exponent is the correct rounding), re-bias the exponent (1023 - 127 = 896)
+template <bool RARE = false>
 __device__ __forceinline__ float f32_of_f64(double d) {
   const unsigned long long p = (unsigned long long)__double_as_longlong(d);
   const unsigned e = (unsigned)(p >> 52) & 0x7FFu;
-  if (e - 897u > 1149u - 897u) return __double2float_rn(d);  // result not surely a normal float
+  if (e - 897u > 1149u - 897u)  // result not surely a normal float: zero, or the conversion
+    return !RARE ? __double2float_rn(d)
+                 : ((p << 1) == 0 ? __uint_as_float((unsigned)(p >> 32)) : cvt_f32_rare(d));
   const unsigned long long r = p + 0x0FFFFFFFull + ((p >> 29) & 1ull);
   const unsigned hi = (unsigned)(r >> 32);
   const unsigned s = hi & 0x80000000u;
@@ -102,10 +119,13 @@ __device__ __forceinline__ float f32_of_f64(double d) {
 }
 
 // float -> double, exact
+template <bool RARE = false>
 __device__ __forceinline__ double f64_of_f32(float f) {
   const unsigned u = __float_as_uint(f);
   const unsigned e = (u >> 23) & 0xFFu;
-  if (e - 1u > 253u) return (double)f;  // zero, subnormal, inf, NaN
+  if (e - 1u > 253u)  // zero, or subnormal, inf, NaN
+    return !RARE ? (double)f
+                 : ((u << 1) == 0 ? __hiloint2double((int)u, 0) : cvt_f64_rare(f));
   const unsigned hi = (u & 0x80000000u) | ((e + 896u) << 20) | ((u & 0x7FFFFFu) >> 3);
   const unsigned lo = u << 29;
   return __hiloint2double((int)hi, (int)lo);
@@ -113,13 +133,13 @@ __device__ __forceinline__ double f64_of_f32(float f) {
 
 // f2_from_double without conversion instructions (bit-identical to it)
 __device__ __forceinline__ f2 f2_split(double d) {
-  const float h = f32_of_f64(d);
-  return f2(h, f32_of_f64(d - f64_of_f32(h)));
+  const float h = f32_of_f64<true>(d);
+  return f2(h, f32_of_f64<true>(d - f64_of_f32<true>(h)));
 }
 
 // f2::to_double without conversion instructions (bit-identical to it)
 __device__ __forceinline__ double f2_to_double(f2 x) {
-  return f64_of_f32(x.hi) + f64_of_f32(x.lo);
+  return f64_of_f32<true>(x.hi) + f64_of_f32<true>(x.lo);
 }
 
 __device__ __forceinline__ bool operator<(f2 a, f2 b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }

@@ -66,6 +66,33 @@ __device__ __forceinline__ f2v operator*(f2v x, f2v y) {
   return quick_two_sum2(p.hi, e);
 }
 
+// Pieces without the final renormalisation (|lo| a few ulps of hi instead of half of one), for
+// values that are only multiplied or summed with others of their sign afterwards: a product in 4
+// operations instead of 7, a product added to a sum in 12 instead of 18.
+__device__ __forceinline__ f2v f2v_prod(f2v x, f2v y) {
+  const f2v p = two_prod2(x.hi, y.hi);
+  return f2v(p.hi, fma2(x.hi, y.lo, fma2(x.lo, y.hi, p.lo)));
+}
+__device__ __forceinline__ f2v f2v_add_prod(f2v s, f2v x, f2v y) {  // s + x y
+  const f2v p = two_prod2(x.hi, y.hi);
+  const f2v t = two_sum2(s.hi, p.hi);
+  const float2 e = add2(add2(s.lo, t.lo), p.lo);
+  return f2v(t.hi, fma2(x.hi, y.lo, fma2(x.lo, y.hi, e)));
+}
+__device__ __forceinline__ f2v f2v_norm(f2v x) { return quick_two_sum2(x.hi, x.lo); }
+// x y + z
+__device__ __forceinline__ f2v f2v_fma(f2v x, f2v y, f2v z) {
+  return f2v_norm(f2v_add_prod(z, x, y));
+}
+// x / y from the approximate reciprocal, one residual (its leading part exact in an FMA) and one
+// correction: 10 operations where the general division below takes 25
+__device__ __forceinline__ f2v f2v_quot(f2v x, f2v y) {
+  const float2 r = make_float2(__fdividef(1.f, y.hi.x), __fdividef(1.f, y.hi.y));
+  const float2 q = mul2(x.hi, r), n = neg2(q);
+  const float2 t = fma2(y.lo, n, add2(fma2(y.hi, n, x.hi), x.lo));
+  return quick_two_sum2(q, mul2(t, r));
+}
+
 // as f2 operator/: approximate reciprocal (one per lane), q1, remainder in float-float, q2
 __device__ __forceinline__ f2v operator/(f2v x, f2v y) {
   const float2 ry = make_float2(__fdividef(1.f, y.hi.x), __fdividef(1.f, y.hi.y));

@@ -13,7 +13,7 @@
 // here: the CFL wave speed, the pack1D stencil gather and the conservation totals.
 #include "common.cuh"
 #include "weno64.cuh"
-#include "weno_face.cuh"
+#include "df64.cuh"
 #include "weno_sweep.cuh"
 #include "weno.cuh"
 
@@ -206,17 +206,36 @@ __global__ void __launch_bounds__(256) divergence_f2_kernel(Grid g, Fields wdot,
     const long fx = i + (nx + 1) * (j + ny * k);
     const long fy = i + nx * (j + (ny + 1) * k);
     const long fz = c;
+    // fields in groups whose 6 fluxes each are loaded before any is used: the rare conversions'
+    // branches keep the compiler from moving loads up across them
+    constexpr int NV = 5 + NCHEM, GR = 5;
 #pragma unroll
-    for (int v = 0; v < 5 + NCHEM; ++v) {
-      const float2 a0 = Fx[v * nfx + fx], a1 = Fx[v * nfx + fx + 1];
-      const float2 b0 = Fy[v * nfy + fy], b1 = Fy[v * nfy + fy + nx];
-      const float2 c0 = Fz[v * nfz + fz], c1 = Fz[v * nfz + fz + nx * ny];
-      const f2 div = (f2(a1.x, a1.y) - f2(a0.x, a0.y)) * idx +
-                     (f2(b1.x, b1.y) - f2(b0.x, b0.y)) * idy +
-                     (f2(c1.x, c1.y) - f2(c0.x, c0.y)) * idz;
-      double* dst = (v < 5) ? (wdot.f[v] + c) : (wdot.f[5] + (v - 5) + (long)NCHEM * c);
-      const double base = G.in_wdot ? *dst : G.c[v];
-      *dst = base - f2_to_double(div);
+    for (int v0 = 0; v0 < NV; v0 += GR) {
+      float2 x[GR][6];
+#pragma unroll
+      for (int q = 0; q < GR; ++q) {
+        const int v = v0 + q;
+        if (v < NV) {
+          x[q][0] = Fx[v * nfx + fx + 1];
+          x[q][1] = Fx[v * nfx + fx];
+          x[q][2] = Fy[v * nfy + fy + nx];
+          x[q][3] = Fy[v * nfy + fy];
+          x[q][4] = Fz[v * nfz + fz + nx * ny];
+          x[q][5] = Fz[v * nfz + fz];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < GR; ++q) {
+        const int v = v0 + q;
+        if (v < NV) {
+          const f2 div = (f2(x[q][0].x, x[q][0].y) - f2(x[q][1].x, x[q][1].y)) * idx +
+                         (f2(x[q][2].x, x[q][2].y) - f2(x[q][3].x, x[q][3].y)) * idy +
+                         (f2(x[q][4].x, x[q][4].y) - f2(x[q][5].x, x[q][5].y)) * idz;
+          double* dst = (v < 5) ? (wdot.f[v] + c) : (wdot.f[5] + (v - 5) + (long)NCHEM * c);
+          const double base = G.in_wdot ? *dst : G.c[v];
+          *dst = base - f2_to_double(div);
+        }
+      }
     }
   }
 }

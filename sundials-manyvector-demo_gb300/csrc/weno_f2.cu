@@ -1,8 +1,12 @@
-// Float-float WENO flux divergence: the per-cell primitive pass and the WV = 0 sweep
-// (float-float weights everywhere), with the entry point that picks the weight variant.
+// Float-float WENO flux divergence: the per-cell primitive pass, the fluid sweep and the entry
+// point that picks the tracers' weights (weno_f2.cuh).
 #include "weno_f2.cuh"
 
 namespace gbmv {
+
+constexpr int kF2MinB = 3;
+constexpr int kF2SharedMinB = 5;
+constexpr int kTracerMinB = 5;
 
 __global__ void __launch_bounds__(256) prims_f2_kernel(Grid g, Fields w, float2* __restrict__ Q2,
                                                        const double* __restrict__ tscale,
@@ -21,7 +25,7 @@ __global__ void __launch_bounds__(256) prims_f2_kernel(Grid g, Fields w, float2*
     // differently from the FP64 form
     bad |= (!(rho > 0.0) ? 1 : 0) | (!(et > 0.0) ? 2 : 0) | (!(p > 0.0) ? 4 : 0);
     double q[kQ2Base] = {rho, mx, my, mz, et, p, mx * ir, my * ir, mz * ir,
-                         sqrt0(g.gamma * p * ir)};
+                         sqrt0_64(g.gamma * p * ir)};
 #pragma unroll
     for (int k = 0; k < kQ2Base; ++k) {
       const f2 v = f2_split(q[k]);
@@ -46,14 +50,215 @@ int prims_f2(const Grid& g, const Fields& w, float2* q2, const double* tscale, i
   return GBMV_OK;
 }
 
+// A face of the fluid sweep in FP64, exactly the FP64 form's arithmetic: fluxes, and half the
+// Lax-Friedrichs speed.
+static __device__ __noinline__ void fluid_face_64(const SweepSet& S, const SweepDir& D, long f,
+                                                  f2 (&out)[5], f2& ha) {
+  long cell[6];
+  bool nall[6], nnorm[6];
+  stencil_of(S, D, f, false, cell, nall, nnorm);
+  Stencil64 T;
+#pragma unroll
+  for (int l = 0; l < 6; ++l) {
+    load_point(D.f, cell[l], nall[l], nnorm[l], T.W[l]);
+    point_prims64(S.gamma, T.W[l][0], T.W[l][1], T.W[l][2], T.W[l][3], T.W[l][4], T.ph[l],
+                  T.hc[l]);
+    T.u[l] = T.W[l][1] / T.W[l][0];
+  }
+  Split64 H;
+  double o[5];
+  fluid_face_flux64(T, S.gamma, H, o);
+#pragma unroll
+  for (int v = 0; v < 5; ++v) out[v] = f2_from_double(o[v]);
+  ha = f2_from_double(half_alpha64(T));
+}
+
+// Fluid face fluxes of the three directions; with tracers, half the Lax-Friedrichs speed is left
+// in the first tracer's flux for the tracer sweep.  MINB: register budget (residency target in
+// 128-thread blocks; the same bits whatever it is).
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB)
+    fluid_flux_f2_kernel(const __grid_constant__ SweepSet S, const float2* __restrict__ Q2, long n,
+                         int nchem) {
+  const int dir = sweep_dir(S);
+  const SweepDir& D = S.d[dir];
+  const int nblk = (dir == 2 ? (int)gridDim.x : S.d[dir + 1].block0) - D.block0;
+  float2* const F = reinterpret_cast<float2*>(D.F);
+  for (long f = (blockIdx.x - D.block0) * (long)blockDim.x + threadIdx.x; f < D.nfaces;
+       f += (long)nblk * blockDim.x) {
+    StencilF2 T;
+    stencil_f2(S, D, f, T);
+    const f2 gm = f2_from_double(S.gamma - 1.0);
+    // a fluid value of point l in face order with its ghost sign (homogeneous Dirichlet negates
+    // every conserved field, so p too; reflecting the normal momentum and velocity)
+    const int src[5] = {0, D.slot[1], D.slot[2], D.slot[3], 4};
+    auto val = [&](int v, int l) {
+      f2 q = q2_load(Q2, n, src[v], T.cell[l]);
+      if (((T.nall ^ (v == 1 ? T.nnorm : 0u)) >> l) & 1u) q = -q;
+      return q;
+    };
+    auto pressure = [&](int l) {
+      const f2 q = q2_load(Q2, n, 5, T.cell[l]);
+      return (T.nall >> l) & 1u ? -q : q;
+    };
+    auto velocity = [&](int l) {
+      const f2 q = q2_load(Q2, n, 6 + D.dir, T.cell[l]);
+      return (T.nnorm >> l) & 1u ? -q : q;
+    };
+    // Lax-Friedrichs speed (src/utilities.cpp:368-380)
+    f2 alpha(0.0);
+#pragma unroll
+    for (int l = 0; l < 6; ++l) {
+      const f2 s = f2_fabs(velocity(l)) + q2_load(Q2, n, 9, T.cell[l]);
+      alpha = (alpha < s) ? s : alpha;
+    }
+    f2 ha = f2_scale(alpha, 0.5f);
+    // Roe average (src/utilities.cpp:298-304) and the left eigenvector rows (:342-364)
+    f2 u, v, w, H, q, c, L00, L01, L02, L03, L04, L30, L31, L40, L41;
+    {
+      const f2 one(1.0);
+      const f2 sL = f2_sqrt0(val(0, 2)), sR = f2_sqrt0(val(0, 3));
+      const f2 iL = one / sL, iR = one / sR, is = one / (sL + sR);
+      u = (val(1, 2) * iL + val(1, 3) * iR) * is;
+      v = (val(2, 2) * iL + val(2, 3) * iR) * is;
+      w = (val(3, 2) * iL + val(3, 3) * iR) * is;
+      H = ((pressure(2) + val(4, 2)) * iL + (pressure(3) + val(4, 3)) * iR) * is;
+      q = f2_scale(u * u + v * v + w * w, 0.5f);
+      c = gm * (H - q);  // the reference's "csnd" (src/utilities.cpp:309)
+      const f2 hc = f2_scale(one / c, 0.5f), hgc = gm * hc, gc = f2_scale(hgc, 2.f), gq = gm * q,
+               gu = gm * u;
+      L00 = hc * (u + gq);
+      L40 = hc * (gq - u);
+      L01 = -(hc * (gu + one));
+      L41 = -(hc * (gu - one));
+      L02 = -(v * hgc);
+      L03 = -(w * hgc);
+      L04 = hgc;
+      L30 = gc * (H - f2_scale(q, 2.f));
+      L31 = u * gc;
+    }
+    bool ok = true;
+    f2v P[5][5];  // [pair][characteristic component]
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const int a = k, b = 5 - k;
+      f2v Wj[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        Wj[m] = f2v(val(m, a), val(m, b));
+        ok = ok && f2v_absmax(Wj[m]) < 1e15f;
+      }
+      const f2v pj = f2v_scale(f2v(pressure(a), pressure(b)), 0.5f);
+      ok = ok && fminf(Wj[0].hi.x, Wj[0].hi.y) > 0.f && f2v_absmax(pj) < 5e14f;
+      const f2 ua = velocity(a), ub = velocity(b);
+      const f2v h = split_pair(ua, ub, ha), uj(ua, ub);
+      const f2v f0 = Wj[0] * h, f1 = f2v_fma(Wj[1], h, pj), f2_ = Wj[2] * h, f3 = Wj[3] * h,
+                f4 = f2v_norm(f2v_add_prod(f2v_prod(Wj[4], h), uj, pj));
+      const f2v X = f2v_norm(
+          f2v_add_prod(f2v_add_prod(f2v_prod(f2v(L02), f2_), f2v(L03), f3), f2v(L04), f4));
+      P[k][0] = f2v_norm(f2v_add_prod(f2v_add_prod(X, f2v(L00), f0), f2v(L01), f1));
+      P[k][1] = f2v_fma(f2v(-v), f0, f2_);
+      P[k][2] = f2v_fma(f2v(-w), f0, f3);
+      P[k][3] = f2v_norm(
+          f2v_add_prod(f2v_add_prod(f2v_scale(X, -2.f), f2v(L30), f0), f2v(L31), f1));
+      P[k][4] = f2v_norm(f2v_add_prod(f2v_add_prod(X, f2v(L40), f0), f2v(L41), f1));
+    }
+    f2 o[5];
+    if (ok) {
+      f2 ff[5];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const f2v r = weno_pair<0>(P[0][i], P[1][i], P[2][i], P[3][i], P[4][i]);
+        ff[i] = r.x() + r.y();
+      }
+      // right eigenvector columns (src/utilities.cpp:318-340)
+      const f2 t = ff[0] + ff[4], s = t + ff[3], cd = c * (ff[4] - ff[0]);
+      o[0] = s;
+      o[1] = u * s + cd;
+      o[2] = v * s + ff[1];
+      o[3] = w * s + ff[2];
+      o[4] = H * t + (u * cd + (v * ff[1] + (w * ff[2] + q * ff[3])));
+    } else {
+      fluid_face_64(S, D, f, o, ha);
+    }
+#pragma unroll
+    for (int m = 0; m < 5; ++m) F[D.slot[m] * D.nfaces + f] = make_float2(o[m].hi, o[m].lo);
+    if (nchem) F[5 * D.nfaces + f] = make_float2(ha.hi, ha.lo);
+  }
+}
+
+// Tracer face fluxes: one thread a face, its tracers one after the other; reads half the
+// Lax-Friedrichs speed that the fluid sweep left in the first tracer's flux.
+template <int WV>
+__global__ void __launch_bounds__(128, WV == 1 ? kTracerMinB : 2)
+    tracer_flux_f2_kernel(const __grid_constant__ SweepSet S, const float2* __restrict__ Q2,
+                          long n, int nchem) {
+  const int dir = sweep_dir(S);
+  const SweepDir& D = S.d[dir];
+  const int nblk = (dir == 2 ? (int)gridDim.x : S.d[dir + 1].block0) - D.block0;
+  float2* const F = reinterpret_cast<float2*>(D.F);
+  for (long f = (blockIdx.x - D.block0) * (long)blockDim.x + threadIdx.x; f < D.nfaces;
+       f += (long)nblk * blockDim.x) {
+    StencilF2 T;
+    stencil_f2(S, D, f, T);
+    f2v h[5];
+    {
+      const float2 t = F[5 * D.nfaces + f];
+      const f2 ha(t.x, t.y);
+      f2 u[6];
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        u[l] = q2_load(Q2, n, 6 + D.dir, T.cell[l]);
+        if ((T.nnorm >> l) & 1u) u[l] = -u[l];
+      }
+#pragma unroll
+      for (int k = 0; k < 5; ++k) h[k] = split_pair(u[k], u[5 - k], ha);
+    }
+#pragma unroll 1
+    for (int c = 0; c < nchem; ++c) {
+      f2 cv[6];
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        cv[l] = q2_load(Q2, n, kQ2Base + c, T.cell[l]);
+        if ((T.nall >> l) & 1u) cv[l] = -cv[l];
+      }
+      const f2 r = tracer_face_flux_f2v<WV>(h, cv);
+      F[(5 + c) * D.nfaces + f] = make_float2(r.hi, r.lo);
+    }
+  }
+}
+
 size_t feuler_f2_prims_floats(const Grid& g) { return (size_t)2 * (kQ2Base + g.nchem) * g.ncell; }
 
 int feuler_f2(const Grid& g, const Fields& w, const Fields& wdot, const ForceTerm& G,
               double* scratch, float* prims, const double* tscale, int* d_status,
               cudaStream_t s, int fast_weights) {
-  float2* q2 = reinterpret_cast<float2*>(prims);
-  if (fast_weights) return feuler_f2_fast(g, w, wdot, G, scratch, q2, tscale, d_status, s);
-  return feuler_f2_wv<0>(g, w, wdot, G, scratch, q2, tscale, d_status, s);
+  float2* const q2 = reinterpret_cast<float2*>(prims);
+  long nf[3];
+  face_counts(g, nf);
+  const long nv = 5 + g.nchem;
+  double* const F[3] = {scratch, scratch + nv * nf[0], scratch + nv * (nf[0] + nf[1])};
+  float2* const F2[3] = {reinterpret_cast<float2*>(F[0]), reinterpret_cast<float2*>(F[1]),
+                         reinterpret_cast<float2*>(F[2])};
+  int rc = prims_f2(g, w, q2, tscale, d_status, s);
+  if (rc != GBMV_OK) return rc;
+  {
+    ProfScope ps("face_flux", s);
+    const int t = sweep_threads(g, nf[0] + nf[1] + nf[2], 128);
+    SweepSet S;
+    const int b = sweep_set(g, w, F, 1, t, (long)kSM * 16, S);
+    if (fast_weights && g.sweep_shared)
+      fluid_flux_f2_kernel<kF2SharedMinB><<<b, t, 0, s>>>(S, q2, g.ncell, g.nchem);
+    else
+      fluid_flux_f2_kernel<kF2MinB><<<b, t, 0, s>>>(S, q2, g.ncell, g.nchem);
+    GBMV_LAUNCH_CHECK("fluid_flux_f2_kernel");
+    if (g.nchem) {
+      if (fast_weights) tracer_flux_f2_kernel<1><<<b, t, 0, s>>>(S, q2, g.ncell, g.nchem);
+      else tracer_flux_f2_kernel<0><<<b, t, 0, s>>>(S, q2, g.ncell, g.nchem);
+      GBMV_LAUNCH_CHECK("tracer_flux_f2_kernel");
+    }
+  }
+  return divergence_f2(g, wdot, F2, G, s);
 }
 
 }  // namespace gbmv

@@ -6,8 +6,8 @@
 // tendency is the derivative only if none of the cell's six faces changes that branch between
 // w - h d, w and w + h d; this kernel marks the cells where one does, so that derivative tests
 // can compare the exact JVP / VJP with finite differences on the smooth entries and count the
-// others.  The branch is evaluated with the face kernel's own expressions (eos_t, sqrt0).
-#include "weno_face.cuh"
+// others.  The branch is evaluated with the face kernel's own expressions (eos64, sqrt0_64).
+#include "weno64.cuh"
 #include "weno_sweep.cuh"
 
 namespace gbmv {
@@ -18,7 +18,6 @@ namespace {
 template <int DIR>
 __device__ __forceinline__ int face_branch(const Grid& g, const Fields& w, const Fields& dw,
                                            double s, long i, long j, long k) {
-  const double gm = g.gamma - 1.0;
   double alpha = 0.0;
   int arg = 0, neg = 0;
 #pragma unroll
@@ -38,9 +37,9 @@ __device__ __forceinline__ int face_branch(const Grid& g, const Fields& w, const
       for (int f = 0; f < 5; ++f) v[f] = -v[f];
     }
     if (nnorm) v[1 + DIR] = -v[1 + DIR];
-    const double p = eos_t<double>(gm, v[0], v[1], v[2], v[3], v[4]);
+    const double p = eos64(g.gamma, v[0], v[1], v[2], v[3], v[4]);
     const double uj = v[1 + DIR] / v[0];
-    const double sp = fabs(uj) + sqrt0<double>(g.gamma * p / v[0]);
+    const double sp = fabs(uj) + sqrt0_64(g.gamma * p / v[0]);
     if (alpha < sp) {
       alpha = sp;
       arg = l;
