@@ -10,63 +10,12 @@
 // one tile's traffic with the others' arithmetic.  (Two-warp CTAs filling their tile with plain
 // loads, a few in flight, left the FP64 pipe 54 % busy in the factorisation and 20 % in the
 // solve: 192,000 blocks 286 and 164 us, now 172 and 64.)
+#include "block_tile.cuh"
 #include "chem.cuh"
+#include "chem_lu.cuh"
 #include "weno64.cuh"
 
 namespace gbmv {
-
-constexpr int kLuThreads = 32;   // blocks per tile = threads per CTA
-constexpr int kLuStride = 102;   // per-block stride of the shared tile (doubles): a multiple of 16
-                                 // bytes, and two-way bank conflicts at most
-constexpr int kVecStride = 11;   // the same for the right-hand-side tile
-
-// Copy of `nb` consecutive blocks of 100 doubles into the shared tile; waits for nothing.
-// 16-byte asynchronous copies where the address allows (caller arrays need only be 8-byte
-// aligned).
-__device__ __forceinline__ void tile_in_async(const double* __restrict__ g, double* sh, long blk0,
-                                              int nb) {
-  const double* src = g + blk0 * 100;
-  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    const unsigned base = (unsigned)__cvta_generic_to_shared(sh);
-#pragma unroll 10
-    for (int c = threadIdx.x; c < nb * 50; c += kLuThreads) {
-      const int b = c / 50, e = c - b * 50;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                       base + (unsigned)(b * (kLuStride * 8) + e * 16)),
-                   "l"(src + 2 * c)
-                   : "memory");
-    }
-  } else {
-    for (int c = threadIdx.x; c < nb * 100; c += kLuThreads)
-      sh[(c / 100) * kLuStride + c % 100] = src[c];
-  }
-}
-__device__ __forceinline__ void tile_in_wait() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncwarp();
-}
-__device__ __forceinline__ void tile_out(double* __restrict__ g, const double* sh, long blk0,
-                                         int nb) {
-  double* dst = g + blk0 * 100;
-  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll 10
-    for (int c = threadIdx.x; c < nb * 50; c += kLuThreads) {
-      const int b = c / 50, e = c - b * 50;
-      reinterpret_cast<double2*>(dst)[c] =
-          *reinterpret_cast<const double2*>(sh + b * kLuStride + 2 * e);
-    }
-  } else {
-    for (int c = threadIdx.x; c < nb * 100; c += kLuThreads)
-      dst[c] = sh[(c / 100) * kLuStride + c % 100];
-  }
-}
-
-// |x| as an ordered integer; NaN counts as 0, as a comparison with it is false.  (Comparisons of
-// doubles run on the FP64 pipe, which bounds the factorisation.)
-__device__ __forceinline__ unsigned long long abs_order(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
-  return b > 0x7ff0000000000000ULL ? 0ULL : b;
-}
 
 // One elimination step KK of LU with partial pivoting (first maximal |pivot|, full-row
 // interchange, the dgetf2 order), fully unrolled through template recursion so the block
@@ -75,12 +24,10 @@ __device__ __forceinline__ unsigned long long abs_order(double x) {
 template <int KK>
 __device__ __forceinline__ void lu_step(double (&A)[100], int (&piv)[10], int& info) {
   int p = KK;
-  // (a NaN diagonal keeps its place: no comparison with it is true)
-  unsigned long long amax =
-      (unsigned long long)__double_as_longlong(A[KK * 10 + KK]) & 0x7fffffffffffffffULL;
+  unsigned long long amax = pivot_size(A[KK * 10 + KK], true);
 #pragma unroll
   for (int r = KK + 1; r < 10; ++r) {
-    const unsigned long long v = abs_order(A[KK * 10 + r]);
+    const unsigned long long v = pivot_size(A[KK * 10 + r], false);
     if (v > amax) { amax = v; p = r; }
   }
   piv[KK] = p;

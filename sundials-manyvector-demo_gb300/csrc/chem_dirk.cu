@@ -70,7 +70,7 @@ __device__ __forceinline__ void dirk_F(const ChemParams& P, const ChemState& S, 
   double k[kNRates], dk[kNRates];
   literal::chem_rates<false>(P, Ts, k, dk);
   double r[21], sp[9];
-  chem_fluxes(k, ya, r);
+  literal::chem_fluxes(k, ya, r);
   literal::chem_species(r, sp);
   const ChemAux Ax{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
 #pragma unroll

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "df64.cuh"
+#include "weno64.cuh"
 
 namespace gbmv {
 
@@ -34,17 +35,30 @@ __device__ constexpr signed char kJacIndex[10][10] = {
     {-1, -1, -1, -1, -1, 38, 39, 40, 41, 42},  {-1, -1, -1, -1, -1, -1, 43, 44, 45, 46},
     {-1, 47, 48, 49, 50, 51, 52, 53, 54, 55},  {56, -1, 57, 58, -1, 59, 60, 61, 62, 63}};
 
+// |x| as an ordered number: comparisons of doubles run on the FP64 pipe, so those compare their
+// bits; a NaN counts as 0 (no comparison with it is true), a NaN diagonal as the largest.
+__device__ __forceinline__ float pivot_size(float x, bool) { return fabsf(x); }
+__device__ __forceinline__ unsigned long long pivot_size(double x, bool diagonal) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+  return !diagonal && b > 0x7ff0000000000000ULL ? 0ULL : b;
+}
+template <bool FAST>
+__device__ __forceinline__ float pivot_rcp(float d) { return 1.f / d; }
+template <bool FAST>
+__device__ __forceinline__ double pivot_rcp(double d) { return FAST ? rcp64_any(d) : 1.0 / d; }
+
 // In-place LU with partial pivoting on a strided per-thread slice A[e*stride] (column-major
-// 10x10), reciprocal pivots on the diagonal; returns 0 or 1 + first zero pivot.
-template <typename R>
+// 10x10), reciprocal pivots on the diagonal; returns 0 or 1 + first zero pivot.  FAST: FP64
+// reciprocals without the IEEE division (within an ulp of it).
+template <typename R, bool FAST = false>
 __device__ __forceinline__ int lu10_strided(R* A, int stride, int (&piv)[10]) {
   int info = 0;
 #pragma unroll 1
   for (int kk = 0; kk < 10; ++kk) {
     int p = kk;
-    R amax = fabs(A[(kk * 10 + kk) * stride]);
+    auto amax = pivot_size(A[(kk * 10 + kk) * stride], true);
     for (int r = kk + 1; r < 10; ++r) {
-      const R v = fabs(A[(kk * 10 + r) * stride]);
+      const auto v = pivot_size(A[(kk * 10 + r) * stride], false);
       if (v > amax) { amax = v; p = r; }
     }
     piv[kk] = p;
@@ -59,7 +73,7 @@ __device__ __forceinline__ int lu10_strided(R* A, int stride, int (&piv)[10]) {
       if (!info) info = kk + 1;
       continue;
     }
-    const R rp = R(1) / d;
+    const R rp = pivot_rcp<FAST>(d);
     A[(kk * 10 + kk) * stride] = rp;
     for (int r = kk + 1; r < 10; ++r) A[(kk * 10 + r) * stride] *= rp;
     for (int col = kk + 1; col < 10; ++col) {

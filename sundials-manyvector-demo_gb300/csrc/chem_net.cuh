@@ -222,32 +222,38 @@ __device__ __forceinline__ void chem_rates(const ChemParams& P, double logT, dou
   }
 }
 
-// The 21 reaction fluxes (rate times reactant product).
-__device__ __forceinline__ void chem_fluxes(const double (&k)[kNRates], const double (&y)[10],
-                                            double (&r)[21]) {
+// The reactant products of the 21 reactions; a flux is its rate times one of them.
+__device__ __forceinline__ void chem_products(const double (&y)[10], double (&p)[21]) {
   const double H2_1 = y[0], H2_2 = y[1], H_1 = y[2], H_2 = y[3], H_m0 = y[4], He_1 = y[5],
                He_2 = y[6], He_3 = y[7], de = y[8];
-  r[0] = k[K01] * H_1 * de;
-  r[1] = k[K02] * H_2 * de;
-  r[2] = k[K03] * He_1 * de;
-  r[3] = k[K04] * He_2 * de;
-  r[4] = k[K05] * He_2 * de;
-  r[5] = k[K06] * He_3 * de;
-  r[6] = k[K07] * H_1 * de;
-  r[7] = k[K08] * H_1 * H_m0;
-  r[8] = k[K09] * H_1 * H_2;
-  r[9] = k[K10] * H2_2 * H_1;
-  r[10] = k[K11] * H2_1 * H_2;
-  r[11] = k[K12] * H2_1 * de;
-  r[12] = k[K13] * H2_1 * H_1;
-  r[13] = k[K14] * H_m0 * de;
-  r[14] = k[K15] * H_1 * H_m0;
-  r[15] = k[K16] * H_2 * H_m0;
-  r[16] = k[K17] * H_2 * H_m0;
-  r[17] = k[K18] * H2_2 * de;
-  r[18] = k[K19] * H2_2 * H_m0;
-  r[19] = k[K21] * H2_1 * H_1 * H_1;
-  r[20] = k[K22] * H_1 * H_1 * H_1;
+  p[0] = H_1 * de;
+  p[1] = H_2 * de;
+  p[2] = He_1 * de;
+  p[3] = He_2 * de;
+  p[4] = p[3];
+  p[5] = He_3 * de;
+  p[6] = p[0];
+  p[7] = H_1 * H_m0;
+  p[8] = H_1 * H_2;
+  p[9] = H2_2 * H_1;
+  p[10] = H2_1 * H_2;
+  p[11] = H2_1 * de;
+  p[12] = H2_1 * H_1;
+  p[13] = H_m0 * de;
+  p[14] = p[7];
+  p[15] = H_2 * H_m0;
+  p[16] = p[15];
+  p[17] = H2_2 * de;
+  p[18] = H2_2 * H_m0;
+  p[19] = p[12] * H_1;
+  p[20] = H_1 * H_1 * H_1;
+}
+// rate table row of each reaction
+__device__ __forceinline__ void chem_fluxes(const double (&k)[kNRates], const double (&p)[21],
+                                            double (&r)[21]) {
+  static_assert(K01 == 0 && K19 == 18 && K21 == 19 && K22 == 20, "rates in reaction order");
+#pragma unroll
+  for (int m = 0; m < 21; ++m) r[m] = k[m] * p[m];
 }
 
 // Net species sources from reaction fluxes (net stoichiometry).
@@ -304,23 +310,146 @@ __device__ __forceinline__ double chem_ge_source(const ChemParams& P, const doub
   return 0.5 * (t.N * t.i2) * t.Hf - A.cie * (H2_1 * h2 + de * L);
 }
 
+// The ge row of the Jacobian by H2_1, H_1, H_2, He_1, He_2, He_3, de (over rho, without
+// 1/mdensity) and by ge (without dT/dge idbin / T).
+struct GeRow {
+  double d0, d2, d3, d5, d6, d7, d8, d9;
+};
+__device__ __forceinline__ void ge_row(const ChemParams& P, const double (&k)[kNRates],
+                                       const double (&dk)[kNRates], const double (&y)[10],
+                                       double T, double h2oda, double md, const GeTerms& t,
+                                       GeRow& g) {
+  const double H2_1 = y[0], H_1 = y[2], H_2 = y[3], He_1 = y[5], He_2 = y[6], He_3 = y[7],
+               de = y[8];
+  const double H1sq = H_1 * H_1;
+  // With D = h2lte / G + 1 and F = ncrn / N + 1 every quotient of the ge row is in G, N and the
+  // two reciprocals: 1/D = G i1, 1/(D G) = i1, 1/F = N i2, 1/(F N) = i2.
+  const double iF = t.N * t.i2, i1h = t.i1 * t.i1 * h2oda, i22 = t.i2 * t.i2;
+  const double lteh = k[H2LTE] * k[H2LTE] * i1h;  // h2lte^2 h2oda / (D G)^2
+  const double hlteh = H2_1 * lteh;
+  const double nf = 0.5 * k[NCRN] * i22 * t.Hf;
+  const double chi = k[CEHI] + k[CIHI], h2c = k[CEHEII] + k[CIHEII] + k[REHEII1] + k[REHEII2],
+               h2d = k[CEHEI] + k[CIHEIS], bd = k[BREM] * de;
+  g.d0 = (nf * k[NCRD2] - k[GAH2] * hlteh - 0.5 * H_1 * k[H2MCOOL] * iF -
+              2.01588 * k[CIECO] * md - k[H2LTE] * h2oda * (t.G * t.i1));
+  g.d2 = (nf * k[NCRD1] - k[GAHI] * hlteh - chi * de +
+              0.5 * (3 * H1sq * k[H2MHEAT] - H2_1 * k[H2MCOOL]) * iF);
+  g.d3 = (-k[GAHP] * hlteh - bd - de * k[REHII]);
+  g.d5 = (-k[GAHE] * hlteh - k[CIHEI] * de);
+  g.d6 = (-bd - de * (h2c + h2d * de));
+  g.d7 = (-4.0 * bd - de * k[REHEIII]);
+  g.d8 = (-k[GAEL] * hlteh - H_1 * chi - H_2 * k[REHII] - He_1 * k[CIHEI] -
+              He_2 * (h2c + 2 * h2d * de) - He_3 * k[REHEIII] -
+              k[BREM] * (H_2 + He_2 + 4.0 * He_3) -
+              k[COMPTON] * P.zp1_4 * (T - (2.73 * P.z + 2.73)));
+  const double dG = H2_1 * dk[GAH2] + H_1 * dk[GAHI] + H_2 * dk[GAHP] + He_1 * dk[GAHE] +
+                    de * dk[GAEL];
+  const double dN = H2_1 * dk[NCRD2] + H_1 * dk[NCRD1];
+  // d/dT of -H2 h2oda h2lte / D and of Hf / (2 F)
+  const double gg = 0.5 * (k[NCRN] * dN - dk[NCRN] * t.N) * i22 * t.Hf +
+                    0.5 * iF * (t.H13 * dk[H2MHEAT] - H2_1 * H_1 * dk[H2MCOOL]) -
+                    H2_1 * (k[H2LTE] * (k[H2LTE] * dG - t.G * dk[H2LTE]) * i1h +
+                            h2oda * dk[H2LTE] * (t.G * t.i1));
+  g.d9 = gg;
+}
+
+// The Newton matrix's part of the Jacobian with every column multiplied by its own variable:
+// put(row, col, v), v = J(row, col) y_col in physical units, without the ge row's 1/mdensity and
+// the ge column's dT/dge idbin / T y_9.  A flux's derivative by a reactant times that reactant is
+// the flux times its order, so the species entries are sums of the fluxes r (no products), and
+// scaling by the Dengo scale and unscaling cancel in them.
+template <class Put>
+__device__ __forceinline__ void chem_matrix(const ChemParams& P, const double (&k)[kNRates],
+                                            const double (&dk)[kNRates], const double (&y)[10],
+                                            const double (&pr)[21], const double (&r)[21],
+                                            double T, const ChemAux& A, const GeTerms& t,
+                                            Put&& put) {
+  const double H2_1 = y[0], H_1 = y[2], H_2 = y[3], He_1 = y[5], He_2 = y[6], He_3 = y[7],
+               de = y[8];
+  const double h2oda = A.h2, md = A.mdens;
+  const double r1516 = r[15] + r[16], r714 = r[7] + r[14], r1314 = r[13] + r[14],
+               r01 = r[0] - r[1], r23 = r[2] - r[3], r45 = r[4] - r[5], r918 = r[9] + r[18];
+  put(0, 0, r[19] - r[10] - r[11] - r[12]);
+  put(0, 1, r918);
+  put(0, 2, fma(3.0, r[20], fma(2.0, r[19], r[7] + r[9] - r[12])));
+  put(0, 3, -r[10]);
+  put(0, 4, r[7] + r[18]);
+  put(0, 8, -r[11]);
+  put(1, 0, r[10]);
+  put(1, 1, -r918 - r[17]);
+  put(1, 2, r[8] - r[9]);
+  put(1, 3, r[8] + r[10] + r[16]);
+  put(1, 4, r[16] - r[18]);
+  put(1, 8, -r[17]);
+  put(2, 0, fma(2.0, r[11] + r[12] - r[19], r[10]));
+  put(2, 1, fma(2.0, r[17], r[18] - r[9]));
+  put(2, 2, fma(-6.0, r[20], fma(-4.0, r[19], fma(2.0, r[12], r[14] - r[7] - r[8] - r[9] - r[0] -
+                                                               r[6]))));
+  put(2, 3, fma(2.0, r[15], r[1] - r[8] + r[10]));
+  put(2, 4, fma(2.0, r[15], r1314 - r[7] + r[18]));
+  put(2, 8, fma(2.0, r[11] + r[17], r[13] - r01 - r[6]));
+  put(3, 0, -r[10]);
+  put(3, 1, r[9]);
+  put(3, 2, r[0] - r[8] + r[9]);
+  put(3, 3, -r[1] - r[8] - r[10] - r1516);
+  put(3, 4, -r1516);
+  put(3, 8, r01);
+  put(4, 1, -r[18]);
+  put(4, 2, r[6] - r714);
+  put(4, 3, -r1516);
+  put(4, 4, -r[7] - r1314 - r1516 - r[18]);
+  put(4, 8, r[6] - r[13]);
+  put(5, 5, -r[2]);
+  put(5, 6, r[3]);
+  put(5, 8, -r23);
+  put(6, 5, r[2]);
+  put(6, 6, -r[3] - r[4]);
+  put(6, 7, r[5]);
+  put(6, 8, r23 - r45);
+  put(7, 6, r[4]);
+  put(7, 7, -r[5]);
+  put(7, 8, r45);
+  put(8, 1, -r[17]);
+  put(8, 2, r[0] - r[6] + r714);
+  put(8, 3, r[16] - r[1]);
+  put(8, 4, r[7] + r1314 + r[16]);
+  put(8, 5, r[2]);
+  put(8, 6, r[4] - r[3]);
+  put(8, 7, -r[5]);
+  put(8, 8, r01 + r23 + r45 - r[6] + r[13] - r[17]);
+  {  // species rows by ge: sources with rates replaced by their bin differences
+    double q[21], s[9];
+    chem_fluxes(dk, pr, q);
+    chem_species(q, s);
+#pragma unroll
+    for (int m = 0; m < 9; ++m) put(m, 9, s[m]);
+  }
+  GeRow g;
+  ge_row(P, k, dk, y, T, h2oda, md, t, g);
+  put(9, 0, g.d0 * H2_1);
+  put(9, 2, g.d2 * H_1);
+  put(9, 3, g.d3 * H_2);
+  put(9, 5, g.d5 * He_1);
+  put(9, 6, g.d6 * He_2);
+  put(9, 7, g.d7 * He_3);
+  put(9, 8, g.d8 * de);
+  put(9, 9, g.d9);
+}
+
 // Analytic Jacobian in physical units, before the inv_scale*scale and time-unit factors;
 // rates k and bin differences dk (chem_rates) at the cell temperature.  Each of the 64 nonzeros is handed to
 // put(row, col, value) once, already multiplied by the factors the reference applies to that
 // entry (1/mdensity on the ge row, dT/dge on the ge column); entries never put are zero.
-// Raw: the ge row's factor and the ge column's, with the idbin / T of the slopes, are left out,
-// for a caller that folds them into its own row and column scaling (one multiply per cell
-// instead of one per entry); else Tge holds dT/dge times idbin / T.
-template <bool Raw = false, class Put>
+// Tge: dT/dge times idbin / T.
+template <class Put>
 __device__ __forceinline__ void chem_jacobian(const ChemParams& P, const double (&k)[kNRates],
                                               const double (&dk)[kNRates], const double (&y)[10],
-                                              double T, double Tge, const ChemAux& A,
-                                              const GeTerms& t, Put&& put) {
+                                              const double (&pr)[21], double T, double Tge,
+                                              const ChemAux& A, const GeTerms& t, Put&& put) {
   const double H2_1 = y[0], H2_2 = y[1], H_1 = y[2], H_2 = y[3], H_m0 = y[4], He_1 = y[5],
                He_2 = y[6], He_3 = y[7], de = y[8];
-  const double z = P.z, h2oda = A.h2, md = A.mdens, imd = A.imdens;
+  const double h2oda = A.h2, md = A.mdens, imd = A.imdens;
 #define SETJ(row, col, expr) put(row, col, (expr))
-#define SETG(col, expr) put(9, col, Raw ? (expr) : (expr) * imd)
   const double H1sq = H_1 * H_1;
   SETJ(0, 0, -k[K11] * H_2 - k[K12] * de - k[K13] * H_1 + k[K21] * H1sq);
   SETJ(0, 1, k[K10] * H_1 + k[K19] * H_m0);
@@ -376,41 +505,21 @@ __device__ __forceinline__ void chem_jacobian(const ChemParams& P, const double 
                  k[K06] * He_3 - k[K07] * H_1 + k[K14] * H_m0 - k[K18] * H2_2);
   {  // species rows by ge: sources with rates replaced by slopes, times dT/dge
     double r[21], s[9];
-    chem_fluxes(dk, y, r);
+    chem_fluxes(dk, pr, r);
     chem_species(r, s);
 #pragma unroll
-    for (int q = 0; q < 9; ++q) put(q, 9, Raw ? s[q] : s[q] * Tge);
+    for (int q = 0; q < 9; ++q) put(q, 9, s[q] * Tge);
   }
-  // With D = h2lte / G + 1 and F = ncrn / N + 1 every quotient of the ge row is in G, N and the
-  // two reciprocals: 1/D = G i1, 1/(D G) = i1, 1/F = N i2, 1/(F N) = i2.
-  const double iF = t.N * t.i2, i1h = t.i1 * t.i1 * h2oda, i22 = t.i2 * t.i2;
-  const double lteh = k[H2LTE] * k[H2LTE] * i1h;  // h2lte^2 h2oda / (D G)^2
-  const double hlteh = H2_1 * lteh;
-  const double nf = 0.5 * k[NCRN] * i22 * t.Hf;
-  const double chi = k[CEHI] + k[CIHI], h2c = k[CEHEII] + k[CIHEII] + k[REHEII1] + k[REHEII2],
-               h2d = k[CEHEI] + k[CIHEIS], bd = k[BREM] * de;
-  SETG(0, nf * k[NCRD2] - k[GAH2] * hlteh - 0.5 * H_1 * k[H2MCOOL] * iF -
-              2.01588 * k[CIECO] * md - k[H2LTE] * h2oda * (t.G * t.i1));
-  SETG(2, nf * k[NCRD1] - k[GAHI] * hlteh - chi * de +
-              0.5 * (3 * H1sq * k[H2MHEAT] - H2_1 * k[H2MCOOL]) * iF);
-  SETG(3, -k[GAHP] * hlteh - bd - de * k[REHII]);
-  SETG(5, -k[GAHE] * hlteh - k[CIHEI] * de);
-  SETG(6, -bd - de * (h2c + h2d * de));
-  SETG(7, -4.0 * bd - de * k[REHEIII]);
-  SETG(8, -k[GAEL] * hlteh - H_1 * chi - H_2 * k[REHII] - He_1 * k[CIHEI] -
-              He_2 * (h2c + 2 * h2d * de) - He_3 * k[REHEIII] -
-              k[BREM] * (H_2 + He_2 + 4.0 * He_3) -
-              k[COMPTON] * P.zp1_4 * (T - (2.73 * z + 2.73)));
-  const double dG = H2_1 * dk[GAH2] + H_1 * dk[GAHI] + H_2 * dk[GAHP] + He_1 * dk[GAHE] +
-                    de * dk[GAEL];
-  const double dN = H2_1 * dk[NCRD2] + H_1 * dk[NCRD1];
-  // d/dT of -H2 h2oda h2lte / D and of Hf / (2 F)
-  const double gg = 0.5 * (k[NCRN] * dN - dk[NCRN] * t.N) * i22 * t.Hf +
-                    0.5 * iF * (t.H13 * dk[H2MHEAT] - H2_1 * H_1 * dk[H2MCOOL]) -
-                    H2_1 * (k[H2LTE] * (k[H2LTE] * dG - t.G * dk[H2LTE]) * i1h +
-                            h2oda * dk[H2LTE] * (t.G * t.i1));
-  put(9, 9, Raw ? gg : gg * imd * Tge);
-#undef SETG
+  GeRow g;
+  ge_row(P, k, dk, y, T, h2oda, md, t, g);
+  put(9, 0, g.d0 * imd);
+  put(9, 2, g.d2 * imd);
+  put(9, 3, g.d3 * imd);
+  put(9, 5, g.d5 * imd);
+  put(9, 6, g.d6 * imd);
+  put(9, 7, g.d7 * imd);
+  put(9, 8, g.d8 * imd);
+  put(9, 9, g.d9 * imd * Tge);
 #undef SETJ
 }
 

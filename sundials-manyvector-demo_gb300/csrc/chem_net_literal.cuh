@@ -166,6 +166,34 @@ __device__ __forceinline__ void chem_rates(const ChemParams& P, double Ts, doubl
   }
 }
 
+// The 21 reaction fluxes (rate times reactant product).
+__device__ __forceinline__ void chem_fluxes(const double (&k)[kNRates], const double (&y)[10],
+                                            double (&r)[21]) {
+  const double H2_1 = y[0], H2_2 = y[1], H_1 = y[2], H_2 = y[3], H_m0 = y[4], He_1 = y[5],
+               He_2 = y[6], He_3 = y[7], de = y[8];
+  r[0] = k[K01] * H_1 * de;
+  r[1] = k[K02] * H_2 * de;
+  r[2] = k[K03] * He_1 * de;
+  r[3] = k[K04] * He_2 * de;
+  r[4] = k[K05] * He_2 * de;
+  r[5] = k[K06] * He_3 * de;
+  r[6] = k[K07] * H_1 * de;
+  r[7] = k[K08] * H_1 * H_m0;
+  r[8] = k[K09] * H_1 * H_2;
+  r[9] = k[K10] * H2_2 * H_1;
+  r[10] = k[K11] * H2_1 * H_2;
+  r[11] = k[K12] * H2_1 * de;
+  r[12] = k[K13] * H2_1 * H_1;
+  r[13] = k[K14] * H_m0 * de;
+  r[14] = k[K15] * H_1 * H_m0;
+  r[15] = k[K16] * H_2 * H_m0;
+  r[16] = k[K17] * H_2 * H_m0;
+  r[17] = k[K18] * H2_2 * de;
+  r[18] = k[K19] * H2_2 * H_m0;
+  r[19] = k[K21] * H2_1 * H_1 * H_1;
+  r[20] = k[K22] * H_1 * H_1 * H_1;
+}
+
 // Net species sources from reaction fluxes (net stoichiometry, reaction order).
 __device__ __forceinline__ void chem_species(const double (&r)[21], double (&s)[9]) {
   s[0] = r[7] + r[9] - r[10] - r[11] - r[12] + r[18] + r[19] + r[20];

@@ -23,6 +23,38 @@ namespace gbmv {
 // seven blocks (seven warps) fit an SM, against six with 64-thread blocks.
 constexpr int kNtThreads = 32;
 
+// entry (row, col) of the Newton matrix: FP32-LU form to the FP64 pattern, FP64 form to the factor
+template <typename LU, int BS>
+__device__ __forceinline__ void put_entry(double* As, LU* L, int row, int col, double a) {
+  if (sizeof(LU) == 4) {
+    const int e = kJacIndex[row][col];
+    if (e >= 0) As[e * BS] = a;
+  } else {
+    L[(col * 10 + row) * BS] = to_lu<LU>(a);
+  }
+}
+
+// The Newton matrix without the column scaling (a rare path): every entry from its own expression
+template <typename LU, int BS>
+static __device__ __noinline__ void newton_matrix_plain(const ChemParams& P, const ChemState& S,
+                                                        long i, const double* __restrict__ y,
+                                                        double T, double dT, double gt, double* As,
+                                                        LU* L) {
+  const long j = i * 10;
+  double ya[10], pr[21], k[kNRates], dk[kNRates];
+#pragma unroll
+  for (int s = 0; s < 10; ++s) ya[s] = y[j + s] * S.scale[j + s];
+  chem_rates<true>(P, log(T), k, dk);
+  chem_products(ya, pr);
+  const ChemAux A{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
+  chem_jacobian(P, k, dk, ya, pr, T, dT * (P.idbin * rcp64_any(T)), A, ge_terms(k, ya),
+                [&](int row, int col, double v) {
+                  put_entry<LU, BS>(As, L, row, col,
+                                    (v * (-gt * S.inv_scale[j + row])) * S.scale[j + col] +
+                                        (row == col ? 1.0 : 0.0));
+                });
+}
+
 template <typename LU, int BS>
 __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState S, long n,
                                                          const double* __restrict__ y,
@@ -74,13 +106,24 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       S.dTs_ge[i] = dTs;
       const ChemAux Ax{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
       double f[10];
+      // The matrix is formed with every column multiplied by its own variable, A diag(z): its
+      // species entries are then plain sums of the reaction fluxes (chem_matrix), and partial
+      // pivoting, which compares within a column, picks the same rows.  The solution is z times
+      // that system's.  Variables that are zero or far from 1 take the unscaled matrix.
+      bool scaled = true;
+#pragma unroll
+      for (int s = 0; s < 10; ++s) {
+        const int e = (__double2hiint(y[j + s]) >> 20) & 0x7FF;
+        scaled = scaled && (unsigned)(e - (1023 - 99)) <= 198u;
+      }
       {  // source and Newton matrix from one rate evaluation (rates and T slopes)
-        double k[kNRates], dk[kNRates];
+        double k[kNRates], dk[kNRates], pr[21], r[21];
         chem_rates<true>(P, logT, k, dk);
         const GeTerms Rg = ge_terms(k, ya);  // shared by the source and the Jacobian's ge row
+        chem_products(ya, pr);
+        chem_fluxes(k, pr, r);
         {
-          double r[21], sp[9];
-          chem_fluxes(k, ya, r);
+          double sp[9];
           chem_species(r, sp);
 #pragma unroll
           for (int s = 0; s < 9; ++s) f[s] = (sp[s] * isc[s]) * tunit;
@@ -90,25 +133,22 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
         }
 #pragma unroll
         for (int s = 0; s < 10; ++s) fout[j + s] = f[s];
-        // A = I - gamma * (J * inv_scale[row] * scale[col] * tunit), FP64 and a float copy;
-        // the ge row's 1/mdensity and the ge column's dT/dge ride on the row and column factors
-        double rf[10];  // -gamma * tunit * inv_scale[row]
-#pragma unroll
-        for (int r = 0; r < 10; ++r) rf[r] = (-gamma * tunit) * isc[r];
-        rf[9] *= Ax.imdens;
-        const double sc9 = sc[9] * dTs * (P.idbin * rcp64_any(Ts));
 #pragma unroll
         for (int e = 0; e < 100; ++e) L[e * BS] = LU(0);  // structural zeros
-        // every structural entry (the diagonal included) is put exactly once
-        chem_jacobian<true>(P, k, dk, ya, Ts, dTs, Ax, Rg, [&](int row, int col, double v) {
-          const double a = (v * rf[row]) * (col == 9 ? sc9 : sc[col]) + (row == col ? 1.0 : 0.0);
-          if (kMixed) {
-            const int e = kJacIndex[row][col];
-            if (e >= 0) As[e * BS] = a;
-          } else {
-            L[(col * 10 + row) * BS] = to_lu<LU>(a);
-          }
-        });
+        if (scaled) {
+          double rf[10];  // -gamma * tunit * inv_scale[row], the ge row's 1/mdensity with it
+#pragma unroll
+          for (int q = 0; q < 10; ++q) rf[q] = (-gamma * tunit) * isc[q];
+          rf[9] *= Ax.imdens;
+          const double t9 = dTs * (P.idbin * rcp64_any(Ts)) * ya[9];
+          // every structural entry (the diagonal included) is put exactly once
+          chem_matrix(P, k, dk, ya, pr, r, Ts, Ax, Rg, [&](int row, int col, double v) {
+            const double u = col == 9 ? v * t9 : v;
+            put_entry<LU, BS>(As, L, row, col, row == col ? fma(u, rf[row], y[j + row]) : u * rf[row]);
+          });
+        } else {
+          newton_matrix_plain<LU, BS>(P, S, i, y, Ts, dTs, gamma * tunit, As, L);
+        }
         if constexpr (kMixed) {  // the FP32 factor's entries, converted with integer
           // instructions after the Jacobian (off the FP64 pipe, which bounds this kernel, and off
           // the Jacobian's dependency chains: 5.45 -> 5.34 ms per 128^3 call; converting inside
@@ -131,7 +171,12 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       // these matrices it changes the pivot order for the worse -- 2.4e-3 against 1.9e-8 after
       // one refinement on the test blocks, reproduced on the oracle's matrices -- so the factor
       // keeps plain partial pivoting.)
-      int info = lu10_strided<LU>(L, BS, piv);
+      float zf[10];  // z for the stopping tests, which are on x
+      if (sizeof(LU) == 4) {
+#pragma unroll
+        for (int s = 0; s < 10; ++s) zf[s] = scaled ? f32_of_f64(y[j + s]) : 1.f;
+      }
+      int info = lu10_strided<LU, true>(L, BS, piv);
       bool fp64_fallback = (sizeof(LU) == 4) && info != 0;
       if (!fp64_fallback) {
         LU xs[10];
@@ -143,7 +188,7 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
 #pragma unroll
         for (int s = 0; s < 10; ++s) {
           x[s] = from_lu(xs[s]);
-          xmax = fmaxf(xmax, fabsf((float)xs[s]));
+          xmax = fmaxf(xmax, fabsf((float)xs[s] * zf[s]));
         }
         if (sizeof(LU) == 4) {
           // iterative refinement against FP64 residuals; a cell stops as soon as its correction
@@ -167,7 +212,7 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
 #pragma unroll
             for (int s = 0; s < 10; ++s) {
               x[s] += from_lu(ds[s]);
-              dmax = fmaxf(dmax, fabsf((float)ds[s]));
+              dmax = fmaxf(dmax, fabsf((float)ds[s] * zf[s]));
             }
             dlast = dmax;
             if (dmax <= 1e-13f * xmax) break;
@@ -183,14 +228,14 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
         double Ad[100];
         for (int e = 0; e < 100; ++e) Ad[e] = 0.0;
         for (int e = 0; e < 64; ++e) Ad[kJacPattern[e][1] * 10 + kJacPattern[e][0]] = As[e * BS];
-        info = lu10_strided<double>(Ad, 1, piv);
+        info = lu10_strided<double, true>(Ad, 1, piv);
 #pragma unroll
         for (int s = 0; s < 10; ++s) x[s] = f[s];
         lus10_strided<double, double>(Ad, 1, piv, x);
       }
       if (info && (sizeof(LU) == 8 || fp64_fallback)) bad = 1;
 #pragma unroll
-      for (int s = 0; s < 10; ++s) xout[j + s] = x[s];
+      for (int s = 0; s < 10; ++s) xout[j + s] = scaled ? x[s] * y[j + s] : x[s];
     }
     if (!queue) i += stride;
   }

@@ -4,9 +4,18 @@
 
 namespace gbmv {
 
-constexpr int kF2MinB = 3;
+#ifndef KF2
+#define KF2 3
+#endif
+#ifndef KTR
+#define KTR 6
+#endif
+#ifndef KTR0
+#define KTR0 5
+#endif
+constexpr int kF2MinB = KF2;
 constexpr int kF2SharedMinB = 5;
-constexpr int kTracerMinB = 5;
+constexpr int kTracerMinB = KTR;
 
 __global__ void __launch_bounds__(256) prims_f2_kernel(Grid g, Fields w, float2* __restrict__ Q2,
                                                        const double* __restrict__ tscale,
@@ -190,7 +199,7 @@ __global__ void __launch_bounds__(128, MINB)
 // Tracer face fluxes: one thread a face, its tracers one after the other; reads half the
 // Lax-Friedrichs speed that the fluid sweep left in the first tracer's flux.
 template <int WV>
-__global__ void __launch_bounds__(128, WV == 1 ? kTracerMinB : 2)
+__global__ void __launch_bounds__(128, WV == 1 ? kTracerMinB : KTR0)
     tracer_flux_f2_kernel(const __grid_constant__ SweepSet S, const float2* __restrict__ Q2,
                           long n, int nchem) {
   const int dir = sweep_dir(S);
