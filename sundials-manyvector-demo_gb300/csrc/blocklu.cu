@@ -17,54 +17,6 @@
 
 namespace gbmv {
 
-// One elimination step KK of LU with partial pivoting (first maximal |pivot|, full-row
-// interchange, the dgetf2 order), fully unrolled through template recursion so the block
-// stays in registers.  The factor keeps 1/U(k,k) on the diagonal (the solve only multiplies);
-// the factored matrix is private to this solver, as MAGMA's is to its own getrs.
-template <int KK>
-__device__ __forceinline__ void lu_step(double (&A)[100], int (&piv)[10], int& info) {
-  int p = KK;
-  unsigned long long amax = pivot_size(A[KK * 10 + KK], true);
-#pragma unroll
-  for (int r = KK + 1; r < 10; ++r) {
-    const unsigned long long v = pivot_size(A[KK * 10 + r], false);
-    if (v > amax) { amax = v; p = r; }
-  }
-  piv[KK] = p;
-#pragma unroll
-  for (int r = KK + 1; r < 10; ++r) {
-    const bool sw = (r == p);
-#pragma unroll
-    for (int col = 0; col < 10; ++col) {
-      const double a = A[col * 10 + KK], b = A[col * 10 + r];
-      A[col * 10 + KK] = sw ? b : a;
-      A[col * 10 + r] = sw ? a : b;
-    }
-  }
-  const double d = A[KK * 10 + KK];
-  if ((__double_as_longlong(d) & 0x7fffffffffffffffLL) == 0) {
-    if (!info) info = KK + 1;
-  } else {
-    const double rp = rcp64_any(d);
-    A[KK * 10 + KK] = rp;
-#pragma unroll
-    for (int r = KK + 1; r < 10; ++r) A[KK * 10 + r] *= rp;
-#pragma unroll
-    for (int col = KK + 1; col < 10; ++col) {
-      const double a = A[col * 10 + KK];
-#pragma unroll
-      for (int r = KK + 1; r < 10; ++r) A[col * 10 + r] -= A[KK * 10 + r] * a;
-    }
-  }
-  if constexpr (KK < 9) lu_step<KK + 1>(A, piv, info);
-}
-
-__device__ __forceinline__ int lu10_regs(double (&A)[100], int (&piv)[10]) {
-  int info = 0;
-  lu_step<0>(A, piv, info);
-  return info;
-}
-
 // Solve with the factor of lu10_regs (row interchanges, unit-lower forward substitution,
 // upper back substitution multiplying by the stored reciprocal pivots).
 __device__ __forceinline__ void lus10(const double* __restrict__ A, const int (&piv)[10],

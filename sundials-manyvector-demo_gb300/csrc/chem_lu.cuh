@@ -110,4 +110,78 @@ __device__ __forceinline__ void lus10_strided(const R* A, int stride, const int 
   }
 }
 
+// One elimination step KK of LU with partial pivoting (first maximal |pivot|, full-row
+// interchange, the dgetf2 order), fully unrolled through template recursion so the block
+// stays in registers.  The factor keeps 1/U(k,k) on the diagonal (the solve only multiplies);
+// the factored matrix is private to this solver, as MAGMA's is to its own getrs.
+template <int KK, typename R>
+__device__ __forceinline__ void lu_step(R (&A)[100], int (&piv)[10], int& info) {
+  int p = KK;
+  auto amax = pivot_size(A[KK * 10 + KK], true);
+#pragma unroll
+  for (int r = KK + 1; r < 10; ++r) {
+    const auto v = pivot_size(A[KK * 10 + r], false);
+    if (v > amax) { amax = v; p = r; }
+  }
+  piv[KK] = p;
+#pragma unroll
+  for (int r = KK + 1; r < 10; ++r) {
+    const bool sw = (r == p);
+#pragma unroll
+    for (int col = 0; col < 10; ++col) {
+      const R a = A[col * 10 + KK], b = A[col * 10 + r];
+      A[col * 10 + KK] = sw ? b : a;
+      A[col * 10 + r] = sw ? a : b;
+    }
+  }
+  const R d = A[KK * 10 + KK];
+  if (pivot_size(d, true) == 0) {
+    if (!info) info = KK + 1;
+  } else {
+    const R rp = pivot_rcp<true>(d);
+    A[KK * 10 + KK] = rp;
+#pragma unroll
+    for (int r = KK + 1; r < 10; ++r) A[KK * 10 + r] *= rp;
+#pragma unroll
+    for (int col = KK + 1; col < 10; ++col) {
+      const R a = A[col * 10 + KK];
+#pragma unroll
+      for (int r = KK + 1; r < 10; ++r) A[col * 10 + r] -= A[KK * 10 + r] * a;
+    }
+  }
+  if constexpr (KK < 9) lu_step<KK + 1>(A, piv, info);
+}
+
+template <typename R>
+__device__ __forceinline__ int lu10_regs(R (&A)[100], int (&piv)[10]) {
+  int info = 0;
+  lu_step<0>(A, piv, info);
+  return info;
+}
+
+// Solve with a factor held in registers (lu10_regs).
+template <typename R>
+__device__ __forceinline__ void lus10_regs(const R (&A)[100], const int (&piv)[10], R (&x)[10]) {
+#pragma unroll
+  for (int kk = 0; kk < 10; ++kk) {
+#pragma unroll
+    for (int r = kk + 1; r < 10; ++r) {
+      const bool sw = (r == piv[kk]);
+      const R a = x[kk], b = x[r];
+      x[kk] = sw ? b : a;
+      x[r] = sw ? a : b;
+    }
+  }
+#pragma unroll
+  for (int col = 0; col < 10; ++col)
+#pragma unroll
+    for (int r = col + 1; r < 10; ++r) x[r] -= A[col * 10 + r] * x[col];
+#pragma unroll
+  for (int col = 9; col >= 0; --col) {
+    x[col] *= A[col * 10 + col];
+#pragma unroll
+    for (int r = 0; r < col; ++r) x[r] -= A[col * 10 + r] * x[col];
+  }
+}
+
 }  // namespace gbmv

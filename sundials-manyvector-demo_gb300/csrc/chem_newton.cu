@@ -18,10 +18,19 @@
 namespace gbmv {
 
 // Threads per block.  Shared memory per cell: the FP32-LU form keeps the 64 structural
-// nonzeros of the FP64 Newton matrix (for the refinement residuals) and the 100-entry FP32
-// factor, 912 bytes; the FP64-LU form only its 100-entry FP64 factor.  With 32-thread blocks
-// seven blocks (seven warps) fit an SM, against six with 64-thread blocks.
+// nonzeros of the FP64 Newton matrix (for the refinement residuals) and the variables, 592 bytes; the FP64-LU form
+// its 100 entries until they are factored.  With 32-thread blocks eight fit an SM, the register
+// limit.
 constexpr int kNtThreads = 32;
+
+// The cell's scaled variables are kept in its shared-memory slice (f may be written over y):
+// after the FP64 matrix entries in the FP32-LU form, in ten places of the FP64 form's matrix
+// that are structurally zero (column-major rows 4-8 of column 0, 5-7 and 9 of column 1, 5 of 2).
+__device__ constexpr int kZeroSlot[10] = {4, 5, 6, 7, 8, 15, 16, 17, 19, 25};
+template <typename LU>
+__device__ __forceinline__ constexpr int z_slot(int s) {
+  return sizeof(LU) == 4 ? 64 + s : kZeroSlot[s];
+}
 
 // entry (row, col) of the Newton matrix: FP32-LU form to the FP64 pattern, FP64 form to the factor
 template <typename LU, int BS>
@@ -37,13 +46,12 @@ __device__ __forceinline__ void put_entry(double* As, LU* L, int row, int col, d
 // The Newton matrix without the column scaling (a rare path): every entry from its own expression
 template <typename LU, int BS>
 static __device__ __noinline__ void newton_matrix_plain(const ChemParams& P, const ChemState& S,
-                                                        long i, const double* __restrict__ y,
-                                                        double T, double dT, double gt, double* As,
-                                                        LU* L) {
+                                                        long i, double T, double dT, double gt,
+                                                        double* As, LU* L) {
   const long j = i * 10;
   double ya[10], pr[21], k[kNRates], dk[kNRates];
 #pragma unroll
-  for (int s = 0; s < 10; ++s) ya[s] = y[j + s] * S.scale[j + s];
+  for (int s = 0; s < 10; ++s) ya[s] = As[z_slot<LU>(s) * BS] * S.scale[j + s];
   chem_rates<true>(P, log(T), k, dk);
   chem_products(ya, pr);
   const ChemAux A{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
@@ -67,10 +75,9 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
                                                          unsigned long long* __restrict__ queue) {
   extern __shared__ unsigned char smem_raw[];
   constexpr bool kMixed = sizeof(LU) == 4;
-  // FP32-LU form: As[e * BS] = FP64 matrix entry e of kJacPattern; L[(col*10+row) * BS] factor
+  // FP32-LU form: As[e * BS] = FP64 matrix entry e of kJacPattern; FP64 form: L[(col*10+row) * BS]
   double* As = reinterpret_cast<double*>(smem_raw) + threadIdx.x;
-  LU* L = reinterpret_cast<LU*>(reinterpret_cast<double*>(smem_raw) + (kMixed ? 64 * BS : 0)) +
-          threadIdx.x;
+  LU* L = reinterpret_cast<LU*>(smem_raw) + threadIdx.x;
   int bad = 0;
   // cells: a grid-stride sweep, or (queue set) 32-cell chunks taken from the shared counter by
   // each one-warp block until every cell is taken (launches on other streams may share it)
@@ -91,8 +98,15 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       const double* __restrict__ sc = S.scale + j;  // re-read through L1: keeps registers free
       const double* __restrict__ isc = S.inv_scale + j;
       double ya[10];
+      bool scaled = true;  // see below
 #pragma unroll
-      for (int s = 0; s < 10; ++s) ya[s] = y[j + s] * sc[s];
+      for (int s = 0; s < 10; ++s) {
+        const double z = y[j + s];
+        ya[s] = z * sc[s];
+        As[z_slot<LU>(s) * BS] = z;
+        const int e = (__double2hiint(z) >> 20) & 0x7FF;
+        scaled = scaled && (unsigned)(e - (1023 - 99)) <= 198u;
+      }
       double Ts = S.Ts[i], dTs = 0.0, logT;
       // mixed form: up to 8 FP32 iterations, then two in FP64.  (One FP64 iteration where
       // the FP32 stage converged measured 5 % faster but left the carried temperature up to
@@ -110,12 +124,6 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       // species entries are then plain sums of the reaction fluxes (chem_matrix), and partial
       // pivoting, which compares within a column, picks the same rows.  The solution is z times
       // that system's.  Variables that are zero or far from 1 take the unscaled matrix.
-      bool scaled = true;
-#pragma unroll
-      for (int s = 0; s < 10; ++s) {
-        const int e = (__double2hiint(y[j + s]) >> 20) & 0x7FF;
-        scaled = scaled && (unsigned)(e - (1023 - 99)) <= 198u;
-      }
       {  // source and Newton matrix from one rate evaluation (rates and T slopes)
         double k[kNRates], dk[kNRates], pr[21], r[21];
         chem_rates<true>(P, logT, k, dk);
@@ -133,8 +141,6 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
         }
 #pragma unroll
         for (int s = 0; s < 10; ++s) fout[j + s] = f[s];
-#pragma unroll
-        for (int e = 0; e < 100; ++e) L[e * BS] = LU(0);  // structural zeros
         if (scaled) {
           double rf[10];  // -gamma * tunit * inv_scale[row], the ge row's 1/mdensity with it
 #pragma unroll
@@ -144,18 +150,10 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
           // every structural entry (the diagonal included) is put exactly once
           chem_matrix(P, k, dk, ya, pr, r, Ts, Ax, Rg, [&](int row, int col, double v) {
             const double u = col == 9 ? v * t9 : v;
-            put_entry<LU, BS>(As, L, row, col, row == col ? fma(u, rf[row], y[j + row]) : u * rf[row]);
+            put_entry<LU, BS>(As, L, row, col, row == col ? fma(u, rf[row], As[z_slot<LU>(row) * BS]) : u * rf[row]);
           });
         } else {
-          newton_matrix_plain<LU, BS>(P, S, i, y, Ts, dTs, gamma * tunit, As, L);
-        }
-        if constexpr (kMixed) {  // the FP32 factor's entries, converted with integer
-          // instructions after the Jacobian (off the FP64 pipe, which bounds this kernel, and off
-          // the Jacobian's dependency chains: 5.45 -> 5.34 ms per 128^3 call; converting inside
-          // the entry loop had measured 1 % slower)
-#pragma unroll
-          for (int e = 0; e < 64; ++e)
-            L[(kJacPattern[e][1] * 10 + kJacPattern[e][0]) * BS] = f32_of_f64(As[e * BS]);
+          newton_matrix_plain<LU, BS>(P, S, i, Ts, dTs, gamma * tunit, As, L);
         }
       }
 #pragma unroll
@@ -174,21 +172,31 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       float zf[10];  // z for the stopping tests, which are on x
       if (sizeof(LU) == 4) {
 #pragma unroll
-        for (int s = 0; s < 10; ++s) zf[s] = scaled ? f32_of_f64(y[j + s]) : 1.f;
+        for (int s = 0; s < 10; ++s) zf[s] = scaled ? f32_of_f64(As[z_slot<LU>(s) * BS]) : 1.f;
       }
-      int info = lu10_strided<LU, true>(L, BS, piv);
+      // the factor lives in registers: in shared memory every elimination step waited on its
+      // loads (7-8 warps per SM); FP32 entries converted with integer instructions
+      LU a[100];
+#pragma unroll
+      for (int e = 0; e < 100; ++e) {
+        const int q = kJacIndex[e % 10][e / 10];
+        if (q < 0) a[e] = LU(0);  // structural zero
+        else if constexpr (kMixed) a[e] = f32_of_f64(As[q * BS]);
+        else a[e] = L[e * BS];
+      }
+      int info = lu10_regs(a, piv);
       bool fp64_fallback = (sizeof(LU) == 4) && info != 0;
       if (!fp64_fallback) {
         LU xs[10];
 #pragma unroll
         for (int s = 0; s < 10; ++s) xs[s] = to_lu<LU>(f[s]);
-        lus10_strided<LU, LU>(L, BS, piv, xs);
+        lus10_regs(a, piv, xs);
         float xmax = 0.f;  // solution size for the stopping tests, from the FP32 solve: the
                            // refinements move it by ~1e-7 relative, far below either threshold
 #pragma unroll
         for (int s = 0; s < 10; ++s) {
           x[s] = from_lu(xs[s]);
-          xmax = fmaxf(xmax, fabsf((float)xs[s] * zf[s]));
+          if (kMixed) xmax = fmaxf(xmax, fabsf((float)xs[s] * zf[s]));
         }
         if (sizeof(LU) == 4) {
           // iterative refinement against FP64 residuals; a cell stops as soon as its correction
@@ -207,7 +215,7 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
             LU ds[10];
 #pragma unroll
             for (int s = 0; s < 10; ++s) ds[s] = to_lu<LU>(rr[s]);
-            lus10_strided<LU, LU>(L, BS, piv, ds);
+            lus10_regs(a, piv, ds);
             float dmax = 0.f;
 #pragma unroll
             for (int s = 0; s < 10; ++s) {
@@ -235,7 +243,7 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       }
       if (info && (sizeof(LU) == 8 || fp64_fallback)) bad = 1;
 #pragma unroll
-      for (int s = 0; s < 10; ++s) xout[j + s] = scaled ? x[s] * y[j + s] : x[s];
+      for (int s = 0; s < 10; ++s) xout[j + s] = scaled ? x[s] * As[z_slot<LU>(s) * BS] : x[s];
     }
     if (!queue) i += stride;
   }
@@ -248,8 +256,7 @@ static int launch_newton(const ChemParams& P, const ChemState& S, long n, const 
                          int* d_info, cudaStream_t s, long blocks, const double* b,
                          unsigned long long* queue) {
   constexpr int BS = kNtThreads;
-  const size_t shm = (size_t)BS * (sizeof(LU) == 4 ? 64 * sizeof(double) + 100 * sizeof(float)
-                                                   : 100 * sizeof(double));
+  const size_t shm = (size_t)BS * (sizeof(LU) == 4 ? 74 : 100) * sizeof(double);
   // a function attribute, not a stream operation: also legal during graph capture
   GBMV_CUDA_TRY(cudaFuncSetAttribute(chem_newton_kernel<LU, BS>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
