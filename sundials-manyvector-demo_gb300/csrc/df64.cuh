@@ -131,8 +131,22 @@ __device__ __forceinline__ double f64_of_f32(float f) {
   return __hiloint2double((int)hi, (int)lo);
 }
 
-// f2_from_double without conversion instructions (bit-identical to it)
+// f2_from_double without conversion instructions (bit-identical to it), and for the common
+// exponents without the FP64 subtraction either: what rounding to hi leaves of the 53-bit
+// significand is a signed integer of 29 bits, whose conversion to float (a 32-bit one) rounds as
+// the conversion of the exact difference would.
 __device__ __forceinline__ f2 f2_split(double d) {
+  const unsigned long long p = (unsigned long long)__double_as_longlong(d);
+  const unsigned e = (unsigned)(p >> 52) & 0x7FFu;
+  if (e - 949u <= 1149u - 949u) {
+    const unsigned long long r = p + 0x0FFFFFFFull + ((p >> 29) & 1ull);
+    const unsigned hi = (unsigned)(r >> 32), s = hi & 0x80000000u;
+    const unsigned h = s | ((((hi >> 20) & 0x7FFu) - 896u) << 23) | ((unsigned)(r >> 29) & 0x7FFFFFu);
+    // p - (r with its low 29 bits cleared), in units of the last place of d
+    const int left = (int)((unsigned)p - ((unsigned)r & 0xE0000000u));
+    return f2(__uint_as_float(h),
+              (float)(s ? -left : left) * __uint_as_float((e - 948u) << 23));
+  }
   const float h = f32_of_f64<true>(d);
   return f2(h, f32_of_f64<true>(d - f64_of_f32<true>(h)));
 }

@@ -155,13 +155,13 @@ __global__ void __launch_bounds__(256) divergence_kernel(Grid g, Fields wdot,
 #pragma unroll
     for (int v = 0; v < 5 + NCHEM; ++v) {
       // (F+ - F-) / d as a multiply by 1/d: the reference divides; the difference is one
-      // rounding, and 45 FP64 divisions per cell would cost more than the rest of this pass
-      const double div = (Fx[v * nfx + fx + 1] - Fx[v * nfx + fx]) * g.inv_d[0] +
-                         (Fy[v * nfy + fy + nx] - Fy[v * nfy + fy]) * g.inv_d[1] +
-                         (Fz[v * nfz + fz + nx * ny] - Fz[v * nfz + fz]) * g.inv_d[2];
+      // rounding, and 45 FP64 divisions per cell would cost more than the rest of this pass.
+      // Subtracted from G as it goes: six FP64 instructions a field
       double* dst = (v < 5) ? (wdot.f[v] + c) : (wdot.f[5] + (v - 5) + (long)NCHEM * c);
-      const double base = G.in_wdot ? *dst : G.c[v];
-      *dst = base - div;
+      double r = G.in_wdot ? *dst : G.c[v];
+      r = fma(Fx[v * nfx + fx] - Fx[v * nfx + fx + 1], g.inv_d[0], r);
+      r = fma(Fy[v * nfy + fy] - Fy[v * nfy + fy + nx], g.inv_d[1], r);
+      *dst = fma(Fz[v * nfz + fz] - Fz[v * nfz + fz + nx * ny], g.inv_d[2], r);
     }
   }
 }
@@ -190,7 +190,7 @@ int divergence(const Grid& g, const Fields& wdot, double* const (&F)[3], const F
 // the float-float forms are set by the primitives pass, which already has the pressure, so this
 // pass reads no state field and needs no division.
 template <int NCHEM>
-__global__ void __launch_bounds__(256) divergence_f2_kernel(Grid g, Fields wdot,
+__global__ void __launch_bounds__(256, 4) divergence_f2_kernel(Grid g, Fields wdot,
                                                             const float2* __restrict__ Fx,
                                                             const float2* __restrict__ Fy,
                                                             const float2* __restrict__ Fz,
@@ -207,8 +207,9 @@ __global__ void __launch_bounds__(256) divergence_f2_kernel(Grid g, Fields wdot,
     const long fy = i + nx * (j + (ny + 1) * k);
     const long fz = c;
     // fields in groups whose 6 fluxes each are loaded before any is used: the rare conversions'
-    // branches keep the compiler from moving loads up across them
-    constexpr int NV = 5 + NCHEM, GR = 5;
+    // branches keep the compiler from moving loads up across them.  128^3 x 15: groups of 2 at 4
+    // blocks per SM 234 us; 3 at 3 257; 1 at 6 292; 5 at 3 295, unbounded 381 (290 before)
+    constexpr int NV = 5 + NCHEM, GR = 2;
 #pragma unroll
     for (int v0 = 0; v0 < NV; v0 += GR) {
       float2 x[GR][6];

@@ -4,18 +4,15 @@
 
 namespace gbmv {
 
-#ifndef KF2
-#define KF2 3
-#endif
-#ifndef KTR
-#define KTR 6
-#endif
-#ifndef KTR0
-#define KTR0 5
-#endif
-constexpr int kF2MinB = KF2;
+// Register budgets of the sweeps (128-thread blocks per SM; the same bits whatever they are).
+// Fluid, 128^3 x 15 GBMV_MIXED_FAST RHS at 2 / 3 / 4 blocks: 2.84 / 2.85 / 3.13 ms.  Beside the
+// chemistry Newton on a second stream (255 registers a thread) 5 leave the Newton's warps room
+// (Grid::sweep_shared).  Tracers: FP32 weights 4 / 5 / 6 / 7 / 8: 2.93 / 2.85 / 2.81 / 2.80 / 2.82
+// ms; float-float weights 2 / 3 / 4 / 5 (GBMV_MIXED): 3.81 / 3.80 / 3.67 / 3.64 ms.
+constexpr int kF2MinB = 3;
 constexpr int kF2SharedMinB = 5;
-constexpr int kTracerMinB = KTR;
+constexpr int kTracerFastMinB = 6;
+constexpr int kTracerMinB = 5;
 
 __global__ void __launch_bounds__(256) prims_f2_kernel(Grid g, Fields w, float2* __restrict__ Q2,
                                                        const double* __restrict__ tscale,
@@ -199,7 +196,7 @@ __global__ void __launch_bounds__(128, MINB)
 // Tracer face fluxes: one thread a face, its tracers one after the other; reads half the
 // Lax-Friedrichs speed that the fluid sweep left in the first tracer's flux.
 template <int WV>
-__global__ void __launch_bounds__(128, WV == 1 ? kTracerMinB : KTR0)
+__global__ void __launch_bounds__(128, WV == 1 ? kTracerFastMinB : kTracerMinB)
     tracer_flux_f2_kernel(const __grid_constant__ SweepSet S, const float2* __restrict__ Q2,
                           long n, int nchem) {
   const int dir = sweep_dir(S);

@@ -36,7 +36,7 @@ __device__ __forceinline__ Dual dfma(double a, Dual b, Dual c) {
   return Dual(fma(a, b.v, c.v), fma(a, b.d, c.d));
 }
 __device__ __forceinline__ Dual drcp(Dual a) {
-  const double r = 1.0 / a.v;
+  const double r = rcp64_any(a.v);
   return Dual(r, -(a.d * (r * r)));
 }
 
@@ -48,7 +48,7 @@ __device__ __forceinline__ void roe_dual(const Dual (&W)[6][5], const Dual (&ph)
                                          RoeDual& R) {
   const double gm = gamma - 1.0;
   const double sL = sqrt0_64(W[2][0].v), sR = sqrt0_64(W[3][0].v);
-  const double rL = 1.0 / sL, rR = 1.0 / sR;
+  const double rL = rcp64_any(sL), rR = rcp64_any(sR);
   const double tL = 0.5 * W[2][0].d * rL, tR = 0.5 * W[3][0].d * rR;  // tangents of the roots
   const Dual iL(rL, -(tL * (rL * rL))), iR(rR, -(tR * (rR * rR)));
   const Dual is = drcp(Dual(sL + sR, tL + tR));

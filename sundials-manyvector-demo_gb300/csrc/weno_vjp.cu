@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
            wb = B.w + fma(ob[3], s, ob[4] * ff[2]), Hb = ob[4] * t, qb = ob[4] * ff[3],
            cb = cdb * d;
     // left eigenvector entries; hc = 1/(2c), hgc = gm hc, gc = 2 hgc
-    const double hc = 0.5 / c, hgc = gm * hc, gq = gm * R.q, gu = gm * u;
+    const double hc = 0.5 * rcp64_any(c), hgc = gm * hc, gq = gm * R.q, gu = gm * u;
     double hcb = fma(B.L00, u + gq, fma(B.L40, gq - u, -fma(B.L01, gu + 1.0, B.L41 * (gu - 1.0))));
     ub = fma(hc, (B.L00 - B.L40) - gm * (B.L01 + B.L41), ub);
     qb = fma(hgc, B.L00 + B.L40, qb);
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
     // Roe averages X = (a iL + b iR) is, iL = 1/sqrt(rhoL), is = 1/(sL + sR)
     {
       const double sL = sqrt0_64(T.W[2][0]), sR = sqrt0_64(T.W[3][0]);
-      const double iL = 1.0 / sL, iR = 1.0 / sR, is = 1.0 / __dadd_rn(sL, sR);
+      const double iL = rcp64_any(sL), iR = rcp64_any(sR), is = rcp64_any(__dadd_rn(sL, sR));
       const double eL = fma(2.0, T.ph[2], T.W[2][4]), eR = fma(2.0, T.ph[3], T.W[3][4]);
       const double xu = ub * is, xv = vb * is, xw = wb * is, xH = Hb * is;
       B.W[2][1] = fma(xu, iL, B.W[2][1]);
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
       const double uadd = su < 0.0 ? -0.5 * B.ha : 0.5 * B.ha;
       double padd = 0.0, radd = 0.0;
       if (sc > 0.0) {
-        const double ir = 1.0 / sr;
+        const double ir = rcp64_any(sr);
         padd = 0.25 * S.gamma * ir * B.ha / sc;
         radd = -(padd * sp) * ir;
       }

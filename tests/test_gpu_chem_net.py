@@ -80,3 +80,28 @@ def test_temperature_at_table_points(cuda, tables):
         # the ge column holds slopes, which step from bin to bin: compare the others
         a, b = Jg[:, :9], Jo[:, :9]
         assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_dirk_residency_leaves_results_alone(cuda, tables, precision):
+    """The integrator's resident warps follow from the number of cells (lines at 20 and 28 warps of
+    cells per SM): the same cells end bit for bit alike in runs of every size."""
+    torch = cuda
+    import gbmv
+    sizes = (1500, 152 * 32 * 20 - 1, 152 * 32 * 20 + 40, 152 * 32 * 28 + 40)
+    y, _ = _state(1500, 960, (10.0, 1e4))
+    ref = None
+    for n in sizes:
+        reps = -(-n // 1500)
+        scale = np.tile(y, (reps, 1))[:n]
+        c = gbmv.Chem(n, tables)
+        c.set_scale(_dev(torch, scale.reshape(-1)))
+        z = torch.ones(10 * n, dtype=torch.float64, device="cuda")
+        assert c.dirk_evolve(0.0, 2e-9, z, 1e11, precision=precision, block=32, rtol=1e-6,
+                             atol=1e-10, maxcor=10, nlscoef=0.01) == 0
+        z = z.view(n, 10)
+        if ref is None:
+            ref = z
+        for k in range(0, n, 1500):
+            m = min(1500, n - k)
+            assert torch.equal(z[k:k + m], ref[:m])
