@@ -17,6 +17,13 @@
 
 namespace gbmv {
 
+// Casts to and from the factor's precision, off the FP64 pipe (60 of a cell's ~900 FP64-pipe
+// instructions were conversions; 96^3 cells 1751 -> 1683 us)
+__device__ __forceinline__ double lu_cast(double x, double*) { return x; }
+__device__ __forceinline__ float lu_cast(double x, float*) { return f32_of_f64<true>(x); }
+__device__ __forceinline__ double lu_back(double x) { return x; }
+__device__ __forceinline__ double lu_back(float x) { return f64_of_f32<true>(x); }
+
 // Threads per block.  Shared memory per cell: the FP32-LU form keeps the 64 structural
 // nonzeros of the FP64 Newton matrix (for the refinement residuals) and the variables, 592 bytes; the FP64-LU form
 // its 100 entries until they are factored.  With 32-thread blocks eight fit an SM, the register
@@ -189,13 +196,13 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       if (!fp64_fallback) {
         LU xs[10];
 #pragma unroll
-        for (int s = 0; s < 10; ++s) xs[s] = to_lu<LU>(f[s]);
+        for (int s = 0; s < 10; ++s) xs[s] = lu_cast(f[s], (LU*)nullptr);
         lus10_regs(a, piv, xs);
         float xmax = 0.f;  // solution size for the stopping tests, from the FP32 solve: the
                            // refinements move it by ~1e-7 relative, far below either threshold
 #pragma unroll
         for (int s = 0; s < 10; ++s) {
-          x[s] = from_lu(xs[s]);
+          x[s] = lu_back(xs[s]);
           if (kMixed) xmax = fmaxf(xmax, fabsf((float)xs[s] * zf[s]));
         }
         if (sizeof(LU) == 4) {
@@ -214,12 +221,12 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
               rr[kJacPattern[e][0]] -= As[e * BS] * x[kJacPattern[e][1]];
             LU ds[10];
 #pragma unroll
-            for (int s = 0; s < 10; ++s) ds[s] = to_lu<LU>(rr[s]);
+            for (int s = 0; s < 10; ++s) ds[s] = lu_cast(rr[s], (LU*)nullptr);
             lus10_regs(a, piv, ds);
             float dmax = 0.f;
 #pragma unroll
             for (int s = 0; s < 10; ++s) {
-              x[s] += from_lu(ds[s]);
+              x[s] += lu_back(ds[s]);
               dmax = fmaxf(dmax, fabsf((float)ds[s] * zf[s]));
             }
             dlast = dmax;

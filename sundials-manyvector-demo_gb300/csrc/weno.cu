@@ -54,7 +54,7 @@ int prims64(const Grid& g, const Fields& w, double* const (&out)[5], int* d_stat
   return GBMV_OK;
 }
 
-// Face fluxes of the three directions (one launch).  Bound by the FP64 pipe: ~1550 instructions
+// Face fluxes of the three directions (one launch).  Bound by the FP64 pipe: 1495 instructions
 // a face at NVAR 15.  PRE: the primitives are read from the cell pass, else formed per stencil
 // point.  SPLIT: two neighbouring threads share a face, each with one Lax-Friedrichs side (the
 // second reads its stencil reversed, which makes its side the plus formula); the same bits.
@@ -80,8 +80,8 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
       load_point(D.f, cell[l], nall[l], nnorm[l], T.W[l]);
       if (PRE) {
         const double p = __ldg(S.ph + cell[l]), u = __ldg(D.vel[0] + cell[l]);
-        T.ph[l] = nall[l] ? -p : p;
-        T.u[l] = nnorm[l] ? -u : u;
+        T.ph[l] = flip_sign(p, nall[l]);
+        T.u[l] = flip_sign(u, nnorm[l]);
         T.hc[l] = __ldg(S.hc + cell[l]);
       } else {
         point_prims64(S.gamma, T.W[l][0], T.W[l][1], T.W[l][2], T.W[l][3], T.W[l][4], T.ph[l],
@@ -95,13 +95,19 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
       fluid_face_flux64(T, S.gamma, H, out);
 #pragma unroll
       for (int v = 0; v < 5; ++v) D.F[D.slot[v] * D.nfaces + f] = out[v];
+      if (NCHEM) {
+#pragma unroll
+        for (int l = 0; l < 5; ++l) {
+          keep64(H.hp[l]);
+          keep64(H.hm[l + 1]);
+        }
+      }
 #pragma unroll 1
       for (int c = 0; c < NCHEM; ++c) {
         double cv[6];
 #pragma unroll
         for (int l = 0; l < 6; ++l) {
-          const double x = __ldg(S.chem + c + (long)NCHEM * cell[l]);
-          cv[l] = nall[l] ? -x : x;
+          cv[l] = flip_sign(__ldg(S.chem + c + (long)NCHEM * cell[l]), nall[l]);
         }
         D.F[(5 + c) * D.nfaces + f] = tracer_face_flux64(H, cv);
       }
@@ -119,13 +125,16 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
 #pragma unroll
       for (int v = 0; v < 5; ++v)
         if (live && (v & 1) == side) D.F[D.slot[v] * D.nfaces + f] = out[v];
+      if (NCHEM) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) keep64(h[k]);
+      }
 #pragma unroll 1
       for (int c = 0; c < NCHEM; ++c) {
         double cv[5];
 #pragma unroll
         for (int l = 0; l < 5; ++l) {
-          const double x = __ldg(S.chem + c + (long)NCHEM * cell[l]);
-          cv[l] = nall[l] ? -x : x;
+          cv[l] = flip_sign(__ldg(S.chem + c + (long)NCHEM * cell[l]), nall[l]);
         }
         Weno64 q;
         double r = weno_prod64(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);

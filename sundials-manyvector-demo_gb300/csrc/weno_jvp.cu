@@ -7,7 +7,7 @@
 //
 // Bound by the FP64 pipe, so the tangents are written out where a generic dual number would
 // spend instructions on constants' zero tangents and on quotients: 40 instructions for the
-// tangent of a reconstruction on top of its 38 (weno_tan64).  96^3 x 9: 5330 -> ~2600 FP64
+// tangent of a reconstruction on top of its 38 (weno_tan64).  96^3 x 9: 5330 -> 2370 FP64
 // instructions a face.
 #include "common.cuh"
 #include "weno.cuh"
@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(128) face_flux_jvp_kernel(const __grid_constan
       ir[l] = rcp64(T.W[l][0]);
       if (PRE) {
         const double p = __ldg(S.ph + cell[l]), x = __ldg(D.vel[0] + cell[l]);
-        T.ph[l] = nall[l] ? -p : p;
-        T.u[l] = nnorm[l] ? -x : x;
+        T.ph[l] = flip_sign(p, nall[l]);
+        T.u[l] = flip_sign(x, nnorm[l]);
         T.hc[l] = __ldg(S.hc + cell[l]);
         v1 = __ldg(D.vel[1] + cell[l]);
         v2 = __ldg(D.vel[2] + cell[l]);
@@ -200,6 +200,15 @@ __global__ void __launch_bounds__(128) face_flux_jvp_kernel(const __grid_constan
         dfma(R.H, t, dfma(R.u, cd, dfma(R.v, ff[1], dfma(R.w, ff[2], R.q * ff[3])))).d};
 #pragma unroll
     for (int v = 0; v < 5; ++v) D.F[D.slot[v] * D.nfaces + f] = o[v];
+    if (NCHEM) {
+#pragma unroll
+      for (int l = 0; l < 5; ++l) {
+        keep64(hp[l].v);
+        keep64(hp[l].d);
+        keep64(hm[l + 1].v);
+        keep64(hm[l + 1].d);
+      }
+    }
 #pragma unroll 1
     for (int c = 0; c < NCHEM; ++c) {
       Dual cv[6];
@@ -207,7 +216,7 @@ __global__ void __launch_bounds__(128) face_flux_jvp_kernel(const __grid_constan
       for (int l = 0; l < 6; ++l) {
         const double x = __ldg(S.chem + c + (long)NCHEM * cell[l]);
         const double dx = __ldg(S.gchem + c + (long)NCHEM * cell[l]);
-        cv[l] = nall[l] ? Dual(-x, -dx) : Dual(x, dx);
+        cv[l] = Dual(flip_sign(x, nall[l]), flip_sign(dx, nall[l]));
       }
       D.F[(5 + c) * D.nfaces + f] =
           tracer_side_tan(cv[0], hp[0], cv[1], hp[1], cv[2], hp[2], cv[3], hp[3], cv[4], hp[4]) +

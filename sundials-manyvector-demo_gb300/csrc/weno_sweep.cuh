@@ -119,12 +119,7 @@ __device__ __forceinline__ void stencil_of(const SweepSet& S, const SweepDir& D,
 __device__ __forceinline__ void load_point(const double* const (&f)[5], long c, bool nall,
                                            bool nnorm, double (&W)[5]) {
 #pragma unroll
-  for (int v = 0; v < 5; ++v) W[v] = __ldg(f[v] + c);
-  if (nall) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) W[v] = -W[v];
-  }
-  if (nnorm) W[1] = -W[1];
+  for (int v = 0; v < 5; ++v) W[v] = flip_sign(__ldg(f[v] + c), nall != (v == 1 && nnorm));
 }
 
 // grid-stride launch size: ceil(n / t) blocks, at least 1, at most 16 per SM

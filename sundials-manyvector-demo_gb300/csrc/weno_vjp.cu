@@ -12,7 +12,7 @@
 // Bound by the FP64 pipe.  The adjoint of a reconstruction works on the neighbour differences
 // and takes the forward weights' products (weno_adj64: 47 instructions after the forward 38; the
 // adjoint of the literal formula took ~250 with its seven divisions), the primitives come from
-// a cell pass, and each point's reciprocal density is formed once.  96^3 x 9: 6120 -> ~2500
+// a cell pass, and each point's reciprocal density is formed once.  96^3 x 9: 6120 -> 2520
 // FP64 instructions a face.
 #include "common.cuh"
 #include "weno.cuh"
@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
     for (int l = 0; l < 6; ++l) {
       load_point(D.f, cell[l], nall[l], nnorm[l], T.W[l]);
       const double p = __ldg(S.ph + cell[l]), x = __ldg(D.vel[0] + cell[l]);
-      T.ph[l] = nall[l] ? -p : p;
-      T.u[l] = nnorm[l] ? -x : x;
+      T.ph[l] = flip_sign(p, nall[l]);
+      T.u[l] = flip_sign(x, nnorm[l]);
       T.hc[l] = __ldg(S.hc + cell[l]);
     }
     int am;
@@ -178,6 +178,11 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
     for (int k = 0; k < 5; ++k) {
       hp[k] = fma(0.5, T.u[k], ha);
       hm[k] = fma(0.5, T.u[5 - k], -ha);
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      keep64(hp[k]);
+      keep64(hm[k]);
     }
     // tracers first: their cotangents of the split factors join the fluid part's
     double hpb[5] = {0, 0, 0, 0, 0}, hmb[5] = {0, 0, 0, 0, 0};
@@ -190,8 +195,7 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
       double cv[6];
 #pragma unroll
       for (int l = 0; l < 6; ++l) {
-        const double x = __ldg(S.chem + c + (long)NCHEM * cell[l]);
-        cv[l] = nall[l] ? -x : x;
+        cv[l] = flip_sign(__ldg(S.chem + c + (long)NCHEM * cell[l]), nall[l]);
       }
       double pb[5], mb[5];
       {
@@ -205,7 +209,7 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
 #pragma unroll
       for (int l = 0; l < 6; ++l) {
         const double b = l == 0 ? pb[0] : (l == 5 ? mb[0] : pb[l] + mb[5 - l]);
-        A[((long)l * NV + 5 + c) * nfaces + f] = nall[l] ? -b : b;
+        A[((long)l * NV + 5 + c) * nfaces + f] = flip_sign(b, nall[l]);
       }
     }
     Adj64 B;
@@ -323,13 +327,10 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
       q[2] = fma(-k, v1, B.W[l][2]);
       q[3] = fma(-k, v2, B.W[l][3]);
       q[4] = B.W[l][4] + k;
-      if (nall[l]) {
 #pragma unroll
-        for (int e = 0; e < 5; ++e) q[e] = -q[e];
-      }
-      if (nnorm[l]) q[1] = -q[1];
-#pragma unroll
-      for (int e = 0; e < 5; ++e) A[((long)l * NV + D.slot[e]) * nfaces + f] = q[e];
+      for (int e = 0; e < 5; ++e)
+        A[((long)l * NV + D.slot[e]) * nfaces + f] =
+            flip_sign(q[e], nall[l] != (e == 1 && nnorm[l]));
     }
   }
 }
