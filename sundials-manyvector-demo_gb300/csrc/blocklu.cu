@@ -72,36 +72,50 @@ __global__ void __launch_bounds__(kLuThreads, 8) block_lu_factor_kernel(long nb,
   if (bad) atomicMax(info_out, 1);
 }
 
+// Two tiles: the next one's copies, right-hand sides and pivots are in flight while this one is
+// solved.  One warp a scheduler keeps the FP64 pipe busy by itself (an instruction's latency is
+// its issue interval), so four such CTAs per SM do where seven with one tile each waited for
+// their loads 46 % of the time: 192,000 blocks 62 -> SOLVE2_US us.
 __global__ void __launch_bounds__(kLuThreads) block_lu_solve_kernel(long nb,
                                                                     const double* __restrict__ LU,
                                                                     const int* __restrict__ piv,
                                                                     const double* b, double* x) {
-  extern __shared__ __align__(16) double sh[];  // LU tile, then the right-hand sides
-  double* shb = sh + kLuThreads * kLuStride;    // [kLuThreads][kVecStride]
-  for (long blk0 = (long)blockIdx.x * kLuThreads; blk0 < nb; blk0 += (long)gridDim.x * kLuThreads) {
-    const int nb_here = (int)((nb - blk0) < kLuThreads ? (nb - blk0) : kLuThreads);
-    tile_in_async(LU, sh, blk0, nb_here);
-    double t[10];  // the right-hand sides: 10 nb_here consecutive doubles
+  extern __shared__ __align__(16) double sh[];   // two LU tiles, then the right-hand sides
+  double* const shb = sh + 2 * kLuThreads * kLuStride;  // [kLuThreads][kVecStride]
+  const long step = (long)gridDim.x * kLuThreads;
+  long blk0 = (long)blockIdx.x * kLuThreads;
+  double t[10];  // right-hand sides of a tile: 10 consecutive doubles a block
+  int p[10];
+  auto count = [&](long at) { return (int)((nb - at) < kLuThreads ? (nb - at) : kLuThreads); };
+  auto fetch = [&](long at, double* tile) {
+    const int m = count(at);
+    tile_in_async(LU, tile, at, m);
 #pragma unroll
     for (int e = 0; e < 10; ++e) {
       const int c = threadIdx.x + e * kLuThreads;
-      t[e] = c < 10 * nb_here ? b[blk0 * 10 + c] : 0.0;
+      t[e] = c < 10 * m ? b[at * 10 + c] : 0.0;
     }
-    int p[10];
-    const int* pg = piv + (blk0 + (threadIdx.x < nb_here ? threadIdx.x : 0)) * 10;
+    const int* pg = piv + (at + (threadIdx.x < m ? threadIdx.x : 0)) * 10;
 #pragma unroll
     for (int e = 0; e < 10; ++e) p[e] = __ldg(pg + e);
+  };
+  if (blk0 < nb) fetch(blk0, sh);
+  for (int buf = 0; blk0 < nb; blk0 += step, buf ^= 1) {
+    const int m = count(blk0);
+    int piv_now[10];
 #pragma unroll
     for (int e = 0; e < 10; ++e) {
       const int c = threadIdx.x + e * kLuThreads;
       shb[(c / 10) * kVecStride + c % 10] = t[e];
+      piv_now[e] = p[e];
     }
     tile_in_wait();
-    if (threadIdx.x < nb_here) {
+    if (blk0 + step < nb) fetch(blk0 + step, sh + (buf ^ 1) * (kLuThreads * kLuStride));
+    if (threadIdx.x < m) {
       double v[10];
 #pragma unroll
       for (int e = 0; e < 10; ++e) v[e] = shb[threadIdx.x * kVecStride + e];
-      lus10(sh + threadIdx.x * kLuStride, p, v);
+      lus10(sh + buf * (kLuThreads * kLuStride) + threadIdx.x * kLuStride, piv_now, v);
 #pragma unroll
       for (int e = 0; e < 10; ++e) shb[threadIdx.x * kVecStride + e] = v[e];
     }
@@ -109,7 +123,7 @@ __global__ void __launch_bounds__(kLuThreads) block_lu_solve_kernel(long nb,
 #pragma unroll
     for (int e = 0; e < 10; ++e) {
       const int c = threadIdx.x + e * kLuThreads;
-      if (c < 10 * nb_here) x[blk0 * 10 + c] = shb[(c / 10) * kVecStride + c % 10];
+      if (c < 10 * m) x[blk0 * 10 + c] = shb[(c / 10) * kVecStride + c % 10];
     }
     __syncwarp();
   }
@@ -157,11 +171,11 @@ int block_lu_factor(long nb, double* A, int* piv, int* d_info, cudaStream_t s) {
 
 int block_lu_solve(long nb, const double* LU, const int* piv, const double* b, double* x,
                    cudaStream_t s) {
-  const size_t shm = sizeof(double) * (kLuStride + kVecStride) * kLuThreads;
+  const size_t shm = sizeof(double) * (2 * kLuStride + kVecStride) * kLuThreads;
   GBMV_CUDA_TRY(cudaFuncSetAttribute(block_lu_solve_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
   ProfScope ps("block_lu_solve", s);
-  block_lu_solve_kernel<<<lu_grid(nb, 7), kLuThreads, shm, s>>>(nb, LU, piv, b, x);
+  block_lu_solve_kernel<<<lu_grid(nb, 4), kLuThreads, shm, s>>>(nb, LU, piv, b, x);
   GBMV_LAUNCH_CHECK("block_lu_solve_kernel");
   return GBMV_OK;
 }

@@ -391,9 +391,16 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
   // to float once
   const size_t tab_doubles = (size_t)kNT * kTSize;
   const size_t gtab_floats = (size_t)8 * kTSize;
+  const size_t ltab_doubles = (size_t)2 * kLogEntries;
   float* gh = (float*)calloc(gtab_floats, sizeof(float));
   double* dh = (double*)calloc(tab_doubles, sizeof(double));
-  if (!gh || !dh) { free(h); free(gh); free(dh); delete c; return GBMV_ENOMEM; }
+  double* lh = (double*)malloc(sizeof(double) * ltab_doubles);
+  if (!gh || !dh || !lh) { free(h); free(gh); free(dh); free(lh); delete c; return GBMV_ENOMEM; }
+  for (int q = 0; q < kLogEntries; ++q) {  // 1/c and log c of each interval's midpoint (chem_log)
+    const double mid = ldexp(1.0 + ((q & 127) + 0.5) / 128.0, (q >> 7) - 2);
+    lh[2 * q] = 1.0 / mid;
+    lh[2 * q + 1] = (double)-logl((long double)lh[2 * q]);
+  }
   for (int b = 0; b + 1 < kTSize; ++b)
     for (int r = 0; r < kNT; ++r) dh[b * kNT + r] = h[(b + 1) * kNT + r] - h[b * kNT + r];
   const int grow[4] = {GAMMAH2_2, DGAMMAH2_2, GAMMAH2_1, DGAMMAH2_1};
@@ -404,14 +411,15 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
       gh[b * 8 + 2 * q + 1] = (float)(hi - lo);
     }
   const size_t per_cell = 10 + 10 + 6;
-  if (cudaMalloc(&c->tab, sizeof(double) * 2 * tab_doubles + sizeof(float) * gtab_floats) !=
-          cudaSuccess ||
+  if (cudaMalloc(&c->tab, sizeof(double) * (2 * tab_doubles + ltab_doubles) +
+                              sizeof(float) * gtab_floats) != cudaSuccess ||
       cudaMalloc(&c->cell, sizeof(double) * per_cell * ncells) != cudaSuccess ||
       cudaMalloc(&c->d_info, 64) != cudaSuccess) {
     cudaGetLastError();
     free(h);
     free(gh);
     free(dh);
+    free(lh);
     cudaFree(c->tab);
     cudaFree(c->cell);
     delete c;
@@ -423,9 +431,12 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
   cudaMemcpy(c->tab, h, sizeof(double) * tab_doubles, cudaMemcpyHostToDevice);
   cudaMemcpy(c->tab + tab_doubles, dh, sizeof(double) * tab_doubles, cudaMemcpyHostToDevice);
   cudaMemcpy(c->tab + 2 * tab_doubles, gh, sizeof(float) * gtab_floats, cudaMemcpyHostToDevice);
+  double* const ltab = c->tab + 2 * tab_doubles + gtab_floats / 2;  // 16-byte aligned
+  cudaMemcpy(ltab, lh, sizeof(double) * ltab_doubles, cudaMemcpyHostToDevice);
   free(h);
   free(gh);
   free(dh);
+  free(lh);
   // constants of cvklu_setup_data (src/raja_primordial_network.cpp:190-194)
   ChemParams& P = c->P;
   P.tab = c->tab;
@@ -437,6 +448,7 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
   P.dbin = (log(P.thi) - log(P.tlo)) / P.nbins;
   P.idbin = (double)(1.0L / (long double)P.dbin);
   P.gtab = reinterpret_cast<const float*>(c->tab + 2 * tab_doubles);  // 16-byte aligned
+  P.ltab = reinterpret_cast<const double2*>(ltab);
   P.dbinf = (float)P.dbin;
   P.idbinf = (float)P.idbin;
   P.lbf = (float)P.lb;

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kLuThreads, 8) chem_jac_kernel(ChemParams P, C
       }
       const double T = S.Ts[i];
       double k[kNRates], dk[kNRates];
-      chem_rates<true>(P, log(T), k, dk);
+      chem_rates<true>(P, chem_log(P, T), k, dk);
       const ChemAux A{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
       const double Tge = S.dTs_ge[i] * (P.idbin * rcp64_any(T));
       double pr[21];
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) chem_jvp_kernel(ChemParams P, ChemState S
     }
     const double T = S.Ts[i];
     double k[kNRates], dk[kNRates];
-    chem_rates<true>(P, log(T), k, dk);
+    chem_rates<true>(P, chem_log(P, T), k, dk);
     const double Tge = S.dTs_ge[i] * (P.idbin * rcp64_any(T));
     double pr[21];
     chem_products(ya, pr);

@@ -36,10 +36,31 @@ struct ChemParams {
   // (float) value and (float)(next - value) of gammaH2_2, dgammaH2_2_dT, gammaH2_1,
   // dgammaH2_1_dT -- the roundings the FP32 iterations apply, done once at setup
   const float* gtab;  // device, gtab[bin * 8 + 2 * table + {0 value, 1 slope}]
+  const double2* ltab;  // device, chem_log's table
   double dbin, idbin, lb, tlo, thi, z, zp1_4;
   float dbinf, idbinf, lbf;  // (float) of dbin, idbin, lb
   int nbins;
 };
+
+// Natural logarithm of a temperature by table and series (P. T. P. Tang, ACM Trans. Math. Softw. 16
+// (1990) 378-400): the entry of the exponent and the seven leading significand bits holds 1/c and
+// log(c) of its interval's midpoint c, r = T/c - 1 is below 2^-8, and six terms of log(1 + r)
+// leave 2^-58.  Eight FP64 instructions where the library's logarithm takes ~25; error within
+// 1.5 units in the last place above T = 2 (absolute error below 2e-15 everywhere, which is what
+// the table position needs).  Temperatures outside [1/4, 2^18) take the library's.
+constexpr int kLogLowHi = 0x3FD00000;  // high word of 1/4
+constexpr int kLogEntries = 20 * 128;
+__device__ __forceinline__ double chem_log(const ChemParams& P, double T) {
+  const unsigned q = (unsigned)(__double2hiint(T) - kLogLowHi) >> 13;
+  if (q >= (unsigned)kLogEntries) return log(T);
+  const double2 e = __ldg(P.ltab + q);
+  const double r = fma(T, e.x, -1.0);
+  double p = fma(r, -1.0 / 6.0, 1.0 / 5.0);
+  p = fma(r, p, -1.0 / 4.0);
+  p = fma(r, p, 1.0 / 3.0);
+  p = fma(r, p, -0.5);
+  return e.y + fma(r * r, p, r);
+}
 
 // Table position of a temperature: bin b (clamped to the table) and the interpolation weight
 // inside it, log T / dbin = b + w (the tables start at T = 1).  The floor is the product rounded
@@ -111,7 +132,7 @@ __device__ __forceinline__ void chem_temp_finish(const ChemParams& P, const Chem
     Ts = P.thi;
     known = false;
   }
-  if (!known) logT = log(Ts);
+  if (!known) logT = chem_log(P, Ts);
   dTs_ge = c.dmh * rcp64_any(kb * slope);
 }
 
@@ -127,7 +148,7 @@ __device__ __forceinline__ void chem_temperature(const ChemParams& P, const doub
   bool known = false;
 #pragma unroll 1
   for (int it = 0; it < 10; ++it) {
-    logT = log(T);
+    logT = chem_log(P, T);
     const double dT = chem_temp_step(P, c, T, logT, slope);
     const double T0 = T;
     T -= dT;
@@ -192,7 +213,7 @@ __device__ __forceinline__ void chem_temperature_mixed(const ChemParams& P, cons
 #pragma unroll 1
   for (int it = nfloat; it < 10; ++it) {
     T0 = Td;
-    logT = log(T0);
+    logT = chem_log(P, T0);
     dT = chem_temp_step(P, c, T0, logT, slope);
     Td = T0 - dT;
   }

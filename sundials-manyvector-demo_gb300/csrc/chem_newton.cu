@@ -59,7 +59,7 @@ static __device__ __noinline__ void newton_matrix_plain(const ChemParams& P, con
   double ya[10], pr[21], k[kNRates], dk[kNRates];
 #pragma unroll
   for (int s = 0; s < 10; ++s) ya[s] = As[z_slot<LU>(s) * BS] * S.scale[j + s];
-  chem_rates<true>(P, log(T), k, dk);
+  chem_rates<true>(P, chem_log(P, T), k, dk);
   chem_products(ya, pr);
   const ChemAux A{S.mdens[i], S.imdens[i], S.cie[i], S.h2[i]};
   chem_jacobian(P, k, dk, ya, pr, T, dT * (P.idbin * rcp64_any(T)), A, ge_terms(k, ya),
