@@ -6,10 +6,10 @@
 // One thread owns one block; the whole 10x10 block lives in registers (fully unrolled through
 // template recursion, compile-time indices), row interchanges are predicated selects.  A CTA is
 // one warp with a tile of 32 consecutive blocks (25.6 KB, contiguous in HBM) brought into shared
-// memory by 16-byte asynchronous copies, all in flight at once; eight such CTAs per SM overlap
+// memory by 16-byte asynchronous copies, all in flight at once; several such CTAs per SM overlap
 // one tile's traffic with the others' arithmetic.  (Two-warp CTAs filling their tile with plain
 // loads, a few in flight, left the FP64 pipe 54 % busy in the factorisation and 20 % in the
-// solve: 192,000 blocks 286 and 164 us, now 172 and 64.)
+// solve: 192,000 blocks 286 and 164 us, now 167 and 58.)
 #include "block_tile.cuh"
 #include "chem.cuh"
 #include "chem_lu.cuh"
@@ -17,8 +17,9 @@
 
 namespace gbmv {
 
-// Solve with the factor of lu10_regs (row interchanges, unit-lower forward substitution,
-// upper back substitution multiplying by the stored reciprocal pivots).
+// Solve with the factor of lu10_regs in shared memory (row interchanges, unit-lower forward
+// substitution, upper back substitution multiplying by the stored reciprocal pivots); columns
+// are read in 16-byte pairs, without bank conflicts at this stride.
 __device__ __forceinline__ void lus10(const double* __restrict__ A, const int (&piv)[10],
                                       double (&x)[10]) {
 #pragma unroll
@@ -31,15 +32,49 @@ __device__ __forceinline__ void lus10(const double* __restrict__ A, const int (&
       x[r] = sw ? a : b;
     }
   }
+  const double2* const C = reinterpret_cast<const double2*>(A);
 #pragma unroll
-  for (int col = 0; col < 10; ++col)
+  for (int col = 0; col < 9; ++col) {
 #pragma unroll
-    for (int r = col + 1; r < 10; ++r) x[r] -= A[col * 10 + r] * x[col];
+    for (int h = (col + 1) / 2; h < 5; ++h) {
+      const double2 v = C[col * 5 + h];
+      if (2 * h > col) x[2 * h] -= v.x * x[col];
+      x[2 * h + 1] -= v.y * x[col];
+    }
+  }
 #pragma unroll
   for (int col = 9; col >= 0; --col) {
-    x[col] *= A[col * 10 + col];
+    double2 v[5];
 #pragma unroll
-    for (int r = 0; r < col; ++r) x[r] -= A[col * 10 + r] * x[col];
+    for (int h = 0; h <= col / 2; ++h) v[h] = C[col * 5 + h];
+    x[col] *= (col & 1) ? v[col / 2].y : v[col / 2].x;
+#pragma unroll
+    for (int r = 0; r < col; ++r) x[r] -= ((r & 1) ? v[r / 2].y : v[r / 2].x) * x[col];
+  }
+}
+
+// ten consecutive doubles of a thread
+__device__ __forceinline__ void load10(const double* g, double (&v)[10]) {
+  if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+#pragma unroll
+    for (int h = 0; h < 5; ++h) {
+      const double2 q = reinterpret_cast<const double2*>(g)[h];
+      v[2 * h] = q.x;
+      v[2 * h + 1] = q.y;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 10; ++e) v[e] = g[e];
+  }
+}
+__device__ __forceinline__ void store10(double* g, const double (&v)[10]) {
+  if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+#pragma unroll
+    for (int h = 0; h < 5; ++h)
+      reinterpret_cast<double2*>(g)[h] = make_double2(v[2 * h], v[2 * h + 1]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 10; ++e) g[e] = v[e];
   }
 }
 
@@ -56,11 +91,16 @@ __global__ void __launch_bounds__(kLuThreads, 8) block_lu_factor_kernel(long nb,
       double a[100];
       int p[10];
       double* mine = sh + threadIdx.x * kLuStride;
+      double2* const m2 = reinterpret_cast<double2*>(mine);
 #pragma unroll
-      for (int e = 0; e < 100; ++e) a[e] = mine[e];
+      for (int e = 0; e < 50; ++e) {
+        const double2 q = m2[e];
+        a[2 * e] = q.x;
+        a[2 * e + 1] = q.y;
+      }
       if (lu10_regs(a, p)) bad = 1;
 #pragma unroll
-      for (int e = 0; e < 100; ++e) mine[e] = a[e];
+      for (int e = 0; e < 50; ++e) m2[e] = make_double2(a[2 * e], a[2 * e + 1]);
       int* pg = piv + (blk0 + threadIdx.x) * 10;
 #pragma unroll
       for (int e = 0; e < 10; ++e) pg[e] = p[e];
@@ -73,57 +113,40 @@ __global__ void __launch_bounds__(kLuThreads, 8) block_lu_factor_kernel(long nb,
 }
 
 // Two tiles: the next one's copies, right-hand sides and pivots are in flight while this one is
-// solved.  One warp a scheduler keeps the FP64 pipe busy by itself (an instruction's latency is
-// its issue interval), so four such CTAs per SM do where seven with one tile each waited for
-// their loads 46 % of the time: 192,000 blocks 62 -> SOLVE2_US us.
+// solved.  One warp a scheduler can keep the FP64 pipe busy by itself (an instruction's latency is
+// its issue interval), so four such CTAs per SM do better than seven with one tile each, as long
+// as little else is issued (192,000 blocks: 62 us with seven one-tile CTAs, 58 here).
 __global__ void __launch_bounds__(kLuThreads) block_lu_solve_kernel(long nb,
                                                                     const double* __restrict__ LU,
                                                                     const int* __restrict__ piv,
                                                                     const double* b, double* x) {
-  extern __shared__ __align__(16) double sh[];   // two LU tiles, then the right-hand sides
-  double* const shb = sh + 2 * kLuThreads * kLuStride;  // [kLuThreads][kVecStride]
+  extern __shared__ __align__(16) double sh[];  // two LU tiles
   const long step = (long)gridDim.x * kLuThreads;
-  long blk0 = (long)blockIdx.x * kLuThreads;
-  double t[10];  // right-hand sides of a tile: 10 consecutive doubles a block
+  double v[10];
   int p[10];
-  auto count = [&](long at) { return (int)((nb - at) < kLuThreads ? (nb - at) : kLuThreads); };
   auto fetch = [&](long at, double* tile) {
-    const int m = count(at);
+    const int m = (int)((nb - at) < kLuThreads ? (nb - at) : kLuThreads);
     tile_in_async(LU, tile, at, m);
+    const long i = at + (threadIdx.x < m ? threadIdx.x : 0);
+    load10(b + i * 10, v);
 #pragma unroll
-    for (int e = 0; e < 10; ++e) {
-      const int c = threadIdx.x + e * kLuThreads;
-      t[e] = c < 10 * m ? b[at * 10 + c] : 0.0;
-    }
-    const int* pg = piv + (at + (threadIdx.x < m ? threadIdx.x : 0)) * 10;
-#pragma unroll
-    for (int e = 0; e < 10; ++e) p[e] = __ldg(pg + e);
+    for (int e = 0; e < 10; ++e) p[e] = __ldg(piv + i * 10 + e);
   };
+  long blk0 = (long)blockIdx.x * kLuThreads;
   if (blk0 < nb) fetch(blk0, sh);
   for (int buf = 0; blk0 < nb; blk0 += step, buf ^= 1) {
-    const int m = count(blk0);
+    double now[10];
     int piv_now[10];
 #pragma unroll
     for (int e = 0; e < 10; ++e) {
-      const int c = threadIdx.x + e * kLuThreads;
-      shb[(c / 10) * kVecStride + c % 10] = t[e];
+      now[e] = v[e];
       piv_now[e] = p[e];
     }
     tile_in_wait();
     if (blk0 + step < nb) fetch(blk0 + step, sh + (buf ^ 1) * (kLuThreads * kLuStride));
-    if (threadIdx.x < m) {
-      double v[10];
-#pragma unroll
-      for (int e = 0; e < 10; ++e) v[e] = shb[threadIdx.x * kVecStride + e];
-      lus10(sh + buf * (kLuThreads * kLuStride) + threadIdx.x * kLuStride, piv_now, v);
-#pragma unroll
-      for (int e = 0; e < 10; ++e) shb[threadIdx.x * kVecStride + e] = v[e];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < 10; ++e) {
-      const int c = threadIdx.x + e * kLuThreads;
-      if (c < 10 * m) x[blk0 * 10 + c] = shb[(c / 10) * kVecStride + c % 10];
+    if (blk0 + threadIdx.x < nb) {
+      lus10(sh + buf * (kLuThreads * kLuStride) + threadIdx.x * kLuStride, piv_now, now);
+      store10(x + (blk0 + threadIdx.x) * 10, now);
     }
     __syncwarp();
   }
@@ -171,7 +194,7 @@ int block_lu_factor(long nb, double* A, int* piv, int* d_info, cudaStream_t s) {
 
 int block_lu_solve(long nb, const double* LU, const int* piv, const double* b, double* x,
                    cudaStream_t s) {
-  const size_t shm = sizeof(double) * (2 * kLuStride + kVecStride) * kLuThreads;
+  const size_t shm = sizeof(double) * 2 * kLuStride * kLuThreads;
   GBMV_CUDA_TRY(cudaFuncSetAttribute(block_lu_solve_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
   ProfScope ps("block_lu_solve", s);
