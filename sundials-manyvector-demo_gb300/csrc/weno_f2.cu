@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(128, MINB)
       L31 = u * gc;
     }
     bool ok = true;
-    f2v P[5][5];  // [pair][characteristic component]
+    const f2 has = f2_scale(ha, kF2Scale);
+    f2v P[5][5];  // [pair][characteristic component], times kF2Scale
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       const int a = k, b = 5 - k;
@@ -154,10 +155,10 @@ __global__ void __launch_bounds__(128, MINB)
         Wj[m] = f2v(val(m, a), val(m, b));
         ok = ok && f2v_absmax(Wj[m]) < 1e15f;
       }
-      const f2v pj = f2v_scale(f2v(pressure(a), pressure(b)), 0.5f);
-      ok = ok && fminf(Wj[0].hi.x, Wj[0].hi.y) > 0.f && f2v_absmax(pj) < 5e14f;
+      const f2v pj = f2v_scale(f2v(pressure(a), pressure(b)), 0.5f * kF2Scale);
+      ok = ok && fminf(Wj[0].hi.x, Wj[0].hi.y) > 0.f && f2v_absmax(pj) < 5e14f * kF2Scale;
       const f2 ua = velocity(a), ub = velocity(b);
-      const f2v h = split_pair(ua, ub, ha), uj(ua, ub);
+      const f2v h = split_pair(ua, ub, has, kF2Scale), uj(ua, ub);
       const f2v f0 = Wj[0] * h, f1 = f2v_fma(Wj[1], h, pj), f2_ = Wj[2] * h, f3 = Wj[3] * h,
                 f4 = f2v_norm(f2v_add_prod(f2v_prod(Wj[4], h), uj, pj));
       const f2v X = f2v_norm(
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(128, MINB)
 #pragma unroll
       for (int i = 0; i < 5; ++i) {
         const f2v r = weno_pair<0>(P[0][i], P[1][i], P[2][i], P[3][i], P[4][i]);
-        ff[i] = r.x() + r.y();
+        ff[i] = f2_scale(r.x() + r.y(), 1.f / kF2Scale);
       }
       // right eigenvector columns (src/utilities.cpp:318-340)
       const f2 t = ff[0] + ff[4], s = t + ff[3], cd = c * (ff[4] - ff[0]);
@@ -210,7 +211,8 @@ __global__ void __launch_bounds__(128, WV == 1 ? kTracerFastMinB : kTracerMinB)
     f2v h[5];
     {
       const float2 t = F[5 * D.nfaces + f];
-      const f2 ha(t.x, t.y);
+      const float sc = WV == 1 ? 1.f : kF2Scale;
+      const f2 ha(sc * t.x, sc * t.y);
       f2 u[6];
 #pragma unroll
       for (int l = 0; l < 6; ++l) {
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(128, WV == 1 ? kTracerFastMinB : kTracerMinB)
         if ((T.nnorm >> l) & 1u) u[l] = -u[l];
       }
 #pragma unroll
-      for (int k = 0; k < 5; ++k) h[k] = split_pair(u[k], u[5 - k], ha);
+      for (int k = 0; k < 5; ++k) h[k] = split_pair(u[k], u[5 - k], ha, sc);
     }
 #pragma unroll 1
     for (int c = 0; c < nchem; ++c) {

@@ -41,17 +41,23 @@ __device__ __forceinline__ float weno_scale(float a, float b, float c) {
   return __int_as_float((127 - two / 2) << 23);
 }
 
+// The float-float reconstructions work on kF2Scale times the fluxes (the split factors and the
+// pressure carry it, so it costs nothing there): the weights' numerator holds eps^4 times a flux
+// difference, whose low part would leave the float range for fluxes below 5e-7; scaled, for fluxes
+// below 3e-23.
+constexpr float kF2Scale = 64.f;
+
 // Both reconstructions of a face (lane x the plus side, lane y the minus side with its stencil
-// reversed): weno_diff64's formula.  The weights' products hold a^4: for a up to 2^25 (jumps up
-// to ~1000) they stay in the float range as they are, beyond that the a_k are scaled by a common
-// power of two, which the weights do not see.  One out-of-line copy serves every reconstruction
-// of a face (the kernel stays inside the instruction cache).
+// reversed), scaled values in and out: weno_diff64's formula.  The weights' products hold a^4: for
+// a up to 2^28 (flux jumps up to ~100) they stay in the float range as they are, beyond that the
+// a_k are scaled by a common power of two, which the weights do not see.  One out-of-line copy
+// serves every reconstruction of a face (the kernel stays inside the instruction cache).
 static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4) {
   const f2v D01 = f0 - f1, D12 = f1 - f2_, D23 = f2_ - f3, D34 = f3 - f4;
   const f2v D23x2 = f2v_scale(D23, 2.f);
   f2v aA, aB, aC;
   {
-    const f2v K{f2(kWenoK)}, eps{f2(kWenoEps)};
+    const f2v K{f2(kWenoK)}, eps{f2(kWenoEps * kF2Scale * kF2Scale)};
     const f2v dA = D23 - D34, dB = D12 - D23, dC = D01 - D12;  // second differences
     const f2v eA = dA + D23x2, eB = D12 + D23, eC = dC - f2v_scale(D12, 2.f);
     aA = f2v_norm(f2v_add_prod(f2v_add_prod(eps, dA, dA), f2v_prod(K, eA), eA));
@@ -60,7 +66,7 @@ static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3
   }
   const float top = fmaxf(fmaxf(fmaxf(aA.hi.x, aB.hi.x), aC.hi.x),
                           fmaxf(fmaxf(aA.hi.y, aB.hi.y), aC.hi.y));
-  if (top > 33554432.f) {
+  if (top > 268435456.f) {
     const float2 s = make_float2(weno_scale(aA.hi.x, aB.hi.x, aC.hi.x),
                                  weno_scale(aA.hi.y, aB.hi.y, aC.hi.y));
     aA = f2v(mul2(aA.hi, s), mul2(aA.lo, s));
@@ -113,15 +119,17 @@ __device__ __forceinline__ f2v weno_plus_f2dv(f2v f0, f2v f1, f2v f2_, f2v f3, f
   return f2_ + f2v(corr, make_float2(0.f, 0.f));
 }
 
-// one lane in FP64
-static __device__ __noinline__ f2 weno_fallback64(f2 f0, f2 f1, f2 f2_, f2 f3, f2 f4) {
-  return f2_from_double(weno_plus64(f0.to_double(), f1.to_double(), f2_.to_double(),
-                                    f3.to_double(), f4.to_double()));
+// one lane in FP64 (s: the values' scale)
+static __device__ __noinline__ f2 weno_fallback64(double s, f2 f0, f2 f1, f2 f2_, f2 f3, f2 f4) {
+  const double t = 1.0 / s;
+  return f2_from_double(s * weno_plus64(t * f0.to_double(), t * f1.to_double(),
+                                        t * f2_.to_double(), t * f3.to_double(),
+                                        t * f4.to_double()));
 }
 __device__ __forceinline__ float f2v_absmax(f2v a) {
   return fmaxf(fabsf(a.hi.x), fabsf(a.hi.y));
 }
-// WV = 0: weights in float-float; WV = 1: the correction form with FP32 weights
+// WV = 0: weights in float-float, scaled values; WV = 1: the correction form with FP32 weights
 template <int WV>
 __device__ __forceinline__ f2v weno_pair(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4) {
   const float mx = fmaxf(fmaxf(fmaxf(f2v_absmax(f0), f2v_absmax(f1)),
@@ -130,23 +138,27 @@ __device__ __forceinline__ f2v weno_pair(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4
     if constexpr (WV == 1) return weno_plus_f2dv(f0, f1, f2_, f3, f4);
     else return weno_plus_f2v(f0, f1, f2_, f3, f4);
   }
-  return f2v(weno_fallback64(f0.x(), f1.x(), f2_.x(), f3.x(), f4.x()),
-             weno_fallback64(f0.y(), f1.y(), f2_.y(), f3.y(), f4.y()));
+  const double s = WV == 1 ? 1.0 : (double)kF2Scale;
+  return f2v(weno_fallback64(s, f0.x(), f1.x(), f2_.x(), f3.x(), f4.x()),
+             weno_fallback64(s, f0.y(), f1.y(), f2_.y(), f3.y(), f4.y()));
 }
 
-// split factors of a pair of points, (u +- alpha)/2: lane x the plus side, lane y the minus side
-__device__ __forceinline__ f2v split_pair(f2 ua, f2 ub, f2 ha) {
-  return f2v_scale(f2v(ua, ub), 0.5f) + f2v(ha, -ha);
+// split factors of a pair of points, s (u +- alpha)/2 with ha = s alpha/2: lane x the plus side,
+// lane y the minus side
+__device__ __forceinline__ f2v split_pair(f2 ua, f2 ub, f2 ha, float s) {
+  return f2v_scale(f2v(ua, ub), 0.5f * s) + f2v(ha, -ha);
 }
 
-// one advected field: pair k holds c_k (u_k + alpha)/2 and c_{5-k} (u_{5-k} - alpha)/2
+// one advected field: pair k holds c_k (u_k + alpha)/2 and c_{5-k} (u_{5-k} - alpha)/2, scaled
+// for WV = 0
 template <int WV>
 __device__ __forceinline__ f2 tracer_face_flux_f2v(const f2v (&h)[5], const f2 (&cv)[6]) {
   f2v a[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) a[k] = f2v(cv[k], cv[5 - k]) * h[k];
   const f2v r = weno_pair<WV>(a[0], a[1], a[2], a[3], a[4]);
-  return r.x() + r.y();
+  const f2 o = r.x() + r.y();
+  return WV == 1 ? o : f2_scale(o, 1.f / kF2Scale);
 }
 
 }  // namespace gbmv
