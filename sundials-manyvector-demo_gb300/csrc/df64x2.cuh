@@ -79,6 +79,10 @@ __device__ __forceinline__ f2v f2v_add_prod(f2v s, f2v x, f2v y) {  // s + x y
   const float2 e = add2(add2(s.lo, t.lo), p.lo);
   return f2v(t.hi, fma2(x.hi, y.lo, fma2(x.lo, y.hi, e)));
 }
+__device__ __forceinline__ f2v f2v_sum(f2v x, f2v y) {  // x + y
+  const f2v s = two_sum2(x.hi, y.hi);
+  return f2v(s.hi, add2(s.lo, add2(x.lo, y.lo)));
+}
 __device__ __forceinline__ f2v f2v_norm(f2v x) { return quick_two_sum2(x.hi, x.lo); }
 // x y + z
 __device__ __forceinline__ f2v f2v_fma(f2v x, f2v y, f2v z) {

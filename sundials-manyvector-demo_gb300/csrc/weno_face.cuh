@@ -58,8 +58,10 @@ static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3
   f2v aA, aB, aC;
   {
     const f2v K{f2(kWenoK)}, eps{f2(kWenoEps * kF2Scale * kF2Scale)};
-    const f2v dA = D23 - D34, dB = D12 - D23, dC = D01 - D12;  // second differences
-    const f2v eA = dA + D23x2, eB = D12 + D23, eC = dC - f2v_scale(D12, 2.f);
+    // (not renormalised: d and e never both cancel against the differences they are built of, so
+    // what a product of them drops stays below 2^-48 of a_k)
+    const f2v dA = f2v_sum(D23, -D34), dB = f2v_sum(D12, -D23), dC = f2v_sum(D01, -D12);
+    const f2v eA = f2v_sum(dA, D23x2), eB = f2v_sum(D12, D23), eC = f2v_sum(dC, f2v_scale(D12, -2.f));
     aA = f2v_norm(f2v_add_prod(f2v_add_prod(eps, dA, dA), f2v_prod(K, eA), eA));
     aB = f2v_norm(f2v_add_prod(f2v_add_prod(eps, dB, dB), f2v_prod(K, eB), eB));
     aC = f2v_norm(f2v_add_prod(f2v_add_prod(eps, dC, dC), f2v_prod(K, eC), eC));
@@ -77,8 +79,8 @@ static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3
   const f2v sA = f2v_prod(PA, PA), sB = f2v_prod(PB, PB), sC = f2v_prod(PC, PC);
   const f2v den = f2v_norm(f2v_add_scaled(f2v_add_scaled(sC, 3.f, sA), 6.f, sB));
   // 3 sA (qA - f2) + 6 sB (qB - f2) + sC (qC - f2)
-  const f2v cA = f2v_scale(D34, 0.5f) - D23x2, cB = -(D12 + D23x2);
-  const f2v cC = f2v_norm(f2v_add_prod(f2v_prod(f2v(f2(1.0 / 3.0)), D01), f2v(f2(-5.0 / 6.0)), D12));
+  const f2v cA = f2v_sum(f2v_scale(D34, 0.5f), -D23x2), cB = -f2v_sum(D12, D23x2);
+  const f2v cC = f2v_add_prod(f2v_prod(f2v(f2(1.0 / 3.0)), D01), f2v(f2(-5.0 / 6.0)), D12);
   const f2v num = f2v_norm(f2v_add_prod(f2v_add_prod(f2v_prod(sA, cA), sB, cB), sC, cC));
   return f2_ + f2v_quot(num, den);
 }
