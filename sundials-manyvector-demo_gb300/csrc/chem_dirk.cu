@@ -442,7 +442,8 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
           for (int s = 0; s < 10; ++s) u[s] = to_lu<LU>(g[s] * pow2(EQ[s * BS]));
           lus10_strided<LU, LU>(L, BS, piv, u);
 #pragma unroll
-          for (int s = 0; s < 10; ++s) dl[s] = from_lu(u[s]) * pow2(EQ[(10 + s) * BS]);
+          for (int s = 0; s < 10; ++s)  // (without REF the column scales are all 1)
+            dl[s] = REF ? from_lu(u[s]) * pow2(EQ[(10 + s) * BS]) : from_lu(u[s]);
           if (REF) {
             for (int it = 0; it < O.refine; ++it) {  // r = g - A dl in FP64, solve, update
               double r[10];
