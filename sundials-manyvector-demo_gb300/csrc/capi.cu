@@ -396,10 +396,17 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
   double* dh = (double*)calloc(tab_doubles, sizeof(double));
   double* lh = (double*)malloc(sizeof(double) * ltab_doubles);
   if (!gh || !dh || !lh) { free(h); free(gh); free(dh); free(lh); delete c; return GBMV_ENOMEM; }
-  for (int q = 0; q < kLogEntries; ++q) {  // 1/c and log c of each interval's midpoint (chem_log)
-    const double mid = ldexp(1.0 + ((q & 127) + 0.5) / 128.0, (q >> 7) - 2);
-    lh[2 * q] = 1.0 / mid;
-    lh[2 * q + 1] = (double)-logl((long double)lh[2 * q]);
+  // 1/c and -log(1/c) of each interval's midpoint c (chem_log); the intervals repeat from one
+  // binade to the next, so 128 logarithms do (a long double one takes ~0.6 us on the Arm host)
+  const long double ln2 = logl(2.0L);
+  for (int k = 0; k < 128; ++k) {
+    const double inv = 1.0 / (1.0 + (k + 0.5) / 128.0);
+    const long double log_inv = logl((long double)inv);
+    for (int q = k; q < kLogEntries; q += 128) {
+      const int e = (q >> 7) - 2;
+      lh[2 * q] = ldexp(inv, -e);
+      lh[2 * q + 1] = (double)(e * ln2 - log_inv);
+    }
   }
   for (int b = 0; b + 1 < kTSize; ++b)
     for (int r = 0; r < kNT; ++r) dh[b * kNT + r] = h[(b + 1) * kNT + r] - h[b * kNT + r];
