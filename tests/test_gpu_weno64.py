@@ -75,3 +75,31 @@ def test_jvp_in_place_matches_out_of_place(cuda, nchem):
     h.fEuler_jvp(0.0, w, d, d)
     for a, b in zip(d, out):
         assert maxnorm_err(a.cpu().numpy(), b.cpu().numpy()) <= 1e-12
+
+
+def test_fp64_sweeps_at_large_densities(cuda):
+    """Flux jumps beyond 2^112 take the scaled weights.  The equations are homogeneous of degree one
+    in the conserved fields and the tracers, and so is the scheme where the weights' 1e-6 is
+    negligible: from densities in 2^60 to 2^200 the right-hand side scales, the derivatives stay.
+    All factors are powers of two, so only the roundings of the scaled weights differ: 1e-12."""
+    torch = cuda
+    import gbmv
+    shape, nchem = (11, 9, 7), 4
+    wl = W.rayleigh_taylor(shape=shape, nchem=nchem, seed=W.SEED_BASE + 703)
+    h = gbmv.Hydro(shape, nchem, (3, 3, 0, 0, 1, 3), wl["gamma"], None)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    v = [torch.rand(f.shape, generator=gen, device="cuda", dtype=torch.float64) - 0.5
+         for f in wl["fields"]]
+    res = []
+    for lam in (2.0 ** 60, 2.0 ** 200):
+        w = [lam * torch.from_numpy(np.ascontiguousarray(f)).cuda() for f in wl["fields"]]
+        f, jv, u = ([torch.empty_like(x) for x in w] for _ in range(3))
+        assert h.fEuler(0.0, w, f) == 0
+        h.fEuler_jvp(0.0, w, v, jv)
+        h.fEuler_vjp(0.0, w, v, u)
+        _, ref = O.feuler([x.cpu().numpy() for x in w], nchem, (3, 3, 0, 0, 1, 3), wl["gamma"], None)
+        for a, r in zip(f, ref):
+            assert maxnorm_err(a.cpu().numpy(), r) <= 1e-12
+        res.append([x.cpu().numpy() / lam for x in f] + [x.cpu().numpy() for x in jv + u])
+    for a, b in zip(*res):
+        assert maxnorm_err(a, b) <= 1e-12
