@@ -72,6 +72,29 @@ ProfScope::~ProfScope() {
 
 using namespace gbmv;
 
+// What a synchronous call reads back, in page-locked host memory that its kernels write directly
+// (status words only where a state is illegal or a block singular): no clearing launch and no copy
+// on the stream, which for a 128 x 3 x 3 right-hand side were 10 of 44 us (the copy into pageable
+// memory is staged by the driver).
+struct HostWords {
+  int flags;       // legal-state mask of the flow; singular block of a chemistry or block handle
+  double sums[2];  // norm, totals
+  unsigned long long speed;
+};
+static bool host_words(HostWords** p) {
+  return cudaHostAlloc(reinterpret_cast<void**>(p), sizeof(HostWords),
+                       cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess;
+}
+// the end of a synchronous call whose launches returned rc (after a failed launch the earlier ones
+// are waited for: they must not write into the next call's words)
+static int finish(int rc, cudaStream_t s) {
+  if (rc && rc != GBMV_ECUDA) return rc;
+  const cudaError_t e = cudaStreamSynchronize(s);
+  if (rc) return rc;
+  return e == cudaSuccess ? GBMV_OK : check_cuda(e, "cudaStreamSynchronize(s)");
+}
+static int flags_of(const HostWords* w) { return *static_cast<const volatile int*>(&w->flags); }
+
 struct gbmv_hydro_s {
   Grid g;
   ForceTerm force;
@@ -80,7 +103,8 @@ struct gbmv_hydro_s {
   float* prims = nullptr;  // float-float per-cell primitives of the mixed form (first use)
   double* adj = nullptr;   // per-face stencil cotangents of the VJP (first use)
   double* cons = nullptr;  // conservation-sum partials (first use)
-  int* d_status = nullptr;
+  int* d_status = nullptr;  // scratch status of the autotuner's launches
+  HostWords* host = nullptr;
   int sweep_threads[3] = {0, 0, 0};  // face-sweep threads per block per precision (0: by size)
   int sweep_shared = 0;               // GBMV_SWEEPS_SHARED register budget
 };
@@ -91,6 +115,7 @@ struct gbmv_chem_s {
   ChemState S{};
   double* tab = nullptr;
   double* cell = nullptr;  // one allocation for all per-cell arrays
+  HostWords* host = nullptr;
   int* d_info = nullptr;               // first word of a 64-byte control block:
   int* d_nfail = nullptr;              //   [0] info, [1] failed cells,
   unsigned long long* d_next = nullptr;  //   [16] DIRK work counter
@@ -213,10 +238,11 @@ int gbmv_hydro_create(const gbmv_grid* grid, gbmv_hydro* out) {
   memset(&h->force, 0, sizeof h->force);
   h->scratch_doubles = feuler_fp64_scratch_doubles(h->g);
   if (cudaMalloc(&h->scratch, h->scratch_doubles * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->d_status, 2 * sizeof(double)) != cudaSuccess) {
+      cudaMalloc(&h->d_status, 2 * sizeof(double)) != cudaSuccess || !host_words(&h->host)) {
     cudaGetLastError();
     set_error("device allocation of %zu flux doubles failed", h->scratch_doubles);
     cudaFree(h->scratch);
+    cudaFree(h->d_status);
     delete h;
     return GBMV_ENOMEM;
   }
@@ -231,6 +257,7 @@ int gbmv_hydro_destroy(gbmv_hydro h) {
   cudaFree(h->adj);
   cudaFree(h->cons);
   cudaFree(h->d_status);
+  cudaFreeHost(h->host);
   delete h;
   return GBMV_OK;
 }
@@ -359,13 +386,10 @@ int gbmv_feuler(gbmv_hydro h, double t, const double* const* w, double* const* w
                 int precision, void* stream) {
   if (!h) return GBMV_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
-  GBMV_CUDA_TRY(cudaMemsetAsync(h->d_status, 0, sizeof(int), s));
-  int rc = gbmv_feuler_async(h, t, w, wdot, precision, 0, h->d_status, stream);
-  if (rc) return rc;
-  int st = 0;
-  GBMV_CUDA_TRY(cudaMemcpyAsync(&st, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
-  GBMV_CUDA_TRY(cudaStreamSynchronize(s));
-  if (st) {
+  h->host->flags = 0;
+  if (int rc = finish(gbmv_feuler_async(h, t, w, wdot, precision, 0, &h->host->flags, stream), s))
+    return rc;
+  if (const int st = flags_of(h->host)) {
     set_error("illegal state (mask %d: 1 density, 2 energy, 4 pressure)", st);
     return GBMV_ILLEGAL_STATE;
   }
@@ -421,7 +445,7 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
   if (cudaMalloc(&c->tab, sizeof(double) * (2 * tab_doubles + ltab_doubles) +
                               sizeof(float) * gtab_floats) != cudaSuccess ||
       cudaMalloc(&c->cell, sizeof(double) * per_cell * ncells) != cudaSuccess ||
-      cudaMalloc(&c->d_info, 64) != cudaSuccess) {
+      cudaMalloc(&c->d_info, 64) != cudaSuccess || !host_words(&c->host)) {
     cudaGetLastError();
     free(h);
     free(gh);
@@ -429,6 +453,7 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
     free(lh);
     cudaFree(c->tab);
     cudaFree(c->cell);
+    cudaFree(c->d_info);
     delete c;
     set_error("device allocation failed for %ld cells", ncells);
     return GBMV_ENOMEM;
@@ -494,6 +519,7 @@ int gbmv_chem_destroy(gbmv_chem c) {
   cudaFree(c->tab);
   cudaFree(c->cell);
   cudaFree(c->d_info);
+  cudaFreeHost(c->host);
   cudaFree(c->dirk_k);
   cudaFree(c->dirk_retry);
   cudaFree(c->dirk_order_buf);
@@ -590,14 +616,12 @@ static int newton_sync(gbmv_chem c, const double* y, const double* b, double* f,
     return GBMV_EINVAL;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  GBMV_CUDA_TRY(cudaMemsetAsync(c->d_info, 0, sizeof(int), s));
-  int rc = chem_newton(c->P, c->S, c->n, y, f, x, gamma, time_units, lu_precision == GBMV_MIXED,
-                       refine, c->d_info, s, c->newton_bps, b);
-  if (rc) return rc;
-  int h = 0;
-  GBMV_CUDA_TRY(cudaMemcpyAsync(&h, c->d_info, sizeof(int), cudaMemcpyDeviceToHost, s));
-  GBMV_CUDA_TRY(cudaStreamSynchronize(s));
-  if (h) { set_error("singular Newton block"); return 1; }
+  c->host->flags = 0;
+  if (int rc = finish(chem_newton(c->P, c->S, c->n, y, f, x, gamma, time_units,
+                                  lu_precision == GBMV_MIXED, refine, &c->host->flags, s,
+                                  c->newton_bps, b), s))
+    return rc;
+  if (flags_of(c->host)) { set_error("singular Newton block"); return 1; }
   return GBMV_OK;
 }
 
@@ -1016,11 +1040,11 @@ int gbmv_block_lu_factor(long nblocks, double* A, int* pivots, void* stream) {
   return GBMV_OK;
 }
 
-// Block linear solver handle: owns the pivots and its own singular-block word.
+// Block linear solver handle: owns the pivots and its own singular-block word (host->flags).
 struct gbmv_block_ls_s {
   long nblocks = 0;
   int* pivots = nullptr;
-  int* d_info = nullptr;
+  HostWords* host = nullptr;
 };
 
 int gbmv_block_ls_create(long nblocks, gbmv_block_ls* out) {
@@ -1030,7 +1054,7 @@ int gbmv_block_ls_create(long nblocks, gbmv_block_ls* out) {
   if (!L) return GBMV_ENOMEM;
   L->nblocks = nblocks;
   if (cudaMalloc(&L->pivots, sizeof(int) * 10 * nblocks) != cudaSuccess ||
-      cudaMalloc(&L->d_info, sizeof(int)) != cudaSuccess) {
+      !host_words(&L->host)) {
     cudaGetLastError();
     cudaFree(L->pivots);
     delete L;
@@ -1044,7 +1068,7 @@ int gbmv_block_ls_create(long nblocks, gbmv_block_ls* out) {
 int gbmv_block_ls_destroy(gbmv_block_ls L) {
   if (!L) return GBMV_OK;
   cudaFree(L->pivots);
-  cudaFree(L->d_info);
+  cudaFreeHost(L->host);
   delete L;
   return GBMV_OK;
 }
@@ -1052,13 +1076,9 @@ int gbmv_block_ls_destroy(gbmv_block_ls L) {
 int gbmv_block_ls_setup(gbmv_block_ls L, double* A, void* stream) {
   if (!L || !A) { set_error("null block solver or matrix"); return GBMV_EINVAL; }
   cudaStream_t s = (cudaStream_t)stream;
-  GBMV_CUDA_TRY(cudaMemsetAsync(L->d_info, 0, sizeof(int), s));
-  int rc = block_lu_factor(L->nblocks, A, L->pivots, L->d_info, s);
-  if (rc) return rc;
-  int h = 0;
-  GBMV_CUDA_TRY(cudaMemcpyAsync(&h, L->d_info, sizeof(int), cudaMemcpyDeviceToHost, s));
-  GBMV_CUDA_TRY(cudaStreamSynchronize(s));
-  if (h) { set_error("singular block"); return 1; }
+  L->host->flags = 0;
+  if (int rc = finish(block_lu_factor(L->nblocks, A, L->pivots, &L->host->flags, s), s)) return rc;
+  if (flags_of(L->host)) { set_error("singular block"); return 1; }
   return GBMV_OK;
 }
 
@@ -1111,13 +1131,11 @@ int gbmv_fexpl(gbmv_hydro h, gbmv_chem c, double t, double* const* w, double* co
   }
   if (!fields_ok(w, 10) || !fields_ok(wdot, 10)) return GBMV_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
-  GBMV_CUDA_TRY(cudaMemsetAsync(h->d_status, 0, sizeof(int), s));
-  int rc = gbmv_fexpl_async(h, c, t, w, wdot, energy_units, precision, h->d_status, stream);
-  if (rc) return rc;
-  int st = 0;
-  GBMV_CUDA_TRY(cudaMemcpyAsync(&st, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
-  GBMV_CUDA_TRY(cudaStreamSynchronize(s));
-  if (st) {
+  h->host->flags = 0;
+  if (int rc = finish(gbmv_fexpl_async(h, c, t, w, wdot, energy_units, precision, &h->host->flags,
+                                       stream), s))
+    return rc;
+  if (const int st = flags_of(h->host)) {
     set_error("illegal state (mask %d: 1 density, 2 energy, 4 pressure)", st);
     return GBMV_ILLEGAL_STATE;
   }
@@ -1350,12 +1368,8 @@ int gbmv_conservation(gbmv_hydro h, const double* const* w, double mass_factor,
   if (int rc = reduction_scratch(h, s, "gbmv_conservation")) return rc;
   Fields W;
   for (int v = 0; v < 6; ++v) W.f[v] = (v < 5) ? const_cast<double*>(w[v]) : nullptr;
-  int rc = conservation_sums(h->g, W, h->cons, s);
-  if (rc) return rc;
-  double t[2];
-  GBMV_CUDA_TRY(cudaMemcpyAsync(t, h->cons + conservation_scratch_doubles() - 2, sizeof t,
-                                cudaMemcpyDeviceToHost, s));
-  GBMV_CUDA_TRY(cudaStreamSynchronize(s));
+  if (int rc = finish(conservation_sums(h->g, W, h->cons, h->host->sums, s), s)) return rc;
+  const volatile double* const t = h->host->sums;
   totals[0] = t[0] * mass_factor;
   totals[1] = t[1] * energy_factor;
   return GBMV_OK;
@@ -1378,11 +1392,8 @@ int gbmv_wrms_norm(gbmv_hydro h, const double* const* v, const double* const* y,
     V.f[k] = const_cast<double*>(v[k]);
     Y.f[k] = const_cast<double*>(y[k]);
   }
-  int rc = wrms_norm(h->g, V, Y, rtol, atol, h->cons, s);
-  if (rc) return rc;
-  GBMV_CUDA_TRY(cudaMemcpyAsync(norm, h->cons + conservation_scratch_doubles() - 2,
-                                sizeof(double), cudaMemcpyDeviceToHost, s));
-  GBMV_CUDA_TRY(cudaStreamSynchronize(s));
+  if (int rc = finish(wrms_norm(h->g, V, Y, rtol, atol, h->cons, h->host->sums, s), s)) return rc;
+  *norm = *static_cast<const volatile double*>(h->host->sums);
   return GBMV_OK;
 }
 
@@ -1418,11 +1429,7 @@ int gbmv_wrms_norm_async(gbmv_hydro h, const double* const* v, const double* con
     V.f[k] = const_cast<double*>(v[k]);
     Y.f[k] = const_cast<double*>(y[k]);
   }
-  int rc = wrms_norm(h->g, V, Y, rtol, atol, h->cons, s);
-  if (rc) return rc;
-  GBMV_CUDA_TRY(cudaMemcpyAsync(d_norm, h->cons + conservation_scratch_doubles() - 2,
-                                sizeof(double), cudaMemcpyDeviceToDevice, s));
-  return GBMV_OK;
+  return wrms_norm(h->g, V, Y, rtol, atol, h->cons, d_norm, s);
 }
 
 int gbmv_print_stats(gbmv_hydro h, const double* const* w, double density_units,
@@ -1453,9 +1460,9 @@ int gbmv_stability(gbmv_hydro h, const double* const* w, double cfl, double* dt_
   unsigned long long* d = reinterpret_cast<unsigned long long*>(h->d_status);  // 8-byte slot
   int rc = wave_speed_max(h->g, W, d, s);
   if (rc) return rc;
-  unsigned long long bits = 0;
-  GBMV_CUDA_TRY(cudaMemcpyAsync(&bits, d, sizeof bits, cudaMemcpyDeviceToHost, s));
+  GBMV_CUDA_TRY(cudaMemcpyAsync(&h->host->speed, d, sizeof *d, cudaMemcpyDeviceToHost, s));
   GBMV_CUDA_TRY(cudaStreamSynchronize(s));
+  const unsigned long long bits = h->host->speed;
   double alpha;
   memcpy(&alpha, &bits, sizeof alpha);
   const double dmin = fmin(fmin(h->g.d[0], h->g.d[1]), h->g.d[2]);

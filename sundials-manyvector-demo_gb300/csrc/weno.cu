@@ -488,22 +488,20 @@ __global__ void __launch_bounds__(256) conservation_final_kernel(const double* _
   if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
-int conservation_sums(const Grid& g, const Fields& w, double* d_scratch, cudaStream_t s) {
+int conservation_sums(const Grid& g, const Fields& w, double* d_scratch, double* out,
+                      cudaStream_t s) {
   conservation_partial_kernel<<<kConsBlocks, 256, 0, s>>>(g.ncell, w.f[0], w.f[4], d_scratch);
   GBMV_LAUNCH_CHECK("conservation_partial_kernel");
-  conservation_final_kernel<<<2, 256, 0, s>>>(d_scratch, d_scratch + 2 * kConsBlocks);
+  conservation_final_kernel<<<2, 256, 0, s>>>(d_scratch, out);
   GBMV_LAUNCH_CHECK("conservation_final_kernel");
   return GBMV_OK;
 }
-
-size_t conservation_scratch_doubles() { return 2 * kConsBlocks + 2; }
 
 // N_VWrmsNorm of the six-component ManyVector (the norm ARKODE's error test and Newton
 // convergence test take, src/imex_chem_hydro_main.cpp:463): ewt = 1 / (rtol |y| + atol) per
 // entry, sum of (v ewt)^2 over the five fluid fields (ncell each) and the chemistry field
 // (nchem ncell), divided by the total length, square root.  Same fixed-grid compensated
-// two-pass reduction as the conservation totals; partials in scratch[0..kConsBlocks), result
-// in scratch[2 kConsBlocks].
+// two-pass reduction as the conservation totals; partials in scratch[0..kConsBlocks).
 __global__ void __launch_bounds__(256) wrms_partial_kernel(long ncell, int nchem, Fields v,
                                                            Fields y, double rtol, double atol,
                                                            double* __restrict__ part) {
@@ -550,11 +548,11 @@ __global__ void __launch_bounds__(256) wrms_final_kernel(const double* __restric
 }
 
 int wrms_norm(const Grid& g, const Fields& v, const Fields& y, double rtol, double atol,
-              double* d_scratch, cudaStream_t s) {
+              double* d_scratch, double* out, cudaStream_t s) {
   wrms_partial_kernel<<<kConsBlocks, 256, 0, s>>>(g.ncell, g.nchem, v, y, rtol, atol, d_scratch);
   GBMV_LAUNCH_CHECK("wrms_partial_kernel");
   const double ntotal = (double)(5 + g.nchem) * (double)g.ncell;
-  wrms_final_kernel<<<1, 256, 0, s>>>(d_scratch, ntotal, d_scratch + 2 * kConsBlocks);
+  wrms_final_kernel<<<1, 256, 0, s>>>(d_scratch, ntotal, out);
   GBMV_LAUNCH_CHECK("wrms_final_kernel");
   return GBMV_OK;
 }

@@ -37,15 +37,14 @@ int divergence_f2(const Grid& g, const Fields& wdot, float2* const (&F)[3], cons
 
 int wave_speed_max(const Grid& g, const Fields& w, unsigned long long* d_out, cudaStream_t s);
 int pack1d(const Grid& g, const Fields& w, int dir, double* out, cudaStream_t s);
-// totals of rho and et into d_scratch[2 * 1024 + 0..1] (scratch: conservation_scratch_doubles)
-size_t conservation_scratch_doubles();
-int conservation_sums(const Grid& g, const Fields& w, double* d_scratch, cudaStream_t s);
-// ManyVector WRMS norm of v with weights 1 / (rtol |y| + atol) into
-// d_scratch[conservation_scratch_doubles() - 2] (scratch: conservation_scratch_doubles)
+// Reductions: every one of a handle shares one scratch of reduction_scratch_doubles(); out is
+// device memory or mapped host memory.  Totals of rho and et into out[0..1];
+int conservation_sums(const Grid& g, const Fields& w, double* d_scratch, double* out,
+                      cudaStream_t s);
+// ManyVector WRMS norm of v with weights 1 / (rtol |y| + atol) into *out;
 int wrms_norm(const Grid& g, const Fields& v, const Fields& y, double rtol, double atol,
-              double* d_scratch, cudaStream_t s);
-// per-field RMS (print_stats) into d_scratch[16 * 1024 + v]; every reduction of a handle shares
-// one scratch of reduction_scratch_doubles() (>= conservation_scratch_doubles())
+              double* d_scratch, double* out, cudaStream_t s);
+// per-field RMS (print_stats) into d_scratch[16 * 1024 + v]
 size_t reduction_scratch_doubles();
 int field_rms(const Grid& g, const Fields& w, double du, double mu, double eu, double* d_scratch,
               cudaStream_t s);

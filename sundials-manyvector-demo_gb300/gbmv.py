@@ -205,8 +205,10 @@ def _dev_ptr(t):
 
 def _stream_ptr(stream):
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    # the current stream without the Stream object around it (3 us of a call's 12 us in Python)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _vec(fields):
