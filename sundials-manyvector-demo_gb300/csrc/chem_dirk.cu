@@ -148,8 +148,9 @@ struct DirkLayout {
   static constexpr size_t kL = 100 * sizeof(LU);                        // factor
   static constexpr size_t kA = REF ? 100 * sizeof(double) : 0;          // FP64 matrix
   static constexpr size_t kEq = sizeof(LU) == 4 ? 20 * sizeof(short) : 0;  // row/col exponents
+  static constexpr size_t kStep = 2 * sizeof(double);                   // step constants
   static constexpr size_t kPiv = 10;                                    // pivots (bytes)
-  static constexpr size_t per_lane = kVec + kEw + kL + kA + kEq + kPiv;
+  static constexpr size_t per_lane = kVec + kEw + kL + kA + kEq + kStep + kPiv;
   static constexpr size_t bytes = per_lane * BS;
 };
 
@@ -264,6 +265,10 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
   p += Lay::kEw * BS;
   short* const EQ = reinterpret_cast<short*>(p) + tid;    // row exponents [0,10), col [10,20)
   p += Lay::kEq * BS;
+  // constants of a step: 1/(h gamma) and the correction of a matrix set up at another h
+  double* const RG = reinterpret_cast<double*>(p) + tid;
+  double* const SC = RG + BS;
+  p += Lay::kStep * BS;
   signed char* const PV = reinterpret_cast<signed char*>(p) + tid;  // pivots
   const unsigned full = 0xffffffffu;
   const bool mixed_temp = O.mixed_temp != 0;
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
   bool jcur = false, force_setup = true, last = false;
   // step start requested / Newton-matrix setup pending (the lane waits for its warp's setup
   // pass) / passes waited
-  bool setup = false, pend = false;
+  bool setup = false, pend = false, base = false;
   int waited = 0;
   const int batch = O.setup_batch;
   const int max_wait = 4 * O.setup_batch;
@@ -335,16 +340,20 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
 #pragma unroll
       for (int s = 0; s < 10; ++s) {
         const double ys = Y[s * BS];
-        EW[s * BS] = (float)(1.0 / (O.rtol * fabs(ys) + O.atol));
+        // (a float: the reciprocal without the IEEE division is as good, at 5 FP64
+        // instructions for 9 -- nearly every pass of a warp has a lane starting a step)
+        EW[s * BS] = (float)rcp64_any(O.rtol * fabs(ys) + O.atol);
         Z[s * BS] = ys;  // trivial predictor
       }
-      const double gam = h * O.T.gamma;
-      if (force_setup || nst >= nst_lp + O.msbp || !(fabs(gam / gp - 1.0) <= O.dgmax)) {
+      const double gam = h * O.T.gamma, ratio = gam / gp;
+      RG[0] = 1.0 / gam;
+      if (force_setup || nst >= nst_lp + O.msbp || !(fabs(ratio - 1.0) <= O.dgmax)) {
         pend = true;
         waited = 0;
       } else {
+        SC[0] = 2.0 / (1.0 + ratio);
         stage = 1;
-        dirk_stage_base<BS>(O, stage, h, Y, K1, KG, kst, B);
+        base = true;
         m = 0;
         phase = kPhNewton;
       }
@@ -388,7 +397,7 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
             }
           } else {
             stage = 1;
-            dirk_stage_base<BS>(O, stage, h, Y, K1, KG, kst, B);
+            base = true;
             m = 0;
             phase = kPhNewton;
           }
@@ -396,6 +405,13 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
       } else if (pend) {
         ++waited;
       }
+    }
+
+    // ---- the base of a stage begun since the last pass, at one place for the lanes that began one
+    // in whatever way (a step without set-up, one after it, a deduced or a stored derivative)
+    if (base) {
+      base = false;
+      dirk_stage_base<BS>(O, stage, h, Y, K1, KG, kst, B);
     }
 
     // ---- one evaluation of F per pass (at Y for the first stage, else at the iterate)
@@ -463,7 +479,7 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
           }
         }
         if (gam != gp) {
-          const double sc = 2.0 / (1.0 + gam / gp);
+          const double sc = SC[0];
 #pragma unroll
           for (int s = 0; s < 10; ++s) dl[s] *= sc;
         }
@@ -490,20 +506,20 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
         ++m;
         ++c_nni;
         if (m > 1) crate = fmax(0.3 * crate, del / delp);
-        const double dcon = fmin(crate, 1.0) * del / O.nlscoef;
-        if (dcon <= 1.0 && O.deduce && stage < ns - 1) {
+        const bool converged = fmin(crate, 1.0) * del <= O.nlscoef;
+        if (converged && O.deduce && stage < ns - 1) {
           // converged intermediate stage, derivative deduced from the stage equation:
           // K_stage = (z - base) / (h gamma), no F evaluation; next stage in this pass.  One
           // reciprocal and ten products: nearly every pass of a warp has a lane deducing, and
           // ten FP64 divisions there cost as much FP64-pipe time as the F evaluations saved
-          const double rg = 1.0 / gam;
+          const double rg = RG[0];
 #pragma unroll
           for (int s = 0; s < 10; ++s)
             KG[((stage - 1) * 10 + s) * kst] = (Z[s * BS] - B[s * BS]) * rg;
           ++stage;
-          dirk_stage_base<BS>(O, stage, h, Y, K1, KG, kst, B);
+          base = true;
           m = 0;
-        } else if (dcon <= 1.0) {
+        } else if (converged) {
           phase = kPhStage;
         } else if ((m > 1 && del > 2.3 * delp) || m >= O.maxcor || !(del == del)) {
           // Newton failure: with a matrix from an earlier step set up a current one at the
@@ -524,7 +540,7 @@ __global__ void __launch_bounds__(BS) chem_dirk_kernel(ChemParams P, ChemState S
 #pragma unroll
         for (int s = 0; s < 10; ++s) KG[((stage - 1) * 10 + s) * kst] = f[s];
         ++stage;  // predictor: the converged value of this stage, already in Z
-        dirk_stage_base<BS>(O, stage, h, Y, K1, KG, kst, B);
+        base = true;
         m = 0;
         phase = kPhNewton;
       } else {  // kPhStage of the last stage: error test
