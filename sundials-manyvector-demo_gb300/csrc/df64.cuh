@@ -67,13 +67,6 @@ __device__ __forceinline__ f2 operator/(f2 x, f2 y) {
 // exact scaling by a power of two
 __device__ __forceinline__ f2 f2_scale(f2 x, float p2) { return f2(x.hi * p2, x.lo * p2); }
 
-// x^2 with the exact square of the high part
-__device__ __forceinline__ f2 f2_sqr(f2 x) {
-  f2 p = two_prod(x.hi, x.hi);
-  const float e = fmaf(2.f * x.hi, x.lo, p.lo);
-  return quick_two_sum(p.hi, e);
-}
-
 // exact split of a double into hi + lo (48 of its 53 significant bits survive)
 __device__ __forceinline__ f2 f2_from_double(double d) {
   const float h = __double2float_rn(d);
@@ -161,7 +154,6 @@ __device__ __forceinline__ bool operator>(f2 a, f2 b) { return b < a; }
 __device__ __forceinline__ bool operator<=(f2 a, f2 b) { return !(b < a); }
 __device__ __forceinline__ bool operator==(f2 a, f2 b) { return a.hi == b.hi && a.lo == b.lo; }
 __device__ __forceinline__ f2 f2_fabs(f2 a) { return a.hi < 0.f ? -a : a; }
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { return a * b + c; }
 
 // square root: FP32 estimate, one Newton correction in float-float
 __device__ __forceinline__ f2 f2_sqrt(f2 a) {

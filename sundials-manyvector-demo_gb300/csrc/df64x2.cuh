@@ -1,7 +1,7 @@
 // Two independent float-float numbers side by side: lane x and lane y of float2 registers,
 // operated on with the paired FP32 instructions of sm_100-class GPUs (__fadd2_rn, __fmul2_rn,
 // __ffma2_rn: one instruction performs the same IEEE round-to-nearest operation on both
-// lanes).  Every operation below is the df64.cuh algorithm of the same name applied to each
+// lanes).  Every operator below is the df64.cuh algorithm of the same name applied to each
 // lane, so lane x of a result equals, bit for bit, what the scalar f2 operation returns for
 // the lane-x operands (and likewise for y), in half the FP32 instructions.
 //
@@ -89,7 +89,7 @@ __device__ __forceinline__ f2v f2v_fma(f2v x, f2v y, f2v z) {
   return f2v_norm(f2v_add_prod(z, x, y));
 }
 // x / y from the approximate reciprocal, one residual (its leading part exact in an FMA) and one
-// correction: 10 operations where the general division below takes 25
+// correction: 10 operations where one with the remainder in float-float takes 25
 __device__ __forceinline__ f2v f2v_quot(f2v x, f2v y) {
   const float2 r = make_float2(__fdividef(1.f, y.hi.x), __fdividef(1.f, y.hi.y));
   const float2 q = mul2(x.hi, r), n = neg2(q);
@@ -97,32 +97,9 @@ __device__ __forceinline__ f2v f2v_quot(f2v x, f2v y) {
   return quick_two_sum2(q, mul2(t, r));
 }
 
-// as f2 operator/: approximate reciprocal (one per lane), q1, remainder in float-float, q2
-__device__ __forceinline__ f2v operator/(f2v x, f2v y) {
-  const float2 ry = make_float2(__fdividef(1.f, y.hi.x), __fdividef(1.f, y.hi.y));
-  const float2 q1 = mul2(x.hi, ry);
-  const f2v r = x - y * f2v(q1, make_float2(0.f, 0.f));
-  const float2 q2 = mul2(r.hi, ry);
-  return quick_two_sum2(q1, q2);
-}
-
 // exact scaling by a power of two
 __device__ __forceinline__ f2v f2v_scale(f2v x, float p2) {
   return f2v(mul2(x.hi, v2(p2)), mul2(x.lo, v2(p2)));
-}
-
-__device__ __forceinline__ f2v f2v_sqr(f2v x) {
-  const f2v p = two_prod2(x.hi, x.hi);
-  const float2 e = fma2(mul2(v2(2.f), x.hi), x.lo, p.lo);
-  return quick_two_sum2(p.hi, e);
-}
-
-// per-lane minimum in the f2 order (hi first, then lo)
-__device__ __forceinline__ f2v f2v_min(f2v a, f2v b) {
-  const bool bx = b.hi.x < a.hi.x || (b.hi.x == a.hi.x && b.lo.x < a.lo.x);
-  const bool by = b.hi.y < a.hi.y || (b.hi.y == a.hi.y && b.lo.y < a.lo.y);
-  return f2v(make_float2(bx ? b.hi.x : a.hi.x, by ? b.hi.y : a.hi.y),
-             make_float2(bx ? b.lo.x : a.lo.x, by ? b.lo.y : a.lo.y));
 }
 
 }  // namespace gbmv

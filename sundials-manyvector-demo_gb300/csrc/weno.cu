@@ -95,13 +95,6 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
       fluid_face_flux64(T, S.gamma, H, out);
 #pragma unroll
       for (int v = 0; v < 5; ++v) D.F[D.slot[v] * D.nfaces + f] = out[v];
-      if (NCHEM) {
-#pragma unroll
-        for (int l = 0; l < 5; ++l) {
-          keep64(H.hp[l]);
-          keep64(H.hm[l + 1]);
-        }
-      }
 #pragma unroll 1
       for (int c = 0; c < NCHEM; ++c) {
         double cv[6];
@@ -125,10 +118,6 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
 #pragma unroll
       for (int v = 0; v < 5; ++v)
         if (live && (v & 1) == side) D.F[D.slot[v] * D.nfaces + f] = out[v];
-      if (NCHEM) {
-#pragma unroll
-        for (int k = 0; k < 5; ++k) keep64(h[k]);
-      }
 #pragma unroll 1
       for (int c = 0; c < NCHEM; ++c) {
         double cv[5];

@@ -5,10 +5,10 @@
 namespace gbmv {
 
 // Register budgets of the sweeps (128-thread blocks per SM; the same bits whatever they are).
-// Fluid, 128^3 x 15 GBMV_MIXED_FAST RHS at 2 / 3 / 4 blocks: 2.84 / 2.85 / 3.13 ms.  Beside the
+// Fluid, 128^3 x 15 GBMV_MIXED_FAST RHS at 2 / 3 / 4 blocks: 2.61 / 2.51 / 2.57 ms.  Beside the
 // chemistry Newton on a second stream (255 registers a thread) 5 leave the Newton's warps room
-// (Grid::sweep_shared).  Tracers: FP32 weights 4 / 5 / 6 / 7 / 8: 2.93 / 2.85 / 2.81 / 2.80 / 2.82
-// ms; float-float weights 2 / 3 / 4 / 5 (GBMV_MIXED): 3.81 / 3.80 / 3.67 / 3.64 ms.
+// (Grid::sweep_shared).  Tracers: FP32 weights 5 / 6 / 7 / 8: 2.53 / 2.51 / 2.51 / 2.53
+// ms; float-float weights 4 / 5 / 6 (128^3 x 9 GBMV_MIXED): 2.34 / 2.32 / 2.32 ms.
 constexpr int kF2MinB = 3;
 constexpr int kF2SharedMinB = 5;
 constexpr int kTracerFastMinB = 6;

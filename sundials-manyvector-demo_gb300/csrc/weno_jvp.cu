@@ -200,15 +200,6 @@ __global__ void __launch_bounds__(128) face_flux_jvp_kernel(const __grid_constan
         dfma(R.H, t, dfma(R.u, cd, dfma(R.v, ff[1], dfma(R.w, ff[2], R.q * ff[3])))).d};
 #pragma unroll
     for (int v = 0; v < 5; ++v) D.F[D.slot[v] * D.nfaces + f] = o[v];
-    if (NCHEM) {
-#pragma unroll
-      for (int l = 0; l < 5; ++l) {
-        keep64(hp[l].v);
-        keep64(hp[l].d);
-        keep64(hm[l + 1].v);
-        keep64(hm[l + 1].d);
-      }
-    }
 #pragma unroll 1
     for (int c = 0; c < NCHEM; ++c) {
       Dual cv[6];

@@ -179,11 +179,6 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
       hp[k] = fma(0.5, T.u[k], ha);
       hm[k] = fma(0.5, T.u[5 - k], -ha);
     }
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      keep64(hp[k]);
-      keep64(hm[k]);
-    }
     // tracers first: their cotangents of the split factors join the fluid part's
     double hpb[5] = {0, 0, 0, 0, 0}, hmb[5] = {0, 0, 0, 0, 0};
 #pragma unroll 1
