@@ -135,6 +135,66 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
   }
 }
 
+// The same for the smallest grids, four threads a face: a lane pair per face as above in each of
+// the block's two warps, which share the characteristic components (76 and 114 of the 190 FP64
+// instructions of a side's reconstructions) and the tracers.  The device
+// time of a right-hand side, two threads a face and four: 128 x 3 x 3 without tracers 26.7 and 24.6
+// us, 10^3 with ten 47.1 and 36.9 (a warp issues its FP64 chain at one instruction per 64 cycles
+// whatever its lanes hold, so only further warps shorten it).  The same bits.
+template <int NCHEM>
+__global__ void __launch_bounds__(64) face_flux64_quad_kernel(const __grid_constant__ SweepSet S) {
+  __shared__ double share[5][16];
+  const int dir = sweep_dir(S);
+  const SweepDir& D = S.d[dir];
+  const int side = threadIdx.x & 1, half = threadIdx.x >> 5, slot = (threadIdx.x & 31) >> 1;
+  long f = (blockIdx.x - D.block0) * 16L + slot;
+  const bool live = f < D.nfaces;
+  if (!live) f = D.nfaces - 1;  // surplus threads repeat the last face and store nothing
+  long cell[6];
+  bool nall[6], nnorm[6];
+  stencil_of(S, D, f, side, cell, nall, nnorm);
+  Stencil64 T;
+#pragma unroll
+  for (int l = 0; l < 6; ++l) {
+    load_point(D.f, cell[l], nall[l], nnorm[l], T.W[l]);
+    T.ph[l] = flip_sign(__ldg(S.ph + cell[l]), nall[l]);
+    T.u[l] = flip_sign(__ldg(D.vel[0] + cell[l]), nnorm[l]);
+    T.hc[l] = __ldg(S.hc + cell[l]);
+  }
+  Roe64 R;
+  roe64(T, S.gamma, R);
+  const double ha = half_alpha64(T);
+  double h[5], ff[5] = {0, 0, 0, 0, 0}, out[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) h[k] = fma(0.5, T.u[k], side ? -ha : ha);
+  if (half) fluid_side64<0, 2>(T, R, h, ff);
+  else fluid_side64<0, 1>(T, R, h, ff);
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const double o = __shfl_xor_sync(0xffffffffu, ff[i], 1);
+    if ((half == 0) == (i == 0 || i == 4) && side == 0) share[i][slot] = ff[i] + o;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 5; ++i) ff[i] = share[i][slot];
+  fluid_back64(R, ff, out);
+#pragma unroll
+  for (int v = 0; v < 5; ++v)
+    if (live && (v & 3) == 2 * half + side) D.F[D.slot[v] * D.nfaces + f] = out[v];
+#pragma unroll 1
+  for (int c = half; c < NCHEM; c += 2) {
+    double cv[5];
+#pragma unroll
+    for (int l = 0; l < 5; ++l) {
+      cv[l] = flip_sign(__ldg(S.chem + c + (long)NCHEM * cell[l]), nall[l]);
+    }
+    Weno64 q;
+    double r = weno_prod64(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
+    r += __shfl_xor_sync(0xffffffffu, r, 1);
+    if (live && side == 0) D.F[(5 + c) * D.nfaces + f] = r;
+  }
+}
+
 template <int NCHEM>
 __global__ void __launch_bounds__(256) divergence_kernel(Grid g, Fields wdot,
                                                          const double* __restrict__ Fx,
@@ -292,14 +352,17 @@ static int launch_fp64(const Grid& g, const Fields& w, const Fields& wdot, const
   {
     ProfScope ps("face_flux", s);
     const bool split = pre && nfaces <= kSplitFaces;
-    const int t = sweep_threads(g, split ? 2 * nfaces : nfaces, 128);
+    const bool quad = split && nfaces <= kQuadFaces;
+    const int per_face = quad ? 4 : (split ? 2 : 1);
+    const int t = quad ? 64 : sweep_threads(g, per_face * nfaces, 128);
     SweepSet S;
-    const int b = sweep_set(g, w, F, split ? 2 : 1, t, split ? 1L << 30 : (long)kSM * 16, S);
+    const int b = sweep_set(g, w, F, per_face, t, split ? 1L << 30 : (long)kSM * 16, S);
     if (pre) {
       const double* const u[3] = {wdot.f[1], wdot.f[2], wdot.f[3]};
       sweep_prims(S, wdot.f[0], u, wdot.f[4]);
     }
-    if (split) face_flux64_kernel<NCHEM, true, true><<<b, t, 0, s>>>(S);
+    if (quad) face_flux64_quad_kernel<NCHEM><<<b, t, 0, s>>>(S);
+    else if (split) face_flux64_kernel<NCHEM, true, true><<<b, t, 0, s>>>(S);
     else if (pre) face_flux64_kernel<NCHEM, true, false><<<b, t, 0, s>>>(S);
     else face_flux64_kernel<NCHEM, false, false><<<b, t, 0, s>>>(S);
     GBMV_LAUNCH_CHECK("face_flux64_kernel");

@@ -103,3 +103,21 @@ def test_fp64_sweeps_at_large_densities(cuda):
         res.append([x.cpu().numpy() / lam for x in f] + [x.cpu().numpy() for x in jv + u])
     for a, b in zip(*res):
         assert maxnorm_err(a, b) <= 1e-12
+
+
+# 4864 faces is the line between four threads a face and two: (11, 11, 12) has 4741 faces, (12, 11,
+# 12) 5160; the Sod tube's grid; odd face counts in every direction
+@pytest.mark.parametrize("shape", [(128, 3, 3), (11, 11, 12), (12, 11, 12), (5, 3, 7)])
+@pytest.mark.parametrize("nchem", [0, 2, 10])
+def test_fp64_small_grids_match_oracle(cuda, shape, nchem):
+    torch = cuda
+    import gbmv
+    bc = (3, 2, 1, 3, 0, 0)
+    wl = W.rayleigh_taylor(shape=shape, nchem=nchem, seed=W.SEED_BASE + 704)
+    st, ref = O.feuler(wl["fields"], nchem, bc, wl["gamma"], None)
+    assert st == 0
+    w = [torch.from_numpy(np.ascontiguousarray(f)).cuda() for f in wl["fields"]]
+    out = [torch.full_like(f, np.nan) for f in w]
+    assert gbmv.Hydro(shape, nchem, bc, wl["gamma"], None).fEuler(0.0, w, out) == 0
+    for a, r in zip(out, ref):
+        assert maxnorm_err(a.cpu().numpy(), r) <= 1e-12
