@@ -417,10 +417,12 @@ def algo_bytes(fam, n):
     ncell, nvar = n ** 3, 15
     nf = (n + 1) * n * n
     return {
-        "face_flux": 8 * nvar * (ncell + nf),           # FP64 form: state in, fluxes out
-        "face_flux_mx": 4 * (16 * ncell + nvar * nf),   # mixed form: FP32 copies in, FP32 fluxes out
+        # FP64 form: state and primitives in, the three directions' fluxes out
+        "face_flux": 8 * ((nvar + 5) * ncell + 3 * nvar * nf),
+        # mixed forms: float pairs of fields and primitives in, of fluxes out
+        "face_flux_mx": 8 * ((nvar + 5) * ncell + 3 * nvar * nf),
         "divergence": 8 * nvar * (3 * nf + ncell) + 8 * 5 * ncell,
-        "prims": 8 * nvar * ncell + 4 * 16 * ncell,
+        "prims": 8 * nvar * ncell + 8 * (nvar + 5) * ncell,
         "chem_rhs": 368 * ncell,
         "chem_jac": (34 * 8 + 800) * ncell,
         "chem_newton": 456 * ncell,
@@ -433,16 +435,15 @@ def algo_bytes(fam, n):
 # Arithmetic per unit of each kernel family, counted by ncu on these kernels
 # (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma} or {fadd,fmul,ffma}: adds + muls +
 # 2 x FMAs, per face or cell, on a 112^3 grid) -- the numerator of the compute
-# roofline; the denominator is the FMA rate measured by gbmv_diag_fma_rate.
+# roofline; the denominator is the FMA rate measured by gbmv_diag_fma_rate.  (The counters do not
+# see paired FP32 instructions, so the float-float sweeps have no entry.)
 FP_COUNTS = {
-    ("fp64", "face_flux"): ("fp64", 3841.3, "face"),
-    ("fp64", "chem_rhs"): ("fp64", 2440.9, "cell"),
-    ("fp64", "chem_jac"): ("fp64", 957.0, "cell"),
-    ("fp64", "block_lu_factor"): ("fp64", 759.0, "cell"),
-    ("mixed", "face_flux"): ("fp32", 25990.0, "face"),
-    ("mixed", "chem_newton"): ("fp64", 1671.1, "cell"),
-    ("mixed_fast", "face_flux"): ("fp32", 16190.0, "face"),
-    ("mixed_fast", "chem_newton"): ("fp64", 1671.1, "cell"),
+    ("fp64", "face_flux"): ("fp64", 2276.0, "face"),
+    ("fp64", "chem_rhs"): ("fp64", 611.3, "cell"),
+    ("fp64", "chem_jac"): ("fp64", 707.1, "cell"),
+    ("fp64", "block_lu_factor"): ("fp64", 729.0, "cell"),
+    ("mixed", "chem_newton"): ("fp64", 1133.2, "cell"),
+    ("mixed_fast", "chem_newton"): ("fp64", 1133.2, "cell"),
 }
 
 
@@ -450,11 +451,11 @@ FP_COUNTS = {
 # L2 (dram__bytes_read.sum + dram__bytes_write.sum per face or cell on a 112^3 grid), scaled by
 # the units of one 128^3 launch for the roofline's `traffic`.
 DRAM_TRAFFIC = {
-    ("fp64", "face_flux"): (248.2, "face"),    # mean of the x / y / z sweeps
-    ("mixed", "face_flux"): (296.5, "face"),
-    ("mixed", "chem_newton"): (471.4, "cell"),
-    ("mixed_fast", "face_flux"): (355.6, "face"),
-    ("mixed_fast", "chem_newton"): (471.4, "cell"),
+    ("fp64", "face_flux"): (287.1, "face"),
+    ("mixed", "face_flux"): (174.2, "face"),       # fluid and tracer sweeps
+    ("mixed", "chem_newton"): (542.6, "cell"),
+    ("mixed_fast", "face_flux"): (174.3, "face"),
+    ("mixed_fast", "chem_newton"): (542.6, "cell"),
     ("fp64", "chem_rhs"): (357.3, "cell"),
 }
 
@@ -553,14 +554,14 @@ def run_gbmv(args):
     traffic, traffic_note = None, None
     if (hform, dom) in DRAM_TRAFFIC:
         per, unit = DRAM_TRAFFIC[(hform, dom)]
-        units = (args.n + 1) * args.n * args.n if unit == "face" else ncell
+        units = 3 * (args.n + 1) * args.n * args.n if unit == "face" else ncell
         traffic = round(per * units, 0)
         traffic_note = (f"bytes per launch: {per} B/{unit} (ncu dram__bytes_read+write, 112^3 "
                         f"capture, state > L2) x {units} {unit}s")
     pipe = None
     if (hform, dom) in FP_COUNTS:
         pname, per_unit, unit = FP_COUNTS[(hform, dom)]
-        units = (args.n + 1) * args.n * args.n if unit == "face" else ncell
+        units = 3 * (args.n + 1) * args.n * args.n if unit == "face" else ncell
         peak_pipe = gbmv.fma_rate(pname == "fp64") / 1e12
         ach = per_unit * units / (avg_ms * 1e-3) / 1e12
         pipe = {"name": pname, "achieved": round(ach, 4), "peak": round(peak_pipe, 4),
@@ -807,7 +808,7 @@ def run_weno(torch, gbmv, grids, steps=3, warmup=2, parity=True):
                  "algorithmic_GBps": round(240.0 * ncell / (ms * 1e-3) / 1e9, 1),
                  "hbm_frac": round(240.0 * ncell / (ms * 1e-3) / 1e9 / hbm_peak, 5)}
             if name == "fp64":
-                fl = FP_COUNTS[("fp64", "face_flux")][1] * faces + 158.4 * ncell
+                fl = FP_COUNTS[("fp64", "face_flux")][1] * faces + 234.4 * ncell
                 r["fp64_pipe_frac"] = round(fl / (ms * 1e-3) / 1e12 / fp64_peak, 4)
             g[name] = r
         g["speedup_mixed_vs_fp64"] = round(g["fp64"]["ms_per_rhs"] / g["mixed"]["ms_per_rhs"], 3)

@@ -117,8 +117,8 @@ int gbmv_feuler_noalloc(const gbmv_grid* grid, const double* force_host, double 
 /* Autotuner of the face sweeps' launch shape (no counterpart in the reference): times the
  * flux divergence of `precision` on the state w with 32, 64 and 128 threads per block and
  * keeps the fastest for this handle and precision (*threads, host, may be NULL, receives it).
- * Each face is computed by one thread on its own, so the choice changes no result.  Without a
- * call the sweeps use 128 threads, fewer on grids too small to give every SM two blocks.
+ * Each face is computed on its own, so the choice changes no result.  Without a call the sweeps
+ * use 128 threads, fewer on grids too small to give every SM two blocks.
  * Synchronous; allocates a temporary output; not during a stream capture. */
 int gbmv_hydro_autotune(gbmv_hydro h, const double* const* w, int precision, int* threads,
                         void* stream);

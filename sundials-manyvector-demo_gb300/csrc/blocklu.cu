@@ -9,7 +9,7 @@
 // memory by 16-byte asynchronous copies, all in flight at once; several such CTAs per SM overlap
 // one tile's traffic with the others' arithmetic.  (Two-warp CTAs filling their tile with plain
 // loads, a few in flight, left the FP64 pipe 54 % busy in the factorisation and 20 % in the
-// solve: 192,000 blocks 286 and 164 us, now 167 and 58.)
+// solve: 192,000 blocks 286 and 164 us, now 165 and 59.)
 #include "block_tile.cuh"
 #include "chem.cuh"
 #include "chem_lu.cuh"

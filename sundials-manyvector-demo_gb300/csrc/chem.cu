@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(128) chem_rhs_kernel(ChemParams P, ChemState S
 
 // One warp a CTA, a block a thread, assembled in a shared tile and written out in order: a
 // thread's entries are 800 bytes apart from its neighbour's, and written directly (with the
-// structural zeros first) they left the FP64 pipe 71 % busy (192,000 cells: 272 -> 214 us).
+// structural zeros first) they left the FP64 pipe 71 % busy (192,000 cells: 272 -> 206 us).
 __global__ void __launch_bounds__(kLuThreads, 8) chem_jac_kernel(ChemParams P, ChemState S, long n,
                                                                  const double* __restrict__ y,
                                                                  double* __restrict__ J,

@@ -1,16 +1,19 @@
 // WENO5 flux divergence (part a): the device implementation of fEuler
 // (src/utilities.cpp:17-253) with in-kernel ghost synthesis for every boundary type.
 //
-// FP64 parity form, two passes:
-//   1. face_flux_kernel<NCHEM, DIR>: one thread per face normal to DIR (all lower faces plus
-//      the upper boundary faces, like the reference's two loops); stencil gathered straight
-//      from the SoA fields with ghost synthesis, flux written to a per-direction scratch array
-//      F_DIR[v][face] (the xflux/yflux/zflux arrays of EulerData, src/euler3D.hpp:497-499,
-//      stored field-major so that the divergence pass reads them coalesced).
-//   2. divergence_kernel<NCHEM>: wdot = G - [(Fx+ - Fx-)/dx + (Fy+ - Fy-)/dy + (Fz+ - Fz-)/dz],
-//      with the legal-state check (src/euler3D.hpp:1405-1414) OR-ed into a status word.
-// The float-float forms (weno_f2*.cu) use divergence_f2_kernel below as their pass 2.  Also
-// here: the CFL wave speed, the pack1D stencil gather and the conservation totals.
+// FP64 parity form, three passes:
+//   1. prims64_kernel: the primitives of every cell into the tendency arrays (which the last pass
+//      overwrites), and the legal-state check (src/euler3D.hpp:1405-1414) OR-ed into a status
+//      word.
+//   2. face_flux64_kernel<NCHEM, PRE, SPLIT>: the faces of the three directions in one launch, a
+//      thread a face (all lower faces plus the upper boundary faces, like the reference's two
+//      loops), two or four threads on small grids; stencil gathered straight from the SoA fields
+//      with ghost synthesis, flux written to a per-direction scratch array F_DIR[v][face] (the
+//      xflux/yflux/zflux arrays of EulerData, src/euler3D.hpp:497-499, stored field-major so that
+//      the divergence pass reads them coalesced).
+//   3. divergence_kernel<NCHEM>: wdot = G - [(Fx+ - Fx-)/dx + (Fy+ - Fy-)/dy + (Fz+ - Fz-)/dz].
+// The float-float forms (weno_f2.cu) use divergence_f2_kernel below as their last pass.  Also
+// here: the CFL wave speed, the pack1D stencil gather, the conservation totals and norms.
 #include "common.cuh"
 #include "weno64.cuh"
 #include "df64.cuh"
@@ -401,7 +404,7 @@ __global__ void __launch_bounds__(256) wave_speed_max_kernel(Grid g, Fields w,
   double m = 0.0;
   for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < g.ncell;
        c += (long)gridDim.x * blockDim.x) {
-    // bound by the FP64 pipe: one reciprocal serves the three quotients (100^3: 92 -> 57 us)
+    // bound by the FP64 pipe: one reciprocal serves the three quotients (100^3: 92 -> 56 us)
     const double mx = w.f[1][c], my = w.f[2][c], mz = w.f[3][c], ir = rcp64_any(w.f[0][c]);
     const double u = fabs(mx * ir);
     const double p = (g.gamma - 1.0) * (w.f[4][c] - (mx * mx + my * my + mz * mz) * (0.5 * ir));
@@ -565,7 +568,7 @@ __global__ void __launch_bounds__(256) wrms_partial_kernel(long ncell, int nchem
     if (n == 0) continue;
     // Four terms are summed plainly before each compensated addition: their rounding is that of
     // the terms themselves, and the FP64 pipe bounds this pass (14 -> 8 instructions a term with
-    // the reciprocal in place of the division; 100^3 x 15: 408 -> 235 us).
+    // the reciprocal in place of the division; 100^3 x 15: 408 -> 228 us).
     const long stride = (long)gridDim.x * blockDim.x;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += 4 * stride) {
       double x = 0.0;
