@@ -27,6 +27,10 @@ __device__ __forceinline__ float2 f2v_diff_hi(f2v a, f2v b) {
   const f2v s = two_sum2(a.hi, neg2(b.hi));
   return add2(s.hi, add2(s.lo, sub2(a.lo, b.lo)));
 }
+__device__ __forceinline__ f2v f2v_times(float c, f2v y) {  // c y, not renormalised
+  const f2v p = two_prod2(v2(c), y.hi);
+  return f2v(p.hi, fma2(v2(c), y.lo, p.lo));
+}
 __device__ __forceinline__ f2v f2v_add_scaled(f2v s, float c, f2v y) {  // s + c y
   const f2v p = two_prod2(v2(c), y.hi);
   const f2v t = two_sum2(s.hi, p.hi);
@@ -57,14 +61,16 @@ static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3
   const f2v D23x2 = f2v_scale(D23, 2.f);
   f2v aA, aB, aC;
   {
-    const f2v K{f2(kWenoK)}, eps{f2(kWenoEps * kF2Scale * kF2Scale)};
-    // (not renormalised: d and e never both cancel against the differences they are built of, so
-    // what a product of them drops stays below 2^-48 of a_k)
-    const f2v dA = f2v_sum(D23, -D34), dB = f2v_sum(D12, -D23), dC = f2v_sum(D01, -D12);
-    const f2v eA = f2v_sum(dA, D23x2), eB = f2v_sum(D12, D23), eC = f2v_sum(dC, f2v_scale(D12, -2.f));
-    aA = f2v_norm(f2v_add_prod(f2v_add_prod(eps, dA, dA), f2v_prod(K, eA), eA));
-    aB = f2v_norm(f2v_add_prod(f2v_add_prod(eps, dB, dB), f2v_prod(K, eB), eB));
-    aC = f2v_norm(f2v_add_prod(f2v_add_prod(eps, dC, dC), f2v_prod(K, eC), eC));
+    // (the t's and k's are not renormalised: they only go into products, and what those drop
+    // stays below 2^-48 of a_k)
+    const f2v eps{f2(kWenoEps * kF2Scale * kF2Scale)};
+    const f2v s23 = f2v_add_prod(eps, f2v_times(39.f / 64.f, D23), D23);
+    const f2v s12 = f2v_add_prod(eps, f2v_times(39.f / 64.f, D12), D12);
+    const f2v tA = f2v_add_scaled(D34, -11.f / 8.f, D23), tB = f2v_add_scaled(D12, -5.f / 8.f, D23),
+              tC = f2v_add_scaled(D01, -11.f / 8.f, D12);
+    aA = f2v_norm(f2v_add_prod(s23, tA, tA));
+    aB = f2v_norm(f2v_add_prod(s23, tB, tB));
+    aC = f2v_norm(f2v_add_prod(s12, tC, tC));
   }
   const float top = fmaxf(fmaxf(fmaxf(aA.hi.x, aB.hi.x), aC.hi.x),
                           fmaxf(fmaxf(aA.hi.y, aB.hi.y), aC.hi.y));
