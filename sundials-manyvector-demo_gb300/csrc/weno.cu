@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
     if constexpr (!SPLIT) {
       Split64 H;
       double out[5];
-      fluid_face_flux64(T, S.gamma, H, out);
+      fluid_face_flux64<(NCHEM > 0)>(T, S.gamma, H, out);
 #pragma unroll
       for (int v = 0; v < 5; ++v) D.F[D.slot[v] * D.nfaces + f] = out[v];
 #pragma unroll 1
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
           cv[l] = flip_sign(__ldg(S.chem + c + (long)NCHEM * cell[l]), nall[l]);
         }
         Weno64 q;
-        double r = weno_prod64(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
+        double r = weno_prod64<true>(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
         r += __shfl_xor_sync(0xffffffffu, r, 1);
         if (live && (c & 1) == side) D.F[(5 + c) * D.nfaces + f] = r;
       }
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
 }
 
 // The same for the smallest grids, four threads a face: a lane pair per face as above in each of
-// the block's two warps, which share the characteristic components (76 and 114 of the 190 FP64
+// the block's two warps, which share the characteristic components (66 and 99 of the 165 FP64
 // instructions of a side's reconstructions) and the tracers.  The device
 // time of a right-hand side, two threads a face and four: 128 x 3 x 3 without tracers 26.7 and 24.6
 // us, 10^3 with ten 47.1 and 36.9 (a warp issues its FP64 chain at one instruction per 64 cycles
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(64) face_flux64_quad_kernel(const __grid_const
       cv[l] = flip_sign(__ldg(S.chem + c + (long)NCHEM * cell[l]), nall[l]);
     }
     Weno64 q;
-    double r = weno_prod64(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
+    double r = weno_prod64<true>(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
     r += __shfl_xor_sync(0xffffffffu, r, 1);
     if (live && side == 0) D.F[(5 + c) * D.nfaces + f] = r;
   }

@@ -73,7 +73,7 @@ static __device__ __noinline__ void fluid_face_64(const SweepSet& S, const Sweep
   }
   Split64 H;
   double o[5];
-  fluid_face_flux64(T, S.gamma, H, o);
+  fluid_face_flux64<false>(T, S.gamma, H, o);
 #pragma unroll
   for (int v = 0; v < 5; ++v) out[v] = f2_from_double(o[v]);
   ha = f2_from_double(half_alpha64(T));

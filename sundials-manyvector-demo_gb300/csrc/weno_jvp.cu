@@ -6,8 +6,8 @@
 // stencil of |u| + c, |u|, the positivity guard of sqrt) take the branch the forward pass took.
 //
 // Bound by the FP64 pipe, so the tangents are written out where a generic dual number would
-// spend instructions on constants' zero tangents and on quotients: 40 instructions for the
-// tangent of a reconstruction on top of its 38 (weno_tan64).  96^3 x 9: 5330 -> 2370 FP64
+// spend instructions on constants' zero tangents and on quotients: 36 instructions for the
+// tangent of a reconstruction on top of its 33 (weno_tan64).  96^3 x 9: 5330 -> 2165 FP64
 // instructions a face.
 #include "common.cuh"
 #include "weno.cuh"

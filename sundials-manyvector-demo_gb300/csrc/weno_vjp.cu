@@ -10,9 +10,9 @@
 // stencil of |u| + c, |u|, the positivity guard of sqrt) take the branch the forward pass took.
 //
 // Bound by the FP64 pipe.  The adjoint of a reconstruction works on the neighbour differences
-// and takes the forward weights' products (weno_adj64: 47 instructions after the forward 38; the
+// and takes the forward weights' products (weno_adj64: 40 instructions after the forward 33; the
 // adjoint of the literal formula took ~250 with its seven divisions), the primitives come from
-// a cell pass, and each point's reciprocal density is formed once.  96^3 x 9: 6120 -> 2520
+// a cell pass, and each point's reciprocal density is formed once.  96^3 x 9: 6120 -> 2350
 // FP64 instructions a face.
 #include "common.cuh"
 #include "weno.cuh"
