@@ -129,7 +129,8 @@ __global__ void __launch_bounds__(128) face_flux64_kernel(const __grid_constant_
           cv[l] = flip_sign(__ldg(S.chem + c + (long)NCHEM * cell[l]), nall[l]);
         }
         Weno64 q;
-        double r = weno_prod64<true>(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
+        double r =
+            weno_prod64<true>(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
         r += __shfl_xor_sync(0xffffffffu, r, 1);
         if (live && (c & 1) == side) D.F[(5 + c) * D.nfaces + f] = r;
       }
@@ -192,7 +193,8 @@ __global__ void __launch_bounds__(64) face_flux64_quad_kernel(const __grid_const
       cv[l] = flip_sign(__ldg(S.chem + c + (long)NCHEM * cell[l]), nall[l]);
     }
     Weno64 q;
-    double r = weno_prod64<true>(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
+    double r =
+        weno_prod64<true>(cv[0], h[0], cv[1], h[1], cv[2], h[2], cv[3], h[3], cv[4], h[4], q);
     r += __shfl_xor_sync(0xffffffffu, r, 1);
     if (live && side == 0) D.F[(5 + c) * D.nfaces + f] = r;
   }
