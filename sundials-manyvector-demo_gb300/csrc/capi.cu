@@ -75,7 +75,7 @@ using namespace gbmv;
 // What a synchronous call reads back, in page-locked host memory that its kernels write directly
 // (status words only where a state is illegal or a block singular): no clearing launch and no copy
 // on the stream, which for a 128 x 3 x 3 right-hand side were 10 of 44 us (the copy into pageable
-// memory is staged by the driver).
+// memory is staged by the CUDA driver).
 struct HostWords {
   int flags;       // legal-state mask of the flow; singular block of a chemistry or block handle
   double sums[2];  // norm, totals

@@ -7,7 +7,7 @@
 //
 // Bound by the FP64 pipe, so the tangents are written out where a generic dual number would
 // spend instructions on constants' zero tangents and on quotients: 36 instructions for the
-// tangent of a reconstruction on top of its 33 (weno_tan64).  96^3 x 9: 5330 -> 2165 FP64
+// tangent of a reconstruction on top of its 33 (weno_tan64).  96^3 x 9: 5330 -> 2135 FP64
 // instructions a face.
 #include "common.cuh"
 #include "weno.cuh"
@@ -71,33 +71,45 @@ __device__ __forceinline__ void roe_dual(const Dual (&W)[6][5], const Dual (&ph)
   R.L31 = 2.0 * (R.u * hgc);
 }
 
-// reconstruction of five duals
-__device__ __forceinline__ Dual weno_dual(Dual f0, Dual f1, Dual f2, Dual f3, Dual f4) {
-  Weno64 w;
-  const double r = weno_diff64(f2.v, f0.v - f1.v, f1.v - f2.v, f2.v - f3.v, f3.v - f4.v, w);
-  return Dual(r, weno_tan64(w, f2.d, f0.d - f1.d, f1.d - f2.d, f2.d - f3.d, f3.d - f4.d));
-}
-
 // fluid_side64 with tangents
 template <int SIDE>
 __device__ __forceinline__ void fluid_side_dual(const Dual (&W)[6][5], const Dual (&ph)[6],
                                                 const Dual (&u)[6], const RoeDual& R,
                                                 const Dual (&h)[5], Dual (&ff)[5]) {
+  const int j0 = SIDE ? 5 : 0, j1 = SIDE ? 4 : 1, j2 = SIDE ? 3 : 2, j3 = SIDE ? 2 : 3,
+            j4 = SIDE ? 1 : 4;
+  Dual g[5][5];  // [field]{central, D01, D12, D23, D34}
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    auto point = [&](int q, Dual hq) {
+      return m == 1 ? dfma(W[q][1], hq, ph[q])
+                    : (m == 4 ? dfma(W[q][4], hq, u[q] * ph[q]) : W[q][m] * hq);
+    };
+    const Dual f1 = point(j1, h[1]), f2 = point(j2, h[2]), f3 = point(j3, h[3]);
+    const Dual r0 = m == 1 ? ph[j0] - f1 : (m == 4 ? dfma(u[j0], ph[j0], -f1) : -f1);
+    const Dual r4 = m == 1 ? f3 - ph[j4] : (m == 4 ? dfma(-u[j4], ph[j4], f3) : f3);
+    g[m][0] = f2;
+    g[m][1] = dfma(W[j0][m], h[0], r0);
+    g[m][2] = f1 - f2;
+    g[m][3] = f2 - f3;
+    g[m][4] = dfma(-W[j4][m], h[4], r4);
+  }
   Dual P[5][5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
-    const int j = SIDE ? 5 - k : k;
-    const Dual f0 = W[j][0] * h[k], f1 = dfma(W[j][1], h[k], ph[j]), f2 = W[j][2] * h[k],
-               f3 = W[j][3] * h[k], f4 = dfma(W[j][4], h[k], u[j] * ph[j]);
-    const Dual X = dfma(R.L02, f2, dfma(R.L03, f3, R.L04 * f4));
-    P[k][0] = dfma(R.L00, f0, dfma(R.L01, f1, X));
-    P[k][1] = dfma(-R.v, f0, f2);
-    P[k][2] = dfma(-R.w, f0, f3);
-    P[k][3] = dfma(R.L30, f0, dfma(-2.0, X, R.L31 * f1));
-    P[k][4] = dfma(R.L40, f0, dfma(R.L41, f1, X));
+    const Dual X = dfma(R.L02, g[2][k], dfma(R.L03, g[3][k], R.L04 * g[4][k]));
+    P[k][0] = dfma(R.L00, g[0][k], dfma(R.L01, g[1][k], X));
+    P[k][1] = dfma(-R.v, g[0][k], g[2][k]);
+    P[k][2] = dfma(-R.w, g[0][k], g[3][k]);
+    P[k][3] = dfma(R.L30, g[0][k], dfma(-2.0, X, R.L31 * g[1][k]));
+    P[k][4] = dfma(R.L40, g[0][k], dfma(R.L41, g[1][k], X));
   }
 #pragma unroll
-  for (int i = 0; i < 5; ++i) ff[i] = weno_dual(P[0][i], P[1][i], P[2][i], P[3][i], P[4][i]);
+  for (int i = 0; i < 5; ++i) {
+    Weno64 w;
+    const double r = weno_diff64(P[0][i].v, P[1][i].v, P[2][i].v, P[3][i].v, P[4][i].v, w);
+    ff[i] = Dual(r, weno_tan64(w, P[0][i].d, P[1][i].d, P[2][i].d, P[3][i].d, P[4][i].d));
+  }
 }
 
 // one tracer's tangent: both sides of c h, the outer points in one difference each
