@@ -438,7 +438,7 @@ def algo_bytes(fam, n):
 # roofline; the denominator is the FMA rate measured by gbmv_diag_fma_rate.  (The counters do not
 # see paired FP32 instructions, so the float-float sweeps have no entry.)
 FP_COUNTS = {
-    ("fp64", "face_flux"): ("fp64", 2276.0, "face"),
+    ("fp64", "face_flux"): ("fp64", 2154.0, "face"),
     ("fp64", "chem_rhs"): ("fp64", 611.3, "cell"),
     ("fp64", "chem_jac"): ("fp64", 707.1, "cell"),
     ("fp64", "block_lu_factor"): ("fp64", 729.0, "cell"),
@@ -451,7 +451,7 @@ FP_COUNTS = {
 # L2 (dram__bytes_read.sum + dram__bytes_write.sum per face or cell on a 112^3 grid), scaled by
 # the units of one 128^3 launch for the roofline's `traffic`.
 DRAM_TRAFFIC = {
-    ("fp64", "face_flux"): (287.1, "face"),
+    ("fp64", "face_flux"): (291.1, "face"),
     ("mixed", "face_flux"): (174.2, "face"),       # fluid and tracer sweeps
     ("mixed", "chem_newton"): (542.6, "cell"),
     ("mixed_fast", "face_flux"): (174.3, "face"),

@@ -57,7 +57,7 @@ int prims64(const Grid& g, const Fields& w, double* const (&out)[5], int* d_stat
   return GBMV_OK;
 }
 
-// Face fluxes of the three directions (one launch).  Bound by the FP64 pipe: 1495 instructions
+// Face fluxes of the three directions (one launch).  Bound by the FP64 pipe: 1355 instructions
 // a face at NVAR 15.  PRE: the primitives are read from the cell pass, else formed per stencil
 // point.  SPLIT: two neighbouring threads share a face, each with one Lax-Friedrichs side (the
 // second reads its stencil reversed, which makes its side the plus formula); the same bits.
