@@ -453,9 +453,9 @@ FP_COUNTS = {
 DRAM_TRAFFIC = {
     ("fp64", "face_flux"): (291.1, "face"),
     ("mixed", "face_flux"): (174.2, "face"),       # fluid and tracer sweeps
-    ("mixed", "chem_newton"): (542.6, "cell"),
+    ("mixed", "chem_newton"): (462.6, "cell"),
     ("mixed_fast", "face_flux"): (174.3, "face"),
-    ("mixed_fast", "chem_newton"): (542.6, "cell"),
+    ("mixed_fast", "chem_newton"): (462.6, "cell"),
     ("fp64", "chem_rhs"): (357.3, "cell"),
 }
 
