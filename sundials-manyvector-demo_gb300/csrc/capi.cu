@@ -81,9 +81,48 @@ struct HostWords {
   double sums[2];  // norm, totals
   unsigned long long speed;
 };
+// A page-locked allocation costs ~0.3 ms, so the handles of a process share one page of 64 slots,
+// kept while the process lives; further handles get an allocation of their own.
+constexpr int kWordSlots = 64;
+constexpr size_t kWordStride = 64;
+static_assert(sizeof(HostWords) <= kWordStride, "a slot holds the words");
+static std::mutex g_words_mu;
+static char* g_words_page = nullptr;
+static unsigned long long g_words_used = 0;
+
 static bool host_words(HostWords** p) {
-  return cudaHostAlloc(reinterpret_cast<void**>(p), sizeof(HostWords),
-                       cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess;
+  const unsigned flags = cudaHostAllocMapped | cudaHostAllocPortable;
+  std::lock_guard<std::mutex> lk(g_words_mu);
+  if (g_words_page) {  // the page does not outlive the context it was made in
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, g_words_page) != cudaSuccess ||
+        a.type != cudaMemoryTypeHost) {
+      cudaGetLastError();
+      g_words_page = nullptr;
+    }
+  }
+  if (!g_words_page) {
+    void* page = nullptr;
+    if (cudaHostAlloc(&page, kWordSlots * kWordStride, flags) != cudaSuccess) return false;
+    g_words_page = static_cast<char*>(page);
+    g_words_used = 0;
+  }
+  for (int k = 0; k < kWordSlots; ++k) {
+    if (g_words_used >> k & 1ULL) continue;
+    g_words_used |= 1ULL << k;
+    *p = reinterpret_cast<HostWords*>(g_words_page + k * kWordStride);
+    return true;
+  }
+  return cudaHostAlloc(reinterpret_cast<void**>(p), sizeof(HostWords), flags) == cudaSuccess;
+}
+static void free_host_words(HostWords* p) {
+  if (!p) return;
+  std::lock_guard<std::mutex> lk(g_words_mu);
+  const char* const c = reinterpret_cast<const char*>(p);
+  if (g_words_page && c >= g_words_page && c < g_words_page + kWordSlots * kWordStride)
+    g_words_used &= ~(1ULL << ((c - g_words_page) / kWordStride));
+  else
+    cudaFreeHost(p);
 }
 // the end of a synchronous call whose launches returned rc (after a failed launch the earlier ones
 // are waited for: they must not write into the next call's words)
@@ -94,6 +133,25 @@ static int finish(int rc, cudaStream_t s) {
   return e == cudaSuccess ? GBMV_OK : check_cuda(e, "cudaStreamSynchronize(s)");
 }
 static int flags_of(const HostWords* w) { return *static_cast<const volatile int*>(&w->flags); }
+
+// chem_log's table, formed once a process: 1/c and -log(1/c) of each interval's midpoint c.  The
+// intervals repeat from one binade to the next, so 128 logarithms do (a long double one takes
+// ~0.6 us on the Arm host).
+struct LogTable {
+  double e[2 * kLogEntries];
+  LogTable() {
+    const long double ln2 = logl(2.0L);
+    for (int k = 0; k < 128; ++k) {
+      const double inv = 1.0 / (1.0 + (k + 0.5) / 128.0);
+      const long double log_inv = logl((long double)inv);
+      for (int q = k; q < kLogEntries; q += 128) {
+        const int x = (q >> 7) - 2;
+        e[2 * q] = ldexp(inv, -x);
+        e[2 * q + 1] = (double)(x * ln2 - log_inv);
+      }
+    }
+  }
+};
 
 struct gbmv_hydro_s {
   Grid g;
@@ -257,7 +315,7 @@ int gbmv_hydro_destroy(gbmv_hydro h) {
   cudaFree(h->adj);
   cudaFree(h->cons);
   cudaFree(h->d_status);
-  cudaFreeHost(h->host);
+  free_host_words(h->host);
   delete h;
   return GBMV_OK;
 }
@@ -418,20 +476,8 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
   const size_t ltab_doubles = (size_t)2 * kLogEntries;
   float* gh = (float*)calloc(gtab_floats, sizeof(float));
   double* dh = (double*)calloc(tab_doubles, sizeof(double));
-  double* lh = (double*)malloc(sizeof(double) * ltab_doubles);
-  if (!gh || !dh || !lh) { free(h); free(gh); free(dh); free(lh); delete c; return GBMV_ENOMEM; }
-  // 1/c and -log(1/c) of each interval's midpoint c (chem_log); the intervals repeat from one
-  // binade to the next, so 128 logarithms do (a long double one takes ~0.6 us on the Arm host)
-  const long double ln2 = logl(2.0L);
-  for (int k = 0; k < 128; ++k) {
-    const double inv = 1.0 / (1.0 + (k + 0.5) / 128.0);
-    const long double log_inv = logl((long double)inv);
-    for (int q = k; q < kLogEntries; q += 128) {
-      const int e = (q >> 7) - 2;
-      lh[2 * q] = ldexp(inv, -e);
-      lh[2 * q + 1] = (double)(e * ln2 - log_inv);
-    }
-  }
+  static const LogTable log_table;
+  if (!gh || !dh) { free(h); free(gh); free(dh); delete c; return GBMV_ENOMEM; }
   for (int b = 0; b + 1 < kTSize; ++b)
     for (int r = 0; r < kNT; ++r) dh[b * kNT + r] = h[(b + 1) * kNT + r] - h[b * kNT + r];
   const int grow[4] = {GAMMAH2_2, DGAMMAH2_2, GAMMAH2_1, DGAMMAH2_1};
@@ -450,7 +496,6 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
     free(h);
     free(gh);
     free(dh);
-    free(lh);
     cudaFree(c->tab);
     cudaFree(c->cell);
     cudaFree(c->d_info);
@@ -464,11 +509,10 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
   cudaMemcpy(c->tab + tab_doubles, dh, sizeof(double) * tab_doubles, cudaMemcpyHostToDevice);
   cudaMemcpy(c->tab + 2 * tab_doubles, gh, sizeof(float) * gtab_floats, cudaMemcpyHostToDevice);
   double* const ltab = c->tab + 2 * tab_doubles + gtab_floats / 2;  // 16-byte aligned
-  cudaMemcpy(ltab, lh, sizeof(double) * ltab_doubles, cudaMemcpyHostToDevice);
+  cudaMemcpy(ltab, log_table.e, sizeof(double) * ltab_doubles, cudaMemcpyHostToDevice);
   free(h);
   free(gh);
   free(dh);
-  free(lh);
   // constants of cvklu_setup_data (src/raja_primordial_network.cpp:190-194)
   ChemParams& P = c->P;
   P.tab = c->tab;
@@ -519,7 +563,7 @@ int gbmv_chem_destroy(gbmv_chem c) {
   cudaFree(c->tab);
   cudaFree(c->cell);
   cudaFree(c->d_info);
-  cudaFreeHost(c->host);
+  free_host_words(c->host);
   cudaFree(c->dirk_k);
   cudaFree(c->dirk_retry);
   cudaFree(c->dirk_order_buf);
@@ -1068,7 +1112,7 @@ int gbmv_block_ls_create(long nblocks, gbmv_block_ls* out) {
 int gbmv_block_ls_destroy(gbmv_block_ls L) {
   if (!L) return GBMV_OK;
   cudaFree(L->pivots);
-  cudaFreeHost(L->host);
+  free_host_words(L->host);
   delete L;
   return GBMV_OK;
 }

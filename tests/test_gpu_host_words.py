@@ -53,3 +53,19 @@ def test_norm_forms_agree(cuda):
         mass, energy = h.check_conservation(y)
         assert abs(mass / y[0].sum().item() - 1) < 1e-14
         assert abs(energy / y[4].sum().item() - 1) < 1e-14
+
+
+def test_more_handles_than_shared_slots(cuda):
+    """Handles beyond the shared page's 64 slots, and slots used again after their handle is gone."""
+    torch = cuda
+    import gbmv
+    n = 5
+    eye = torch.eye(10, device="cuda", dtype=torch.float64).repeat(n, 1, 1)
+    bad = eye.clone()
+    bad[2, 7, 7] = 0.0
+    for _ in range(2):
+        ls = [gbmv.BlockLinearSolver(n) for _ in range(70)]
+        for k in (0, 1, 63, 64, 69):
+            assert ls[k].setup(bad.clone().view(-1)) == 1
+        assert all(x.setup(eye.clone().view(-1)) == 0 for x in ls)
+        del ls
