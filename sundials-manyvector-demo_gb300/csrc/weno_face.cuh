@@ -52,10 +52,14 @@ __device__ __forceinline__ float weno_scale(float a, float b, float c) {
 constexpr float kF2Scale = 64.f;
 
 // Both reconstructions of a face (lane x the plus side, lane y the minus side with its stencil
-// reversed), scaled values in and out: weno_diff64's formula.  The weights' products hold a^4: for
-// a up to 2^28 (flux jumps up to ~100) they stay in the float range as they are, beyond that the
-// a_k are scaled by a common power of two, which the weights do not see.  One out-of-line copy
-// serves every reconstruction of a face (the kernel stays inside the instruction cache).
+// reversed), scaled values in and out: weno_diff64's formula.  The weights' products hold a^4 and
+// the numerator a candidate's correction beside it.  With a_k <= A, every |D23| and |D12| is below
+// 1.29 sqrt(A) and |D34|, |D01| below 2.77 sqrt(A), so |cA| + |cB| + |cC| < 9.8 sqrt(A) and the
+// numerator stays below 9.8 A^4.5: 2^125 for A = 2^27 (the denominator below 10 A^4 = 2^112).
+// Beyond, the a_k are scaled by a common power of two, which the weights do not see.  One
+// out-of-line copy serves every reconstruction of a face (the kernel stays inside the instruction
+// cache).
+constexpr float kF2Big = 134217728.f;  // 2^27
 static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4) {
   const f2v D01 = f0 - f1, D12 = f1 - f2_, D23 = f2_ - f3, D34 = f3 - f4;
   const f2v D23x2 = f2v_scale(D23, 2.f);
@@ -74,7 +78,7 @@ static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3
   }
   const float top = fmaxf(fmaxf(fmaxf(aA.hi.x, aB.hi.x), aC.hi.x),
                           fmaxf(fmaxf(aA.hi.y, aB.hi.y), aC.hi.y));
-  if (top > 268435456.f) {
+  if (top > kF2Big) {
     const float2 s = make_float2(weno_scale(aA.hi.x, aB.hi.x, aC.hi.x),
                                  weno_scale(aA.hi.y, aB.hi.y, aC.hi.y));
     aA = f2v(mul2(aA.hi, s), mul2(aA.lo, s));
