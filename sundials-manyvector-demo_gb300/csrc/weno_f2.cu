@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(128, MINB)
       const f2v h = split_pair(ua, ub, has, kF2Scale), uj(ua, ub);
       const f2v f0 = Wj[0] * h, f1 = f2v_fma(Wj[1], h, pj), f2_ = Wj[2] * h, f3 = Wj[3] * h,
                 f4 = f2v_norm(f2v_add_prod(f2v_prod(Wj[4], h), uj, pj));
+      ok = ok && f2v_absmax(f4) < 1e30f;  // the energy flux, the largest: no overflow below
       const f2v X = f2v_norm(
           f2v_add_prod(f2v_add_prod(f2v_prod(f2v(L02), f2_), f2v(L03), f3), f2v(L04), f4));
       P[k][0] = f2v_norm(f2v_add_prod(f2v_add_prod(X, f2v(L00), f0), f2v(L01), f1));
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(128, MINB)
       f2 ff[5];
 #pragma unroll
       for (int i = 0; i < 5; ++i) {
-        const f2v r = weno_pair<0>(P[0][i], P[1][i], P[2][i], P[3][i], P[4][i]);
+        const f2v r = weno_pair(P[0][i], P[1][i], P[2][i], P[3][i], P[4][i]);
         ff[i] = f2_scale(r.x() + r.y(), 1.f / kF2Scale);
       }
       // right eigenvector columns (src/utilities.cpp:318-340)
@@ -192,6 +193,29 @@ __global__ void __launch_bounds__(128, MINB)
   }
 }
 
+// The reconstructions of a tracer whose split fluxes pass the range of the scaled arithmetic, from
+// the start and without the scale (ha: half the Lax-Friedrichs speed).
+template <int WV>
+static __device__ __noinline__ f2 tracer_large(const SweepSet& S, const SweepDir& D, long f,
+                                               const float2* __restrict__ Q2, long n, int c,
+                                               f2 ha) {
+  StencilF2 T;
+  stencil_f2(S, D, f, T);
+  f2 u[6], v[6];
+#pragma unroll
+  for (int l = 0; l < 6; ++l) {
+    u[l] = q2_load(Q2, n, 6 + D.dir, T.cell[l]);
+    v[l] = q2_load(Q2, n, kQ2Base + c, T.cell[l]);
+    if ((T.nnorm >> l) & 1u) u[l] = -u[l];
+    if ((T.nall >> l) & 1u) v[l] = -v[l];
+  }
+  f2v a[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) a[k] = f2v(v[k], v[5 - k]) * split_pair(u[k], u[5 - k], ha, 1.f);
+  const f2v r = weno_large<WV>(a[0], a[1], a[2], a[3], a[4]);
+  return r.x() + r.y();
+}
+
 // Tracer face fluxes: one thread a face, its tracers one after the other; reads half the
 // Lax-Friedrichs speed that the fluid sweep left in the first tracer's flux.
 template <int WV>
@@ -205,8 +229,8 @@ __global__ void __launch_bounds__(128, WV == 1 ? kTracerFastMinB : kTracerMinB)
     StencilF2 T;
     stencil_f2(S, D, f, T);
     f2v h[5];
+    const float2 t = F[5 * D.nfaces + f];
     {
-      const float2 t = F[5 * D.nfaces + f];
       const float sc = WV == 1 ? 1.f : kF2Scale;
       const f2 ha(sc * t.x, sc * t.y);
       f2 u[6];
@@ -226,7 +250,8 @@ __global__ void __launch_bounds__(128, WV == 1 ? kTracerFastMinB : kTracerMinB)
         cv[l] = q2_load(Q2, n, kQ2Base + c, T.cell[l]);
         if ((T.nall >> l) & 1u) cv[l] = -cv[l];
       }
-      const f2 r = tracer_face_flux_f2v<WV>(h, cv);
+      f2 r;
+      if (!tracer_face_flux_f2v<WV>(h, cv, r)) r = tracer_large<WV>(S, D, f, Q2, n, c, f2(t.x, t.y));
       F[(5 + c) * D.nfaces + f] = make_float2(r.hi, r.lo);
     }
   }

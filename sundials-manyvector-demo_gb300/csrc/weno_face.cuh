@@ -47,12 +47,13 @@ __device__ __forceinline__ float weno_scale(float a, float b, float c) {
 
 // The float-float reconstructions work on kF2Scale times the fluxes (the split factors and the
 // pressure carry it, so it costs nothing there): the weights' numerator holds eps^4 times a flux
-// difference, whose low part would leave the float range for fluxes below 5e-7; scaled, for fluxes
-// below 3e-23.
-constexpr float kF2Scale = 64.f;
+// difference, whose low part would leave the float range for small fluxes.  Scaled so that eps is
+// near 1 (0.79), the numerator leaves it where the fluxes' own float pairs do.  (Scale 64: errors
+// of 1e-7 at fluxes of 1e-30, 1e-3 at 1e-34; 1024: 2e-14 and 7e-11, as ratios of the a_k had.)
+constexpr float kF2Scale = 1024.f;
 
 // Both reconstructions of a face (lane x the plus side, lane y the minus side with its stencil
-// reversed), scaled values in and out: weno_diff64's formula.  The weights' products hold a^4 and
+// reversed), values scaled by s in and out, s2 = s^2: weno_diff64's formula.  The weights' products hold a^4 and
 // the numerator a candidate's correction beside it.  With a_k <= A, every |D23| and |D12| is below
 // 1.29 sqrt(A) and |D34|, |D01| below 2.77 sqrt(A), so |cA| + |cB| + |cC| < 9.8 sqrt(A) and the
 // numerator stays below 9.8 A^4.5: 2^125 for A = 2^27 (the denominator below 10 A^4 = 2^112).
@@ -60,14 +61,15 @@ constexpr float kF2Scale = 64.f;
 // out-of-line copy serves every reconstruction of a face (the kernel stays inside the instruction
 // cache).
 constexpr float kF2Big = 134217728.f;  // 2^27
-static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4) {
+static __device__ __noinline__ f2v weno_plus_f2v(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4,
+                                                 float s2) {
   const f2v D01 = f0 - f1, D12 = f1 - f2_, D23 = f2_ - f3, D34 = f3 - f4;
   const f2v D23x2 = f2v_scale(D23, 2.f);
   f2v aA, aB, aC;
   {
     // (the t's and k's are not renormalised: they only go into products, and what those drop
     // stays below 2^-48 of a_k)
-    const f2v eps{f2(kWenoEps * kF2Scale * kF2Scale)};
+    const f2v eps = f2v_scale(f2v(f2(kWenoEps)), s2);
     const f2v s23 = f2v_add_prod(eps, f2v_times(39.f / 64.f, D23), D23);
     const f2v s12 = f2v_add_prod(eps, f2v_times(39.f / 64.f, D12), D12);
     const f2v tA = f2v_add_scaled(D34, -11.f / 8.f, D23), tB = f2v_add_scaled(D12, -5.f / 8.f, D23),
@@ -131,28 +133,35 @@ __device__ __forceinline__ f2v weno_plus_f2dv(f2v f0, f2v f1, f2v f2_, f2v f3, f
   return f2_ + f2v(corr, make_float2(0.f, 0.f));
 }
 
-// one lane in FP64 (s: the values' scale)
-static __device__ __noinline__ f2 weno_fallback64(double s, f2 f0, f2 f1, f2 f2_, f2 f3, f2 f4) {
-  const double t = 1.0 / s;
-  return f2_from_double(s * weno_plus64(t * f0.to_double(), t * f1.to_double(),
-                                        t * f2_.to_double(), t * f3.to_double(),
-                                        t * f4.to_double()));
+// one lane in FP64
+static __device__ __noinline__ f2 weno_fallback64(f2 f0, f2 f1, f2 f2_, f2 f3, f2 f4) {
+  return f2_from_double(weno_plus64(f0.to_double(), f1.to_double(), f2_.to_double(),
+                                    f3.to_double(), f4.to_double()));
 }
 __device__ __forceinline__ float f2v_absmax(f2v a) {
   return fmaxf(fabsf(a.hi.x), fabsf(a.hi.y));
 }
-// WV = 0: weights in float-float, scaled values; WV = 1: the correction form with FP32 weights
+// unscaled values of any size (a rare path): WV = 0 with weights in float-float, WV = 1 in
+// correction form with FP32 weights; in FP64 beyond 1e18
 template <int WV>
-__device__ __forceinline__ f2v weno_pair(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4) {
+static __device__ __noinline__ f2v weno_large(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4) {
   const float mx = fmaxf(fmaxf(fmaxf(f2v_absmax(f0), f2v_absmax(f1)),
                                fmaxf(f2v_absmax(f2_), f2v_absmax(f3))), f2v_absmax(f4));
   if (mx < 1e18f) {
     if constexpr (WV == 1) return weno_plus_f2dv(f0, f1, f2_, f3, f4);
-    else return weno_plus_f2v(f0, f1, f2_, f3, f4);
+    else return weno_plus_f2v(f0, f1, f2_, f3, f4, 1.f);
   }
-  const double s = WV == 1 ? 1.0 : (double)kF2Scale;
-  return f2v(weno_fallback64(s, f0.x(), f1.x(), f2_.x(), f3.x(), f4.x()),
-             weno_fallback64(s, f0.y(), f1.y(), f2_.y(), f3.y(), f4.y()));
+  return f2v(weno_fallback64(f0.x(), f1.x(), f2_.x(), f3.x(), f4.x()),
+             weno_fallback64(f0.y(), f1.y(), f2_.y(), f3.y(), f4.y()));
+}
+// the float-float reconstructions of values scaled by kF2Scale
+__device__ __forceinline__ f2v weno_pair(f2v f0, f2v f1, f2v f2_, f2v f3, f2v f4) {
+  const float mx = fmaxf(fmaxf(fmaxf(f2v_absmax(f0), f2v_absmax(f1)),
+                               fmaxf(f2v_absmax(f2_), f2v_absmax(f3))), f2v_absmax(f4));
+  if (mx < 1e18f) return weno_plus_f2v(f0, f1, f2_, f3, f4, kF2Scale * kF2Scale);
+  const float t = 1.f / kF2Scale;
+  return f2v_scale(weno_large<0>(f2v_scale(f0, t), f2v_scale(f1, t), f2v_scale(f2_, t),
+                                 f2v_scale(f3, t), f2v_scale(f4, t)), kF2Scale);
 }
 
 // split factors of a pair of points, s (u +- alpha)/2 with ha = s alpha/2: lane x the plus side,
@@ -161,16 +170,34 @@ __device__ __forceinline__ f2v split_pair(f2 ua, f2 ub, f2 ha, float s) {
   return f2v_scale(f2v(ua, ub), 0.5f * s) + f2v(ha, -ha);
 }
 
-// one advected field: pair k holds c_k (u_k + alpha)/2 and c_{5-k} (u_{5-k} - alpha)/2, scaled
-// for WV = 0
+// the larger of two magnitudes, NaN if either is
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float f2v_absmax_nan(f2v a) {
+  return max_nan(fabsf(a.hi.x), fabsf(a.hi.y));
+}
+// one advected field: pair k holds c_k (u_k + alpha)/2 and c_{5-k} (u_{5-k} - alpha)/2; h: the
+// split factors, scaled for WV = 0.  Returns whether the products are in range: beyond 1e18, or
+// past the float range (NaN), the caller takes tracer_large.
 template <int WV>
-__device__ __forceinline__ f2 tracer_face_flux_f2v(const f2v (&h)[5], const f2 (&cv)[6]) {
+__device__ __forceinline__ bool tracer_face_flux_f2v(const f2v (&h)[5], const f2 (&cv)[6],
+                                                     f2& out) {
+  constexpr float kS = WV == 1 ? 1.f : kF2Scale;
   f2v a[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) a[k] = f2v(cv[k], cv[5 - k]) * h[k];
-  const f2v r = weno_pair<WV>(a[0], a[1], a[2], a[3], a[4]);
-  const f2 o = r.x() + r.y();
-  return WV == 1 ? o : f2_scale(o, 1.f / kF2Scale);
+  const float mx = max_nan(max_nan(max_nan(f2v_absmax_nan(a[0]), f2v_absmax_nan(a[1])),
+                                   max_nan(f2v_absmax_nan(a[2]), f2v_absmax_nan(a[3]))),
+                           f2v_absmax_nan(a[4]));
+  if (!(mx < 1e18f)) return false;
+  f2v r;
+  if constexpr (WV == 1) r = weno_plus_f2dv(a[0], a[1], a[2], a[3], a[4]);
+  else r = weno_plus_f2v(a[0], a[1], a[2], a[3], a[4], kS * kS);
+  out = f2_scale(r.x() + r.y(), 1.f / kS);
+  return true;
 }
 
 }  // namespace gbmv

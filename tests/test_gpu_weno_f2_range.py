@@ -1,8 +1,9 @@
 """The float-float reconstructions between the sizes at which their arithmetic changes, against the
-oracle: linear ramps whose jumps per cell cross the point where the weights are scaled.  The states
-keep velocities and sound speeds near 1, so the mixed form's parity bar is 1e-9 of the largest
-tendency (its roundings are 2^-46, times the flux over its difference, ~100 here); the FP64 form's
-own error is held to 1e-11, so that a broken reference could not pass."""
+oracle: linear ramps whose jumps per cell cross the point where the weights are scaled, and tracers
+at both ends of the float range.  The ramps keep velocities and sound speeds near 1, so the mixed
+form's parity bar is 1e-9 of the largest tendency (its roundings are 2^-46, times the flux over its
+difference, ~100 here); the FP64 form's own error is held to 1e-11, so that a broken reference could
+not pass."""
 import numpy as np
 import pytest
 
@@ -55,3 +56,34 @@ def test_ramps_across_the_scaling_of_the_weights(cuda, fluid, lo, hi):
     shape, bc = (12, 30, 20), (1, 1, 0, 0, 1, 1)
     fields = _ramp_state(shape, 2, lo, hi, fluid)
     _check(cuda, shape, 2, bc, fields, 1e-9, (gbmv.MIXED, gbmv.MIXED_FAST))
+
+
+def _tracer_state(shape, nchem, size, seed):
+    """Uniform density and pressure, velocities of a few tenths, tracers of the given size."""
+    rng = np.random.default_rng(seed)
+    nx, ny, nz = shape
+    rho = np.ones((nz, ny, nx))
+    u = rng.uniform(-0.3, 0.3, (3, nz, ny, nx))
+    f = [rho, u[0], u[1], u[2], 1.0 / (GAMMA - 1.0) + 0.5 * (u * u).sum(0)]
+    f.append(size * rng.uniform(0.5, 1.5, (nz, ny, nx, nchem)))
+    return f
+
+
+# fluxes whose float pairs reach the end of the float range, where the pairs themselves lose bits
+# (2^-149 absolute: a few dozen such roundings make a tendency); FP32 weights keep the contract's 1e-6
+@pytest.mark.parametrize("size", [1e-18, 1e-24, 1e-28, 1e-30, 1e-32, 1e-34, 1e-36])
+def test_small_tracers(cuda, size):
+    import gbmv
+    shape, bc = (17, 12, 9), (3, 3, 0, 0, 1, 1)
+    fields = _tracer_state(shape, 2, size, 7)
+    _check(cuda, shape, 2, bc, fields, 1e-12 + 64 * 2.0 ** -149 / size, (gbmv.MIXED,
+                                                                        gbmv.MIXED_FAST))
+
+
+# on both sides of the FP64 fallback (fluxes of 1e18, 1e15 scaled) up to the end of the float range
+@pytest.mark.parametrize("size", [1e12, 7e14, 2e15, 1e16, 1e17, 3e18, 1e20, 1e30, 5e36])
+def test_large_tracers(cuda, size):
+    import gbmv
+    shape, bc = (5, 4, 3), (3, 3, 0, 0, 1, 1)
+    fields = _tracer_state(shape, 2, size, 8)
+    _check(cuda, shape, 2, bc, fields, 1e-12, (gbmv.MIXED, gbmv.MIXED_FAST))
