@@ -554,11 +554,24 @@ int conservation_sums(const Grid& g, const Fields& w, double* d_scratch, double*
   return GBMV_OK;
 }
 
+// s + x for non-negative numbers, the addition's rounding error added to c: Dekker's sum of the
+// larger and the smaller, four FP64 instructions where two_sum_acc takes seven for the same error.
+// The order is found on the bits, which for non-negative doubles is integer work (comparisons of
+// doubles run on the FP64 pipe).
+__device__ __forceinline__ void pos_sum_acc(double& s, double& c, double x) {
+  const bool swap = __double_as_longlong(x) > __double_as_longlong(s);
+  const double a = swap ? x : s, b = swap ? s : x;
+  const double t = a + b;
+  c += b - (t - a);
+  s = t;
+}
+
 // N_VWrmsNorm of the six-component ManyVector (the norm ARKODE's error test and Newton
 // convergence test take, src/imex_chem_hydro_main.cpp:463): ewt = 1 / (rtol |y| + atol) per
 // entry, sum of (v ewt)^2 over the five fluid fields (ncell each) and the chemistry field
 // (nchem ncell), divided by the total length, square root.  Same fixed-grid compensated
-// two-pass reduction as the conservation totals; partials in scratch[0..kConsBlocks).
+// two-pass reduction as the conservation totals, every term compensated; partials in
+// scratch[0..kConsBlocks).
 __global__ void __launch_bounds__(256) wrms_partial_kernel(long ncell, int nchem, Fields v,
                                                            Fields y, double rtol, double atol,
                                                            double* __restrict__ part) {
@@ -568,21 +581,20 @@ __global__ void __launch_bounds__(256) wrms_partial_kernel(long ncell, int nchem
     const double* __restrict__ vk = v.f[k];
     const double* __restrict__ yk = y.f[k];
     if (n == 0) continue;
-    // Four terms are summed plainly before each compensated addition: their rounding is that of
-    // the terms themselves, and the FP64 pipe bounds this pass (14 -> 8 instructions a term with
-    // the reciprocal in place of the division; 100^3 x 15: 408 -> 228 us).
+    // Bound by the FP64 pipe: 11 instructions a term, five of them the weight's reciprocal and
+    // four the compensated addition (an IEEE division and two_sum_acc: 18).  100^3 x 15: 408 us
+    // with those, 296 now; 228 with one compensation for four terms, which was up to an ulp off.
+    // Four terms at a time keep enough loads in flight.
     const long stride = (long)gridDim.x * blockDim.x;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += 4 * stride) {
-      double x = 0.0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const long e = i + j * stride;
         if (e < n) {
           const double q = vk[e] * rcp64_any(fma(rtol, fabs(yk[e]), atol));
-          x = fma(q, q, x);
+          pos_sum_acc(s0, c0, q * q);
         }
       }
-      two_sum_acc(s0, c0, x);
     }
   }
   double a = s0 + c0;
