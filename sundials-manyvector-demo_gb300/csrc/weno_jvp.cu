@@ -50,7 +50,7 @@ __device__ __forceinline__ void roe_dual(const Dual (&W)[6][5], const Dual (&ph)
   const double sL = sqrt0_64(W[2][0].v), sR = sqrt0_64(W[3][0].v);
   const double rL = rcp64_any(sL), rR = rcp64_any(sR);
   const double tL = 0.5 * W[2][0].d * rL, tR = 0.5 * W[3][0].d * rR;  // tangents of the roots
-  const Dual iL(rL, -(tL * (rL * rL))), iR(rR, -(tR * (rR * rR)));
+  const Dual iL(rL, -(tL * rL) * rL), iR(rR, -(tR * rR) * rR);
   const Dual is = drcp(Dual(sL + sR, tL + tR));
   R.u = dfma(W[2][1], iL, W[3][1] * iR) * is;
   R.v = dfma(W[2][2], iL, W[3][2] * iR) * is;
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(128) face_flux_jvp_kernel(const __grid_constan
       for (int v = 0; v < 5; ++v) W[l][v] = Dual(T.W[l][v], t[v]);
       // u = m / rho;  p/2 = (gamma-1)/2 (E - |m|^2 / (2 rho))
       const double x = T.u[l], q = 0.5 * fma(x, x, fma(v1, v1, v2 * v2));
-      u[l] = Dual(x, fma(-x, t[0], t[1]) * ir[l]);
+      u[l] = Dual(x, over64(fma(-x, t[0], t[1]), T.W[l][0], ir[l]));
       ph[l] = Dual(T.ph[l], 0.5 * gm *
                    fma(q, t[0], fma(-x, t[1], fma(-v1, t[2], fma(-v2, t[3], t[4])))));
     }
@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(128) face_flux_jvp_kernel(const __grid_constan
     // (c/2)^2 = gamma (p/2) / (2 rho), so d(c/2) = gamma / (4 rho) (dp/2 - (p/2) drho/rho) / (c/2)
     int am;
     const double ha = half_alpha64(T, &am);
-    double su = T.u[0], du = u[0].d, sp = T.ph[0], dp = ph[0].d, sr = W[0][0].d, si = ir[0],
-           sc = T.hc[0];
+    double su = T.u[0], du = u[0].d, sp = T.ph[0], dp = ph[0].d, sv = T.W[0][0], sr = W[0][0].d,
+           si = ir[0], sc = T.hc[0];
 #pragma unroll
     for (int l = 1; l < 6; ++l) {
       const bool m = l == am;
@@ -181,12 +181,14 @@ __global__ void __launch_bounds__(128) face_flux_jvp_kernel(const __grid_constan
       du = m ? u[l].d : du;
       sp = m ? T.ph[l] : sp;
       dp = m ? ph[l].d : dp;
+      sv = m ? T.W[l][0] : sv;
       sr = m ? W[l][0].d : sr;
       si = m ? ir[l] : si;
       sc = m ? T.hc[l] : sc;
     }
     double dha = su < 0.0 ? -0.5 * du : 0.5 * du;
-    if (sc > 0.0) dha += 0.25 * S.gamma * si * fma(-(sp * si), sr, dp) / sc;
+    if (sc > 0.0)
+      dha += 0.25 * S.gamma * over64(fma(-over64(sp, sv, si), sr, dp), sv, si) / sc;
     Dual hp[6], hm[6];
 #pragma unroll
     for (int l = 0; l < 6; ++l) {

@@ -279,9 +279,9 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
       const double sb2 = -is * fma(ub, u, fma(vb, v, fma(wb, w, Hb * R.H)));
       // d iL = -iL^2 dsL, dsL = drho iL / 2
       if (T.W[2][0] > 0.0)
-        B.W[2][0] = fma(0.5 * iL, fma(-(iL * iL), iLb, sb2), B.W[2][0]);
+        B.W[2][0] = fma(0.5 * iL, fma(-iL, iL * iLb, sb2), B.W[2][0]);
       if (T.W[3][0] > 0.0)
-        B.W[3][0] = fma(0.5 * iR, fma(-(iR * iR), iRb, sb2), B.W[3][0]);
+        B.W[3][0] = fma(0.5 * iR, fma(-iR, iR * iRb, sb2), B.W[3][0]);
     }
     // half the Lax-Friedrichs speed at its point: ha = |u|/2 + c/2,
     // d(c/2) = gamma / (4 rho) (d(p/2) - (p/2) drho / rho) / (c/2)
@@ -298,9 +298,9 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
       const double uadd = su < 0.0 ? -0.5 * B.ha : 0.5 * B.ha;
       double padd = 0.0, radd = 0.0;
       if (sc > 0.0) {
-        const double ir = rcp64_any(sr);
-        padd = 0.25 * S.gamma * ir * B.ha / sc;
-        radd = -(padd * sp) * ir;
+        const double ir = rcp64(sr);
+        padd = 0.25 * S.gamma * over64(B.ha, sr, ir) / sc;
+        radd = -over64(padd * sp, sr, ir);
       }
 #pragma unroll
       for (int l = 0; l < 6; ++l) {
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(128) face_flux_vjp_kernel(const __grid_constan
     for (int l = 0; l < 6; ++l) {
       const double ir = rcp64(T.W[l][0]), x = T.u[l], v1 = __ldg(D.vel[1] + cell[l]),
                    v2 = __ldg(D.vel[2] + cell[l]);
-      const double k = 0.5 * gm * B.ph[l], m = B.u[l] * ir;
+      const double k = 0.5 * gm * B.ph[l], m = over64(B.u[l], T.W[l][0], ir);
       double q[5];
       q[0] = fma(k, 0.5 * fma(x, x, fma(v1, v1, v2 * v2)), fma(-m, x, B.W[l][0]));
       q[1] = fma(-k, x, B.W[l][1] + m);

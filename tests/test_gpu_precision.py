@@ -31,3 +31,37 @@ def test_wrms_terms_are_compensated(cuda, big, small):
     mean = (Fraction(big) ** 2 + 3 * Fraction(small) ** 2) / 4
     exact = (Decimal(mean.numerator) / Decimal(mean.denominator)).sqrt()
     assert abs(Decimal(got) - exact) <= Decimal(math.ulp(got)) * Decimal("0.75")
+
+
+@pytest.mark.parametrize("rho_vacuum", [1.2e-308, 1e-310])
+def test_derivatives_beside_a_subnormal_density(cuda, rho_vacuum):
+    """A near-vacuum cell whose density is below the range of the approximate reciprocal (the first's
+    reciprocal is a double still): the products elsewhere are those beside one of 1e-290 (both
+    vanish beside the neighbours' numbers; 1e-10 leaves their roundings a wide margin)."""
+    torch = cuda
+    import gbmv
+    shape, bc = (9, 8, 7), (0, 0, 1, 1, 3, 3)
+    rng = np.random.default_rng(3)
+    n = (shape[2], shape[1], shape[0])
+    w0 = [rng.uniform(0.5, 1.5, n)] + [rng.uniform(-0.2, 0.2, n) for _ in range(3)]
+    w0.append(rng.uniform(2.0, 3.0, n))
+    d0, v0 = ([rng.standard_normal(n) for _ in range(5)] for _ in range(2))
+    at = (3, 4, 4)
+    other = np.ones(n, dtype=bool)
+    other[at] = False
+    h = gbmv.Hydro(shape, 0, bc, 1.4, None)
+    out = []
+    for rho in (rho_vacuum, 1e-290):
+        for f, x in zip(w0, (rho, 0.0, 0.0, 0.0, 2.5 * rho)):
+            f[at] = x
+        for f in d0:
+            f[at] = 0.0
+        w, dw, v = ([torch.from_numpy(f).cuda() for f in g] for g in (w0, d0, v0))
+        jv, vj = ([torch.full_like(f, np.nan) for f in w] for _ in range(2))
+        assert h.fEuler_jvp(0.0, w, dw, jv) == 0
+        assert h.fEuler_vjp(0.0, w, v, vj) == 0
+        out.append([x.cpu().numpy() for x in jv + vj])
+    for k, (a, b) in enumerate(zip(*out)):
+        a, b = a[other], b[other]
+        assert np.isfinite(b).all(), k
+        assert np.max(np.abs(a - b)) <= 1e-10 * np.max(np.abs(b)), k
