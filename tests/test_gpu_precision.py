@@ -65,3 +65,16 @@ def test_derivatives_beside_a_subnormal_density(cuda, rho_vacuum):
         a, b = a[other], b[other]
         assert np.isfinite(b).all(), k
         assert np.max(np.abs(a - b)) <= 1e-10 * np.max(np.abs(b)), k
+
+
+def test_wave_speed_at_a_tiny_density(cuda):
+    """A density whose reciprocal is not a double: the speed is that of the quotients."""
+    torch = cuda
+    import gbmv
+    shape = (4, 3, 3)
+    h = gbmv.Hydro(shape, 0, (0,) * 6, 1.4, None)
+    w = [torch.full((3, 3, 4), x, dtype=torch.float64, device="cuda")
+         for x in (1e-310, 5e-311, 0.0, 0.0, 1e-310)]
+    alpha = 0.5 + math.sqrt(1.4 * 0.4)
+    dt = 0.5 * 0.25 / alpha
+    assert abs(h.stability(w, 0.5) - dt) <= 1e-12 * dt
