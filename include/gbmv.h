@@ -598,6 +598,12 @@ int gbmv_diag_fma_rate(int fp64, double* flops_per_s);
 int gbmv_diag_convert_check(const double* d_in, long n, unsigned long long* mismatches,
                             void* stream);
 
+/* The FP64 functions the kernels evaluate in place of divisions and logarithms, at the n device
+ * doubles x: d_out[0..n) = 1/x (any x), [n..2n) = 2/x (normal x and 1/x), [2n..3n) = 3/x as the
+ * derivative sweeps divide by a density, [3n..4n) = log x as the chemistry takes it of a
+ * temperature.  Asynchronous.  (No counterpart in the reference.) */
+int gbmv_diag_math(gbmv_chem c, const double* d_x, long n, double* d_out, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -586,6 +586,11 @@ double* gbmv_chem_state(gbmv_chem c, int which) {
   }
 }
 
+int gbmv_diag_math(gbmv_chem c, const double* d_x, long n, double* d_out, void* stream) {
+  if (!c || !d_x || !d_out || n < 0) { set_error("bad diagnostic arguments"); return GBMV_EINVAL; }
+  return diag_math(c->P, d_x, n, d_out, (cudaStream_t)stream);
+}
+
 int gbmv_chem_prepare(gbmv_chem c, double* chem, void* stream) {
   if (!c || !chem) return GBMV_EINVAL;
   return chem_prepare(c->S, chem, c->n, (cudaStream_t)stream);

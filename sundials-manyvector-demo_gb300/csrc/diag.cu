@@ -2,7 +2,9 @@
 // the FP64 (and FP32) fused multiply-add rate of the SIMT pipes.  Each thread runs 8
 // independent FMA chains for a fixed number of iterations; flops = 2 * FMAs.
 #include "common.cuh"
+#include "chem_net.cuh"
 #include "df64.cuh"
+#include "weno64.cuh"
 
 namespace gbmv {
 
@@ -77,6 +79,27 @@ __global__ void __launch_bounds__(256) convert_check_kernel(const double* __rest
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, off);
   if ((threadIdx.x & 31) == 0 && mine) atomicAdd(bad, mine);
+}
+
+__global__ void __launch_bounds__(256) math_kernel(ChemParams P, const double* __restrict__ in,
+                                                   long n, double* __restrict__ out) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
+       i += (long)gridDim.x * blockDim.x) {
+    const double x = in[i];
+    out[i] = rcp64_any(x);
+    out[n + i] = rcp_twice(x);
+    out[2 * n + i] = over64(3.0, x, rcp64(x));
+    out[3 * n + i] = chem_log(P, x);
+  }
+}
+
+int diag_math(const ChemParams& P, const double* in, long n, double* out, cudaStream_t s) {
+  long b = (n + 255) / 256;
+  if (b > (long)kSM * 8) b = (long)kSM * 8;
+  if (b < 1) b = 1;
+  math_kernel<<<(int)b, 256, 0, s>>>(P, in, n, out);
+  GBMV_LAUNCH_CHECK("math_kernel");
+  return GBMV_OK;
 }
 
 }  // namespace gbmv

@@ -163,6 +163,7 @@ SIGNATURES = [
     ("gbmv_launch_count", C.c_long, []),
     ("gbmv_diag_fma_rate", C.c_int, [C.c_int, _P]),
     ("gbmv_diag_convert_check", C.c_int, [_VP, C.c_long, C.POINTER(C.c_ulonglong), _VP]),
+    ("gbmv_diag_math", C.c_int, [_VP, _VP, C.c_long, _VP, _VP]),
     ("gbmv_profile_enable", C.c_int, [C.c_int]),
     ("gbmv_profile_reset", C.c_int, []),
     ("gbmv_profile_get", C.c_int, [C.c_char_p, _P, C.POINTER(C.c_long)]),
@@ -681,6 +682,15 @@ def convert_check(d) -> int:
     _check(load().gbmv_diag_convert_check(_dev_ptr(d), d.numel(), C.byref(out), None),
            "gbmv_diag_convert_check")
     return int(out.value)
+
+
+def diag_math(chem: Chem, x):
+    """1/x, 2/x, 3/x and log x of the doubles of the CUDA tensor x, as the kernels evaluate them."""
+    import torch
+    out = torch.empty((4, x.numel()), dtype=torch.float64, device=x.device)
+    _check(load().gbmv_diag_math(chem.c, _dev_ptr(x), x.numel(), _dev_ptr(out),
+                                 _stream_ptr(None)), "gbmv_diag_math")
+    return out
 
 
 def fma_rate(fp64: bool = True) -> float:

@@ -78,3 +78,43 @@ def test_wave_speed_at_a_tiny_density(cuda):
     alpha = 0.5 + math.sqrt(1.4 * 0.4)
     dt = 0.5 * 0.25 / alpha
     assert abs(h.stability(w, 0.5) - dt) <= 1e-12 * dt
+
+
+def _ulps(got, exact):
+    """Error of the doubles got against extended-precision numbers, in units in the last place."""
+    ulp = np.spacing(np.abs(exact).astype(np.float64)).astype(np.longdouble)
+    return np.abs((got.astype(np.longdouble) - exact) / ulp)
+
+
+def _functions(torch, tables, x):
+    import gbmv
+    c = gbmv.Chem(1, tables)
+    return gbmv.diag_math(c, torch.from_numpy(x).cuda()).cpu().numpy()
+
+
+def _doubles(rng, n, lo, hi):
+    """Doubles of either sign, exponents lo .. hi - 1: random, and the ends of a binade."""
+    m = 1.0 + rng.integers(0, 1 << 52, n) * 2.0 ** -52
+    m[:n // 8] = 1.0
+    m[n // 8:n // 4] = 2.0 - 2.0 ** -52
+    return np.ldexp(m, rng.integers(lo, hi, n)) * rng.choice([-1.0, 1.0], n)
+
+
+# r (1 + e + e^2) with |e| < 2^-20: half a unit for the last rounding, 2^-60 for e^3
+def test_reciprocals(cuda, tables):
+    rng = np.random.default_rng(1)
+    one = np.longdouble(1)
+    x = _doubles(rng, 1 << 19, -1021, 1021)
+    r, _, q, _ = _functions(cuda, tables, x)
+    assert _ulps(r, one / x).max() <= 0.51
+    assert _ulps(q, 3 * one / x).max() <= 1.6  # 3 r: the reciprocal's rounding and the product's
+    x = _doubles(rng, 1 << 19, -1000, 1000)
+    assert _ulps(_functions(cuda, tables, x)[1], 2 * one / x).max() <= 0.51
+    # outside the approximate instruction's range: the division, bit for bit
+    x = np.concatenate([_doubles(rng, 4096, -1074, -1021), _doubles(rng, 4096, 1021, 1024),
+                        [5e-324, -5e-324, 0.0, -0.0, np.inf, -np.inf, np.nan]])
+    r, _, q, _ = _functions(cuda, tables, x)
+    with np.errstate(divide="ignore", over="ignore"):
+        ok = np.abs(x) != np.ldexp(1.0, -1021)
+        assert np.array_equal(r[ok], (1.0 / x)[ok], equal_nan=True)
+        assert np.array_equal(q[ok], (3.0 / x)[ok], equal_nan=True)
