@@ -134,20 +134,26 @@ static int finish(int rc, cudaStream_t s) {
 }
 static int flags_of(const HostWords* w) { return *static_cast<const volatile int*>(&w->flags); }
 
-// chem_log's table, formed once a process: 1/c and -log(1/c) of each interval's midpoint c.  The
-// intervals repeat from one binade to the next, so 128 logarithms do (a long double one takes
+// chem_log's table, formed once a process: 1/c to 21 bits, for c near each interval's midpoint, and
+// log(c) = -log(1/c) as a double and what is left of it (its high word in the low word of 1/c).
+// The intervals repeat from one binade to the next, so 128 logarithms do (a long double one takes
 // ~0.6 us on the Arm host).
 struct LogTable {
   double e[2 * kLogEntries];
   LogTable() {
+    auto bits = [](double x) { uint64_t b; memcpy(&b, &x, 8); return b; };
+    auto number = [](uint64_t b) { double x; memcpy(&x, &b, 8); return x; };
+    const uint64_t high = 0xFFFFFFFF00000000ULL;
     const long double ln2 = logl(2.0L);
     for (int k = 0; k < 128; ++k) {
-      const double inv = 1.0 / (1.0 + (k + 0.5) / 128.0);
+      const double inv = number((bits(1.0 / (1.0 + (k + 0.5) / 128.0)) + 0x80000000ULL) & high);
       const long double log_inv = logl((long double)inv);
       for (int q = k; q < kLogEntries; q += 128) {
         const int x = (q >> 7) - 2;
-        e[2 * q] = ldexp(inv, -x);
-        e[2 * q + 1] = (double)(x * ln2 - log_inv);
+        const long double log_c = x * ln2 - log_inv;
+        const double hi = (double)log_c, lo = (double)(log_c - hi);
+        e[2 * q] = number(bits(ldexp(inv, -x)) | bits(lo) >> 32);
+        e[2 * q + 1] = hi;
       }
     }
   }

@@ -44,22 +44,23 @@ struct ChemParams {
 
 // Natural logarithm of a temperature by table and series (P. T. P. Tang, ACM Trans. Math. Softw. 16
 // (1990) 378-400): the entry of the exponent and the seven leading significand bits holds 1/c and
-// log(c) of its interval's midpoint c, r = T/c - 1 is below 2^-8, and six terms of log(1 + r)
-// leave 2^-58.  Eight FP64 instructions where the library's logarithm takes ~25; error within
-// 1.5 units in the last place above T = 2 (absolute error below 2e-15 everywhere, which is what
-// the table position needs).  Temperatures outside [1/4, 2^18) take the library's.
+// log(c) near its interval's midpoint c, r = T/c - 1 is below 2^-7.99, and six terms of log(1 + r)
+// leave 2^-58.  1/c has 21 bits; its low word holds the high word of what log(c) has beyond a
+// double, so that the last addition's rounding is the only other error (0.5 units in the last
+// place above T = 2; 1.5 with log(c) a double, one FP64 instruction less).  Nine FP64 instructions
+// where the library's logarithm takes ~25.  Temperatures outside [1/4, 2^18) take the library's.
 constexpr int kLogLowHi = 0x3FD00000;  // high word of 1/4
 constexpr int kLogEntries = 20 * 128;
 __device__ __forceinline__ double chem_log(const ChemParams& P, double T) {
   const unsigned q = (unsigned)(__double2hiint(T) - kLogLowHi) >> 13;
   if (q >= (unsigned)kLogEntries) return log(T);
   const double2 e = __ldg(P.ltab + q);
-  const double r = fma(T, e.x, -1.0);
+  const double r = fma(T, __hiloint2double(__double2hiint(e.x), 0), -1.0);
   double p = fma(r, -1.0 / 6.0, 1.0 / 5.0);
   p = fma(r, p, -1.0 / 4.0);
   p = fma(r, p, 1.0 / 3.0);
   p = fma(r, p, -0.5);
-  return e.y + fma(r * r, p, r);
+  return e.y + fma(r * r, p, r + __hiloint2double(__double2loint(e.x), 0));
 }
 
 // Table position of a temperature: bin b (clamped to the table) and the interpolation weight

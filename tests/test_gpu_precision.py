@@ -118,3 +118,19 @@ def test_reciprocals(cuda, tables):
         ok = np.abs(x) != np.ldexp(1.0, -1021)
         assert np.array_equal(r[ok], (1.0 / x)[ok], equal_nan=True)
         assert np.array_equal(q[ok], (3.0 / x)[ok], equal_nan=True)
+
+
+def test_temperature_logarithm(cuda, tables):
+    """Six terms of the series leave 2^-58 absolute; the table's entry carries more bits than a
+    double, so the last addition's rounding is the only other error."""
+    rng = np.random.default_rng(2)
+    inside = np.exp2(rng.uniform(-2.0, 18.0, 1 << 19))
+    edges = np.ldexp(1.0 + np.arange(129) / 128.0, 0)[None] * np.exp2(np.arange(-2, 17))[:, None]
+    edges = np.concatenate([edges.ravel(), np.nextafter(edges, 0).ravel()])
+    x = np.concatenate([inside, edges[(edges >= 0.25) & (edges < 2.0 ** 18)]])
+    exact = np.log(x.astype(np.longdouble))
+    got = _functions(cuda, tables, x)[3]
+    half = 0.5 * np.spacing(np.abs(exact).astype(np.float64))
+    assert np.all(np.abs(got - exact) <= 1.01 * half + 2.0 ** -57.5)
+    x = np.concatenate([np.exp2(rng.uniform(-40, -2.01, 4096)), np.exp2(rng.uniform(18.0, 60, 4096))])
+    assert _ulps(_functions(cuda, tables, x)[3], np.log(x.astype(np.longdouble))).max() <= 1.0
