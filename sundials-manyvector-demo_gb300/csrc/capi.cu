@@ -774,6 +774,7 @@ static int dirk_store(gbmv_chem c, DirkOpts* O, cudaStream_t s) {
   }
   O->kstore = c->dirk_k;
   O->kstore_lanes = c->dirk_k_lanes;
+  O->cells = c->n;
   if (!c->dirk_retry) {  // the FP32 form's second pass: start state, Ts, failed-cell list
     if (capturing(s)) {
       set_error("the first DIRK call allocates its buffers: make it before any capture");
@@ -858,6 +859,7 @@ static int dirk_opts(const gbmv_dirk_opts* o, double t0, double tout, double tun
   for (int q = 0; q < 8; ++q) O->fz[q] = nullptr;
   O->kstore = nullptr;
   O->kstore_lanes = 0;
+  O->cells = 0;
   O->list_in = nullptr;
   O->list_in_n = nullptr;
   O->y_init = nullptr;
@@ -873,10 +875,10 @@ static int ck(cudaError_t e, const char* where) {
 
 // Block-size autotuner: integrates a sample of the cells (the first min(n, 65536), their
 // temperature state saved and restored) once per candidate, 32 and 64 threads, and keeps the
-// fastest.  (128 is accepted as an explicit option but not a candidate: on the 64^3
-// static-chemistry run it measured 2.49 s against 2.27-2.30 s for 32 and 64 in the FP64 form
-// and no better in the mixed one, while a sample run -- under two cells per lane, so mostly
-// its slowest cells -- cannot tell them apart.)
+// fastest; a sample runs at the resident warps that all the cells get.  (128 is accepted as an
+// explicit option but not a candidate: on the 64^3 static-chemistry run it measured 2.49 s against
+// 2.27-2.30 s for 32 and 64 in the FP64 form and no better in the mixed one, while a sample run --
+// a few cells per lane, so mostly its slowest cells -- cannot tell them apart.)
 static int dirk_autotune(gbmv_chem c, const double* y, const DirkOpts& O, int mixed,
                          cudaStream_t s) {
   const long ns = c->n < 65536 ? c->n : 65536;

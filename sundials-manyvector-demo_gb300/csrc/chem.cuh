@@ -94,6 +94,7 @@ struct DirkOpts {
   // kstore_lanes lanes; K_0 stays in shared memory
   double* kstore;
   long kstore_lanes;
+  long cells;  // host only: cells that set the residency (a sample runs as the whole would), 0: n
   // cell lists.  list_in: null = cells 0..n-1, else the *list_in_n cells list_in[...], each
   // started from y_init / Ts_init (Ts at [cell], dTs/dge at [n + cell]) instead of the in-out
   // state.  list_out: null = failed cells are counted in nfail, else appended to list_out.

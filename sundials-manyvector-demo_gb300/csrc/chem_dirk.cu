@@ -667,7 +667,7 @@ static int launch_dirk(const ChemParams& P, const ChemState& S, long n, double* 
   // latency that more warps hide counts (mixed form, 4 / 5 / 8 warps per SM: 32^3 cells 44.1 /
   // 49.3 / 58.7 ms, 44^3 74.6 / 75.6 / 80.4, 48^3 90.8 / 90.3 / 95.0, 52^3 109.0 / 107.1 / 109.6,
   // 64^3 183 / 179 / 175).
-  const long warps = n / (32L * nsm);
+  const long warps = (O.cells ? O.cells : n) / (32L * nsm);
   const int cap = (warps < 20 ? 4 : (warps < 28 ? 5 : 64)) * 32 / BS;
   if (per_sm > cap && cap > 0) per_sm = cap;
   long blocks = (long)nsm * per_sm;
