@@ -664,12 +664,14 @@ static int launch_dirk(const ChemParams& P, const ChemState& S, long n, double* 
   // Resident warps by the cells there are for each SM.  The launch ends with its costliest cells,
   // and a warp that shares its scheduler's FP64 pipe runs them at half speed, so with few cells
   // per lane one warp a scheduler, refilled from the cost order, ends sooner; with many the
-  // latency that more warps hide counts (mixed form, 4 / 5 / 8 warps per SM: 32^3 cells 44.1 /
-  // 49.3 / 58.7 ms, 44^3 74.6 / 75.6 / 80.4, 48^3 90.8 / 90.3 / 95.0, 52^3 109.0 / 107.1 / 109.6,
-  // 64^3 183 / 179 / 175).
+  // latency that more warps hide counts.  Blocks of 32; ms at 4 / 5 / 8 warps per SM, mixed form:
+  // 32^3 cells 42.8 / 47.1 / 57.0, 40^3 60.7 / 61.8 / 66.4, 48^3 88.3 / 87.3 / 90.2, 64^3 179.7 /
+  // 173.4 / 166.1; FP64 form, of which 5 fit: 32^3 67.1 / 71.9, 40^3 97.5 / 97.7, 44^3 115.4 /
+  // 116.2, 48^3 140.8 / 139.2, 52^3 170.0 / 165.3.  Rounded up for larger blocks (64 threads, 48^3,
+  // 4 / 6 warps: mixed 88.3 / 87.4, FP64 142.1 / 139.6).
   const long warps = (O.cells ? O.cells : n) / (32L * nsm);
-  const int cap = (warps < 20 ? 4 : (warps < 28 ? 5 : 64)) * 32 / BS;
-  if (per_sm > cap && cap > 0) per_sm = cap;
+  const int cap = ((warps < 20 ? 4 : (warps < 28 ? 5 : 64)) * 32 + BS - 1) / BS;
+  if (per_sm > cap) per_sm = cap;
   long blocks = (long)nsm * per_sm;
   const long need = (n + BS - 1) / BS;
   if (blocks > need) blocks = need;
