@@ -14,6 +14,7 @@
 
 #include "butcher.cuh"
 #include "chem.cuh"
+#include "host_words.h"
 #include "weno.cuh"
 
 namespace gbmv {
@@ -72,58 +73,7 @@ ProfScope::~ProfScope() {
 
 using namespace gbmv;
 
-// What a synchronous call reads back, in page-locked host memory that its kernels write directly
-// (status words only where a state is illegal or a block singular): no clearing launch and no copy
-// on the stream, which for a 128 x 3 x 3 right-hand side were 10 of 44 us (the copy into pageable
-// memory is staged by the CUDA driver).
-struct HostWords {
-  int flags;       // legal-state mask of the flow; singular block of a chemistry or block handle
-  double sums[2];  // norm, totals
-  unsigned long long speed;
-};
-// A page-locked allocation costs ~0.3 ms, so the handles of a process share one page of 64 slots,
-// kept while the process lives; further handles get an allocation of their own.
-constexpr int kWordSlots = 64;
-constexpr size_t kWordStride = 64;
-static_assert(sizeof(HostWords) <= kWordStride, "a slot holds the words");
-static std::mutex g_words_mu;
-static char* g_words_page = nullptr;
-static unsigned long long g_words_used = 0;
-
-static bool host_words(HostWords** p) {
-  const unsigned flags = cudaHostAllocMapped | cudaHostAllocPortable;
-  std::lock_guard<std::mutex> lk(g_words_mu);
-  if (g_words_page) {  // the page does not outlive the context it was made in
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, g_words_page) != cudaSuccess ||
-        a.type != cudaMemoryTypeHost) {
-      cudaGetLastError();
-      g_words_page = nullptr;
-    }
-  }
-  if (!g_words_page) {
-    void* page = nullptr;
-    if (cudaHostAlloc(&page, kWordSlots * kWordStride, flags) != cudaSuccess) return false;
-    g_words_page = static_cast<char*>(page);
-    g_words_used = 0;
-  }
-  for (int k = 0; k < kWordSlots; ++k) {
-    if (g_words_used >> k & 1ULL) continue;
-    g_words_used |= 1ULL << k;
-    *p = reinterpret_cast<HostWords*>(g_words_page + k * kWordStride);
-    return true;
-  }
-  return cudaHostAlloc(reinterpret_cast<void**>(p), sizeof(HostWords), flags) == cudaSuccess;
-}
-static void free_host_words(HostWords* p) {
-  if (!p) return;
-  std::lock_guard<std::mutex> lk(g_words_mu);
-  const char* const c = reinterpret_cast<const char*>(p);
-  if (g_words_page && c >= g_words_page && c < g_words_page + kWordSlots * kWordStride)
-    g_words_used &= ~(1ULL << ((c - g_words_page) / kWordStride));
-  else
-    cudaFreeHost(p);
-}
+static WordPool g_words;
 // the end of a synchronous call whose launches returned rc (after a failed launch the earlier ones
 // are waited for: they must not write into the next call's words)
 static int finish(int rc, cudaStream_t s) {
@@ -168,7 +118,7 @@ struct gbmv_hydro_s {
   double* adj = nullptr;   // per-face stencil cotangents of the VJP (first use)
   double* cons = nullptr;  // conservation-sum partials (first use)
   int* d_status = nullptr;  // scratch status of the autotuner's launches
-  HostWords* host = nullptr;
+  WordSlot host;
   int sweep_threads[3] = {0, 0, 0};  // face-sweep threads per block per precision (0: by size)
   int sweep_shared = 0;               // GBMV_SWEEPS_SHARED register budget
 };
@@ -179,7 +129,7 @@ struct gbmv_chem_s {
   ChemState S{};
   double* tab = nullptr;
   double* cell = nullptr;  // one allocation for all per-cell arrays
-  HostWords* host = nullptr;
+  WordSlot host;
   int* d_info = nullptr;               // first word of a 64-byte control block:
   int* d_nfail = nullptr;              //   [0] info, [1] failed cells,
   unsigned long long* d_next = nullptr;  //   [16] DIRK work counter
@@ -302,7 +252,7 @@ int gbmv_hydro_create(const gbmv_grid* grid, gbmv_hydro* out) {
   memset(&h->force, 0, sizeof h->force);
   h->scratch_doubles = feuler_fp64_scratch_doubles(h->g);
   if (cudaMalloc(&h->scratch, h->scratch_doubles * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->d_status, 2 * sizeof(double)) != cudaSuccess || !host_words(&h->host)) {
+      cudaMalloc(&h->d_status, 2 * sizeof(double)) != cudaSuccess || !g_words.take(&h->host)) {
     cudaGetLastError();
     set_error("device allocation of %zu flux doubles failed", h->scratch_doubles);
     cudaFree(h->scratch);
@@ -321,7 +271,7 @@ int gbmv_hydro_destroy(gbmv_hydro h) {
   cudaFree(h->adj);
   cudaFree(h->cons);
   cudaFree(h->d_status);
-  free_host_words(h->host);
+  g_words.give(&h->host);
   delete h;
   return GBMV_OK;
 }
@@ -450,10 +400,10 @@ int gbmv_feuler(gbmv_hydro h, double t, const double* const* w, double* const* w
                 int precision, void* stream) {
   if (!h) return GBMV_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
-  h->host->flags = 0;
-  if (int rc = finish(gbmv_feuler_async(h, t, w, wdot, precision, 0, &h->host->flags, stream), s))
+  h->host.w->flags = 0;
+  if (int rc = finish(gbmv_feuler_async(h, t, w, wdot, precision, 0, &h->host.w->flags, stream), s))
     return rc;
-  if (const int st = flags_of(h->host)) {
+  if (const int st = flags_of(h->host.w)) {
     set_error("illegal state (mask %d: 1 density, 2 energy, 4 pressure)", st);
     return GBMV_ILLEGAL_STATE;
   }
@@ -497,7 +447,7 @@ int gbmv_chem_create(long ncells, const double* tables_host, double current_z, g
   if (cudaMalloc(&c->tab, sizeof(double) * (2 * tab_doubles + ltab_doubles) +
                               sizeof(float) * gtab_floats) != cudaSuccess ||
       cudaMalloc(&c->cell, sizeof(double) * per_cell * ncells) != cudaSuccess ||
-      cudaMalloc(&c->d_info, 64) != cudaSuccess || !host_words(&c->host)) {
+      cudaMalloc(&c->d_info, 64) != cudaSuccess || !g_words.take(&c->host)) {
     cudaGetLastError();
     free(h);
     free(gh);
@@ -569,7 +519,7 @@ int gbmv_chem_destroy(gbmv_chem c) {
   cudaFree(c->tab);
   cudaFree(c->cell);
   cudaFree(c->d_info);
-  free_host_words(c->host);
+  g_words.give(&c->host);
   cudaFree(c->dirk_k);
   cudaFree(c->dirk_retry);
   cudaFree(c->dirk_order_buf);
@@ -671,12 +621,12 @@ static int newton_sync(gbmv_chem c, const double* y, const double* b, double* f,
     return GBMV_EINVAL;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  c->host->flags = 0;
+  c->host.w->flags = 0;
   if (int rc = finish(chem_newton(c->P, c->S, c->n, y, f, x, gamma, time_units,
-                                  lu_precision == GBMV_MIXED, refine, &c->host->flags, s,
+                                  lu_precision == GBMV_MIXED, refine, &c->host.w->flags, s,
                                   c->newton_bps, b), s))
     return rc;
-  if (flags_of(c->host)) { set_error("singular Newton block"); return 1; }
+  if (flags_of(c->host.w)) { set_error("singular Newton block"); return 1; }
   return GBMV_OK;
 }
 
@@ -1101,7 +1051,7 @@ int gbmv_block_lu_factor(long nblocks, double* A, int* pivots, void* stream) {
 struct gbmv_block_ls_s {
   long nblocks = 0;
   int* pivots = nullptr;
-  HostWords* host = nullptr;
+  WordSlot host;
 };
 
 int gbmv_block_ls_create(long nblocks, gbmv_block_ls* out) {
@@ -1111,7 +1061,7 @@ int gbmv_block_ls_create(long nblocks, gbmv_block_ls* out) {
   if (!L) return GBMV_ENOMEM;
   L->nblocks = nblocks;
   if (cudaMalloc(&L->pivots, sizeof(int) * 10 * nblocks) != cudaSuccess ||
-      !host_words(&L->host)) {
+      !g_words.take(&L->host)) {
     cudaGetLastError();
     cudaFree(L->pivots);
     delete L;
@@ -1125,7 +1075,7 @@ int gbmv_block_ls_create(long nblocks, gbmv_block_ls* out) {
 int gbmv_block_ls_destroy(gbmv_block_ls L) {
   if (!L) return GBMV_OK;
   cudaFree(L->pivots);
-  free_host_words(L->host);
+  g_words.give(&L->host);
   delete L;
   return GBMV_OK;
 }
@@ -1133,9 +1083,9 @@ int gbmv_block_ls_destroy(gbmv_block_ls L) {
 int gbmv_block_ls_setup(gbmv_block_ls L, double* A, void* stream) {
   if (!L || !A) { set_error("null block solver or matrix"); return GBMV_EINVAL; }
   cudaStream_t s = (cudaStream_t)stream;
-  L->host->flags = 0;
-  if (int rc = finish(block_lu_factor(L->nblocks, A, L->pivots, &L->host->flags, s), s)) return rc;
-  if (flags_of(L->host)) { set_error("singular block"); return 1; }
+  L->host.w->flags = 0;
+  if (int rc = finish(block_lu_factor(L->nblocks, A, L->pivots, &L->host.w->flags, s), s)) return rc;
+  if (flags_of(L->host.w)) { set_error("singular block"); return 1; }
   return GBMV_OK;
 }
 
@@ -1188,11 +1138,11 @@ int gbmv_fexpl(gbmv_hydro h, gbmv_chem c, double t, double* const* w, double* co
   }
   if (!fields_ok(w, 10) || !fields_ok(wdot, 10)) return GBMV_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
-  h->host->flags = 0;
-  if (int rc = finish(gbmv_fexpl_async(h, c, t, w, wdot, energy_units, precision, &h->host->flags,
+  h->host.w->flags = 0;
+  if (int rc = finish(gbmv_fexpl_async(h, c, t, w, wdot, energy_units, precision, &h->host.w->flags,
                                        stream), s))
     return rc;
-  if (const int st = flags_of(h->host)) {
+  if (const int st = flags_of(h->host.w)) {
     set_error("illegal state (mask %d: 1 density, 2 energy, 4 pressure)", st);
     return GBMV_ILLEGAL_STATE;
   }
@@ -1425,8 +1375,8 @@ int gbmv_conservation(gbmv_hydro h, const double* const* w, double mass_factor,
   if (int rc = reduction_scratch(h, s, "gbmv_conservation")) return rc;
   Fields W;
   for (int v = 0; v < 6; ++v) W.f[v] = (v < 5) ? const_cast<double*>(w[v]) : nullptr;
-  if (int rc = finish(conservation_sums(h->g, W, h->cons, h->host->sums, s), s)) return rc;
-  const volatile double* const t = h->host->sums;
+  if (int rc = finish(conservation_sums(h->g, W, h->cons, h->host.w->sums, s), s)) return rc;
+  const volatile double* const t = h->host.w->sums;
   totals[0] = t[0] * mass_factor;
   totals[1] = t[1] * energy_factor;
   return GBMV_OK;
@@ -1449,8 +1399,8 @@ int gbmv_wrms_norm(gbmv_hydro h, const double* const* v, const double* const* y,
     V.f[k] = const_cast<double*>(v[k]);
     Y.f[k] = const_cast<double*>(y[k]);
   }
-  if (int rc = finish(wrms_norm(h->g, V, Y, rtol, atol, h->cons, h->host->sums, s), s)) return rc;
-  *norm = *static_cast<const volatile double*>(h->host->sums);
+  if (int rc = finish(wrms_norm(h->g, V, Y, rtol, atol, h->cons, h->host.w->sums, s), s)) return rc;
+  *norm = *static_cast<const volatile double*>(h->host.w->sums);
   return GBMV_OK;
 }
 
@@ -1517,9 +1467,9 @@ int gbmv_stability(gbmv_hydro h, const double* const* w, double cfl, double* dt_
   unsigned long long* d = reinterpret_cast<unsigned long long*>(h->d_status);  // 8-byte slot
   int rc = wave_speed_max(h->g, W, d, s);
   if (rc) return rc;
-  GBMV_CUDA_TRY(cudaMemcpyAsync(&h->host->speed, d, sizeof *d, cudaMemcpyDeviceToHost, s));
+  GBMV_CUDA_TRY(cudaMemcpyAsync(&h->host.w->speed, d, sizeof *d, cudaMemcpyDeviceToHost, s));
   GBMV_CUDA_TRY(cudaStreamSynchronize(s));
-  const unsigned long long bits = h->host->speed;
+  const unsigned long long bits = h->host.w->speed;
   double alpha;
   memcpy(&alpha, &bits, sizeof alpha);
   const double dmin = fmin(fmin(h->g.d[0], h->g.d[1]), h->g.d[2]);
