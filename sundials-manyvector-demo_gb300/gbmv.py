@@ -208,8 +208,12 @@ def _stream_ptr(stream):
     import torch
     if stream is not None:
         return stream.cuda_stream
-    # the current stream without the Stream object around it (3 us of a call's 12 us in Python)
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # the current stream without the Stream object around it (3 us of a call's 12 us in Python),
+    # where this torch has that call; it is not part of its public interface
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return torch.cuda.current_stream().cuda_stream
+    return raw(torch.cuda.current_device())
 
 
 def _vec(fields):
