@@ -82,6 +82,10 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
                                                          unsigned long long* __restrict__ queue) {
   extern __shared__ unsigned char smem_raw[];
   constexpr bool kMixed = sizeof(LU) == 4;
+  // variables whose columns are scaled by them: 2^-kRange to 2^kRange.  FP32 entries take products
+  // of two such scales with the matrix' own range and stay in the float range (at 2^+-99, variables
+  // over 56 decades and no refinement, the median cell lost every digit; plain 3e-4)
+  constexpr unsigned kRange = kMixed ? 40 : 99;
   // FP32-LU form: As[e * BS] = FP64 matrix entry e of kJacPattern; FP64 form: L[(col*10+row) * BS]
   double* As = reinterpret_cast<double*>(smem_raw) + threadIdx.x;
   LU* L = reinterpret_cast<LU*>(smem_raw) + threadIdx.x;
@@ -112,7 +116,7 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
         ya[s] = z * sc[s];
         As[z_slot<LU>(s) * BS] = z;
         const int e = (__double2hiint(z) >> 20) & 0x7FF;
-        scaled = scaled && (unsigned)(e - (1023 - 99)) <= 198u;
+        scaled = scaled && (unsigned)(e - (1023 - kRange)) <= 2u * kRange;
       }
       double Ts = S.Ts[i], dTs = 0.0, logT;
       // mixed form: up to 8 FP32 iterations, then two in FP64.  (One FP64 iteration where
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(BS) chem_newton_kernel(ChemParams P, ChemState
       // The matrix is formed with every column multiplied by its own variable, A diag(z): its
       // species entries are then plain sums of the reaction fluxes (chem_matrix), and partial
       // pivoting, which compares within a column, picks the same rows.  The solution is z times
-      // that system's.  Variables that are zero or far from 1 take the unscaled matrix.
+      // that system's.  Variables that are zero or far from 1 (kRange) take the unscaled matrix.
       {  // source and Newton matrix from one rate evaluation (rates and T slopes)
         double k[kNRates], dk[kNRates], pr[21], r[21];
         chem_rates<true>(P, logT, k, dk);
