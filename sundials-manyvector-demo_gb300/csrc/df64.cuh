@@ -19,7 +19,6 @@ struct f2 {
   __host__ __device__ constexpr explicit f2(double d) : hi((float)d), lo((float)(d - (double)(float)d)) {}
   __host__ __device__ constexpr explicit f2(int i) : hi((float)i), lo(0.f) {}
   __device__ __forceinline__ static f2 from(float x) { return f2(x, 0.f); }
-  __device__ __forceinline__ float to_float() const { return hi + lo; }
   __device__ __forceinline__ double to_double() const { return (double)hi + (double)lo; }
 };
 

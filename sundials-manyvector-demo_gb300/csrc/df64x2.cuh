@@ -33,7 +33,6 @@ struct f2v {
   __device__ __forceinline__ explicit f2v(f2 a) : hi(v2(a.hi)), lo(v2(a.lo)) {}
   __device__ __forceinline__ f2 x() const { return f2(hi.x, lo.x); }
   __device__ __forceinline__ f2 y() const { return f2(hi.y, lo.y); }
-  __device__ __forceinline__ float2 to_float() const { return add2(hi, lo); }
 };
 
 __device__ __forceinline__ f2v quick_two_sum2(float2 a, float2 b) {  // |a| >= |b| per lane

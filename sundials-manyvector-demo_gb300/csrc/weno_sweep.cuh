@@ -35,44 +35,6 @@ __device__ __forceinline__ void face_coords(long f, const Grid& g, long& i, long
   split3(f, g.n[0] + (DIR == 0), g.n[1] + (DIR == 1), i, j, k);
 }
 
-// cells and ghost signs of the six stencil points of face f
-template <int DIR>
-__device__ __forceinline__ void stencil(const Grid& g, long f, long (&cell)[6], bool (&nall)[6],
-                                        bool (&nnorm)[6], long (&ijk)[3]) {
-  long i, j, k;
-  face_coords<DIR>(f, g, i, j, k);
-  ijk[0] = i;
-  ijk[1] = j;
-  ijk[2] = k;
-#pragma unroll
-  for (int l = 0; l < 6; ++l) {
-    long q[3] = {i, j, k};
-    q[DIR] = ghost_src(q[DIR] - 3 + l, g.n[DIR], g.bc[2 * DIR], g.bc[2 * DIR + 1], &nall[l],
-                       &nnorm[l]);
-    cell[l] = q[0] + g.n[0] * (q[1] + g.n[1] * q[2]);
-  }
-}
-
-// the five fluid values of a stencil point in face order (normal momentum in slot 1, the
-// direction swap of src/utilities.cpp:283-285), ghost signs applied
-template <int DIR>
-__device__ __forceinline__ void load_point(const Fields& w, long c, bool nall, bool nnorm,
-                                           double (&W)[5]) {
-  double q[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) q[v] = __ldg(w.f[v] + c);
-  if (nall) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) q[v] = -q[v];
-  }
-  if (nnorm) q[1 + DIR] = -q[1 + DIR];
-  W[0] = q[0];
-  W[1] = q[1 + DIR];
-  W[2] = (DIR == 1) ? q[1] : q[2];
-  W[3] = (DIR == 2) ? q[1] : q[3];
-  W[4] = q[4];
-}
-
 // One direction of a sweep that takes the direction at run time: one kernel body serves the
 // three, and one launch covers the faces of all of them (SweepSet), so small grids wait for one
 // sweep instead of three in a row.  Field order as load_point: normal momentum in slot 1.
