@@ -8,10 +8,9 @@
 
 namespace gbmv {
 
-// Casts to and from the factor's precision.  These stay conversion instructions: the Newton
-// and DIRK kernels run few warps per SM and are latency-bound, and the integer-instruction
-// conversions of df64.cuh (which win in the throughput-bound float-float passes) lengthen
-// their dependency chains (measured 1 % slower fused Newton, 8 % slower mixed DIRK).
+// Casts to and from the factor's precision in the integrator.  These stay conversion instructions:
+// it runs few warps per SM and is latency-bound, and the integer-instruction conversions of
+// df64.cuh lengthen its dependency chains (8 % slower).  The fused Newton has casts of its own.
 template <typename LU>
 __device__ __forceinline__ LU to_lu(double x) { return (LU)x; }
 __device__ __forceinline__ double from_lu(float x) { return (double)x; }

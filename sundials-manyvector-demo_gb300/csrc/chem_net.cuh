@@ -208,7 +208,7 @@ __device__ __forceinline__ void chem_temperature_mixed(const ChemParams& P, cons
     T = T - dT;
     if (fabsf(dT) <= 1e-5f * T) break;
   }
-  // remaining iterations (and dT/dge) in FP64: exactly chem_temperature's loop body
+  // remaining iterations (and dT/dge) in FP64: chem_temperature's step without its early end
   const ChemTemp c = chem_temp_setup(y);
   double Td = (double)T, T0 = Td, slope = 0.0, dT = 0.0;
 #pragma unroll 1

@@ -6,7 +6,8 @@
 // tendency is the derivative only if none of the cell's six faces changes that branch between
 // w - h d, w and w + h d; this kernel marks the cells where one does, so that derivative tests
 // can compare the exact JVP / VJP with finite differences on the smooth entries and count the
-// others.  The branch is evaluated with the face kernel's own expressions (eos64, sqrt0_64).
+// others.  The branch is evaluated on |u| + c as the reference does; the face kernels compare half of
+// it, fma(1/2, |u|, c/2), so speeds that agree to a rounding may be ordered otherwise there.
 #include "weno64.cuh"
 #include "weno_sweep.cuh"
 
