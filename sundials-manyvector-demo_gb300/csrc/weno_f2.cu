@@ -4,7 +4,8 @@
 
 namespace gbmv {
 
-// Register budgets of the sweeps (128-thread blocks per SM; the same bits whatever they are).
+// Register budgets of the sweeps (128-thread blocks per SM; the same bits whatever they are; timed
+// with un-normalised projections: 2.51 ms is 2.54 with the normalised ones).
 // Fluid, 128^3 x 15 GBMV_MIXED_FAST RHS at 2 / 3 / 4 blocks: 2.61 / 2.51 / 2.57 ms.  Beside the
 // chemistry Newton on a second stream (255 registers a thread) 5 leave the Newton's warps room
 // (Grid::sweep_shared).  Tracers: FP32 weights 5 / 6 / 7 / 8: 2.53 / 2.51 / 2.51 / 2.53

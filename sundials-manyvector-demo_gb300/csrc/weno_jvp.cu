@@ -7,7 +7,7 @@
 //
 // Bound by the FP64 pipe, so the tangents are written out where a generic dual number would
 // spend instructions on constants' zero tangents and on quotients: 36 instructions for the
-// tangent of a reconstruction on top of its 33 (weno_tan64).  96^3 x 9: 5330 -> 2135 FP64
+// tangent of a reconstruction on top of its 33 (weno_tan64).  96^3 x 9: 5330 -> 2139 FP64
 // instructions a face.
 #include "common.cuh"
 #include "weno.cuh"
